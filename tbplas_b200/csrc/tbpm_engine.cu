@@ -28,6 +28,7 @@
 #include "tbpm_pair_kernels.cuh"
 #include "tbpm_more_kernels.cuh"
 #include "tbpm_scan.cuh"
+#include "tbpm_poly_kernels.cuh"
 
 
 namespace tbpm {
@@ -247,12 +248,12 @@ void ensure_partials(tbpm_ctx* c, size_t n_doubles) {
   c->partials.ensure(std::max(n_doubles, floor_doubles) * sizeof(double));
 }
 
-// Launch shapes of the three compiled modes of the Chebyshev-term kernel, and
+// Launch shapes of the four compiled modes of the Chebyshev-term kernel, and
 // for each mode whether the shared-memory ring kernel runs it.
 struct TermTiles {
-  Tile t[3];
-  bool ring[3] = {false, false, false};
-  RingShape rs[3] = {};
+  Tile t[4];
+  bool ring[4] = {false, false, false, false};
+  RingShape rs[4] = {};
   const int* win = nullptr;  // window records (ring_window_kernel); null: no windows
 };
 
@@ -297,7 +298,7 @@ RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win
     off += tile;
   }
   s.acc_off = -1;
-  if (mode >= 1) {
+  if (mode == 1 || mode == 2) {
     s.acc_off = off;
     off += tile;
   }
@@ -327,7 +328,7 @@ RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win
   s.cap = cap;
   s.bar_off = S * off;
   s.smem_bytes = s.bar_off + 2 * S * 8;
-  // MODE 2 reduces its partials in the stage buffers
+  // MODE 2 and 3 reduce their partials in the stage buffers
   if ((size_t)s.bar_off < (size_t)kRingConsumers * V * 3 * sizeof(double)) return RingShape{};
   return s;
 }
@@ -394,6 +395,7 @@ TermTiles term_tiles(tbpm_ctx* c, int64_t n_rows, int tpr, int ref_tpr = 0) {
   tt.t[0] = pick_tile(c, n_rows, tpr, cheb_term_kernel<R, V, 0>, 0, th);
   tt.t[1] = pick_tile(c, n_rows, tpr, cheb_term_kernel<R, V, 1>, 0, th);
   tt.t[2] = pick_tile(c, n_rows, tpr, cheb_term_kernel<R, V, 2>, V * 3 * sizeof(double), th);
+  tt.t[3] = pick_tile(c, n_rows, tpr, cheb_term_kernel<R, V, 3>, V * 2 * sizeof(double), th);
   // row windows (term_kernel 4) where every mode's window layout fits and the
   // plan exists.  (Measured on B200, 2048^2 graphene, 16 states: 31.3 ms per
   // step against 28.2 ms with gathers; each row of p_{k-1} is staged by three
@@ -416,10 +418,12 @@ TermTiles term_tiles(tbpm_ctx* c, int64_t n_rows, int tpr, int ref_tpr = 0) {
                      (n_rows + kRingConsumers / tpr - 1) / (kRingConsumers / tpr) <
                          2 * (int64_t)num_sms(c->device);
   if (c->opts.term_kernel != 1 && !small) {
-    for (int m = 0; m < 3; ++m) {
-      const RingShape rs = ring_shape<R, V>(c, tpr, m, ref_tpr, win);
+    for (int m = 0; m < 4; ++m) {
+      // mode 3 always gathers
+      const RingShape rs = ring_shape<R, V>(c, tpr, m, ref_tpr, win && m < 3);
       if (rs.stages == 0) continue;
-      const int per_sm = win ? (m == 0   ? ring_blocks_per_sm<R, V, 0, true>(c, rs)
+      const int per_sm = m == 3 ? ring_blocks_per_sm<R, V, 3, false>(c, rs)
+                         : win ? (m == 0   ? ring_blocks_per_sm<R, V, 0, true>(c, rs)
                                 : m == 1 ? ring_blocks_per_sm<R, V, 1, true>(c, rs)
                                          : ring_blocks_per_sm<R, V, 2, true>(c, rs))
                              : (m == 0   ? ring_blocks_per_sm<R, V, 0, false>(c, rs)
@@ -443,7 +447,7 @@ TermTiles term_tiles(tbpm_ctx* c, int64_t n_rows, int tpr, int ref_tpr = 0) {
 // Returns the grid of the launch (needed by the finalize of mode 2).
 template <typename R, int V>
 int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
-  const int mode = a.partials ? 2 : (a.c.nflush > 0 ? 1 : 0);
+  const int mode = a.partials ? (a.acc ? 2 : 3) : (a.c.nflush > 0 ? 1 : 0);
   const Tile& t = tt.t[mode];
   if (tt.ring[mode]) {
     RingArgs<R, V> ra;
@@ -452,7 +456,9 @@ int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
     ra.status = c->status.as<unsigned int>();
     ra.win = tt.win;
     const size_t smem = (size_t)ra.s.smem_bytes;
-    if (tt.win) {
+    if (mode == 3) {
+      cheb_ring_kernel<R, V, 3, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+    } else if (tt.win) {
       if (mode == 2)
         cheb_ring_kernel<R, V, 2, true><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
       else if (mode == 1)
@@ -466,6 +472,9 @@ int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
     } else {
       cheb_ring_kernel<R, V, 0, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
     }
+  } else if (mode == 3) {
+    const size_t smem = (size_t)t.threads * V * 2 * sizeof(double);
+    cheb_term_kernel<R, V, 3><<<t.grid, t.threads, smem, c->stream>>>(a);
   } else if (mode == 2) {
     const size_t smem = (size_t)t.threads * V * 3 * sizeof(double);
     cheb_term_kernel<R, V, 2><<<t.grid, t.threads, smem, c->stream>>>(a);
@@ -1036,6 +1045,359 @@ void read_out(tbpm_ctx* c, std::vector<double>& host, size_t n_doubles) {
     TBPM_CK(cudaMemcpy(host.data(), c->out.p, n_doubles * sizeof(double), cudaMemcpyDeviceToHost));
 }
 
+// ---- polynomial routes (tbpm_poly_kernels.cuh) --------------------------------
+
+// Shortest run that takes a polynomial route.  Below it the whole run is a few
+// milliseconds to a second, and time stepping keeps its results bit for bit
+// equal to those of sessions (checkpoints) and of the other term kernels.
+constexpr int kPolyMinSteps = 64;
+// Largest deviation |P(x) - exp(-i tau x)| over the spectrum for which powers
+// of P count as unitary (the default Bessel precision leaves 1e-14).
+constexpr double kPolyUnitary = 1e-12;
+// The recurrence runs on y = H/a with a this much above the Gershgorin bound: at
+// the edge of [-1, 1] a rounding error grows by 1/sin(theta) per term, 7 here,
+// against k at the very edge; the margin costs 1% more terms.
+constexpr double kPolyMargin = 1.01;
+// With a norm-check threshold below this the check would see the rounding of
+// the time steps themselves; such a run is time-stepped.
+constexpr double kPolyMinThr = 1e-11;
+
+struct PolyPlan {
+  float alpha = 0;         // 2/a, a float, so that both precisions run the same y = H/a
+  long double a = 0;       // 2/alpha
+  double tau = 0;          // P(x) ~ exp(-i tau x)
+  const double* bes = nullptr;
+  int n_bes = 0;
+};
+
+const Spectrum& ham_spectrum(tbpm_ctx* c) {
+  Spectrum& sp = c->spec;
+  const Ham& h = c->ham;
+  if (sp.gen == h.gen && h.gen != 0) return sp;
+  c->poly.ensure(256);
+  TBPM_CK(cudaMemsetAsync(c->poly.p, 0, 16, c->stream));
+  const int grid = (int)std::min<int64_t>(blocks_for(h.n, 256), (int64_t)num_sms(c->device) * 16);
+  auto launch = [&](auto tag) {
+    using R = decltype(tag);
+    using C = typename Cx<R>::t;
+    // values that are conjugates in FP64 stay so when rounded to FP32
+    const double tol = sizeof(R) == 8 ? 1e-14 : 1.2e-7;
+    ham_spectrum_kernel<R><<<grid, 256, 0, c->stream>>>(
+        h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<C>(),
+        h.has_diag ? h.diag.as<C>() : nullptr, h.n, tol, c->poly.as<unsigned long long>());
+  };
+  if (h.prec == TBPM_PREC_FP64)
+    launch(double{});
+  else
+    launch(float{});
+  TBPM_CK(cudaGetLastError());
+  c->launches++;
+  unsigned long long info[2];
+  TBPM_CK(cudaMemcpyAsync(info, c->poly.p, sizeof info, cudaMemcpyDeviceToHost, c->stream));
+  TBPM_CK(cudaStreamSynchronize(c->stream));
+  std::memcpy(&sp.bound, &info[0], sizeof(double));
+  sp.hermitian = info[1] == 0;
+  sp.gen = h.gen;
+  return sp;
+}
+
+// P(x) = sum_k w_k T_k(x), w_k = (2 - delta_k0) (-i)^k bes_k (propagation.f90:33-48)
+void step_polynomial(const PolyPlan& pp, long double x, long double* re, long double* im) {
+  long double t0 = 1.0L, t1 = x;
+  *re = pp.bes[0];
+  *im = 0.0L;
+  for (int k = 1; k < pp.n_bes; ++k) {
+    const long double w = 2.0L * pp.bes[k] * t1;
+    switch (k & 3) {
+      case 0: *re += w; break;
+      case 1: *im -= w; break;
+      case 2: *re -= w; break;
+      default: *im += w; break;
+    }
+    const long double t2 = 2.0L * x * t1 - t0;
+    t0 = t1;
+    t1 = t2;
+  }
+}
+
+// Whether powers of the step polynomial of `bes` on the resident Hamiltonian may
+// be expanded over the whole run: H Hermitian, its spectrum bounded, and P
+// unitary on it.  Everything else (a series for another operator, a rescale
+// factor below the spectral radius, a non-Hermitian H) is time-stepped as before.
+bool poly_route(tbpm_ctx* c, const double* bes, int n_bes, int n_timestep, int chk_step,
+                double chk_thr, PolyPlan* pp) {
+  if (n_timestep < kPolyMinSteps) return false;
+  const bool check = chk_step >= 2 && chk_step <= n_timestep;
+  if (check && !(effective_thr(c, chk_thr) >= kPolyMinThr)) return false;
+  const Spectrum& sp = ham_spectrum(c);
+  if (!sp.hermitian || !(sp.bound < 4.0)) return false;
+  const double want = 2.0 / std::max(sp.bound * kPolyMargin, 1.0 / 1024);
+  float alpha = (float)want;
+  if ((double)alpha > want) alpha = std::nextafter(alpha, 0.0f);
+  pp->alpha = alpha;
+  pp->a = 2.0L / (long double)alpha;
+  pp->bes = bes;
+  pp->n_bes = n_bes;
+  double tau = 0.0;  // -i P'(0) / P(0), T_k'(0) = k sin(k pi / 2)
+  for (int k = 1; k < n_bes; k += 2) tau += 2.0 * k * bes[k];
+  pp->tau = tau;
+  if (!(std::fabs(tau) < 1e3)) return false;
+  for (int j = 0; j <= 64; ++j) {
+    const long double x = pp->a * (long double)(j - 32) / 32.0L;
+    long double re, im;
+    step_polynomial(*pp, x, &re, &im);
+    const long double dr = re - cosl(tau * x), di = im + sinl(tau * x);
+    if (!(std::fabs((double)dr) <= kPolyUnitary && std::fabs((double)di) <= kPolyUnitary))
+      return false;
+  }
+  return true;
+}
+
+// Number of Chebyshev coefficients of exp(-i z y) on [-1, 1] above 1e-17, i.e.
+// one more than the last k with |J_k(z)| > 1e-17 (Miller's downward recurrence
+// normalised by J_0 + 2 sum J_2k = 1).
+int bessel_degree(double z) {
+  z = std::max(std::fabs(z), 1e-2);
+  const int top = (int)(z + 30 * std::cbrt(z) + 40);
+  std::vector<double> J(top + 2, 0.0);
+  J[top] = 1e-300;
+  for (int k = top; k > 0; --k) {
+    J[k - 1] = 2.0 * k / z * J[k] - J[k + 1];
+    if (std::fabs(J[k - 1]) > 1e200)
+      for (int q = k - 1; q <= top; ++q) J[q] *= 1e-200;
+  }
+  double norm = J[0];
+  for (int k = 2; k <= top; k += 2) norm += 2.0 * J[k];
+  int last = 2;
+  for (int k = 0; k <= top; ++k)
+    if (std::fabs(J[k] / norm) > 1e-17) last = k;
+  return last + 1;
+}
+
+// The powers' bases at the M Gauss-Chebyshev nodes of [-a, a], in extended
+// precision: an error of a node's phase grows with the power.
+std::vector<PolyNode> poly_nodes(const PolyPlan& pp, int M) {
+  const long double pi = 3.14159265358979323846264338327950288L;
+  std::vector<PolyNode> nodes(M);
+  for (int j = 0; j < M; ++j) {
+    long double re, im;
+    step_polynomial(pp, pp.a * cosl(pi * (j + 0.5L) / M), &re, &im);
+    const long double turns = atan2l(im, re) / (2.0L * pi);
+    nodes[j].hi = (double)turns;
+    nodes[j].lo = (double)(turns - (long double)nodes[j].hi);
+    nodes[j].lnabs = (double)(0.5L * log1pl(re * re + im * im - 1.0L));
+  }
+  return nodes;
+}
+
+// Arguments of term k of p_k = (2/a) H p_{k-1} - p_{k-2} on two buffers: p_k
+// overwrites p_{k-2}.
+template <typename R, int V>
+TermArgs<R, V> poly_term(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr, Pack<R, V>* A,
+                         Pack<R, V>* X) {
+  const Ham& h = c->ham;
+  TermArgs<R, V> a{};
+  a.indptr = h.indptr.as<int32_t>();
+  a.indices = h.indices.as<int32_t>();
+  a.hop = h.hop.as<typename Cx<R>::t>();
+  a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
+  a.n_rows = h.n;
+  a.tpr = tpr;
+  a.gather = (k & 1) ? A : X;
+  a.pout = (k & 1) ? X : A;
+  a.pin = k >= 2 ? a.pout : nullptr;
+  a.c.alpha_re = (k == 1 ? 0.5 : 1.0) * (double)pp.alpha;
+  a.c.beta = k >= 2 ? -1.0 : 0.0;
+  return a;
+}
+
+double matrix_bytes(const Ham& h) {
+  const double s = h.prec == TBPM_PREC_FP64 ? 16 : 8;
+  return (double)(h.n + 1) * 4 + (double)h.nnz * (4 + s) + (h.has_diag ? (double)h.n * s : 0.0);
+}
+
+#ifndef TBPM_PERSIST_MB
+#define TBPM_PERSIST_MB 48
+#endif
+#ifndef TBPM_PERSIST_ITEMS
+#define TBPM_PERSIST_ITEMS 8
+#endif
+// All K terms in one cooperative launch (cheb_persist_kernel) when the vectors
+// and the matrix stay in L2 and a thread has few items; false when it does not apply.
+template <typename R, int V>
+bool launch_persist(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A, Pack<R, V>* X,
+                    double* sums) {
+  const tbpm_options& o = c->opts;
+  if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return false;
+  const Ham& h = c->ham;
+  const int tpr = ld / V;
+  constexpr int TMAX = kPersistThreads<R, V>;
+  if (tpr > TMAX) return false;
+  const double bytes = matrix_bytes(h) + 2.0 * (double)h.n * ld * 2 * sizeof(R);
+  const int sms = num_sms(c->device);
+  if (bytes > TBPM_PERSIST_MB * 1e6 || h.n * tpr > (int64_t)TBPM_PERSIST_ITEMS * sms * TMAX)
+    return false;
+  const int64_t per_sm = (h.n + sms - 1) / sms;
+  const int rpp = (int)std::min<int64_t>(std::max<int64_t>(per_sm, (128 + tpr - 1) / tpr),
+                                         TMAX / tpr);
+  const int threads = rpp * tpr;
+  const int grid = (int)std::min<int64_t>(sms, (h.n + rpp - 1) / rpp);
+  const size_t smem = (size_t)threads * V * 2 * sizeof(double);
+  static bool attr_set[64] = {false};
+  const int dev = c->device;
+  if (dev < 0 || dev >= 64) return false;
+  if (!attr_set[dev]) {
+    TBPM_CK(cudaFuncSetAttribute(cheb_persist_kernel<R, V>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
+    attr_set[dev] = true;
+  }
+  const int64_t n_vals = (int64_t)K * ld * 2;
+  ensure_partials(c, (size_t)n_vals * grid);
+  unsigned int* bar = c->ctr.as<unsigned int>() + 12;
+  TBPM_CK(cudaMemsetAsync(bar, 0, sizeof(unsigned int), c->stream));
+  PersistArgs<R, V> a;
+  a.indptr = h.indptr.as<int32_t>();
+  a.indices = h.indices.as<int32_t>();
+  a.hop = h.hop.as<typename Cx<R>::t>();
+  a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
+  a.n_rows = h.n;
+  a.tpr = tpr;
+  a.p0 = A;
+  a.p1 = X;
+  a.alpha = pp.alpha;
+  a.n_terms = K;
+  a.partials = c->partials.as<double>();
+  a.bar = bar;
+  a.status = c->status.as<unsigned int>();
+  // cooperative: every block is resident, the barrier cannot wait on a block
+  // that has not started
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TBPM_CK(cudaLaunchKernelEx(&cfg, cheb_persist_kernel<R, V>, a));
+  reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+      c->partials.as<double>(), grid, n_vals, sums);
+  TBPM_CK(cudaGetLastError());
+  c->launches += 2;
+  c->model_bytes += K * (matrix_bytes(h) + 3.0 * (double)h.n * ld * 2 * sizeof(R));
+  return true;
+}
+
+// Terms 1..K with the products of every term: sums[((k-1)*ld + col)*2 + q],
+// q = 0: <p_k|p_k>, 1: Re <p_k|p_{k-1}>.  p_0 is in A, X is scratch.
+template <typename R, int V>
+void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A,
+                          Pack<R, V>* X, double* sums) {
+  if (launch_persist<R, V>(c, pp, K, ld, A, X, sums)) return;
+  const int tpr = ld / V;
+  const TermTiles tt = term_tiles<R, V>(c, c->ham.n, tpr);
+  const int grid = tt.t[3].grid;
+  const int64_t per_term = (int64_t)ld * 2 * grid;
+  // block partials of as many terms as fit 64 MB, then one reduction of them all
+  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(K, (64ll << 20) / (per_term * 8)));
+  ensure_partials(c, (size_t)chunk * per_term);
+  const double bytes = matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R);
+  for (int k0 = 1; k0 <= K; k0 += chunk) {
+    const int m = std::min(chunk, K - k0 + 1);
+    for (int i = 0; i < m; ++i) {
+      TermArgs<R, V> a = poly_term<R, V>(c, pp, k0 + i, tpr, A, X);
+      a.partials = c->partials.as<double>() + (int64_t)i * per_term;
+      launch_term<R, V>(c, tt, a);
+      c->model_bytes += bytes;
+    }
+    const int64_t n_vals = (int64_t)m * ld * 2;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), grid, n_vals, sums + (int64_t)(k0 - 1) * ld * 2);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+  }
+}
+
+// Moments of n_cols columns -> correlation functions and norms in c->out (the
+// rows of moment_curve_kernel); mu, rho: n_cols*M doubles each.
+void enqueue_moment_curves(tbpm_ctx* c, const PolyPlan& pp, int M, int T, int n_cols,
+                           const double* sums, int64_t stride, const double* mu0,
+                           int mu0_stride, double* mu, double* rho, PolyNode* nodes,
+                           int chk_step) {
+  const int64_t total = (int64_t)n_cols * M;
+  moment_gather_kernel<<<(int)std::min<int64_t>(blocks_for(total, 256), 4096), 256, 0,
+                         c->stream>>>(sums, stride, mu0, mu0_stride, n_cols, M, mu);
+  const unsigned cg = (unsigned)((n_cols + kMomentCols - 1) / kMomentCols);
+  moment_density_kernel<<<dim3((unsigned)M, cg), 128, 0, c->stream>>>(mu, n_cols, M, rho);
+  TBPM_CK(cudaGetLastError());
+  // (the host evaluates the nodes while the terms run)
+  const std::vector<PolyNode> host = poly_nodes(pp, M);
+  TBPM_CK(cudaMemcpyAsync(nodes, host.data(), sizeof(PolyNode) * M, cudaMemcpyHostToDevice,
+                          c->stream));
+  moment_curve_kernel<<<dim3((unsigned)(T + 3), cg), 128, 0, c->stream>>>(
+      nodes, rho, n_cols, M, T, 1, std::max(chk_step - 1, 1), c->out.as<double>());
+  TBPM_CK(cudaGetLastError());
+  c->launches += 3;
+}
+
+// dos_batch by moments of the whole run: C(t) = <wf0|P(H)^t|wf0>.
+template <typename R, int V>
+void dos_moments(tbpm_ctx* c, const PolyPlan& pp, int ns, const StateKeys* keys,
+                 const double* host_wf0, int n_timestep, int chk_step, double chk_thr, int n_avg,
+                 double* corr, double* corr_per_state, int state_offset) {
+  const int T = n_timestep;
+  const int M = std::max(4, bessel_degree(pp.tau * (double)pp.a * T));
+  const int K = M / 2;
+  c->graph.reset();
+  c->sess.active = false;
+  const size_t vb = (size_t)c->ham.n * ns * 2 * sizeof(R);
+  c->A.ensure(vb);
+  c->X.ensure(vb);
+  c->ctr.ensure(16 * sizeof(int));
+  c->small.ensure(sizeof(double) * kMaxCols * 3);
+  c->out.ensure((size_t)(T + 3) * ns * 2 * sizeof(double));
+  const size_t n_sums = (size_t)K * ns * 2, n_mu = (size_t)ns * M;
+  c->poly.ensure((n_sums + 2 * n_mu) * sizeof(double) + sizeof(PolyNode) * M);
+  double* sums = c->poly.as<double>();
+  double* mu = sums + n_sums;
+  double* rho = mu + n_mu;
+  PolyNode* nodes = reinterpret_cast<PolyNode*>(rho + n_mu);
+  auto* A = c->A.as<Pack<R, V>>();
+  auto* X = c->X.as<Pack<R, V>>();
+  if (keys)
+    gen_states<R, V>(c, *keys, ns, c->opts.state_kind, A);
+  else
+    upload_states<R>(c, host_wf0, ns, ns, 0, A);
+  reset_counters(c, 2);
+  enqueue_corr<R, V>(c, A, nullptr, ns, 0, c->small.as<double>(), counters(c, 2));
+  enqueue_moment_terms<R, V>(c, pp, K, ns, A, X, sums);
+  enqueue_moment_curves(c, pp, M, T, ns, sums, (int64_t)ns * 2, c->small.as<double>() + 2, 3, mu,
+                        rho, nodes, chk_step);
+  std::vector<double> host;
+  read_out(c, host, (size_t)(T + 3) * ns * 2);
+  // check_norm as in dos_batch: after chk_step - 1 steps against after the first
+  if (chk_step >= 2 && chk_step <= T) {
+    const double thr = effective_thr(c, chk_thr);
+    for (int b = 0; b < ns; ++b)
+      if (const int bad = norm_broken(host[((size_t)(T + 2) * ns + b) * 2],
+                                      host[((size_t)(T + 1) * ns + b) * 2], thr))
+        raise_norm("tbpm_dos", chk_step, bad);
+  }
+  for (int b = 0; b < ns; ++b)
+    for (int t = 0; t <= T; ++t) {
+      const double* v = &host[((size_t)t * ns + b) * 2];
+      corr[2 * t] += v[0] / n_avg;
+      corr[2 * t + 1] += v[1] / n_avg;
+      if (corr_per_state) {
+        double* o = corr_per_state + 2 * ((size_t)(state_offset + b) * (T + 1) + t);
+        o[0] = v[0];
+        o[1] = v[1];
+      }
+    }
+}
+
 // ---- DOS ----------------------------------------------------------------------
 
 template <typename R, int V>
@@ -1278,6 +1640,117 @@ void dos_segmented_run(tbpm_ctx* c, const Expansion& ex, const std::vector<int64
       corr[2 * ((size_t)k * (n_timestep + 1) + t)] = re;
       corr[2 * ((size_t)k * (n_timestep + 1) + t) + 1] = im;
     }
+}
+
+// dos_segmented_run by moments: the terms of all realisations run as one block
+// row-interleaved state block, seg_dots_kernel forms the two products of every
+// term per (segment, state).
+template <typename R, int V>
+bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<int64_t>& off,
+                           int ns, int seed, int n_timestep, int chk_step, double chk_thr,
+                           double* corr, double* corr_per_state) {
+  using C = typename Cx<R>::t;
+  const int n_seg = (int)off.size() - 1;
+  const int n_cols = n_seg * ns;
+  const int T = n_timestep;
+  const int64_t n = c->ham.n;
+  const int M = std::max(4, bessel_degree(pp.tau * (double)pp.a * T));
+  const int K = M / 2;
+  // a batch of very many tiny realisations would need more moments than states
+  if ((n_cols + kMomentCols - 1) / kMomentCols > 65535 || (double)n_cols * M * 32 > 4e9)
+    return false;
+  int64_t max_len = 0;
+  for (int k = 0; k < n_seg; ++k) max_len = std::max<int64_t>(max_len, off[k + 1] - off[k]);
+  const int64_t rows_per_chunk = 4096;
+  const int n_chunks = (int)std::max<int64_t>(1, (max_len + rows_per_chunk - 1) / rows_per_chunk);
+  const int rpp = std::max(1, 256 / ns);
+  const int threads = rpp * ns;
+  c->graph.reset();
+  c->sess.active = false;
+  const size_t vb = (size_t)n * ns * sizeof(C);
+  c->A.ensure(vb);
+  c->X.ensure(vb);
+  c->ctr.ensure(16 * sizeof(int));
+  c->seg.ensure(sizeof(int64_t) * off.size());
+  TBPM_CK(cudaMemcpyAsync(c->seg.p, off.data(), sizeof(int64_t) * off.size(),
+                          cudaMemcpyHostToDevice, c->stream));
+  const int64_t per_term = (int64_t)n_cols * 2 * n_chunks;
+  const int chunk =
+      (int)std::max<int64_t>(1, std::min<int64_t>(K + 1, (64ll << 20) / (per_term * 8)));
+  ensure_partials(c, (size_t)chunk * per_term);
+  c->small.ensure(sizeof(double) * std::max<size_t>((size_t)n_cols, kMaxCols * 2));
+  c->out.ensure((size_t)(T + 3) * n_cols * 2 * sizeof(double));
+  const size_t n_sums = (size_t)(K + 1) * n_cols * 2, n_mu = (size_t)n_cols * M;
+  c->poly.ensure((n_sums + 2 * n_mu) * sizeof(double) + sizeof(PolyNode) * M);
+  double* sums = c->poly.as<double>();
+  double* mu = sums + n_sums;
+  double* rho = mu + n_mu;
+  PolyNode* nodes = reinterpret_cast<PolyNode*>(rho + n_mu);
+  auto* A = c->A.as<Pack<R, V>>();
+  auto* X = c->X.as<Pack<R, V>>();
+  const dim3 grid(n_chunks, n_seg);
+  reset_counters(c, 1);
+  seg_state_kernel<R><<<grid, threads, 0, c->stream>>>(
+      c->seg.as<int64_t>(), ns, (long long)seed, c->opts.state_kind, rows_per_chunk, 0, nullptr,
+      nullptr, c->partials.as<double>());
+  TBPM_CK(cudaGetLastError());
+  launch_finalize(c, n_chunks, n_cols, counters(c, 1), c->small.as<double>());
+  seg_state_kernel<R><<<grid, threads, 0, c->stream>>>(
+      c->seg.as<int64_t>(), ns, (long long)seed, c->opts.state_kind, rows_per_chunk, 1,
+      c->small.as<double>(), reinterpret_cast<C*>(A), nullptr);
+  TBPM_CK(cudaGetLastError());
+  c->launches += 2;
+  const int tpr = ns / V;
+  const TermTiles tt = term_tiles<R, V>(c, n, tpr);
+  const double bytes = matrix_bytes(c->ham) + 5.0 * (double)vb;
+  for (int k0 = 0; k0 <= K; k0 += chunk) {  // row 0 of the sums: <p_0|p_0>
+    const int m = std::min(chunk, K + 1 - k0);
+    for (int i = 0; i < m; ++i) {
+      const int k = k0 + i;
+      Pack<R, V>* x = (k & 1) ? X : A;
+      Pack<R, V>* y = (k & 1) || k == 0 ? A : X;
+      if (k >= 1) launch_term<R, V>(c, tt, poly_term<R, V>(c, pp, k, tpr, A, X));
+      seg_dots_kernel<R><<<grid, threads, 0, c->stream>>>(
+          c->seg.as<int64_t>(), ns, rows_per_chunk, reinterpret_cast<const C*>(x),
+          reinterpret_cast<const C*>(y), c->partials.as<double>() + (int64_t)i * per_term);
+      TBPM_CK(cudaGetLastError());
+      c->launches++;
+      c->model_bytes += bytes;
+    }
+    const int64_t n_vals = (int64_t)m * n_cols * 2;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), n_chunks, n_vals, sums + (int64_t)k0 * n_cols * 2);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+  }
+  enqueue_moment_curves(c, pp, M, T, n_cols, sums + (int64_t)n_cols * 2, (int64_t)n_cols * 2,
+                        sums, 2, mu, rho, nodes, chk_step);
+  std::vector<double> host;
+  read_out(c, host, (size_t)(T + 3) * n_cols * 2);
+  if (chk_step >= 2 && chk_step <= T) {
+    const double thr = effective_thr(c, chk_thr);
+    for (int v = 0; v < n_cols; ++v)
+      if (const int bad = norm_broken(host[((size_t)(T + 2) * n_cols + v) * 2],
+                                      host[((size_t)(T + 1) * n_cols + v) * 2], thr))
+        raise_norm("tbpm_dos_segmented", chk_step, bad);
+  }
+  for (int k = 0; k < n_seg; ++k)
+    for (int t = 0; t <= T; ++t) {
+      double re = 0, im = 0;
+      for (int b = 0; b < ns; ++b) {
+        const double* v = &host[((size_t)t * n_cols + k * ns + b) * 2];
+        re += v[0] / ns;
+        im += v[1] / ns;
+        if (corr_per_state) {
+          double* o = corr_per_state + 2 * (((size_t)k * ns + b) * (T + 1) + t);
+          o[0] = v[0];
+          o[1] = v[1];
+        }
+      }
+      corr[2 * ((size_t)k * (T + 1) + t)] = re;
+      corr[2 * ((size_t)k * (T + 1) + t) + 1] = im;
+    }
+  return true;
 }
 
 // ---- AC ---------------------------------------------------------------------
@@ -2191,6 +2664,8 @@ void drv_dos(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, int n
   c->model_bytes = 0;
   std::fill(corr, corr + 2 * (size_t)(n_timestep + 1), 0.0);
   const Expansion ex = time_step_expansion(bes, n_bes);
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   const int B = batch_size(c);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int ns = std::min(B, n_states - s0);
@@ -2203,8 +2678,12 @@ void drv_dos(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, int n
     const double* hw = wf0 ? wf0 + 2 * (size_t)s0 * c->ham.n : nullptr;
     dispatch(c->ham.prec, pick_V(c->ham.prec, ns, ns, c->opts.vector_width), [&](auto tag) {
       using P = decltype(tag);
-      dos_batch<typename P::Real, P::V>(c, ex, ns, kp, hw, n_timestep, chk_step, chk_thr,
-                                        n_states, corr, corr_per_state, s0, n_states);
+      if (poly)
+        dos_moments<typename P::Real, P::V>(c, pp, ns, kp, hw, n_timestep, chk_step, chk_thr,
+                                            n_states, corr, corr_per_state, s0);
+      else
+        dos_batch<typename P::Real, P::V>(c, ex, ns, kp, hw, n_timestep, chk_step, chk_thr,
+                                          n_states, corr, corr_per_state, s0, n_states);
     });
   }
 }
@@ -2650,9 +3129,15 @@ void drv_dos_segmented(tbpm_ctx* c, const double* bes, int n_bes, const int64_t*
   c->launches = 0;
   c->model_bytes = 0;
   const Expansion ex = time_step_expansion(bes, n_bes);
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   dispatch(c->ham.prec, pick_V(c->ham.prec, n_states, n_states, c->opts.vector_width),
            [&](auto tag) {
              using P = decltype(tag);
+             if (poly && dos_segmented_moments<typename P::Real, P::V>(
+                             c, pp, off, n_states, seed, n_timestep, chk_step, chk_thr, corr,
+                             corr_per_state))
+               return;
              dos_segmented_run<typename P::Real, P::V>(c, ex, off, n_states, seed, n_timestep,
                                                        chk_step, chk_thr, corr, corr_per_state);
            });

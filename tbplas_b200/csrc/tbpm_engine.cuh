@@ -132,6 +132,14 @@ struct PairRequest {
   int kind = 0;
 };
 
+// What the polynomial routes need to know of a Hamiltonian (ham_spectrum_kernel),
+// valid while gen equals the Hamiltonian's.
+struct Spectrum {
+  uint64_t gen = 0;
+  bool hermitian = false;
+  double bound = 0;  // Gershgorin: every eigenvalue lies in [-bound, bound]
+};
+
 struct Session {
   bool active = false;
   int kind = 0;  // 1 = DOS
@@ -158,6 +166,8 @@ struct tbpm_ctx {
   std::vector<std::unique_ptr<tbpm::WindowPlan>> windows;  // ring window plans, by tile height
   std::vector<tbpm::PairRequest> pair_requests;
   tbpm::DevMem pair_tmp;  // scratch of the plan build
+  tbpm::Spectrum spec;
+  tbpm::DevMem poly;  // sums, moments, nodes and weights of the polynomial routes
   int64_t launches = 0;
   double model_bytes = 0;
   tbpm::Session sess;

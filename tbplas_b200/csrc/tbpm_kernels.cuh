@@ -49,12 +49,14 @@ struct TermArgs {
   Pack<R, V>* acc;           // accumulator (null when nflush == 0)
   const Pack<R, V>* ref;     // correlation reference (null: no partials)
   int ref_tpr;               // packs per row of ref; lanes >= ref_tpr correlate to 0
-  double* partials;          // [(col*3 + v) * gridDim.x + block]
+  double* partials;          // [(col*nv + v) * gridDim.x + block], nv = 3 (mode 2) or 2 (mode 3)
   TermCoef c;
 };
 
 // Kernel modes: 0 = recurrence only, 1 = recurrence + accumulator flush,
-// 2 = flush + correlation/norm partials (last term of a time step).  Each
+// 2 = flush + correlation/norm partials (last term of a time step), 3 =
+// recurrence + partials of <p_k|p_k> and Re <p_k|p_{k-1}> per column (moments:
+// both factors are in registers, so they cost no memory traffic).  Each
 // mode is compiled separately so the common mode-0 terms keep few registers.
 // Blocks have at most 256 threads; the minimum resident blocks per SM bound
 // the registers per thread (4 blocks: 64 registers).
@@ -133,10 +135,10 @@ __global__ void __launch_bounds__(256, (TermBounds<R, MODE, V>::min_blocks))
   const unsigned neg_bits = (unsigned)(a.c.neg_mask >> (lane * V)) & ((1u << V) - 1u);
   const unsigned set_bits = (unsigned)(a.c.set_mask >> (lane * V)) & ((1u << V) - 1u);
   const R beta = (R)a.c.beta;
-  const int nflush = MODE >= 1 ? a.c.nflush : 0;
+  const int nflush = MODE == 1 || MODE == 2 ? a.c.nflush : 0;
   constexpr bool do_corr = MODE == 2;
   const bool ref_lane = do_corr && a.ref != nullptr && lane < a.ref_tpr;
-  const bool need_own = a.diag != nullptr || nflush >= 2;
+  const bool need_own = MODE == 3 || a.diag != nullptr || nflush >= 2;
 
   double cre[V], cim[V], nrm[V];
 #pragma unroll
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(256, (TermBounds<R, MODE, V>::min_blocks))
           const char* p = reinterpret_cast<const char*>(a.pin);
           prefetch_l2(p + rp * row_bytes, tile, p, p + a.n_rows * row_bytes);
         }
-        if (MODE >= 1 && !a.c.acc_init) {
+        if ((MODE == 1 || MODE == 2) && !a.c.acc_init) {
           const char* q = reinterpret_cast<const char*>(a.acc);
           prefetch_l2(q + rp * row_bytes, tile, q, q + a.n_rows * row_bytes);
         }
@@ -261,17 +263,26 @@ __global__ void __launch_bounds__(256, (TermBounds<R, MODE, V>::min_blocks))
         }
       }
     }
+    if (MODE == 3) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
+        nrm[v] += xr * xr + xi * xi;
+        cre[v] += xr * (double)own.v[2 * v] + xi * (double)own.v[2 * v + 1];
+      }
+    }
     if (a.pout) stcs_pack(a.pout + e, pk);
   }
 
-  if (do_corr) {
-    const int width = tpr * V * 3;
+  if (MODE >= 2) {
+    constexpr int NV = MODE == 3 ? 2 : 3;
+    const int width = tpr * V * NV;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-      double* s = smem + slot * width + (lane * V + v) * 3;
-      s[0] = cre[v];
-      s[1] = cim[v];
-      s[2] = nrm[v];
+      double* s = smem + slot * width + (lane * V + v) * NV;
+      s[0] = MODE == 3 ? nrm[v] : cre[v];
+      s[1] = MODE == 3 ? cre[v] : cim[v];
+      if (NV == 3) s[2] = nrm[v];
     }
     __syncthreads();
     tree_reduce_slots(smem, rpp, width, slot, lane, tpr);
@@ -280,8 +291,8 @@ __global__ void __launch_bounds__(256, (TermBounds<R, MODE, V>::min_blocks))
       for (int v = 0; v < V; ++v) {
         const int col = lane * V + v;
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
-          a.partials[(int64_t)(col * 3 + q) * gridDim.x + blockIdx.x] = smem[col * 3 + q];
+        for (int q = 0; q < NV; ++q)
+          a.partials[(int64_t)(col * NV + q) * gridDim.x + blockIdx.x] = smem[col * NV + q];
       }
     }
   }

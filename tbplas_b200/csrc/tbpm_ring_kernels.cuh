@@ -4,8 +4,9 @@
 // The term computes the same values in the same order as cheb_term_kernel
 // (tbpm_kernels.cuh): p_k = alpha*(H p_{k-1}) + beta*p_{k-2}, H = D + O, with the
 // deferred Bessel/Fermi-weighted flush of up to three pending terms into the
-// accumulator and, in MODE 2, the <ref|psi> / <psi|psi> block partials.  Only
-// the way the operands reach the threads differs.
+// accumulator and, in MODE 2, the <ref|psi> / <psi|psi> block partials, in MODE
+// 3 those of <p_k|p_k> and Re <p_k|p_{k-1}>.  Only the way the operands reach
+// the threads differs.
 //
 // A block is one producer warp and kRingConsumerWarps consumer warps.  The
 // persistent grid walks row tiles grid-stride; tile i of a block goes to stage
@@ -194,8 +195,8 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
   const int tid = threadIdx.x;
   const uint32_t full0 = ring_smem(rsm + sh.bar_off);
   const uint32_t empty0 = full0 + 8u * (uint32_t)S;
-  const int nflush = MODE >= 1 ? a.c.nflush : 0;
-  const bool need_own = a.diag != nullptr || nflush >= 2;
+  const int nflush = MODE == 1 || MODE == 2 ? a.c.nflush : 0;
+  const bool need_own = MODE == 3 || a.diag != nullptr || nflush >= 2;
   const bool add_acc = nflush > 0 && !a.c.acc_init;
   const int64_t row_bytes = (int64_t)tpr * sizeof(Pack<R, V>);
   const bool ref_staged = MODE == 2 && a.ref != nullptr && sh.ref_off >= 0;
@@ -491,6 +492,14 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
           pk.v[2 * v] = fma(ar, sre[v], fma(-ai, sim[v], beta * pm2.v[2 * v]));
           pk.v[2 * v + 1] = fma(ar, sim[v], fma(ai, sre[v], beta * pm2.v[2 * v + 1]));
         }
+        if (MODE == 3) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
+            nrm[v] += xr * xr + xi * xi;
+            cre[v] += xr * (double)own.v[2 * v] + xi * (double)own.v[2 * v + 1];
+          }
+        }
         if (a.pout) stcs_pack(a.pout + e, pk);
         if (nflush > 0) {
           Pack<R, V> acc;
@@ -537,19 +546,20 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
     }
   }
 
-  if constexpr (MODE == 2) {
-    // block partials of the correlation and norm, reduced in a fixed order over
-    // the rows of a tile; the stage buffers are free (every copy was consumed)
+  if constexpr (MODE >= 2) {
+    // block partials of the products, reduced in a fixed order over the rows
+    // of a tile; the stage buffers are free (every copy was consumed)
+    constexpr int NV = MODE == 3 ? 2 : 3;
     __syncthreads();
     double* red = reinterpret_cast<double*>(rsm);
-    const int width = tpr * V * 3;
+    const int width = tpr * V * NV;
     if (tid < kRingConsumers && slot < TR) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        double* p = red + slot * width + (lane * V + v) * 3;
-        p[0] = cre[v];
-        p[1] = cim[v];
-        p[2] = nrm[v];
+        double* p = red + slot * width + (lane * V + v) * NV;
+        p[0] = MODE == 3 ? nrm[v] : cre[v];
+        p[1] = MODE == 3 ? cre[v] : cim[v];
+        if (NV == 3) p[2] = nrm[v];
       }
     }
     __syncthreads();
@@ -559,8 +569,8 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
       for (int v = 0; v < V; ++v) {
         const int col = lane * V + v;
 #pragma unroll
-        for (int q = 0; q < 3; ++q)
-          a.partials[(int64_t)(col * 3 + q) * gridDim.x + blockIdx.x] = red[col * 3 + q];
+        for (int q = 0; q < NV; ++q)
+          a.partials[(int64_t)(col * NV + q) * gridDim.x + blockIdx.x] = red[col * NV + q];
       }
     }
   }

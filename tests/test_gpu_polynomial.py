@@ -1,0 +1,181 @@
+"""Long runs (64 time steps or more) evaluate functions of a Hermitian H from
+Chebyshev vectors over the whole run (tbpm_poly_kernels.cuh) instead of step by
+step.  Every case is compared with the time-stepping CPU oracle on the same
+inputs: FP64 to the relative 1e-10 of the other parity tests, FP32 states to
+their 3e-5; calls that must keep time stepping (a non-Hermitian matrix, long
+rows, a series that is not unitary) are compared the same way.
+"""
+
+import math
+
+import numpy as np
+import pytest
+
+import tbplas_b200 as tb
+from tbplas_b200 import _native as nat
+from tbplas_b200.fortran import f2py
+from oracle import oracle
+
+from conftest import bessel_series, rel_err, unit_states
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-10, "fp32": 3e-5}
+
+
+@pytest.fixture(autouse=True)
+def _backend():
+    f2py.set_backend(precision="fp64", batch=16, device=0, state_kind="exp", term_kernel=0,
+                     use_graphs=True, vector_width=0, threads_per_block=0, rows_per_tile=0)
+    yield
+    f2py.set_backend(precision="fp64", batch=16, term_kernel=0, vector_width=0)
+
+
+@pytest.fixture(scope="module")
+def flake():
+    """A ragged open sample with vacancies in a field."""
+    s = tb.make_graphene_sample(19, 23, disorder=1.0, vacancy_rate=0.02, pbc=False, rescale=9.0,
+                                seed=3)
+    s.set_magnetic_field(60.0)
+    return s.build_ham_csr()
+
+
+def _random_hermitian(n, degree, seed):
+    """A sparse Hermitian matrix with rows of very different lengths, unsorted
+    columns, and its largest row sum below 0.95."""
+    rng = np.random.default_rng(seed)
+    rows = [dict() for _ in range(n)]
+    for r in range(n):
+        for c in rng.integers(0, n, rng.integers(0, degree)):
+            if c != r:
+                v = complex(rng.standard_normal(), rng.standard_normal())
+                rows[r][int(c)] = v
+                rows[int(c)][r] = v.conjugate()
+        rows[r][r] = complex(rng.standard_normal())
+    top = max(sum(abs(v) for v in row.values()) for row in rows)
+    ip = np.zeros(n + 1, dtype=np.int32)
+    ix, hv = [], []
+    for r, row in enumerate(rows):
+        keys = list(row)
+        rng.shuffle(keys)
+        ip[r + 1] = ip[r] + len(keys)
+        ix += keys
+        hv += [row[k] * 0.95 / top for k in keys]
+    return ip, np.array(ix, dtype=np.int32), np.array(hv, dtype=np.complex128)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("kernel", [0, 1, 2])
+@pytest.mark.parametrize("ns", [1, 3, 16])
+def test_dos_long_run(flake, prec, kernel, ns):
+    """One launch for all terms (0), the grid-stride kernel (1), the ring (2);
+    with the norm check inside the run."""
+    h = flake
+    wf0 = unit_states(ns, h.shape[0], seed=ns)
+    bes = bessel_series(math.pi)
+    f2py.set_backend(precision=prec, term_kernel=kernel)
+    got, per = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, 130, 128, 1e-9,
+                                    per_state=True)
+    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 130, wf0=wf0)
+    assert rel_err(got, ref) < TOL[prec]
+    assert np.allclose(per.mean(axis=0), got, rtol=0, atol=1e-14)
+
+
+@pytest.mark.parametrize("n,degree", [(1, 1), (2, 2), (37, 3), (700, 9), (3001, 14)])
+@pytest.mark.parametrize("width", [0, 1])
+def test_dos_long_run_of_general_matrices(n, degree, width):
+    """Rows with no entries up to tens of them, unsorted columns."""
+    ip, ix, hv = _random_hermitian(n, degree, seed=n)
+    wf0 = unit_states(4, n, seed=5)
+    bes = bessel_series(math.pi)
+    for kernel in (0, 1, 2):
+        f2py.set_backend(vector_width=width, term_kernel=kernel)
+        got = f2py.tbpm_dos_states(bes, ip, ix, hv, wf0, 64, 128, 1e-9)
+        ref = oracle.tbpm_dos(bes, ip, ix, hv, 64, wf0=wf0)
+        assert rel_err(got, ref) < 1e-10
+
+
+def test_dos_long_run_several_items_per_thread():
+    """32,768 orbitals x 16 states: several items per thread of the one-launch
+    kernel, device-generated states."""
+    s = tb.make_graphene_sample(128, 128, disorder=1.0, rescale=9.0, seed=11)
+    h = s.build_ham_csr()
+    bes = bessel_series(math.pi)
+    got = f2py.tbpm_dos(bes, h.indptr, h.indices, h.data, 7, 64, 16, "", 0, 128, 1e-9)
+    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 64, seed=7, n_samples=16)
+    assert rel_err(got, ref) < 1e-10
+
+
+def test_dos_other_time_steps(flake):
+    """Half and twice the usual time step, a negative one, and a rescale factor
+    far above the spectral radius."""
+    h = flake
+    wf0 = unit_states(2, h.shape[0], seed=1)
+    for z, scale in ((math.pi / 2, 1.0), (2 * math.pi, 1.0), (-math.pi, 1.0), (math.pi, 0.02)):
+        bes = [(-1) ** k * b for k, b in enumerate(bessel_series(-z))] if z < 0 \
+            else bessel_series(z)
+        got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data * scale, wf0, 96, 90, 1e-9)
+        ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data * scale, 96, wf0=wf0)
+        assert rel_err(got, ref) < 1e-10
+
+
+def test_calls_that_keep_time_stepping(flake):
+    """A non-Hermitian matrix, a row of 80 entries, a series cut at 1e-6 (its
+    step is not unitary to rounding)."""
+    h = flake
+    n = h.shape[0]
+    wf0 = unit_states(2, n, seed=2)
+    bes = bessel_series(math.pi)
+    skew = h.data.copy()
+    skew[11] *= 1 + 1e-9
+    cut = bessel_series(math.pi, precision=1e-6)
+    star = np.zeros((n, n), dtype=complex)
+    star[5, 100:180] = 0.005j
+    star[100:180, 5] = -0.005j
+    import scipy.sparse as sp
+    hs = sp.csr_matrix(h + sp.csr_matrix(star)) * 0.9
+    for b, ip, ix, hv in ((bes, h.indptr, h.indices, skew), (bes, hs.indptr, hs.indices, hs.data),
+                          (cut, h.indptr, h.indices, h.data)):
+        got = f2py.tbpm_dos_states(b, ip, ix, hv, wf0, 70, 200, 1e-9)
+        ref = oracle.tbpm_dos(b, ip, ix, hv, 70, wf0=wf0)
+        assert rel_err(got, ref) < 1e-10
+
+
+def test_norm_errors_of_long_runs(flake):
+    """What check_norm refuses is refused: a rescale factor below the spectral
+    radius, a series that loses norm, a NaN in a state."""
+    h = flake
+    n = h.shape[0]
+    wf0 = unit_states(2, n, seed=4)
+    bes = bessel_series(math.pi)
+    with pytest.raises(nat.NormError):
+        f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data * 4.5, wf0, 80, 64, 1e-9)
+    with pytest.raises(nat.NormError):
+        f2py.tbpm_dos_states(np.asarray(bes) * (1 - 1e-8), h.indptr, h.indices, h.data, wf0, 80,
+                             64, 1e-9)
+    wf0[1, 3] = np.nan
+    with pytest.raises(nat.NanError):
+        f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, 80, 64, 1e-9)
+    got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0[:1], 80, 64, 1e-9)
+    assert rel_err(got, oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 80,
+                                        wf0=wf0[:1])) < 1e-10
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("ns", [1, 4])
+def test_packed_realisations_long_run(prec, ns):
+    samples = [tb.make_graphene_sample(nx, ny, disorder=w, vacancy_rate=v, rescale=10.0, seed=i)
+               for i, (nx, ny, w, v) in enumerate([(6, 5, 0.0, 0.0), (9, 7, 1.5, 0.02),
+                                                   (70, 40, 3.0, 0.01)])]
+    packed = tb.pack_samples(samples)
+    bes = bessel_series(math.pi)
+    f2py.set_backend(precision=prec)
+    corr, per = f2py.tbpm_dos_segmented(bes, packed.indptr, packed.indices, packed.data,
+                                        packed.offsets, ns, 1337, 72, 64, 1e-9, per_state=True)
+    for k, s in enumerate(samples):
+        h = s.build_ham_csr()
+        for b in range(ns):
+            ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 72,
+                                  seed=1337 * (k * ns + b + 1), n_samples=1)
+            assert rel_err(per[k, b], ref) < TOL[prec]
+        assert np.allclose(corr[k], per[k].mean(axis=0), rtol=0, atol=1e-14)

@@ -1190,11 +1190,56 @@ std::vector<PolyNode> poly_nodes(const PolyPlan& pp, int M) {
   return nodes;
 }
 
-// Arguments of term k of p_k = (2/a) H p_{k-1} - p_{k-2} on two buffers: p_k
-// overwrites p_{k-2}.
+// w[k] with P(x)^m = sum_k w[k] (-i)^k T_k(x/a), k < bessel_degree: the even
+// coefficients of a power of P are real, the odd ones imaginary, and the
+// nodes j and M-1-j differ only in the sign of x, so half of them suffice.
+std::vector<double> power_weights(const PolyPlan& pp, int m) {
+  const int M = std::max(4, bessel_degree(pp.tau * (double)pp.a * m));
+  const std::vector<PolyNode> nodes = poly_nodes(pp, M);
+  const double pi = 3.14159265358979323846;
+  std::vector<double> re(M), im(M), tab(4 * (size_t)M);
+  for (int j = 0; j < M; ++j) {
+    const long double t = (long double)m * ((long double)nodes[j].hi + nodes[j].lo);
+    const long double f = 2 * 3.14159265358979323846264338327950288L * (t - roundl(t));
+    const double g = std::exp(m * nodes[j].lnabs);
+    re[j] = g * (double)cosl(f);
+    im[j] = g * (double)sinl(f);
+  }
+  for (int q = 0; q < 4 * M; ++q) tab[q] = std::cos(pi * q / (2.0 * M));
+  std::vector<double> w(M);
+  for (int k = 0; k < M; ++k) {
+    const std::vector<double>& f = (k & 1) ? im : re;
+    double s = 0.0;
+    for (int j = 0; j < M / 2; ++j)
+      s += f[j] * tab[(size_t)((int64_t)k * (2 * j + 1) % (4 * M))];
+    s *= 2.0;
+    if (M & 1) s += f[M / 2] * tab[(size_t)((int64_t)k * M % (4 * M))];
+    s *= (k ? 2.0 : 1.0) / M;
+    // (-i)^k: 1, -i, -1, i
+    const int q = k & 3;
+    w[k] = (q == 0 || q == 3) ? s : -s;
+  }
+  return w;
+}
+
+// m time steps as one expansion on y = H/a: p_k = (-i)^k T_k(y) psi.
+Expansion power_expansion(const PolyPlan& pp, int m) {
+  Expansion e;
+  e.w[0] = power_weights(pp, m);
+  e.w[1] = e.w[0];
+  e.n_terms = (int)e.w[0].size();
+  e.alpha1_im = -0.5 * (double)pp.alpha;
+  e.alpha_im = -(double)pp.alpha;
+  e.beta = 1.0;
+  return e;
+}
+
+// Arguments of the term p_k = (2/a) H p_{k-1} - p_{k-2} (k >= 1), or, with
+// `turn`, of the same vectors times (-i)^k.
 template <typename R, int V>
-TermArgs<R, V> poly_term(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr, Pack<R, V>* A,
-                         Pack<R, V>* X) {
+TermArgs<R, V> poly_term(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr,
+                         const Pack<R, V>* pm1, const Pack<R, V>* pm2, Pack<R, V>* pk,
+                         bool turn = false) {
   const Ham& h = c->ham;
   TermArgs<R, V> a{};
   a.indptr = h.indptr.as<int32_t>();
@@ -1203,12 +1248,24 @@ TermArgs<R, V> poly_term(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr, 
   a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
   a.n_rows = h.n;
   a.tpr = tpr;
-  a.gather = (k & 1) ? A : X;
-  a.pout = (k & 1) ? X : A;
-  a.pin = k >= 2 ? a.pout : nullptr;
-  a.c.alpha_re = (k == 1 ? 0.5 : 1.0) * (double)pp.alpha;
-  a.c.beta = k >= 2 ? -1.0 : 0.0;
+  a.gather = pm1;
+  a.pin = k >= 2 ? pm2 : nullptr;
+  a.pout = pk;
+  const double alpha = (k == 1 ? 0.5 : 1.0) * (double)pp.alpha;
+  if (turn)
+    a.c.alpha_im = -alpha;
+  else
+    a.c.alpha_re = alpha;
+  a.c.beta = k >= 2 ? (turn ? 1.0 : -1.0) : 0.0;
   return a;
+}
+
+// The same on two buffers, p_0 in A: p_k overwrites p_{k-2}.
+template <typename R, int V>
+TermArgs<R, V> poly_term2(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr, Pack<R, V>* A,
+                          Pack<R, V>* X) {
+  Pack<R, V>* dst = (k & 1) ? X : A;
+  return poly_term<R, V>(c, pp, k, tpr, (k & 1) ? A : X, dst, dst);
 }
 
 double matrix_bytes(const Ham& h) {
@@ -1307,7 +1364,7 @@ void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R
   for (int k0 = 1; k0 <= K; k0 += chunk) {
     const int m = std::min(chunk, K - k0 + 1);
     for (int i = 0; i < m; ++i) {
-      TermArgs<R, V> a = poly_term<R, V>(c, pp, k0 + i, tpr, A, X);
+      TermArgs<R, V> a = poly_term2<R, V>(c, pp, k0 + i, tpr, A, X);
       a.partials = c->partials.as<double>() + (int64_t)i * per_term;
       launch_term<R, V>(c, tt, a);
       c->model_bytes += bytes;
@@ -1325,19 +1382,20 @@ void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R
 void enqueue_moment_curves(tbpm_ctx* c, const PolyPlan& pp, int M, int T, int n_cols,
                            const double* sums, int64_t stride, const double* mu0,
                            int mu0_stride, double* mu, double* rho, PolyNode* nodes,
-                           int chk_step) {
+                           int chk_step, int t_ref = 1, bool have_nodes = false) {
   const int64_t total = (int64_t)n_cols * M;
   moment_gather_kernel<<<(int)std::min<int64_t>(blocks_for(total, 256), 4096), 256, 0,
                          c->stream>>>(sums, stride, mu0, mu0_stride, n_cols, M, mu);
   const unsigned cg = (unsigned)((n_cols + kMomentCols - 1) / kMomentCols);
   moment_density_kernel<<<dim3((unsigned)M, cg), 128, 0, c->stream>>>(mu, n_cols, M, rho);
   TBPM_CK(cudaGetLastError());
-  // (the host evaluates the nodes while the terms run)
-  const std::vector<PolyNode> host = poly_nodes(pp, M);
-  TBPM_CK(cudaMemcpyAsync(nodes, host.data(), sizeof(PolyNode) * M, cudaMemcpyHostToDevice,
-                          c->stream));
+  if (!have_nodes) {  // the host evaluates them while the terms run
+    const std::vector<PolyNode> host = poly_nodes(pp, M);
+    TBPM_CK(cudaMemcpyAsync(nodes, host.data(), sizeof(PolyNode) * M, cudaMemcpyHostToDevice,
+                            c->stream));
+  }
   moment_curve_kernel<<<dim3((unsigned)(T + 3), cg), 128, 0, c->stream>>>(
-      nodes, rho, n_cols, M, T, 1, std::max(chk_step - 1, 1), c->out.as<double>());
+      nodes, rho, n_cols, M, T, t_ref, std::max(chk_step - 1, 1), c->out.as<double>());
   TBPM_CK(cudaGetLastError());
   c->launches += 3;
 }
@@ -1709,7 +1767,7 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
       const int k = k0 + i;
       Pack<R, V>* x = (k & 1) ? X : A;
       Pack<R, V>* y = (k & 1) || k == 0 ? A : X;
-      if (k >= 1) launch_term<R, V>(c, tt, poly_term<R, V>(c, pp, k, tpr, A, X));
+      if (k >= 1) launch_term<R, V>(c, tt, poly_term2<R, V>(c, pp, k, tpr, A, X));
       seg_dots_kernel<R><<<grid, threads, 0, c->stream>>>(
           c->seg.as<int64_t>(), ns, rows_per_chunk, reinterpret_cast<const C*>(x),
           reinterpret_cast<const C*>(y), c->partials.as<double>() + (int64_t)i * per_term);
@@ -1753,14 +1811,159 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
   return true;
 }
 
+// ---- several time steps per expansion (combine_kernel) ---------------------------
+
+// Weights of P^1 .. P^m; the last one's length is the number of vectors.
+struct StepsPlan {
+  int m = 0;
+  std::vector<std::vector<double>> w;
+};
+
+StepsPlan steps_plan(const PolyPlan& pp, int m) {
+  StepsPlan sp;
+  sp.m = m;
+  for (int j = 1; j <= m; ++j) sp.w.push_back(power_weights(pp, j));
+  return sp;
+}
+
+// states[j] = P(H)^(j+1) psi, j < m <= sp.m, for blocks of ld columns.  psi may be
+// states[sp.m-1].  ring: window + 2 blocks for the vectors of the recurrence; the
+// outputs are updated once per `window` vectors (at most kCombineWindow).
+template <typename R, int V>
+void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, int ld,
+                   Pack<R, V>* psi, const std::vector<Pack<R, V>*>& ring,
+                   const std::vector<Pack<R, V>*>& states) {
+  using C = typename Cx<R>::t;
+  const int64_t n = c->ham.n;
+  const double vb = (double)n * ld * sizeof(C);
+  const int tpr = ld / V;
+  const int window = (int)ring.size() - 2;
+  const TermTiles tt = term_tiles<R, V>(c, n, tpr);
+  const double term_bytes = matrix_bytes(c->ham) + 3.0 * vb;
+  auto vec = [&](int k) { return k == 0 ? psi : ring[k % ring.size()]; };
+  const int n_vec = (int)sp.w[m - 1].size();
+  CombineArgs<R> a{};
+  a.total = n * ld;
+  a.m = m;
+  for (int j = 0; j < m; ++j) a.out[j] = reinterpret_cast<C*>(states[j]);
+  const int grid = blocks_for(a.total, 256);
+  for (int k0 = 0; k0 < n_vec; k0 += window) {
+    const int len = std::min(window, n_vec - k0);
+    for (int q = 0; q < len; ++q) {
+      const int k = k0 + q;
+      if (k >= 1) {
+        launch_term<R, V>(c, tt,
+                          poly_term<R, V>(c, pp, k, tpr, vec(k - 1), k >= 2 ? vec(k - 2) : nullptr,
+                                          vec(k), true));
+        c->model_bytes += term_bytes;
+      }
+      a.p[q] = reinterpret_cast<const C*>(vec(k));
+    }
+    a.np = len;
+    // outputs are ordered by degree: those that end before this window are done
+    a.j0 = 0;
+    while (a.j0 < m - 1 && (int)sp.w[a.j0].size() <= k0) ++a.j0;
+    a.init = k0 == 0 ? 0xffffffffu : 0u;
+    for (int j = 0; j < m; ++j)
+      for (int q = 0; q < kCombineWindow; ++q)
+        a.w[j][q] = q < len && k0 + q < (int)sp.w[j].size() ? sp.w[j][k0 + q] : 0.0;
+    if (m <= 4)
+      combine_kernel<R, 4><<<grid, 256, 0, c->stream>>>(a);
+    else if (m <= 8)
+      combine_kernel<R, 8><<<grid, 256, 0, c->stream>>>(a);
+    else
+      combine_kernel<R, 16><<<grid, 256, 0, c->stream>>>(a);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    c->model_bytes += vb * (len + (m - a.j0) * (k0 == 0 ? 1 : 2));
+  }
+}
+
+// Time steps per expansion and vectors per update for blocks of vb bytes.
+struct StepsShape {
+  int m = 0;  // 0: none fits
+  int window = 0;
+};
+
+// The largest shape whose states and ring, beside `other` bytes, fit the memory
+// that is free or held by the buffers they go into.  Model of a step of phase
+// pi/2 in passes over the block (time stepping: 57): 20 at (16, 16), 24 at
+// (8, 16), 27 at (8, 8), 36 at (4, 8).
+StepsShape steps_that_fit(size_t vb, size_t other, size_t held) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return StepsShape{};
+  }
+  const size_t reserve = (size_t)2 << 30;
+  for (const StepsShape s : {StepsShape{16, 16}, StepsShape{8, 16}, StepsShape{8, 8},
+                             StepsShape{4, 8}})
+    if (vb * (size_t)(s.m + s.window + 2) + other + reserve <= free_b + held) return s;
+  return StepsShape{};
+}
+
+// Blocks of several steps can fill the device; they are given back after the
+// call when they hold more than this.
+constexpr size_t kKeepBytes = (size_t)8 << 30;
+void trim(DevMem& m) {
+  if (m.bytes > kKeepBytes) m.release();
+}
+
+// Room for the blocks of enqueue_steps behind the block in c->A (ld columns; X
+// and Y serve as two blocks of the ring), reserved before c->A is filled.
+template <typename R>
+StepsShape steps_room(tbpm_ctx* c, const PolyPlan* pp, int ld, int ref_ld) {
+  if (!pp) return StepsShape{};
+  const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
+  const size_t ref = (size_t)c->ham.n * ref_ld * 2 * sizeof(R);
+  const StepsShape s =
+      steps_that_fit(vb, vb + ref, c->A.bytes + c->X.bytes + c->Y.bytes + c->wf0.bytes);
+  if (s.m > 0) c->A.ensure(vb * (size_t)(1 + s.window + s.m));
+  return s;
+}
+
+// Propagates the block in c->A by enqueue_steps and hands every state to `each`.
+template <typename R, int V>
+struct StepsRun {
+  const PolyPlan* pp;
+  StepsPlan sp;
+  int ld;
+  Pack<R, V>* psi = nullptr;
+  std::vector<Pack<R, V>*> ring, states;
+
+  StepsRun(tbpm_ctx* c, const PolyPlan* plan, const StepsShape& s, int ld_) : pp(plan), ld(ld_) {
+    if (s.m == 0) return;
+    const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
+    auto block = [&](int i) { return reinterpret_cast<Pack<R, V>*>(c->A.as<char>() + vb * i); };
+    sp = steps_plan(*plan, s.m);
+    psi = block(0);
+    ring = {c->X.as<Pack<R, V>>(), c->Y.as<Pack<R, V>>()};
+    for (int q = 0; q < s.window; ++q) ring.push_back(block(1 + q));
+    for (int j = 0; j < s.m; ++j) states.push_back(block(1 + s.window + j));
+  }
+
+  template <class F>
+  void run(tbpm_ctx* c, int n_steps, F&& each) {
+    while (n_steps > 0) {
+      const int m = std::min(n_steps, sp.m);
+      enqueue_steps<R, V>(c, *pp, sp, m, ld, psi, ring, states);
+      for (int j = 0; j < m; ++j) each(states[j]);
+      if (m < sp.m) std::swap(states[m - 1], states[sp.m - 1]);
+      psi = states[sp.m - 1];
+      n_steps -= m;
+    }
+  }
+};
+
 // ---- AC ---------------------------------------------------------------------
 
 template <typename R, int V>
 void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, int nb,
               const StateKeys* keys, const double* host_wf0, int n_timestep, int chk_step,
-              double chk_thr, int n_avg, double* corr) {
+              double chk_thr, int n_avg, double* corr, const PolyPlan* pp) {
   const int ld = 3 * nb;
   c->graph.reset();
+  const StepsShape shape = steps_room<R>(c, pp, ld, nb);
   ensure_vectors(c, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * nb * 9 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
@@ -1784,12 +1987,12 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
   const Tile tj = pick_tile(c, h.n, nb, jcorr_kernel<R>, 9 * sizeof(double));
   const size_t smem_j = (size_t)tj.threads * 9 * sizeof(double);
   reset_counters(c, 0);
-  auto jcorr = [&]() {
+  auto jcorr = [&](const Pack<R, V>* x) {
     ensure_partials(c, (size_t)nb * 9 * tj.grid);
     jcorr_kernel<R><<<tj.grid, tj.threads, smem_j, c->stream>>>(
         h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<typename Cx<R>::t>(),
         h.dx.as<R>(), h.dy.as<R>(), h.rescale, h.n, tj.rows_per_tile, nb,
-        reinterpret_cast<const typename Cx<R>::t*>(A), c->partials.as<double>());
+        reinterpret_cast<const typename Cx<R>::t*>(x), c->partials.as<double>());
     TBPM_CK(cudaGetLastError());
     c->launches++;
     c->model_bytes += (double)(h.n + 1) * 4 + (double)h.nnz * (4 + 4 * sizeof(R)) +
@@ -1798,19 +2001,26 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
   };
   // row 0: after the Fermi operators (t = 1, not accumulated; its psi2 norm is
   // the norm reference of tbpm.f90:307)
-  jcorr();
+  jcorr(A);
   auto step = [&]() {
     enqueue_expansion<R, V>(c, ex_time, ld, A, X, Y, nullptr, 0, nullptr, Counters{});
-    jcorr();
+    jcorr(A);
   };
   const double thr = effective_thr(c, chk_thr);
   std::vector<double> host;
   int done = 0;  // propagation steps enqueued; row r = after r steps
   const bool check = chk_step >= 2 && chk_step <= n_timestep;
   const auto key = plan_key(c, 2, ld, V, ex_time);
+  StepsRun<R, V> many(c, pp, shape, ld);
+  auto advance = [&](int n_steps) {
+    if (shape.m > 0)
+      many.run(c, n_steps, jcorr);
+    else
+      run_steps(c, n_steps, key, step);
+  };
   if (check) {
     // at t == chk_step psi2 has been propagated chk_step-2 times
-    run_steps(c, chk_step - 2, key, step);
+    advance(chk_step - 2);
     done = chk_step - 2;
     read_out(c, host, (size_t)(done + 1) * nb * 9);
     for (int b = 0; b < nb; ++b) {
@@ -1820,7 +2030,7 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
         raise_norm("tbpm_accond", chk_step, bad_);
     }
   }
-  run_steps(c, (n_timestep - 1) - done, key, step);
+  advance((n_timestep - 1) - done);
   const int rows = std::max(n_timestep, 1);
   read_out(c, host, (size_t)rows * nb * 9);
   // corr(k, t) for t = 2..n_timestep is row t-1 (tbpm.f90:346-349)
@@ -1860,12 +2070,135 @@ void qe_project_attr(size_t bytes) {
   qe_smem_attr(qe_project_kernel<R>, bytes);
 }
 
+// Phase 1 on the polynomial route: QE_i = f_i(H) wf0 by the energies' filters
+// (filter_values_kernel), and the DOS correlation from the moments of the same
+// vectors' first half.  dos (complex [T] per state, interleaved [t][nb]) may be null.
+template <typename R, int V>
+void dc_filter(tbpm_ctx* c, const PolyPlan& pp, int nb, const Pack<R, V>* W, int T, double t_step,
+               const std::vector<double>& en_sel, int chk_step, double chk_thr, const char* who,
+               std::vector<double>* dos) {
+  using C = typename Cx<R>::t;
+  const int64_t n = c->ham.n;
+  const int n_en = (int)en_sel.size();
+  const int M = std::max(4, bessel_degree(pp.tau * (double)pp.a * T));
+  const int K = M / 2;
+  const int last = n_en > 0 ? M - 1 : K;  // last Chebyshev vector needed
+  const size_t vb = (size_t)n * nb * sizeof(C);
+  constexpr int slots = kFilterWindow + 2;
+  c->A.ensure(vb * slots);
+  c->out.ensure((size_t)(T + 3) * nb * 2 * sizeof(double));
+  c->small.ensure(sizeof(double) * kMaxCols * 3);
+  const size_t n_sums = (size_t)K * nb * 2, n_mu = (size_t)nb * M, n_f = (size_t)M * n_en;
+  const size_t n_c = (size_t)T * n_en;  // window and phase factors (complex)
+  c->poly.ensure((n_sums + 2 * n_mu + 2 * n_f + 2 * n_c) * sizeof(double) + sizeof(PolyNode) * M);
+  double2* factors = c->poly.as<double2>();
+  double* sums = c->poly.as<double>() + 2 * n_c;
+  double* mu = sums + n_sums;
+  double* rho = mu + n_mu;
+  double* f = rho + n_mu;
+  double* coef = f + n_f;
+  PolyNode* nodes = reinterpret_cast<PolyNode*>(coef + n_f);
+  const std::vector<PolyNode> host_nodes = poly_nodes(pp, M);
+  TBPM_CK(cudaMemcpyAsync(nodes, host_nodes.data(), sizeof(PolyNode) * M, cudaMemcpyHostToDevice,
+                          c->stream));
+  if (n_en > 0) {
+    // Hanning window and phases as the time-stepped phase 1 forms them
+    std::vector<double2> hf(n_c);
+    const double pi = 3.14159265358979323846;
+    for (int tt = 1; tt <= T; ++tt) {
+      const double Wh = 0.5 * (1 + std::cos(pi * tt / T));
+      for (int i = 0; i < n_en; ++i) {
+        const double x = en_sel[i] * (double)tt * t_step;
+        hf[(size_t)(tt - 1) * n_en + i] = make_double2(Wh * std::cos(x), Wh * std::sin(x));
+      }
+    }
+    TBPM_CK(cudaMemcpyAsync(factors, hf.data(), sizeof(double2) * n_c, cudaMemcpyHostToDevice,
+                            c->stream));
+    filter_values_kernel<<<dim3((unsigned)((M + 31) / 32), (unsigned)((n_en + 7) / 8)), 256, 0,
+                           c->stream>>>(nodes, M, factors, n_en, T, f);
+    filter_coef_kernel<<<dim3((unsigned)M, (unsigned)((n_en + 255) / 256)), 256, 0, c->stream>>>(
+        f, M, n_en, coef);
+    TBPM_CK(cudaGetLastError());
+    c->launches += 2;
+    TBPM_CK(cudaStreamSynchronize(c->stream));  // the host vectors go out of scope
+  }
+  reset_counters(c, 2);
+  enqueue_corr<R, V>(c, W, nullptr, nb, 0, c->small.as<double>(), counters(c, 2));
+  const int tpr = nb / V;
+  const TermTiles tt = term_tiles<R, V>(c, n, tpr);
+  const int grid3 = tt.t[3].grid;
+  const int64_t per_term = (int64_t)nb * 2 * grid3;
+  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(K, (64ll << 20) / (per_term * 8)));
+  ensure_partials(c, (size_t)chunk * per_term);
+  auto vec = [&](int k) -> Pack<R, V>* {
+    return k == 0 ? const_cast<Pack<R, V>*>(W)
+                  : reinterpret_cast<Pack<R, V>*>(c->A.as<char>() + vb * (k % slots));
+  };
+  const double term_bytes = matrix_bytes(c->ham) + 3.0 * (double)vb;
+  C* qe = c->qe.as<C>();
+  const int rt = qe_mma_rows(nb);
+  const int64_t tiles = (n + rt - 1) / rt;
+  const int groups = ((n_en + 7) / 8 + kQeMmaWarps * kQeMmaMT - 1) / (kQeMmaWarps * kQeMmaMT);
+  const dim3 qgrid((unsigned)std::min<int64_t>(tiles, (int64_t)num_sms(c->device) * 4),
+                   (unsigned)std::max(groups, 1));
+  const size_t qsmem = qe_filter_smem(nb);
+  qe_smem_attr(qe_filter_mma_kernel<R>, qsmem);
+  int pend = 0;  // terms whose block partials wait for their reduction
+  FilterPtrs<R> win{};
+  int w0 = 0;  // first vector of the window
+  for (int k = 0; k <= last; ++k) {
+    if (k >= 1) {
+      TermArgs<R, V> a = poly_term<R, V>(c, pp, k, tpr, vec(k - 1), k >= 2 ? vec(k - 2) : nullptr,
+                                         vec(k));
+      if (k <= K) a.partials = c->partials.as<double>() + (int64_t)pend * per_term;
+      launch_term<R, V>(c, tt, a);
+      c->model_bytes += term_bytes;
+      if (k <= K && (++pend == chunk || k == K)) {
+        const int64_t n_vals = (int64_t)pend * nb * 2;
+        reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+            c->partials.as<double>(), grid3, n_vals, sums + (int64_t)(k - pend) * nb * 2);
+        TBPM_CK(cudaGetLastError());
+        c->launches++;
+        pend = 0;
+      }
+    }
+    if (n_en == 0) continue;
+    win.p[k - w0] = reinterpret_cast<const C*>(vec(k));
+    if (k - w0 + 1 == kFilterWindow || k == last) {
+      qe_filter_mma_kernel<R><<<qgrid, kQeMmaWarps * 32, qsmem, c->stream>>>(
+          qe, n, n_en, nb, win, k - w0 + 1, coef + (int64_t)w0 * n_en, w0 == 0 ? 1 : 0);
+      TBPM_CK(cudaGetLastError());
+      c->launches++;
+      c->model_bytes += (double)n * n_en * nb * sizeof(C) * (w0 == 0 ? 1 : 2) +
+                        (double)(k - w0 + 1) * (double)vb;
+      w0 = k + 1;
+    }
+  }
+  const bool check = chk_step >= 2 && chk_step <= T;
+  if (!dos && !check) return;
+  enqueue_moment_curves(c, pp, M, T, nb, sums, (int64_t)nb * 2, c->small.as<double>() + 2, 3, mu,
+                        rho, nodes, chk_step, 0, true);
+  std::vector<double> host;
+  read_out(c, host, (size_t)(T + 3) * nb * 2);
+  if (check) {
+    // tbpm.f90:611-614: after chk_step - 1 steps against <wf0|wf0>; P and its
+    // conjugate have the same norms
+    const double thr = effective_thr(c, chk_thr);
+    for (int b = 0; b < nb; ++b)
+      if (const int bad = norm_broken(host[((size_t)(T + 2) * nb + b) * 2],
+                                      host[((size_t)(T + 1) * nb + b) * 2], thr))
+        raise_norm(who, chk_step, bad);
+  }
+  if (dos) dos->assign(host.begin() + (size_t)nb * 2, host.begin() + (size_t)(T + 1) * nb * 2);
+}
+
 template <typename R, int V>
 void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int nb,
               const StateKeys* keys, const double* host_wf0, int n_timestep, double t_step,
               const std::vector<double>& en_sel, int chk_step, double chk_thr, int n_avg,
               int n_energies, double* dos_corr, double* dc_corr, double* qe_acc = nullptr,
-              const char* who = "tbpm_dccond", int en_out0 = 0, bool add_dos = true) {
+              const char* who = "tbpm_dccond", int en_out0 = 0, bool add_dos = true,
+              const PolyPlan* pp = nullptr) {
   using C = typename Cx<R>::t;
   const Ham& h = c->ham;
   const int64_t n = h.n;
@@ -1875,9 +2208,11 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   const int T2 = std::min(8, std::max(n_timestep, 1));           // phase-2 window
   const size_t vb = (size_t)n * ld * 2 * sizeof(R);
   c->graph.reset();
-  c->X.ensure(vb);
-  c->Y.ensure(vb);
-  c->A.ensure(vb * (size_t)(std::max(T1, T2) + 1));
+  if (!pp) {
+    c->X.ensure(vb);
+    c->Y.ensure(vb);
+    c->A.ensure(vb * (size_t)(std::max(T1, T2) + 1));
+  }
   c->wf0.ensure((size_t)n * nb * 2 * sizeof(R));
   c->ctr.ensure(16 * sizeof(int));
   c->out.ensure((size_t)std::max(n_timestep, 1) * ld * 3 * sizeof(double));
@@ -1886,102 +2221,114 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   c->qe.ensure(qe_bytes);
   c->coef.ensure(sizeof(double2) * (size_t)kMaxWindow * std::max(n_en, 1));
   auto slot = [&](int s) { return reinterpret_cast<Pack<R, V>*>(c->A.as<char>() + vb * s); };
-  auto* X = c->X.as<Pack<R, V>>();
-  auto* Y = c->Y.as<Pack<R, V>>();
   auto* W = c->wf0.as<Pack<R, V>>();
   C* qe = c->qe.as<C>();
   if (keys)
     gen_states<R, V>(c, *keys, nb, c->opts.state_kind, W);
   else
     upload_states<R>(c, host_wf0, nb, nb, 0, W);
-  // wf_t_pos = wf_t_neg = wf0 in the slot read by the first step
-  dup_columns_kernel<R><<<blocks_for(n * nb, 256), 256, 0, c->stream>>>(
-      reinterpret_cast<const C*>(W), n, nb, reinterpret_cast<C*>(slot(T1 - 1)));
-  TBPM_CK(cudaGetLastError());
-  c->launches++;
-  // norm_ref = <wf0|wf0> (tbpm.f90:606) for every column
-  reset_counters(c, 2);
-  enqueue_corr<R, V>(c, slot(T1 - 1), nullptr, ld, 0, c->small.as<double>(), counters(c, 2));
-  std::vector<double> norm_ref(3 * ld);
-  TBPM_CK(cudaMemcpyAsync(norm_ref.data(), c->small.p, norm_ref.size() * sizeof(double),
-                          cudaMemcpyDeviceToHost, c->stream));
-  TBPM_CK(cudaStreamSynchronize(c->stream));
-  const double thr = effective_thr(c, chk_thr);
-  reset_counters(c, 0);
-  const bool check = chk_step >= 2 && chk_step <= n_timestep;
-  std::vector<double2> coef_host((size_t)kMaxWindow * std::max(n_en, 1));
   std::vector<double> host;
-  const double pi = 3.14159265358979323846;
-  // ---- phase 1: +/- dt propagation, DOS correlation, QE accumulation ----
   std::optional<Phase> phase;
   phase.emplace("tbpm_dccond: quasi-eigenstates");
   int t = 1;
-  bool first_window = true;
-  while (t <= n_timestep) {
-    int len = std::min(T1, n_timestep - t + 1);
-    if (check && t <= chk_step - 1 && t + len - 1 > chk_step - 1) len = chk_step - t;
-    for (int tau = 0; tau < len; ++tau) {
-      Pack<R, V>* in = slot(tau == 0 ? T1 - 1 : tau - 1);
-      enqueue_expansion<R, V>(c, ex_pm, ld, in, X, Y, W, nb, c->out.as<double>(),
-                              counters(c, 0), slot(tau));
-    }
-    if (n_en > 0) {
-      for (int tau = 0; tau < len; ++tau) {
-        const int tt = t + tau;
-        const double Wh = 0.5 * (1 + std::cos(pi * tt / n_timestep));  // Hanning
-        for (int i = 0; i < n_en; ++i) {
-          const double x = en_sel[i] * (double)tt * t_step;
-          coef_host[(size_t)tau * n_en + i] = make_double2(Wh * std::cos(x), Wh * std::sin(x));
+  if (pp) {
+    std::vector<double> dos;
+    dc_filter<R, V>(c, *pp, nb, W, n_timestep, t_step, en_sel, chk_step, chk_thr, who,
+                    dos_corr && add_dos ? &dos : nullptr);
+    if (dos_corr && add_dos)
+      for (int b = 0; b < nb; ++b)
+        for (int tt = 1; tt <= n_timestep; ++tt) {
+          dos_corr[2 * (tt - 1)] += dos[((size_t)(tt - 1) * nb + b) * 2] / n_avg;
+          dos_corr[2 * (tt - 1) + 1] += dos[((size_t)(tt - 1) * nb + b) * 2 + 1] / n_avg;
         }
+  } else {
+    auto* X = c->X.as<Pack<R, V>>();
+    auto* Y = c->Y.as<Pack<R, V>>();
+    // wf_t_pos = wf_t_neg = wf0 in the slot read by the first step
+    dup_columns_kernel<R><<<blocks_for(n * nb, 256), 256, 0, c->stream>>>(
+        reinterpret_cast<const C*>(W), n, nb, reinterpret_cast<C*>(slot(T1 - 1)));
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    // norm_ref = <wf0|wf0> (tbpm.f90:606) for every column
+    reset_counters(c, 2);
+    enqueue_corr<R, V>(c, slot(T1 - 1), nullptr, ld, 0, c->small.as<double>(), counters(c, 2));
+    std::vector<double> norm_ref(3 * ld);
+    TBPM_CK(cudaMemcpyAsync(norm_ref.data(), c->small.p, norm_ref.size() * sizeof(double),
+                            cudaMemcpyDeviceToHost, c->stream));
+    TBPM_CK(cudaStreamSynchronize(c->stream));
+    const double thr = effective_thr(c, chk_thr);
+    reset_counters(c, 0);
+    const bool check = chk_step >= 2 && chk_step <= n_timestep;
+    std::vector<double2> coef_host((size_t)kMaxWindow * std::max(n_en, 1));
+    const double pi = 3.14159265358979323846;
+    // ---- phase 1: +/- dt propagation, DOS correlation, QE accumulation ----
+    bool first_window = true;
+    while (t <= n_timestep) {
+      int len = std::min(T1, n_timestep - t + 1);
+      if (check && t <= chk_step - 1 && t + len - 1 > chk_step - 1) len = chk_step - t;
+      for (int tau = 0; tau < len; ++tau) {
+        Pack<R, V>* in = slot(tau == 0 ? T1 - 1 : tau - 1);
+        enqueue_expansion<R, V>(c, ex_pm, ld, in, X, Y, W, nb, c->out.as<double>(),
+                                counters(c, 0), slot(tau));
       }
-      TBPM_CK(cudaMemcpyAsync(c->coef.p, coef_host.data(), sizeof(double2) * len * n_en,
-                              cudaMemcpyHostToDevice, c->stream));
-      StatePtrs<R> win{};
-      for (int tau = 0; tau < len; ++tau) win.p[tau] = reinterpret_cast<const C*>(slot(tau));
-      const int64_t total = n * n_en * nb;
-      if (TBPM_QE_MMA) {
-        // FP64 tensor-path products (qe_accum_mma_kernel)
-        const int rt = qe_mma_rows(nb);
-        const int64_t tiles = (n + rt - 1) / rt;
-        const int groups = ((n_en + 7) / 8 + kQeMmaWarps * kQeMmaMT - 1) / (kQeMmaWarps * kQeMmaMT);
-        const dim3 grid((unsigned)std::min<int64_t>(tiles, (int64_t)num_sms(c->device) * 4),
-                        (unsigned)groups);
-        const size_t qsmem = qe_mma_smem(nb);
-        qe_smem_attr(qe_accum_mma_kernel<R>, qsmem);
-        qe_accum_mma_kernel<R><<<grid, kQeMmaWarps * 32, qsmem, c->stream>>>(
-            qe, n, n_en, nb, win, len, c->coef.as<double2>(), first_window ? 1 : 0,
-            reinterpret_cast<const C*>(W));
-      } else {
-        const int qthreads = qe_accum_threads(n_en, nb);
-        const int n_chunks = (n_en * nb + kQeG * qthreads - 1) / (kQeG * qthreads);
-        const int64_t tiles = (n + qe_accum_rows<R>(nb) - 1) / qe_accum_rows<R>(nb);
-        const dim3 grid((unsigned)std::min<int64_t>(tiles, (int64_t)kSMs * 16),
-                        (unsigned)n_chunks);
-        const size_t qsmem = qe_accum_smem<R>(n_en, nb);
-        qe_accum_attr<R>(qsmem);
-        qe_accum_kernel<R><<<grid, qthreads, qsmem, c->stream>>>(
-            qe, n, n_en, nb, win, len, c->coef.as<double2>(), first_window ? 1 : 0,
-            reinterpret_cast<const C*>(W));
+      if (n_en > 0) {
+        for (int tau = 0; tau < len; ++tau) {
+          const int tt = t + tau;
+          const double Wh = 0.5 * (1 + std::cos(pi * tt / n_timestep));  // Hanning
+          for (int i = 0; i < n_en; ++i) {
+            const double x = en_sel[i] * (double)tt * t_step;
+            coef_host[(size_t)tau * n_en + i] = make_double2(Wh * std::cos(x), Wh * std::sin(x));
+          }
+        }
+        TBPM_CK(cudaMemcpyAsync(c->coef.p, coef_host.data(), sizeof(double2) * len * n_en,
+                                cudaMemcpyHostToDevice, c->stream));
+        StatePtrs<R> win{};
+        for (int tau = 0; tau < len; ++tau) win.p[tau] = reinterpret_cast<const C*>(slot(tau));
+        const int64_t total = n * n_en * nb;
+        if (TBPM_QE_MMA) {
+          // FP64 tensor-path products (qe_accum_mma_kernel)
+          const int rt = qe_mma_rows(nb);
+          const int64_t tiles = (n + rt - 1) / rt;
+          const int groups = ((n_en + 7) / 8 + kQeMmaWarps * kQeMmaMT - 1) / (kQeMmaWarps * kQeMmaMT);
+          const dim3 grid((unsigned)std::min<int64_t>(tiles, (int64_t)num_sms(c->device) * 4),
+                          (unsigned)groups);
+          const size_t qsmem = qe_mma_smem(nb);
+          qe_smem_attr(qe_accum_mma_kernel<R>, qsmem);
+          qe_accum_mma_kernel<R><<<grid, kQeMmaWarps * 32, qsmem, c->stream>>>(
+              qe, n, n_en, nb, win, len, c->coef.as<double2>(), first_window ? 1 : 0,
+              reinterpret_cast<const C*>(W));
+        } else {
+          const int qthreads = qe_accum_threads(n_en, nb);
+          const int n_chunks = (n_en * nb + kQeG * qthreads - 1) / (kQeG * qthreads);
+          const int64_t tiles = (n + qe_accum_rows<R>(nb) - 1) / qe_accum_rows<R>(nb);
+          const dim3 grid((unsigned)std::min<int64_t>(tiles, (int64_t)kSMs * 16),
+                          (unsigned)n_chunks);
+          const size_t qsmem = qe_accum_smem<R>(n_en, nb);
+          qe_accum_attr<R>(qsmem);
+          qe_accum_kernel<R><<<grid, qthreads, qsmem, c->stream>>>(
+              qe, n, n_en, nb, win, len, c->coef.as<double2>(), first_window ? 1 : 0,
+              reinterpret_cast<const C*>(W));
+        }
+        TBPM_CK(cudaGetLastError());
+        c->launches++;
+        c->model_bytes += (double)total * 2 * sizeof(R) * (first_window ? 1 : 2) +
+                          (double)len * n * ld * 2 * sizeof(R);
       }
-      TBPM_CK(cudaGetLastError());
-      c->launches++;
-      c->model_bytes += (double)total * 2 * sizeof(R) * (first_window ? 1 : 2) +
-                        (double)len * n * ld * 2 * sizeof(R);
-    }
-    // the window ring: the next window reads the last state from slot T1-1
-    if (len != T1 && t + len - 1 < n_timestep)
-      TBPM_CK(cudaMemcpyAsync(slot(T1 - 1), slot(len - 1), vb, cudaMemcpyDeviceToDevice,
-                              c->stream));
-    TBPM_CK(cudaStreamSynchronize(c->stream));  // coef_host is reused
-    first_window = false;
-    t += len;
-    if (check && t == chk_step) {
-      // tbpm.f90:611-614: at t == chk_step the states after chk_step-1 steps
-      read_out(c, host, (size_t)(chk_step - 1) * ld * 3);
-      for (int b = 0; b < ld; ++b) {
-        const double nv = host[((size_t)(chk_step - 2) * ld + b) * 3 + 2];
-        if (const int bad_ = norm_broken(nv, norm_ref[(size_t)b * 3 + 2], thr))
-          raise_norm(who, chk_step, bad_);
+      // the window ring: the next window reads the last state from slot T1-1
+      if (len != T1 && t + len - 1 < n_timestep)
+        TBPM_CK(cudaMemcpyAsync(slot(T1 - 1), slot(len - 1), vb, cudaMemcpyDeviceToDevice,
+                                c->stream));
+      TBPM_CK(cudaStreamSynchronize(c->stream));  // coef_host is reused
+      first_window = false;
+      t += len;
+      if (check && t == chk_step) {
+        // tbpm.f90:611-614: at t == chk_step the states after chk_step-1 steps
+        read_out(c, host, (size_t)(chk_step - 1) * ld * 3);
+        for (int b = 0; b < ld; ++b) {
+          const double nv = host[((size_t)(chk_step - 2) * ld + b) * 3 + 2];
+          if (const int bad_ = norm_broken(nv, norm_ref[(size_t)b * 3 + 2], thr))
+            raise_norm(who, chk_step, bad_);
+        }
       }
     }
   }
@@ -2008,8 +2355,8 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
     TBPM_CK(cudaStreamSynchronize(c->stream));
     return;
   }
-  read_out(c, host, (size_t)n_timestep * ld * 3);
-  if (add_dos)
+  if (!pp) read_out(c, host, (size_t)n_timestep * ld * 3);
+  if (!pp && add_dos)
     for (int b = 0; b < nb; ++b)
       for (int tt = 1; tt <= n_timestep; ++tt) {
         dos_corr[2 * (tt - 1)] += host[((size_t)(tt - 1) * ld + b) * 3 + 0] / n_avg;
@@ -2048,8 +2395,31 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   TBPM_CK(cudaStreamSynchronize(c->stream));
   std::vector<double> amp(n_ib);
   for (int ib = 0; ib < n_ib; ++ib) amp[ib] = std::hypot(proj[2 * ib], proj[2 * ib + 1]);
-  // wf0_J = [J_x wf0 | J_y wf0] (tbpm.f90:654-655) in slot T (the propagated block)
-  Pack<R, V>* wj = slot(std::max(T1, T2));
+  // wf0_J = [J_x wf0 | J_y wf0] (tbpm.f90:654-655), propagated step by step, or
+  // several steps per expansion where their blocks fit beside QE
+  StepsShape shape;
+  if (pp) {
+    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes);
+    if (shape.m > 0) {
+      c->A.ensure(vb * (size_t)(shape.m + shape.window + 2 + T2));
+    } else {
+      c->X.ensure(vb);
+      c->Y.ensure(vb);
+      c->A.ensure(vb * (size_t)(T2 + 1));
+    }
+  }
+  std::vector<Pack<R, V>*> ring, states, us;
+  for (int q = 0; q < T2; ++q) us.push_back(slot(q));
+  StepsPlan sp;
+  if (shape.m > 0) {
+    sp = steps_plan(*pp, std::min(shape.m, std::max(n_timestep - 1, 1)));
+    for (int q = 0; q < shape.window + 2; ++q) ring.push_back(slot(T2 + q));
+    for (int q = 0; q < sp.m; ++q) states.push_back(slot(T2 + shape.window + 2 + q));
+  } else {
+    states.push_back(slot(pp ? T2 : std::max(T1, T2)));
+  }
+  Pack<R, V>* wj = states.back();
+  int made = 0, used = 0;  // states of the current expansion
   jj_apply_kernel<R><<<blocks_for(n * ld, 256), 256, 0, c->stream>>>(
       h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<C>(), h.dx.as<R>(), h.dy.as<R>(),
       h.rescale, n, nb, reinterpret_cast<const C*>(W), nb, 0, 0, reinterpret_cast<C*>(wj));
@@ -2062,15 +2432,24 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
     StatePtrs<R> u{};
     for (int tau = 0; tau < len; ++tau) {
       const int tt = t + tau;
-      if (tt >= 2)
-        enqueue_expansion<R, V>(c, ex_fwd, ld, wj, X, Y, nullptr, 0, nullptr, Counters{});
-      C* us = reinterpret_cast<C*>(slot(tau));
+      if (tt >= 2 && shape.m > 0) {
+        if (used == made) {
+          made = std::min(sp.m, n_timestep - tt + 1);
+          used = 0;
+          enqueue_steps<R, V>(c, *pp, sp, made, ld, wj, ring, states);
+        }
+        wj = states[used++];
+      } else if (tt >= 2) {
+        enqueue_expansion<R, V>(c, ex_fwd, ld, wj, c->X.as<Pack<R, V>>(), c->Y.as<Pack<R, V>>(),
+                                nullptr, 0, nullptr, Counters{});
+      }
+      C* uq = reinterpret_cast<C*>(us[tau]);
       jj_apply_kernel<R><<<blocks_for(n * ld, 256), 256, 0, c->stream>>>(
           h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<C>(), h.dx.as<R>(),
-          h.dy.as<R>(), h.rescale, n, nb, reinterpret_cast<const C*>(wj), ld, 0, nb, us);
+          h.dy.as<R>(), h.rescale, n, nb, reinterpret_cast<const C*>(wj), ld, 0, nb, uq);
       TBPM_CK(cudaGetLastError());
       c->launches++;
-      u.p[tau] = us;
+      u.p[tau] = uq;
     }
     qe_project_kernel<R><<<pgrid2, pthreads, psmem, c->stream>>>(
         qe, n, rows_per_tile, n_en, nb, u, len, 0, nullptr, c->partials.as<double>());
@@ -2110,11 +2489,13 @@ template <typename R, int V>
 void dynpol_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, int nb,
                   int nq, const QBlock& qb, const double* sx, const double* sy, const double* sz,
                   const StateKeys* keys, const double* host_wf0, int n_timestep, int chk_step,
-                  double chk_thr, int n_avg, int q0, int n_q_total, double* corr) {
+                  double chk_thr, int n_avg, int q0, int n_q_total, double* corr,
+                  const PolyPlan* pp) {
   using C = typename Cx<R>::t;
   const int ld = (nq + 1) * nb;
   const int tpr = nq * nb;
   c->graph.reset();
+  const StepsShape shape = steps_room<R>(c, pp, ld, nb);
   ensure_vectors(c, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * tpr * 3 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
@@ -2137,32 +2518,39 @@ void dynpol_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fer
   const Tile td = pick_tile(c, h.n, tpr, dens_corr_kernel<R>, 3 * sizeof(double));
   const size_t smem = (size_t)td.threads * 3 * sizeof(double);
   reset_counters(c, 0);
-  auto dcorr = [&]() {
+  auto dcorr = [&](const Pack<R, V>* x) {
     ensure_partials(c, (size_t)tpr * 3 * td.grid);
     dens_corr_kernel<R><<<td.grid, td.threads, smem, c->stream>>>(
-        reinterpret_cast<const C*>(A), sx, sy, sz, qb, nq, nb, h.n, c->partials.as<double>());
+        reinterpret_cast<const C*>(x), sx, sy, sz, qb, nq, nb, h.n, c->partials.as<double>());
     TBPM_CK(cudaGetLastError());
     c->launches++;
     c->model_bytes += (double)h.n * ld * 2 * sizeof(R) + (double)h.n * 24;
     launch_finalize(c, td.grid, tpr * 3, counters(c, 0), c->out.as<double>());
   };
-  dcorr();  // t = 1 (tbpm.f90:463-470); its psi2 norm is the norm reference
+  dcorr(A);  // t = 1 (tbpm.f90:463-470); its psi2 norm is the norm reference
   auto step = [&]() {
     enqueue_expansion<R, V>(c, ex_time, ld, A, X, Y, nullptr, 0, nullptr, Counters{});
-    dcorr();
+    dcorr(A);
   };
   auto key = plan_key(c, 5, ld, V, ex_time);
   key_push(key, nq);
   key_push(key, sx);
   for (int k = 0; k < nq; ++k)
     for (int d = 0; d < 3; ++d) key_push(key, qb.q[k][d]);
+  StepsRun<R, V> many(c, pp, shape, ld);
+  auto advance = [&](int n_steps) {
+    if (shape.m > 0)
+      many.run(c, n_steps, dcorr);
+    else
+      run_steps(c, n_steps, key, step);
+  };
   const double thr = effective_thr(c, chk_thr);
   std::vector<double> host;
   int done = 0;
   const bool check = chk_step >= 2 && chk_step <= n_timestep;
   if (check) {
     // tbpm.f90:479: at t == chk_step psi2 has been propagated chk_step-2 times
-    run_steps(c, chk_step - 2, key, step);
+    advance(chk_step - 2);
     done = chk_step - 2;
     read_out(c, host, (size_t)(done + 1) * tpr * 3);
     for (int b = 0; b < nb; ++b) {
@@ -2172,7 +2560,7 @@ void dynpol_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fer
         raise_norm("tbpm_dyn_pol", chk_step, bad_);
     }
   }
-  run_steps(c, (n_timestep - 1) - done, key, step);
+  advance((n_timestep - 1) - done);
   read_out(c, host, (size_t)n_timestep * tpr * 3);
   for (int k = 0; k < nq; ++k)
     for (int b = 0; b < nb; ++b)
@@ -2352,7 +2740,7 @@ void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
 // ---- psi(t) -------------------------------------------------------------------
 
 template <typename R>
-void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* psi0, const int32_t* time_log,
+void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, const double* psi0, const int32_t* time_log,
                int n_log, int n_timestep, int chk_step, double chk_thr, double* psi_t) {
   constexpr int V = 1;
   c->graph.reset();
@@ -2370,16 +2758,34 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* psi0, const int32
   };
   const auto key = plan_key(c, 3, 1, V, ex);
   const double thr = effective_thr(c, chk_thr);
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   std::vector<double> host;
   int done = 0;  // steps enqueued
+  int rows = 0;  // rows of c->out after the initial one
   int ptr = 0;
+  int jump_m = 0;
+  Expansion jump;
   // tbpm.f90:1071-1092: at iteration t the state after t-1 steps is logged if
-  // requested, checked at t == chk_step, then propagated.
+  // requested, checked at t == chk_step, then propagated.  Between two such
+  // times the state is not needed: on the polynomial route the m steps are one
+  // expansion of about tau*a*m terms (512 x 480 graphene, one state, 64 steps
+  // between frames: 260 terms instead of 1216).
   auto advance_to = [&](int target) {
-    if (target > done) {
+    if (target <= done) return;
+    if (poly) {
+      if (target - done != jump_m) {
+        jump_m = target - done;
+        jump = power_expansion(pp, jump_m);
+      }
+      enqueue_expansion<R, V>(c, jump, 1, A, X, Y, nullptr, 0, c->out.as<double>(),
+                              counters(c, 0));
+      ++rows;
+    } else {
       run_steps(c, target - done, key, step);
-      done = target;
+      rows += target - done;
     }
+    done = target;
   };
   for (int t = 1; t <= n_timestep; ++t) {
     if (ptr < n_log && time_log[ptr] == t - 1) {
@@ -2390,8 +2796,8 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* psi0, const int32
     }
     if (t == chk_step) {
       advance_to(t - 1);
-      read_out(c, host, (size_t)(done + 1) * 3);
-      if (const int bad_ = norm_broken(host[(size_t)done * 3 + 2], host[2], thr))
+      read_out(c, host, (size_t)(rows + 1) * 3);
+      if (const int bad_ = norm_broken(host[(size_t)rows * 3 + 2], host[2], thr))
         raise_norm("tbpm_psi_t", t, bad_);
     }
   }
@@ -2705,6 +3111,8 @@ void drv_ac(tbpm_ctx* c, const double* bes, int n_bes, double beta, double mu,
   const int nomf = fermi_coef(nr_fermi, beta, mu, true, fermi_precision, comf);
   if (nf < 3 || nomf < 3) throw Error{TBPM_ERR_ARG, "Fermi expansion shorter than 3 terms"};
   const Expansion ex_time = time_step_expansion(bes, n_bes);
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   const int B = std::min(batch_size(c), kMaxCols / 3);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
@@ -2721,9 +3129,10 @@ void drv_ac(tbpm_ctx* c, const double* bes, int n_bes, double beta, double mu,
     dispatch(c->ham.prec, pick_V(c->ham.prec, 3 * nb, nb, c->opts.vector_width), [&](auto tag) {
       using P = decltype(tag);
       ac_batch<typename P::Real, P::V>(c, ex_time, ex_fermi, nb, kp, hw, n_timestep, chk_step,
-                                       chk_thr, n_states, corr);
+                                       chk_thr, n_states, corr, poly ? &pp : nullptr);
     });
   }
+  trim(c->A);
 }
 
 
@@ -2794,6 +3203,8 @@ void drv_dc_part(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, i
     }
     (void)cudaGetLastError();
   }
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;
@@ -2815,10 +3226,12 @@ void drv_dc_part(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, i
                  dc_batch<typename P::Real, P::V>(c, ex_pm, ex_fwd, nb, kp, hw, n_timestep,
                                                   t_step, part, chk_step, chk_thr, n_avg,
                                                   n_energies, dos_corr, dc_corr, nullptr,
-                                                  "tbpm_dccond", e0, e0 == 0);
+                                                  "tbpm_dccond", e0, e0 == 0,
+                                                  poly ? &pp : nullptr);
                });
     }
   }
+  trim(c->A);
 }
 
 void drv_dc(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, int n_states,
@@ -2852,6 +3265,8 @@ void drv_dyn_pol(tbpm_ctx* c, const double* bes, int n_bes, double beta, double 
   const int nomf = fermi_coef(nr_fermi, beta, mu, true, fermi_precision, comf);
   if (nf < 3 || nomf < 3) throw Error{TBPM_ERR_ARG, "Fermi expansion shorter than 3 terms"};
   const Expansion ex_time = time_step_expansion(bes, n_bes);
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   const int64_t n = c->ham.n;
   DevMem sites;
   sites.ensure((size_t)n * 3 * sizeof(double));
@@ -2883,11 +3298,12 @@ void drv_dyn_pol(tbpm_ctx* c, const double* bes, int n_bes, double beta, double 
         using P = decltype(tag);
         dynpol_batch<typename P::Real, P::V>(c, ex_time, ex_fermi, nb, nq, qb, dsx, dsx + n,
                                              dsx + 2 * n, kp, hw, n_timestep, chk_step, chk_thr,
-                                             n_states, q0, n_q, corr);
+                                             n_states, q0, n_q, corr, poly ? &pp : nullptr);
       });
     }
   }
   c->graph.reset();  // the graphs refer to the site buffer of this call
+  trim(c->A);
 }
 
 void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0,
@@ -2922,6 +3338,8 @@ void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf
     }
     (void)cudaGetLastError();
   }
+  PolyPlan pp;
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;
@@ -2937,7 +3355,8 @@ void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf
       using P = decltype(tag);
       dc_batch<typename P::Real, P::V>(c, ex_pm, ex_fwd, nb, kp, hw, n_timestep, t_step, en_sel,
                                        chk_step, chk_thr, n_states, n_energies, nullptr,
-                                       nullptr, acc.as<double>(), "tbpm_eigenstates");
+                                       nullptr, acc.as<double>(), "tbpm_eigenstates", 0, true,
+                                       poly ? &pp : nullptr);
     });
   }
   // acc[r][i] is the Fortran (n_energies, n) layout of wf_QE
@@ -3160,9 +3579,9 @@ void drv_psi_t(tbpm_ctx* c, const double* bes, int n_bes, const double* psi0,
   c->model_bytes = 0;
   const Expansion ex = time_step_expansion(bes, n_bes);
   if (c->ham.prec == TBPM_PREC_FP64)
-    psi_t_run<double>(c, ex, psi0, time_log, n_log, n_timestep, chk_step, chk_thr, psi_t);
+    psi_t_run<double>(c, ex, bes, n_bes, psi0, time_log, n_log, n_timestep, chk_step, chk_thr, psi_t);
   else
-    psi_t_run<float>(c, ex, psi0, time_log, n_log, n_timestep, chk_step, chk_thr, psi_t);
+    psi_t_run<float>(c, ex, bes, n_bes, psi0, time_log, n_log, n_timestep, chk_step, chk_thr, psi_t);
 }
 
 void drv_random_states(tbpm_ctx* c, int64_t n, int seed, int first_sample, int n_states,

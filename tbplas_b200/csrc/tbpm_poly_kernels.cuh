@@ -20,8 +20,15 @@
 //  moment_curve_kernel    C(t) = sum_j P(x_j)^t rho_j, and the norms.
 //  cheb_persist_kernel    all terms of a small problem in one launch.
 //  seg_dots_kernel        the two products per (segment, state) of packed samples.
+//  filter_values_kernel,  the quasi-eigenstates' energy filters on the nodes and
+//  filter_coef_kernel     their Chebyshev coefficients.
+//  qe_filter_mma_kernel   QE += (filter coefficients) x (a window of Chebyshev
+//                         vectors) on mma.sync f64.
+//  combine_kernel         the states after 1..m time steps from the Chebyshev
+//                         vectors of one expansion.
 #pragma once
 
+#include "tbpm_dc_kernels.cuh"
 #include "tbpm_kernels.cuh"
 #include "tbpm_seg_kernels.cuh"
 
@@ -437,6 +444,287 @@ __global__ void __launch_bounds__(256) seg_dots_kernel(const int64_t* seg_off, i
     for (int q = 0; q < 2; ++q)
       partials[(((int64_t)seg * ns + col) * 2 + q) * gridDim.x + blockIdx.x] = smem[col * 2 + q];
   }
+}
+
+// ---- quasi-eigenstates as energy filters ---------------------------------------
+
+// Phase 1 of tbpm_dccond (tbpm.f90:600-638) accumulates
+//   QE_i = wf0 + sum_t W(t) [e^{i E_i t dt} P(H)^t + e^{-i E_i t dt} conj(P)(H)^t] wf0,
+// W(t) = (1 + cos(pi t / T)) / 2: a real function f_i of H.  With its Chebyshev
+// coefficients, QE_i = sum_k c_ki T_k(H/a) wf0 needs one block of Chebyshev
+// vectors (3.0 products with H per time step) instead of the forward and the
+// backward propagation of 19 products each.
+
+// The window and phase factors c_ti = W(t) e^{i E_i t dt} are taken as the same
+// doubles that time stepping multiplies with (far from the spectrum QE_i is a
+// small difference of them), and the powers of P come from extended-precision
+// phases, so the filters carry no more rounding than the sums over t did.
+
+// s + e += v without loss (two-sum)
+__device__ __forceinline__ void filter_add(double* s, double* e, double v) {
+  const double t = *s + v;
+  const double z = t - *s;
+  *e += (*s - (t - z)) + (v - z);
+  *s = t;
+}
+
+// f[j*n_en + i] = 1 + 2 Re sum_t c[(t-1)*n_en + i] P(x_j)^t.  Block: 32 nodes x 8
+// energies; per 32 time steps the powers of the nodes are formed once and
+// shared by the energies.
+static __global__ void __launch_bounds__(256) filter_values_kernel(const PolyNode* nodes, int M,
+                                                                   const double2* c, int n_en,
+                                                                   int T, double* f) {
+  __shared__ double pre[32][33], pim[32][33];
+  __shared__ double2 cc[32][8];
+  const int jj = threadIdx.x & 31, ii = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + jj;
+  const int i = blockIdx.y * 8 + ii;
+  PolyNode p = {0.0, 0.0, 0.0};
+  if (j < M) p = nodes[j];
+  double s = 0.0, e = 0.0;
+  for (int t0 = 1; t0 <= T; t0 += 32) {
+    __syncthreads();
+    for (int q = ii; q < 32; q += 8) {
+      const double t = (double)(t0 + q);
+      double re, im;
+      node_power(p, t, &re, &im);
+      const double g = 1.0 + t * p.lnabs;  // |P|^t, lnabs of the order of rounding
+      pre[q][jj] = re * g;
+      pim[q][jj] = im * g;
+    }
+    {
+      const int q = threadIdx.x >> 3, k = threadIdx.x & 7;
+      const int ik = blockIdx.y * 8 + k;
+      cc[q][k] = t0 + q <= T && ik < n_en ? c[(int64_t)(t0 + q - 1) * n_en + ik]
+                                          : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q)
+      filter_add(&s, &e, cc[q][ii].x * pre[q][jj] - cc[q][ii].y * pim[q][jj]);
+  }
+  if (j < M && i < n_en) f[(int64_t)j * n_en + i] = 1.0 + 2.0 * (s + e);
+}
+
+// c[k*n_en + i] = (2 - delta_k0)/M sum_j f[j*n_en + i] cos(k theta_j).  Block: one
+// k and up to 256 energies; the threads left over split the nodes.
+static __global__ void __launch_bounds__(256) filter_coef_kernel(const double* f, int M, int n_en,
+                                                                 double* c) {
+  __shared__ double cs[256];
+  __shared__ double red[2][256];
+  const int k = blockIdx.x;
+  const int i0 = blockIdx.y * 256;
+  const int ni = min(256, n_en - i0);
+  const int parts = 256 / ni;
+  const int part = threadIdx.x / ni;
+  const int i = threadIdx.x - part * ni;
+  double s = 0.0, e = 0.0;
+  for (int j0 = 0; j0 < M; j0 += 256) {
+    __syncthreads();
+    if (j0 + threadIdx.x < M) cs[threadIdx.x] = node_cos(k, j0 + threadIdx.x, M);
+    __syncthreads();
+    if (part < parts) {
+      const int nj = min(256, M - j0);
+      for (int j = part; j < nj; j += parts)
+        filter_add(&s, &e, cs[j] * f[(int64_t)(j0 + j) * n_en + i0 + i]);
+    }
+  }
+  red[0][threadIdx.x] = s;
+  red[1][threadIdx.x] = e;
+  __syncthreads();
+  if (threadIdx.x < ni) {
+    double t = 0.0, r = 0.0;
+    for (int q = 0; q < parts; ++q) {
+      filter_add(&t, &r, red[0][q * ni + threadIdx.x]);
+      r += red[1][q * ni + threadIdx.x];
+    }
+    c[(int64_t)k * n_en + i0 + threadIdx.x] = (k ? 2.0 : 1.0) / M * (t + r);
+  }
+}
+
+constexpr int kFilterWindow = 32;  // Chebyshev vectors folded into QE per pass
+
+template <typename R>
+struct FilterPtrs {
+  const typename Cx<R>::t* p[kFilterWindow];
+};
+
+// Shared memory of qe_filter_mma_kernel: the window's values of a tile,
+// [tau][pair], rows padded by 4 pairs (64 bytes), so that the four tau of a
+// fragment load lie in different banks.
+constexpr int kFilterPad = 4;
+__host__ __device__ constexpr size_t qe_filter_smem(int nb) {
+  return (size_t)kFilterWindow * (qe_mma_rows(nb) * nb + kFilterPad) * sizeof(double2);
+}
+
+// QE[r][i][b] (+)= sum_{tau < T} c[tau][i] p_tau[r][b], c real: per tile of
+// (row, state) pairs a real product A (energies x 32) . B (32 x (pair, re/im)),
+// with the fragments and the split over warps of qe_accum_mma_kernel (whose
+// +/- windows need 2 x 16 coefficients for 16 steps).  A window of 32 vectors
+// per pass over QE: at 16 the pass over QE (32 bytes a complex128 element
+// against 32 FMAs) was the longer side.  A warp's QE elements of the next
+// column tile are loaded before the products of the current one.
+template <typename R>
+__global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_filter_mma_kernel(
+    typename Cx<R>::t* qe, int64_t n_rows, int n_en, int nb,
+    const __grid_constant__ FilterPtrs<R> win, int T, const double* coef, int init) {
+  using C = typename Cx<R>::t;
+  extern __shared__ double2 qsm[];
+  const int RT = qe_mma_rows(nb);
+  const int P = RT * nb;  // pairs of a tile; P % 4 == 0
+  const int PS = P + kFilterPad;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int n_mt = (n_en + 7) / 8;
+  const int mt_b = blockIdx.y * kQeMmaWarps * kQeMmaMT;
+  const int n_mt_b = min(kQeMmaWarps * kQeMmaMT, n_mt - mt_b);
+  const int n_mg = (n_mt_b + kQeMmaMT - 1) / kQeMmaMT;
+  const int mg = warp % n_mg;
+  const int nt_first = warp / n_mg;
+  const int nt_step = (kQeMmaWarps - mg + n_mg - 1) / n_mg;
+  const int mt0 = mt_b + mg * kQeMmaMT;
+  double afr[kQeMmaMT][kFilterWindow / 4];
+#pragma unroll
+  for (int m = 0; m < kQeMmaMT; ++m) {
+    const int i = (mt0 + m) * 8 + g;
+#pragma unroll
+    for (int st = 0; st < kFilterWindow / 4; ++st) {
+      const int tau = 4 * st + t;
+      afr[m][st] = i < n_en && tau < T ? coef[(int64_t)tau * n_en + i] : 0.0;
+    }
+  }
+  for (int64_t r0 = (int64_t)blockIdx.x * RT; r0 < n_rows; r0 += (int64_t)gridDim.x * RT) {
+    const int nr = (int)min((int64_t)RT, n_rows - r0);
+    const int np = nr * nb;  // pairs in range
+    auto load_c = [&](int nt, C* v) {
+      const int pc = 4 * nt + t;
+      const int rr = pc / nb, bb = pc - rr * nb;
+#pragma unroll
+      for (int m = 0; m < kQeMmaMT; ++m) {
+        const int i = (mt0 + m) * 8 + g;
+        v[m].x = v[m].y = (R)0;
+        if (!init && nt < P / 4 && pc < np && i < n_en)
+          v[m] = qe[((r0 + rr) * n_en + i) * nb + bb];
+      }
+    };
+    C cv[kQeMmaMT];
+    load_c(nt_first, cv);
+    __syncthreads();  // the previous tile's values are consumed
+    for (int q = threadIdx.x; q < kFilterWindow * P; q += blockDim.x) {
+      const int tau = q / P;
+      const int pr = q - tau * P;
+      double2 v = make_double2(0.0, 0.0);
+      if (tau < T && pr < np) {
+        const C x = ldg_c(win.p[tau] + r0 * nb + pr);
+        v = make_double2((double)x.x, (double)x.y);
+      }
+      qsm[tau * PS + pr] = v;
+    }
+    __syncthreads();
+    for (int nt = nt_first; nt < P / 4; nt += nt_step) {
+      // B fragment: B[k = 4*s + t][n = g]; column g is pair 4*nt + g/2, part g&1
+      const double* b = reinterpret_cast<const double*>(qsm + 4 * nt) + g;
+      double bfr[kFilterWindow / 4];
+#pragma unroll
+      for (int st = 0; st < kFilterWindow / 4; ++st) bfr[st] = b[(4 * st + t) * 2 * PS];
+      double c0[kQeMmaMT], c1[kQeMmaMT];
+#pragma unroll
+      for (int m = 0; m < kQeMmaMT; ++m) {
+        c0[m] = (double)cv[m].x;
+        c1[m] = (double)cv[m].y;
+      }
+      load_c(nt + nt_step, cv);
+#pragma unroll
+      for (int m = 0; m < kQeMmaMT; ++m) {
+        if (mt0 + m < n_mt) {
+#pragma unroll
+          for (int st = 0; st < kFilterWindow / 4; ++st)
+            dmma_8x8x4(c0[m], c1[m], afr[m][st], bfr[st]);
+        }
+      }
+      const int pc = 4 * nt + t;
+      const int rr = pc / nb, bb = pc - rr * nb;
+#pragma unroll
+      for (int m = 0; m < kQeMmaMT; ++m) {
+        const int i = (mt0 + m) * 8 + g;
+        if (pc < np && i < n_en) {
+          C o;
+          o.x = (R)c0[m];
+          o.y = (R)c1[m];
+          qe[((r0 + rr) * n_en + i) * nb + bb] = o;
+        }
+      }
+    }
+  }
+}
+
+// ---- several time steps from one expansion ----------------------------------------
+
+constexpr int kCombineWindow = 16;  // Chebyshev vectors per pass
+constexpr int kCombineSteps = 16;   // most time steps per expansion
+constexpr int kCombineBatch = 8;    // vectors loaded together
+
+template <typename R>
+struct CombineArgs {
+  const typename Cx<R>::t* p[kCombineWindow];
+  typename Cx<R>::t* out[kCombineSteps];
+  double w[kCombineSteps][kCombineWindow];  // zero where an output has no such term
+  int64_t total;                            // values of a block
+  int np;                                   // vectors of this pass
+  int j0, m;                                // outputs j0 <= j < m take part
+  unsigned int init;                        // bit j: out_j starts here (is not read)
+};
+
+// out_j[e] (+)= sum_tau w[j][tau] p_tau[e] for up to 16 outputs: the states
+// after 1..m time steps all come from the same Chebyshev vectors, so m steps of
+// phase tau take n(m tau) products with H instead of m n(tau) (AC: 57 instead of
+// 240 for 16 steps).  One complex value per thread; the weights are
+// compile-time offsets into the parameter bank.  Sums in FP64.  Bound by memory: 16
+// values read for 32 FMAs each, 9 TB/s of reads at the FP64 peak.
+// p_0 may be out_{m-1}: a thread reads every p of its value before it writes.
+template <typename R, int M>
+__global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__ CombineArgs<R> a) {
+  using C = typename Cx<R>::t;
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.total) return;
+  double re[M], im[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    re[j] = im[j] = 0.0;
+    if (j >= a.j0 && j < a.m && !((a.init >> j) & 1u)) {
+      const C o = a.out[j][e];
+      re[j] = (double)o.x;
+      im[j] = (double)o.y;
+    }
+  }
+#pragma unroll
+  for (int q0 = 0; q0 < kCombineWindow; q0 += kCombineBatch) {
+    if (q0 < a.np) {
+      C p[kCombineBatch];
+#pragma unroll
+      for (int q = 0; q < kCombineBatch; ++q) {
+        p[q].x = p[q].y = (R)0;
+        if (q0 + q < a.np) p[q] = a.p[q0 + q][e];
+      }
+#pragma unroll
+      for (int q = 0; q < kCombineBatch; ++q) {
+        const double x = (double)p[q].x, y = (double)p[q].y;
+#pragma unroll
+        for (int j = 0; j < M; ++j) {
+          re[j] = fma(a.w[j][q0 + q], x, re[j]);
+          im[j] = fma(a.w[j][q0 + q], y, im[j]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < M; ++j)
+    if (j >= a.j0 && j < a.m) {
+      C o;
+      o.x = (R)re[j];
+      o.y = (R)im[j];
+      a.out[j][e] = o;
+    }
 }
 
 }  // namespace tbpm

@@ -179,3 +179,143 @@ def test_packed_realisations_long_run(prec, ns):
                                   seed=1337 * (k * ns + b + 1), n_samples=1)
             assert rel_err(per[k, b], ref) < TOL[prec]
         assert np.allclose(corr[k], per[k].mean(axis=0), rtol=0, atol=1e-14)
+
+
+@pytest.fixture(scope="module")
+def sample():
+    s = tb.make_graphene_sample(9, 11, disorder=1.0, rescale=9.0, seed=21)
+    s.set_magnetic_field(30.0)
+    return s
+
+
+@pytest.mark.parametrize("n_t,log", [(64, [0, 64]), (150, [0, 1, 2, 17, 90, 149]),
+                                     (80, [79, 80]), (300, [7, 299])])
+def test_psi_t_jumps(sample, n_t, log):
+    """One expansion per logged interval, with and without the norm check."""
+    h = sample.build_ham_csr()
+    psi0 = unit_states(1, h.shape[0], seed=41)[0]
+    bes = bessel_series(math.pi)
+    got = f2py.tbpm_psi_t(bes, h.indptr, h.indices, h.data, psi0, np.array(log), n_t, 128, 1e-9)
+    ref = oracle.tbpm_psi_t(bes, h.indptr, h.indices, h.data, psi0, np.array(log), n_t)
+    assert rel_err(got, ref) < 1e-10
+    psi0[3] = np.nan
+    with pytest.raises(nat.NanError):
+        f2py.tbpm_psi_t(bes, h.indptr, h.indices, h.data, psi0, np.array(log), n_t, 60, 1e-9)
+
+
+def _energies(s, tnr, limits):
+    e = np.array([0.5 * i * s.energy_range / tnr - s.energy_range / 2. for i in range(2 * tnr)])
+    return e, np.where((e >= limits[0]) & (e <= limits[1]))[0]
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 5e-5)])
+@pytest.mark.parametrize("ns,n_en", [(1, 1), (3, 9), (4, 70), (2, 300)])
+def test_eigenstates_long_run(sample, prec, tol, ns, n_en):
+    """1 to 300 energies: one to ten groups of energy tiles, odd state counts."""
+    h = sample.build_ham_csr()
+    wf = unit_states(ns, h.shape[0], seed=6)
+    t_step = 2 * math.pi / sample.energy_range
+    energies = np.linspace(-2.0, 2.0, n_en) + 0.01
+    bes = bessel_series(math.pi)
+    f2py.set_backend(precision=prec)
+    got = f2py.tbpm_eigenstates_states(bes, h.indptr, h.indices, h.data, wf, 66, t_step, energies,
+                                       64, 1e-9)
+    ref = oracle.tbpm_eigenstates(bes, h.indptr, h.indices, h.data, 66, t_step, energies, wf0=wf)
+    assert rel_err(got, ref) < tol
+
+
+@pytest.mark.parametrize("ns,tnr,batch", [(1, 64, 16), (3, 89, 2), (5, 70, 16)])
+def test_dc_long_run(sample, ns, tnr, batch):
+    """Filters for phase 1, several steps per expansion in phase 2 (remainders
+    of 16 steps and of 8-step projections), several batches."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf0 = unit_states(ns, ip.size - 1, seed=31)
+    energies, sel = _energies(sample, tnr, (-2.0, 2.0))
+    bes = bessel_series(math.pi)
+    t_step = 2 * math.pi / sample.energy_range
+    f2py.set_backend(batch=batch)
+    dos, dc = f2py.tbpm_dccond_states(bes, ip, ix, hv, sample.rescale, dx, dy, wf0, tnr, t_step,
+                                      energies, sel, 60, 1e-9)
+    rdos, rdc = oracle.tbpm_dccond(bes, ip, ix, hv, sample.rescale, dx, dy, tnr, t_step, energies,
+                                   sel, wf0=wf0)
+    assert rel_err(dos, rdos) < 1e-10
+    assert rel_err(dc, rdc) < 1e-10
+
+
+def test_dc_long_run_without_energies(sample):
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf0 = unit_states(2, ip.size - 1, seed=31)
+    bes = bessel_series(math.pi)
+    args = (bes, ip, ix, hv, sample.rescale, dx, dy)
+    t_step = 2 * math.pi / sample.energy_range
+    none = np.zeros(0, dtype=np.int32)
+    dos, dc = f2py.tbpm_dccond_states(*args, wf0, 64, t_step, np.zeros(3), none, 60, 1e-9)
+    rdos, _ = oracle.tbpm_dccond(*args, 64, t_step, np.zeros(3), none, wf0=wf0)
+    assert rel_err(dos, rdos) < 1e-10 and not dc.any()
+    wf0[0, 0] = np.inf
+    with pytest.raises(nat.NanError):
+        f2py.tbpm_dccond_states(*args, wf0, 64, t_step, np.zeros(3), none, 60, 1e-9)
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 2e-5)])
+@pytest.mark.parametrize("ns,tnr,chk", [(1, 64, 200), (3, 70, 64), (4, 97, 2)])
+def test_ac_long_run(sample, prec, tol, ns, tnr, chk):
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf0 = unit_states(ns, ip.size - 1, seed=21)
+    bes = bessel_series(math.pi / 2)
+    beta = sample.rescale / (tb.KB * 3000.0)
+    f2py.set_backend(precision=prec)
+    got = f2py.tbpm_accond_states(bes, beta, 0.05, ip, ix, hv, sample.rescale, dx, dy, wf0, tnr,
+                                  2**15, 1e-12, chk, 1e-9)
+    ref = oracle.tbpm_accond(bes, beta, 0.05, ip, ix, hv, sample.rescale, dx, dy, tnr, wf0=wf0)
+    assert np.all(got[:, 0] == 0)
+    assert rel_err(got, ref) < tol
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 2e-5)])
+def test_dyn_pol_long_run(sample, prec, tol):
+    h = sample.build_ham_csr()
+    pos = sample.orb_pos
+    q = [[1.3, 0.2, 0.0], [0.0, 2.0, 0.0], [0.5, 0.5, 0.0]]
+    wf = unit_states(3, h.shape[0], seed=5)
+    bes = bessel_series(math.pi / 2)
+    beta = sample.rescale / (tb.KB * 3000.0)
+    f2py.set_backend(precision=prec)
+    got = f2py.tbpm_dyn_pol_states(bes, beta, 0.0, h.indptr, h.indices, h.data, pos[:, 0],
+                                   pos[:, 1], pos[:, 2], q, wf, 75, 2**15, 1e-12, 64, 1e-9)
+    ref = oracle.tbpm_dyn_pol(bes, beta, 0.0, h.indptr, h.indices, h.data, pos[:, 0], pos[:, 1],
+                              pos[:, 2], q, 75, wf0=wf)
+    assert rel_err(got, ref) < tol
+
+
+def test_steps_per_expansion_follow_the_free_memory():
+    """The same AC run with less and less free device memory (16, 8, 8 and 4
+    steps per expansion, then step by step): equal to rounding."""
+    import torch
+    s = tb.make_graphene_sample(192, 192, disorder=1.0, rescale=9.0, seed=2)
+    ip, ix, hv, dx, dy = s.build_ham_dxy()
+    n = ip.size - 1
+    wf0 = unit_states(8, n, seed=3)
+    bes = bessel_series(math.pi / 2)
+    beta = s.rescale / (tb.KB * 6000.0)
+    vb = n * 24 * 16
+    args = (bes, beta, 0.0, ip, ix, hv, s.rescale, dx, dy, wf0, 64, 2**15, 1e-12, 128, 1e-9)
+    ctx = nat.Context(0)  # holds no buffers yet: the process-wide context is left aside
+    nat._contexts, kept = {0: ctx}, nat._contexts
+    try:
+        want = f2py.tbpm_accond_states(*args)
+        ctx.close()
+        for blocks in (30, 24, 16, 8):
+            nat._contexts[0] = ctx = nat.Context(0)
+            f2py._ctx()
+            torch.cuda.synchronize()
+            free, _ = torch.cuda.mem_get_info(0)
+            hold = torch.empty(free - (2 << 30) - int(blocks * vb) - (64 << 20),
+                               dtype=torch.uint8, device="cuda")
+            got = f2py.tbpm_accond_states(*args)
+            del hold
+            torch.cuda.empty_cache()
+            ctx.close()
+            assert rel_err(got, want) < 1e-12
+    finally:
+        nat._contexts = kept

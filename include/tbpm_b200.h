@@ -303,7 +303,7 @@ int tbpm_eigenstates_states(tbpm_ctx* ctx, const double* bes, int n_bes, const i
  * the ket side.  mu: complex128 (n_kernel, n_kernel) Fortran order,
  * mu(m, n) = g_m g_n <T_m(H) J_x psi | J_dir T_n(H) psi> averaged over the
  * states (g: Jackson kernel).  The n_kernel^2 inner products run as complex
- * GEMMs (cuBLAS, loaded on first use); memory: (n_kernel + 134) vectors. */
+ * GEMMs of this library; memory: (n_kernel + 134) vectors. */
 int tbpm_kbdc(tbpm_ctx* ctx, int seed, const int32_t* indptr, const int32_t* indices,
               const double* hop, int64_t n_rows, int64_t nnz, double h_rescale,
               const double* dx, const double* dy, int n_ran_samples, int n_kernel,
@@ -319,12 +319,17 @@ int tbpm_kbdc_states(tbpm_ctx* ctx, const int32_t* indptr, const int32_t* indice
  * with propagation.f90:85-155 (SUBROUTINE Haydock_coef), averaged over
  * n_samples start vectors whose amplitudes on the sites are wf_sites
  * (complex128 [n_samples][n_sites]).  coefa: complex128[n_depth],
- * coefb: float64[n_depth].  The Green function and LDOS on the energy grid
- * (funcs.f90:152-172) are evaluated by the caller. */
+ * coefb: float64[n_depth].  tbpm_haydock_green evaluates the Green function. */
 int tbpm_haydock_coef(tbpm_ctx* ctx, const int32_t* indptr, const int32_t* indices,
                       const double* hop, int64_t n_rows, int64_t nnz, double h_rescale,
                       const int32_t* site_indices, int n_sites, const double* wf_sites,
                       int n_samples, int n_depth, double* coefa, double* coefb);
+
+/* Green function G00(E + i delta) of the Haydock continued fraction
+ * (funcs.f90:152-172 green_function) from tbpm_haydock_coef's coefficients:
+ * energies float64[n_energies], g complex128[n_energies].  Host arrays. */
+int tbpm_haydock_green(tbpm_ctx* ctx, const double* coefa, const double* coefb, int n_depth,
+                       const double* energies, int n_energies, double delta, double* g);
 
 /* cond_from_trace -- replaces analysis.f90:6-69 (SUBROUTINE cond_from_trace,
  * with kpm.f90:31-56 get_gamma_mn) as called from Analyzer.calc_hall_cond

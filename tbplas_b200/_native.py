@@ -47,7 +47,7 @@ EXPORTED_SYMBOLS = (
     "tbpm_eigenstates_states", "tbpm_kbdc", "tbpm_kbdc_states", "tbpm_haydock_coef",
     "tbpm_cond_from_trace", "tbpm_session_export", "tbpm_session_dos_resume",
     "tbpm_nn_gemm_tn_mma", "tbpm_nn_tc_status", "tbpm_trig_sums", "tbpm_trig_cumtrapz",
-    "tbpm_selftest_wait_timeout", "tbpm_dccond_accumulate",
+    "tbpm_selftest_wait_timeout", "tbpm_dccond_accumulate", "tbpm_haydock_green",
 )
 
 
@@ -199,6 +199,7 @@ _SIGNATURES = {
                                   _c_int, _c_int, _c_int, _vp]),
     "tbpm_haydock_coef": (_c_int, [_vp, _vp, _vp, _vp, _c_i64, _c_i64, _c_dbl, _vp, _c_int,
                                    _vp, _c_int, _c_int, _vp, _vp]),
+    "tbpm_haydock_green": (_c_int, [_vp, _vp, _vp, _c_int, _vp, _c_int, _c_dbl, _vp]),
     "tbpm_session_export": (_c_int, [_vp, _vp, _vp]),
     "tbpm_session_dos_resume": (_c_int, [_vp, _vp, _c_int, _c_int, _vp, _vp, _vp, _vp, _c_int,
                                          _c_int]),

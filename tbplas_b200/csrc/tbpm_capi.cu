@@ -62,6 +62,8 @@ void drv_kbdc(tbpm_ctx* c, const double* wf0, int n_states, int seed, int rank,
               int n_ran_samples, int n_kernel, int direction, double* mu);
 void drv_haydock(tbpm_ctx* c, const int32_t* sites, int n_sites, const double* wf_sites,
                  int n_samples, int n_depth, double h_rescale, double* coefa, double* coefb);
+void drv_haydock_green(tbpm_ctx* c, const double* coefa, const double* coefb, int n_depth,
+                       const double* energies, int n_e, double delta, double* g);
 void drv_cond_from_trace(tbpm_ctx* c, const double* mu_mn, int nk, const double* mu, int n_mu,
                          double h_rescale, double beta, int ne_integral, double* cond);
 void drv_supercell_ham(tbpm_ctx* c, const tbpm_supercell* sc, int layout, double cutoff,
@@ -328,6 +330,13 @@ int tbpm_haydock_coef(tbpm_ctx* c, const int32_t* indptr, const int32_t* indices
     maybe_upload(c, indptr, indices, hop, n_rows, nnz, nullptr, nullptr, h_rescale);
     tbpm::drv_haydock(c, site_indices, n_sites, wf_sites, n_samples, n_depth, h_rescale, coefa,
                       coefb);
+  });
+}
+
+int tbpm_haydock_green(tbpm_ctx* c, const double* coefa, const double* coefb, int n_depth,
+                       const double* energies, int n_energies, double delta, double* g) {
+  return guarded(c, [&] {
+    tbpm::drv_haydock_green(c, coefa, coefb, n_depth, energies, n_energies, delta, g);
   });
 }
 

@@ -1273,6 +1273,24 @@ double matrix_bytes(const Ham& h) {
   return (double)(h.n + 1) * 4 + (double)h.nnz * (4 + s) + (h.has_diag ? (double)h.n * s : 0.0);
 }
 
+// Launch of a kernel with a grid barrier: every block is resident at once, so the
+// barrier cannot wait on a block that has not started.
+template <class K, class Args>
+void launch_cooperative(tbpm_ctx* c, K kernel, int grid, int threads, size_t smem,
+                        const Args& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TBPM_CK(cudaLaunchKernelEx(&cfg, kernel, args));
+}
+
 #ifndef TBPM_PERSIST_MB
 #define TBPM_PERSIST_MB 48
 #endif
@@ -1326,19 +1344,7 @@ bool launch_persist(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* 
   a.partials = c->partials.as<double>();
   a.bar = bar;
   a.status = c->status.as<unsigned int>();
-  // cooperative: every block is resident, the barrier cannot wait on a block
-  // that has not started
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TBPM_CK(cudaLaunchKernelEx(&cfg, cheb_persist_kernel<R, V>, a));
+  launch_cooperative(c, cheb_persist_kernel<R, V>, grid, threads, smem, a);
   reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
       c->partials.as<double>(), grid, n_vals, sums);
   TBPM_CK(cudaGetLastError());
@@ -2638,14 +2644,17 @@ void kbdc_state(tbpm_ctx* c, int nk, int direction, const double* g_dev, double 
     TBPM_CK(cudaGetLastError());
     c->launches++;
   };
-  // ket side: Q_j = J_a T_j(H) psi  (tbpm.f90:905-929)
+  // ket side: Q_j = J_a T_j(H) psi  (tbpm.f90:905-929), with T_{j+1} from the same
+  // pass over the matrix
   C* t[3] = {ring, ring + n, ring + 2 * n};
   TBPM_CK(cudaMemcpyAsync(t[0], psi, vb, cudaMemcpyDeviceToDevice, c->stream));
   for (int j = 0; j < nk; ++j) {
-    C* tj = t[j % 3];
-    if (j == 1) hmv(1.0, 0.0, t[0], nullptr, tj);
-    if (j >= 2) hmv(2.0, -1.0, t[(j - 1) % 3], t[(j - 2) % 3], tj);
-    cur(dj, tj, Q + (size_t)j * n);
+    cheb_current_kernel<R><<<grid, 256, 0, c->stream>>>(
+        h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<C>(), diag, dj, h.rescale, n,
+        j == 0 ? 1.0 : 2.0, j == 0 ? 0.0 : -1.0, t[j % 3], j == 0 ? nullptr : t[(j + 2) % 3],
+        j + 1 < nk ? t[(j + 1) % 3] : nullptr, Q + (size_t)j * n);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
   }
   // bra side in chunks: P_i = T_i(H) J_x psi, then mu[i0:i0+kc, :] += P^H Q
   C* carry[2] = {ring + 3 * n, ring + 4 * n};
@@ -2668,9 +2677,13 @@ void kbdc_state(tbpm_ctx* c, int nk, int direction, const double* g_dev, double 
     // a short last chunk may take more slices than the full chunks it was sized for
     c->qe.ensure((size_t)sp.slices * m * nk * sizeof(double2));
     ws = c->qe.as<double2>();
-    pq_gemm_kernel<R><<<dim3((nk + kPqTile - 1) / kPqTile, (m + kPqTile - 1) / kPqTile,
-                             sp.slices),
-                        256, 0, c->stream>>>(P, Q, n, m, nk, sp.rows, ws);
+    const dim3 pgrid((nk + kPqTile - 1) / kPqTile, (m + kPqTile - 1) / kPqTile, sp.slices);
+    if constexpr (sizeof(R) == 8) {
+      qe_smem_attr(pq_dmma_kernel, kPqSmem);
+      pq_dmma_kernel<<<pgrid, 128, kPqSmem, c->stream>>>(P, Q, n, m, nk, sp.rows, ws);
+    } else {
+      pq_gemm_kernel<R><<<pgrid, 256, 0, c->stream>>>(P, Q, n, m, nk, sp.rows, ws);
+    }
     TBPM_CK(cudaGetLastError());
     pq_reduce_kernel<<<(int)std::min<int64_t>(blocks_for((int64_t)m * nk, 256), 4096), 256, 0,
                        c->stream>>>(ws, sp.slices, m, nk, i0, g_dev, scale, mu_dev);
@@ -2685,7 +2698,7 @@ void kbdc_state(tbpm_ctx* c, int nk, int direction, const double* g_dev, double 
     }
   }
   c->model_bytes += (double)nk * (2.0 * ((double)(h.n + 1) * 4 + (double)h.nnz * (4 + 2 * sizeof(R))) +
-                                  4.0 * n * sizeof(C)) +
+                                  7.0 * n * sizeof(C)) +
                     2.0 * (double)nk * n * sizeof(C);
 }
 
@@ -2697,44 +2710,34 @@ template <typename R>
 void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
   using C = typename Cx<R>::t;
   const Ham& h = c->ham;
-  const int64_t n = h.n;
-  const int grid = (int)std::min<int64_t>(blocks_for(n, 256), (int64_t)kSMs * 8);
-  ensure_partials(c, (size_t)2 * grid);
-  double* part = c->partials.as<double>();
-  C* v[3] = {c->wf0.as<C>(), c->X.as<C>(), c->Y.as<C>()};
-  const C* diag = h.has_diag ? h.diag.as<C>() : nullptr;
-  double* a = sc;              // [2 * n_depth]
-  double* b = sc + 2 * n_depth;  // [n_depth]
-  C* p1 = v[0];  // n_i-1 (n1 at depth 0)
-  C* p2 = v[0];  // n_i
-  C* pb = v[1];
-  C* spare = v[2];
-  for (int d = 0; d < n_depth; ++d) {
-    haydock_apply_kernel<R><<<grid, 256, 0, c->stream>>>(h.indptr.as<int32_t>(),
-                                                         h.indices.as<int32_t>(), h.hop.as<C>(),
-                                                         diag, n, h_rescale, p2, pb, part);
-    small_reduce_kernel<<<1, 256, 0, c->stream>>>(part, grid, 2, 0, a + 2 * d);
-    haydock_orth_kernel<R><<<grid, 256, 0, c->stream>>>(n, a + 2 * d,
-                                                        d ? b + d - 1 : nullptr, p2, p1, pb,
-                                                        part);
-    small_reduce_kernel<<<1, 256, 0, c->stream>>>(part, grid, 1, 1, b + d);
-    C* dst = d == 0 ? spare : pb;  // n2 = m2 / b1 into its own vector at depth 0
-    scale_inv_kernel<R><<<grid, 256, 0, c->stream>>>(n, b + d, pb, dst);
-    TBPM_CK(cudaGetLastError());
-    c->launches += 5;
-    if (d == 0) {
-      p1 = v[0];
-      p2 = spare;
-      // pb keeps its buffer
-    } else {
-      C* sw = p1;
-      p1 = p2;
-      p2 = pb;
-      pb = sw;
-    }
-  }
-  c->model_bytes += (double)n_depth * ((double)(h.n + 1) * 4 + (double)h.nnz * (4 + 2 * sizeof(R)) +
-                                       9.0 * n * sizeof(C));
+  // enough threads for one row each, spread over the SMs
+  const int sms = num_sms(c->device);
+  const int64_t per_sm = (h.n + sms - 1) / sms;
+  const int threads =
+      (int)std::min<int64_t>(kHaydockThreads, std::max<int64_t>(128, (per_sm + 31) / 32 * 32));
+  const int grid = (int)std::min<int64_t>(sms, (h.n + threads - 1) / threads);
+  ensure_partials(c, (size_t)3 * grid);
+  c->ctr.ensure(16 * sizeof(int));
+  HaydockArgs<R> a;
+  a.indptr = h.indptr.as<int32_t>();
+  a.indices = h.indices.as<int32_t>();
+  a.hop = h.hop.as<C>();
+  a.diag = h.has_diag ? h.diag.as<C>() : nullptr;
+  a.n_rows = h.n;
+  a.rescale = h_rescale;
+  a.w0 = c->wf0.as<C>();
+  a.w1 = c->X.as<C>();
+  a.y = c->Y.as<C>();
+  a.n_depth = n_depth;
+  a.a = sc;
+  a.b = sc + 2 * n_depth;
+  a.partials = c->partials.as<double>();
+  a.bar = c->ctr.as<unsigned int>() + 12;
+  a.status = c->status.as<unsigned int>();
+  TBPM_CK(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), c->stream));
+  launch_cooperative(c, haydock_kernel<R>, grid, threads, 0, a);
+  c->launches++;
+  c->model_bytes += (double)n_depth * (matrix_bytes(h) + 6.0 * h.n * sizeof(C));
 }
 
 // ---- psi(t) -------------------------------------------------------------------
@@ -3475,12 +3478,35 @@ void drv_haydock(tbpm_ctx* c, const int32_t* sites, int n_sites, const double* w
     TBPM_CK(cudaMemcpyAsync(host.data(), sc.p, host.size() * sizeof(double),
                             cudaMemcpyDeviceToHost, c->stream));
     TBPM_CK(cudaStreamSynchronize(c->stream));
+    check_status(c);
     for (int d = 0; d < n_depth; ++d) {
       coefa[2 * d] += host[2 * d] / n_samples;
       coefa[2 * d + 1] += host[2 * d + 1] / n_samples;
       coefb[d] += host[2 * (size_t)n_depth + d] / n_samples;
     }
   }
+}
+
+// G00(E + i delta) on the energies from the recursion's coefficients.
+void drv_haydock_green(tbpm_ctx* c, const double* coefa, const double* coefb, int n_depth,
+                       const double* energies, int n_e, double delta, double* g) {
+  Phase phase("tbpm_haydock_green");
+  if (!coefa || !coefb || !energies || !g || n_depth < 1 || n_e < 1)
+    throw Error{TBPM_ERR_ARG, "coefficients, energies and an output required"};
+  const size_t n_in = 3 * (size_t)n_depth + n_e;
+  c->small.ensure(sizeof(double) * (n_in + 2 * (size_t)n_e + 1));
+  double* in = c->small.as<double>();
+  double2* out = reinterpret_cast<double2*>(in + ((n_in + 1) & ~(size_t)1));
+  std::vector<double> host(coefa, coefa + 2 * (size_t)n_depth);
+  host.insert(host.end(), coefb, coefb + n_depth);
+  host.insert(host.end(), energies, energies + n_e);
+  TBPM_CK(cudaMemcpyAsync(in, host.data(), sizeof(double) * n_in, cudaMemcpyHostToDevice,
+                          c->stream));
+  haydock_green_kernel<<<blocks_for(n_e, 64), 64, 0, c->stream>>>(
+      in, in + 2 * n_depth, n_depth, in + 3 * n_depth, n_e, delta, out);
+  TBPM_CK(cudaGetLastError());
+  TBPM_CK(cudaMemcpyAsync(g, out, sizeof(double2) * n_e, cudaMemcpyDeviceToHost, c->stream));
+  TBPM_CK(cudaStreamSynchronize(c->stream));
 }
 
 void drv_cond_from_trace(tbpm_ctx* c, const double* mu_mn, int nk, const double* mu, int n_mu,

@@ -192,129 +192,247 @@ __global__ void current_vec_kernel(const int32_t* indptr, const int32_t* indices
   }
 }
 
-// Haydock step, part 1: pb = rescale * H p2 and partials of <p2|pb>
-// (partials[v * gridDim.x + block], v = re, im)
+// One ket step of the Kubo-Bastin moments: y = alpha*(H x) + beta*z (y null: not
+// formed) and q = J_d x, from one pass over the matrix and one gather of x.
 template <typename R>
-__global__ void __launch_bounds__(256) haydock_apply_kernel(
+__global__ void __launch_bounds__(256) cheb_current_kernel(
     const int32_t* indptr, const int32_t* indices, const typename Cx<R>::t* hop,
-    const typename Cx<R>::t* diag, int64_t n_rows, double rescale, const typename Cx<R>::t* p2,
-    typename Cx<R>::t* pb, double* partials) {
-  __shared__ double red[2][256];
-  double cr = 0.0, ci = 0.0;
+    const typename Cx<R>::t* diag, const R* d, double rescale, int64_t n_rows, double alpha,
+    double beta, const typename Cx<R>::t* x, const typename Cx<R>::t* z, typename Cx<R>::t* y,
+    typename Cx<R>::t* q) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows;
        r += (int64_t)gridDim.x * blockDim.x) {
-    double vr = 0.0, vi = 0.0;
-    if (diag) {
-      const typename Cx<R>::t d = diag[r], w = p2[r];
-      vr = (double)d.x * (double)w.x - (double)d.y * (double)w.y;
-      vi = (double)d.x * (double)w.y + (double)d.y * (double)w.x;
+    double vr = 0.0, vi = 0.0, cr = 0.0, ci = 0.0;
+    typename Cx<R>::t zz;
+    zz.x = zz.y = (R)0;
+    if (y && beta != 0.0) zz = z[r];
+    if (y && diag) {
+      const typename Cx<R>::t g = diag[r], w = x[r];
+      vr = (double)g.x * (double)w.x - (double)g.y * (double)w.y;
+      vi = (double)g.x * (double)w.y + (double)g.y * (double)w.x;
     }
     const int j0 = __ldg(indptr + r), j1 = __ldg(indptr + r + 1);
+#pragma unroll 4
     for (int j = j0; j < j1; ++j) {
       const typename Cx<R>::t h = ldg_c(hop + j);
-      const typename Cx<R>::t w = ldg_c(p2 + __ldg(indices + j));
+      const double dd = (double)__ldg(d + j);
+      const typename Cx<R>::t w = ldg_c(x + __ldg(indices + j));
       vr += (double)h.x * (double)w.x - (double)h.y * (double)w.y;
       vi += (double)h.x * (double)w.y + (double)h.y * (double)w.x;
+      const double jr = -rescale * (double)h.y * dd, ji = rescale * (double)h.x * dd;
+      cr += jr * (double)w.x - ji * (double)w.y;
+      ci += jr * (double)w.y + ji * (double)w.x;
     }
-    vr *= rescale;
-    vi *= rescale;
     typename Cx<R>::t o;
-    o.x = (R)vr;
-    o.y = (R)vi;
-    pb[r] = o;
-    const typename Cx<R>::t s = p2[r];
-    const double sr = (double)s.x, si = (double)s.y;
-    cr += sr * (double)o.x + si * (double)o.y;
-    ci += sr * (double)o.y - si * (double)o.x;
-  }
-  red[0][threadIdx.x] = cr;
-  red[1][threadIdx.x] = ci;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      red[0][threadIdx.x] += red[0][threadIdx.x + w];
-      red[1][threadIdx.x] += red[1][threadIdx.x + w];
+    o.x = (R)cr;
+    o.y = (R)ci;
+    q[r] = o;
+    if (y) {
+      o.x = (R)(alpha * vr + beta * (double)zz.x);
+      o.y = (R)(alpha * vi + beta * (double)zz.y);
+      y[r] = o;
     }
-    __syncthreads();
   }
+}
+
+// ---- Haydock recursion ------------------------------------------------------
+
+template <typename R>
+struct HaydockArgs {
+  const int32_t* indptr;
+  const int32_t* indices;
+  const typename Cx<R>::t* hop;
+  const typename Cx<R>::t* diag;
+  int64_t n_rows;
+  double rescale;
+  typename Cx<R>::t* w0;  // start vector (overwritten)
+  typename Cx<R>::t* w1;
+  typename Cx<R>::t* y;
+  int n_depth;
+  double* a;         // [2 * n_depth]
+  double* b;         // [n_depth]
+  double* partials;  // [3 * gridDim.x]: <v|y> (re, im), <w|w>
+  unsigned int* bar;     // grid barrier, zero on entry
+  unsigned int* status;  // bit 0: a bounded wait ran out
+};
+
+constexpr int kHaydockThreads = 1024;
+constexpr unsigned long long kHaydockWaitNs = 2000000000ull;  // 2 s per wait
+
+// Arrival of the block on the grid barrier and bounded wait for `want` arrivals;
+// false when the wait ran out.  Every thread of the block calls it.
+__device__ __forceinline__ bool haydock_barrier(unsigned int* bar, unsigned int want,
+                                                unsigned int* status, int* stop) {
+  __threadfence();
+  __syncthreads();
   if (threadIdx.x == 0) {
-    partials[blockIdx.x] = red[0][0];
-    partials[gridDim.x + blockIdx.x] = red[1][0];
-  }
-}
-
-// Haydock step, part 2: pb = -a*p2 - b_prev*p1 + pb (a = coef[0..1] complex,
-// b_prev = *bprev, absent when bprev is null) and partials of <pb|pb>
-template <typename R>
-__global__ void __launch_bounds__(256) haydock_orth_kernel(int64_t n_rows, const double* a,
-                                                           const double* bprev,
-                                                           const typename Cx<R>::t* p2,
-                                                           const typename Cx<R>::t* p1,
-                                                           typename Cx<R>::t* pb,
-                                                           double* partials) {
-  __shared__ double red[256];
-  const double ar = -a[0], ai = -a[1];
-  const double bb = bprev ? -*bprev : 0.0;
-  double nn = 0.0;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    const typename Cx<R>::t x = p2[r], z = pb[r];
-    double vr = ar * (double)x.x - ai * (double)x.y;
-    double vi = ar * (double)x.y + ai * (double)x.x;
-    if (bprev) {
-      const typename Cx<R>::t y = p1[r];
-      vr += bb * (double)y.x;
-      vi += bb * (double)y.y;
+    atomicAdd(bar, 1u);
+    unsigned long long t0 = 0;
+    for (unsigned int spin = 0;; ++spin) {
+      unsigned int seen;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+      if (seen >= want) break;
+      if ((spin & 255u) == 255u) {
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (t0 == 0) t0 = now;
+        if (now - t0 > kHaydockWaitNs) {
+          atomicOr(status, 1u);
+          *stop = 1;
+          break;
+        }
+      }
     }
-    vr += (double)z.x;
-    vi += (double)z.y;
-    typename Cx<R>::t o;
-    o.x = (R)vr;
-    o.y = (R)vi;
-    pb[r] = o;
-    nn += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
+    __threadfence();
   }
-  red[threadIdx.x] = nn;
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partials[blockIdx.x] = red[0];
+  return *stop == 0;
 }
 
-// Fixed-order sum of n_parts partials of n_vals values into out (one block);
-// mode 1 takes the square root of value 0 (a norm).
-__global__ void __launch_bounds__(256) small_reduce_kernel(const double* partials, int n_parts,
-                                                           int n_vals, int mode, double* out) {
-  __shared__ double red[256];
-  for (int v = 0; v < n_vals; ++v) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n_parts; i += blockDim.x) s += partials[v * n_parts + i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[v] = (mode == 1 && v == 0) ? sqrt(red[0]) : red[0];
-    __syncthreads();
+// Sum of a block's per-thread values (in every thread of warp 0), fixed order.
+__device__ __forceinline__ double haydock_block_sum(double v, double* red) {
+  for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x < 32) {
+    t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+    for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
   }
+  __syncthreads();
+  return t;
 }
 
-// y = x / *b (b on the device)
+// Sum over the grid's partials, read past L1 (other blocks wrote them in this
+// launch), in the same order in every block; in every thread.
+__device__ __forceinline__ double haydock_grid_sum(const double* p, int n, double* bcast) {
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    for (int i = threadIdx.x; i < n; i += 32) t += __ldcg(p + i);
+    for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+    if (threadIdx.x == 0) *bcast = t;
+  }
+  __syncthreads();
+  const double t = *bcast;
+  __syncthreads();
+  return t;
+}
+
+__device__ __forceinline__ double2 ldcg_c(const double2* p) { return __ldcg(p); }
+__device__ __forceinline__ float2 ldcg_c(const float2* p) { return __ldcg(p); }
+
+// The whole recursion (propagation.f90:85-155) in one cooperative launch.  With
+// w the unnormalised vector and v = w / b_{d-1}:
+//   y = rescale H v, a_d = <v|y>;  w' = y - a_d v - b_{d-1} v_prev, b_d = |w'|.
+// Two grid barriers per depth (one per inner product) replace five launches, and
+// the division by b_d is folded into the next depth instead of taking a pass:
+// the matrix and 6 vector passes instead of 9.  512 x 512 graphene fits L2, so a
+// depth is bound by the two barrier round trips and L2: 16.5 us (measured; the
+// five launches took 35 us).
 template <typename R>
-__global__ void scale_inv_kernel(int64_t n_rows, const double* b, const typename Cx<R>::t* x,
-                                 typename Cx<R>::t* y) {
-  const double s = *b;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_rows;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    const typename Cx<R>::t v = x[r];
-    typename Cx<R>::t o;
-    o.x = (R)((double)v.x / s);
-    o.y = (R)((double)v.y / s);
-    y[r] = o;
+__global__ void __launch_bounds__(kHaydockThreads, 1)
+    haydock_kernel(const __grid_constant__ HaydockArgs<R> k) {
+  using C = typename Cx<R>::t;
+  __shared__ double red[32];
+  __shared__ double bcast;
+  __shared__ int stop;
+  if (threadIdx.x == 0) stop = 0;
+  __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned int want = 0;
+  double s = 1.0, s_prev = 0.0, b_prev = 0.0;  // v = s w, v_prev = s_prev w_prev
+  C* w = k.w0;
+  C* w_prev = k.w1;
+  for (int d = 0; d < k.n_depth; ++d) {
+    double cr = 0.0, ci = 0.0;
+    for (int64_t r = r0; r < k.n_rows; r += stride) {
+      const int j0 = __ldg(k.indptr + r), j1 = __ldg(k.indptr + r + 1);
+      const C own = ldcg_c(w + r);
+      double vr = 0.0, vi = 0.0;
+      if (k.diag) {
+        const C g = ldg_c(k.diag + r);
+        vr = (double)g.x * (double)own.x - (double)g.y * (double)own.y;
+        vi = (double)g.x * (double)own.y + (double)g.y * (double)own.x;
+      }
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        const C h = ldg_c(k.hop + j);
+        const C x = ldcg_c(w + __ldg(k.indices + j));
+        vr += (double)h.x * (double)x.x - (double)h.y * (double)x.y;
+        vi += (double)h.x * (double)x.y + (double)h.y * (double)x.x;
+      }
+      C o;
+      o.x = (R)(vr * s * k.rescale);
+      o.y = (R)(vi * s * k.rescale);
+      k.y[r] = o;
+      const double xr = s * (double)own.x, xi = s * (double)own.y;
+      cr += xr * (double)o.x + xi * (double)o.y;
+      ci += xr * (double)o.y - xi * (double)o.x;
+    }
+    const double tr = haydock_block_sum(cr, red);
+    const double ti = haydock_block_sum(ci, red);
+    if (threadIdx.x == 0) {
+      k.partials[blockIdx.x] = tr;
+      k.partials[gridDim.x + blockIdx.x] = ti;
+    }
+    want += gridDim.x;
+    if (!haydock_barrier(k.bar, want, k.status, &stop)) return;
+    const double ar = haydock_grid_sum(k.partials, gridDim.x, &bcast);
+    const double ai = haydock_grid_sum(k.partials + gridDim.x, gridDim.x, &bcast);
+    double nn = 0.0;
+    for (int64_t r = r0; r < k.n_rows; r += stride) {
+      const C x = ldcg_c(w + r), z = ldcg_c(k.y + r);
+      const double xr = s * (double)x.x, xi = s * (double)x.y;
+      double vr = (double)z.x - (ar * xr - ai * xi);
+      double vi = (double)z.y - (ar * xi + ai * xr);
+      if (d > 0) {
+        const C p = ldcg_c(w_prev + r);
+        vr -= b_prev * (s_prev * (double)p.x);
+        vi -= b_prev * (s_prev * (double)p.y);
+      }
+      C o;
+      o.x = (R)vr;
+      o.y = (R)vi;
+      w_prev[r] = o;
+      nn += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
+    }
+    const double tn = haydock_block_sum(nn, red);
+    if (threadIdx.x == 0) k.partials[2 * gridDim.x + blockIdx.x] = tn;
+    want += gridDim.x;
+    if (!haydock_barrier(k.bar, want, k.status, &stop)) return;
+    const double b = sqrt(haydock_grid_sum(k.partials + 2 * gridDim.x, gridDim.x, &bcast));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      k.a[2 * d] = ar;
+      k.a[2 * d + 1] = ai;
+      k.b[d] = b;
+    }
+    C* t = w;
+    w = w_prev;
+    w_prev = t;
+    s_prev = s;
+    s = 1.0 / b;
+    b_prev = b;
   }
+}
+
+// G00(E + i delta) of the continued fraction (funcs.f90:152-172), one thread per energy.
+static __global__ void haydock_green_kernel(const double* a, const double* b, int n_depth,
+                                            const double* energies, int n_e, double delta,
+                                            double2* g) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_e) return;
+  const double e = energies[i];
+  double gr = 0.0, gi = 0.0;
+  for (int d = n_depth - 1; d >= 0; --d) {
+    const double b2 = b[d] * b[d];
+    const double zr = e - a[2 * d] - b2 * gr;
+    const double zi = delta - a[2 * d + 1] - b2 * gi;
+    const double q = 1.0 / (zr * zr + zi * zi);
+    gr = zr * q;
+    gi = -zi * q;
+  }
+  g[i] = make_double2(gr, gi);
 }
 
 }  // namespace tbpm

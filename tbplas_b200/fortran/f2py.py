@@ -460,7 +460,9 @@ def ldos_haydock(site_indices, delta, e_range, s_indptr, s_indices, s_hop, h_res
     a, b = haydock_coef(sites, s_indptr, s_indices, s_hop, h_rescale, n_depth, wf)
     tnr = int(n_timestep)
     energy = np.array([0.5 * i * e_range / tnr for i in range(-tnr, tnr + 1)])
-    g = green_function(energy, delta, a, b)
+    g = np.zeros(energy.shape, dtype=np.complex128)
+    _ctx().call("tbpm_haydock_green", nat.ptr(a), nat.ptr(b), a.size, nat.ptr(energy),
+                energy.size, float(delta), nat.ptr(g))
     return energy, -1.0 / np.pi * g.imag
 
 

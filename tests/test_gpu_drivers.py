@@ -252,3 +252,48 @@ def test_dyn_pol_on_device_sample_equals_host_route(tmp_path):
     a = _solver(dev, cfg, tmp_path, "dev").calc_corr_dyn_pol()
     b = _solver(host, cfg, tmp_path, "host").calc_corr_dyn_pol()
     assert rel_err(a, b) < 1e-12
+
+
+def test_haydock_several_rows_per_thread():
+    """More rows than the one-launch recursion has threads (148 blocks of 1024),
+    and the Green function against its numpy evaluation."""
+    s = tb.make_graphene_sample(290, 271, disorder=1.0, rescale=9.0, seed=4)
+    h = s.build_ham_csr()
+    assert h.shape[0] > 148 * 1024
+    w = unit_states(1, 2, seed=8)
+    a, b = f2py.haydock_coef([5, 70000], h.indptr, h.indices, h.data, s.rescale, 40, w)
+    ra, rb = oracle.haydock_coef([5, 70000], h.indptr, h.indices, h.data, s.rescale, 40, w)
+    assert rel_err(a, ra) < FP64_TOL and rel_err(b, rb) < FP64_TOL
+    e, ldos = f2py.ldos_haydock([5], 0.02, s.energy_range, h.indptr, h.indices, h.data,
+                                s.rescale, 3, 40, 33, 2, "")
+    wf = f2py.random_states(1, 3, 2, rank=0, n_ran_samples=2)
+    a, b = f2py.haydock_coef([5], h.indptr, h.indices, h.data, s.rescale, 40, wf)
+    g = f2py.green_function(e, 0.02, a, b)
+    assert e.size == 67 and rel_err(ldos, -g.imag / np.pi) < 1e-12
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (3, 2), (20, 33)])
+def test_haydock_small_samples(nx, ny):
+    s = tb.make_graphene_sample(nx, ny, disorder=1.0, rescale=9.0, seed=4)
+    h = s.build_ham_csr()
+    depth = min(20, h.shape[0])
+    w = unit_states(2, 1, seed=8)
+    a, b = f2py.haydock_coef([1], h.indptr, h.indices, h.data, s.rescale, depth, w)
+    ra, rb = oracle.haydock_coef([1], h.indptr, h.indices, h.data, s.rescale, depth, w)
+    n = max(1, depth - 1)  # the last b of an exhausted space is rounding
+    assert rel_err(a[:n], ra[:n]) < FP64_TOL and rel_err(b[:n - 1], rb[:n - 1]) < FP64_TOL \
+        if n > 1 else rel_err(a[:1], ra[:1]) < FP64_TOL
+
+
+@pytest.mark.parametrize("nk", [2, 63, 64, 65, 129, 200])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (13, 17), (60, 57)])
+def test_kbdc_tile_edges(nk, nx, ny):
+    """Moment counts around the 64 x 64 tiles and the 128-column chunks, row
+    counts that are no multiples of the 16-row stages, one slice and many."""
+    s = tb.make_graphene_sample(nx, ny, disorder=1.0, rescale=9.0, seed=5)
+    s.set_magnetic_field(25.0)
+    ip, ix, hop, dx, dy = s.build_ham_dxy()
+    wf = unit_states(1, ip.size - 1, seed=7)
+    gpu = f2py.tbpm_kbdc_states(ip, ix, hop, s.rescale, dx, dy, wf, nk, 2)
+    ref = oracle.tbpm_kbdc(ip, ix, hop, s.rescale, dx, dy, nk, 2, wf0=wf)
+    assert rel_err(gpu, ref) < FP64_TOL

@@ -530,7 +530,8 @@ void build_pair_plan(tbpm_ctx* c, PairPlan& p, const PairRequest& q) {
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t b_list = al((size_t)nt * kPairDeps * 4), b_t = al((size_t)nt * 4),
                b_t1 = al((size_t)(nt + 1) * 4), b_off = al((size_t)(nt + 2) * 8);
-  c->pair_tmp.ensure(2 * b_list + 3 * b_t + 2 * b_t1 + b_off + 256);
+  const size_t b_scan = al(scan_bytes(nt + 1));
+  c->pair_tmp.ensure(2 * b_list + 3 * b_t + 2 * b_t1 + b_off + 256 + b_scan);
   char* w = c->pair_tmp.as<char>();
   int* fwd = reinterpret_cast<int*>(w);
   int* rev = reinterpret_cast<int*>(w += b_list);
@@ -564,7 +565,7 @@ void build_pair_plan(tbpm_ctx* c, PairPlan& p, const PairRequest& q) {
   pair_merge_kernel<<<gt, 256, 0, st>>>(fwd, fcnt, rev, rcnt, nt, margin, near,
                                         p.deps.as<int>(), ready, cnt_b, flags2, flags2 + 1);
   TBPM_CK(cudaGetLastError());
-  scan_counts(cnt_b, nt + 1, off_b, st);
+  scan_counts(cnt_b, nt + 1, off_b, reinterpret_cast<int64_t*>(w + 256), st);
   pair_seq_kernel<<<gt, 256, 0, st>>>(h.indptr.as<int32_t>(), h.n, TR, nt, ready, off_b, g_cnt,
                                       p.seq.as<int4>());
   TBPM_CK(cudaGetLastError());
@@ -2980,8 +2981,8 @@ void ham_upload(tbpm_ctx* c, const int32_t* indptr, const int32_t* indices, cons
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t b_ip = al((size_t)(n + 1) * 4), b_ix = al(nz * 4), b_hop = al(nz * 16);
   const size_t b_d = with_dxy ? al(nz * 8) : 0, b_cnt = al((size_t)n * 4);
-  const size_t b_off = al((size_t)(n + 1) * 8), b_fl = 256;
-  c->raw.ensure(b_ip + b_ix + b_hop + 2 * b_d + b_cnt + b_off + b_fl);
+  const size_t b_off = al((size_t)(n + 1) * 8), b_fl = 256, b_scan = al(scan_bytes(n));
+  c->raw.ensure(b_ip + b_ix + b_hop + 2 * b_d + b_cnt + b_off + b_fl + b_scan);
   char* q = c->raw.as<char>();
   int32_t* rip = reinterpret_cast<int32_t*>(q);
   int32_t* rix = reinterpret_cast<int32_t*>(q += b_ip);
@@ -3011,7 +3012,7 @@ void ham_upload(tbpm_ctx* c, const int32_t* indptr, const int32_t* indices, cons
   const unsigned bad = (unsigned)(host_flags[0] & 0xffffffffu);
   if (bad & 1u) throw Error{TBPM_ERR_ARG, "indptr must be non-decreasing"};
   if (bad & 2u) throw Error{TBPM_ERR_ARG, "column index out of range"};
-  const int64_t n_off = scan_counts(cnt, n, offs, st);
+  const int64_t n_off = scan_counts(cnt, n, offs, reinterpret_cast<int64_t*>(q + b_fl), st);
   const bool has_diag = host_flags[1] > 0;
   const size_t rs = c->opts.precision == TBPM_PREC_FP64 ? 8 : 4;
   h.indptr.ensure((size_t)(n + 1) * 4);
@@ -3271,7 +3272,8 @@ void drv_dyn_pol(tbpm_ctx* c, const double* bes, int n_bes, double beta, double 
   PolyPlan pp;
   const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   const int64_t n = c->ham.n;
-  DevMem sites;
+  ScratchScope scope(c->scratch);
+  TempMem sites(c->scratch);
   sites.ensure((size_t)n * 3 * sizeof(double));
   double* dsx = sites.as<double>();
   TBPM_CK(cudaMemcpyAsync(dsx, sx, n * 8, cudaMemcpyHostToDevice, c->stream));
@@ -3325,7 +3327,8 @@ void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf
   const int64_t n = c->ham.n;
   const std::vector<double> en_sel(energies, energies + n_energies);
   const Expansion ex_fwd = time_step_expansion(bes, n_bes);
-  DevMem acc;
+  ScratchScope scope(c->scratch);
+  TempMem acc(c->scratch);
   acc.ensure((size_t)n * n_energies * sizeof(double));
   TBPM_CK(cudaMemsetAsync(acc.p, 0, (size_t)n * n_energies * sizeof(double), c->stream));
   int B = std::min(batch_size(c), kMaxCols / 2);
@@ -3401,7 +3404,8 @@ void drv_kbdc(tbpm_ctx* c, const double* wf0, int n_states, int seed, int rank,
   const double cotq = std::cos(q) / std::sin(q);
   for (int k = 1; k < n_kernel; ++k)
     g[k] = ((double)(n_kernel - k) * std::cos(q * k) + cotq * std::sin(q * k)) / n_kernel;
-  DevMem gdev, mdev;
+  ScratchScope scope(c->scratch);
+  TempMem gdev(c->scratch), mdev(c->scratch);
   gdev.ensure(sizeof(double) * n_kernel);
   mdev.ensure(sizeof(double2) * (size_t)n_kernel * n_kernel);
   TBPM_CK(cudaMemcpyAsync(gdev.p, g.data(), sizeof(double) * n_kernel, cudaMemcpyHostToDevice,
@@ -3451,7 +3455,8 @@ void drv_haydock(tbpm_ctx* c, const int32_t* sites, int n_sites, const double* w
   c->wf0.ensure((size_t)n * cs);
   c->X.ensure((size_t)n * cs);
   c->Y.ensure((size_t)n * cs);
-  DevMem dsites, dvals, sc;
+  ScratchScope scope(c->scratch);
+  TempMem dsites(c->scratch), dvals(c->scratch), sc(c->scratch);
   dsites.ensure(sizeof(int32_t) * n_sites);
   dvals.ensure(sizeof(double2) * n_sites);
   sc.ensure(sizeof(double) * 3 * (size_t)n_depth);
@@ -3516,7 +3521,8 @@ void drv_cond_from_trace(tbpm_ctx* c, const double* mu_mn, int nk, const double*
   if ((size_t)nk * 2 * sizeof(double) > 200 * 1024)
     throw Error{TBPM_ERR_ARG, "n_kernel too large for the trace kernel (max 12800)"};
   const int ne = ne_integral - 1;
-  DevMem dmu, dsum;
+  ScratchScope scope(c->scratch);
+  TempMem dmu(c->scratch), dsum(c->scratch);
   dmu.ensure(sizeof(double2) * (size_t)nk * nk);
   dsum.ensure(sizeof(double) * ne);
   TBPM_CK(cudaMemcpyAsync(dmu.p, mu_mn, sizeof(double2) * (size_t)nk * nk,

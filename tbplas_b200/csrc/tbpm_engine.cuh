@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -52,6 +53,56 @@ struct DevMem {
   DevMem(const DevMem&) = delete;
   DevMem& operator=(const DevMem&) = delete;
   ~DevMem() { release(); }
+};
+
+// Scratch of a context for the temporaries of one call (tables of the supercell
+// builder, counts, per-call outputs).  A call's cudaMalloc / cudaFree pairs cost
+// 50 to 200 us each, and a free waits for the device; so the sum a call has
+// asked for is kept as one block for the next call, up to kKeep bytes.  Work on
+// a context is ordered by its stream, so the next call may reuse it at once.
+struct Scratch {
+  static constexpr size_t kKeep = (size_t)512 << 20;
+  DevMem block;
+  size_t used = 0, want = 0;
+};
+
+// One temporary: a part of the scratch block, or an allocation of its own where
+// the block is too small.  Valid inside a ScratchScope.
+struct TempMem {
+  Scratch& s;
+  void* p = nullptr;
+  DevMem own;
+  explicit TempMem(Scratch& sc) : s(sc) {}
+  void ensure(size_t n) {
+    n = (std::max<size_t>(n, 16) + 255) & ~(size_t)255;
+    s.want += n;
+    if (s.used + n <= s.block.bytes) {
+      p = static_cast<char*>(s.block.p) + s.used;
+      s.used += n;
+    } else {
+      own.ensure(n);
+      p = own.p;
+    }
+  }
+  template <typename T>
+  T* as() const {
+    return reinterpret_cast<T*>(p);
+  }
+};
+
+// The temporaries of one call; at its end the block grows to what they needed.
+struct ScratchScope {
+  Scratch& s;
+  explicit ScratchScope(Scratch& sc) : s(sc) { s.used = s.want = 0; }
+  ~ScratchScope() {
+    if (s.want <= s.block.bytes || s.want > Scratch::kKeep) return;
+    try {
+      s.block.ensure(s.want);
+    } catch (const Error&) {  // no room: the next call allocates singly again
+    }
+  }
+  ScratchScope(const ScratchScope&) = delete;
+  ScratchScope& operator=(const ScratchScope&) = delete;
 };
 
 // H = D + O: the diagonal D (on-site terms, dense complex[N]) and the
@@ -167,6 +218,8 @@ struct tbpm_ctx {
   std::vector<tbpm::PairRequest> pair_requests;
   tbpm::DevMem pair_tmp;  // scratch of the plan build
   tbpm::Spectrum spec;
+  tbpm::Scratch scratch;
+  tbpm::DevMem wts;   // weights of an expansion that runs in one launch
   tbpm::DevMem poly;  // sums, moments, nodes and weights of the polynomial routes
   int64_t launches = 0;
   double model_bytes = 0;

@@ -72,14 +72,18 @@ __global__ void scan_add_kernel(int64_t* off, int64_t n, const int64_t* tsum) {
   if (i < n) off[i] += tsum[blockIdx.x];
 }
 
+// bytes of workspace scan_counts needs
+size_t scan_bytes(int64_t n) {
+  return (size_t)std::max<int64_t>((n + kScanTile - 1) / kScanTile, 1) * 8;
+}
+
 // exclusive scan of count[0..n) into off[0..n] (off[n] = total); returns total
-int64_t scan_counts(const int32_t* count, int64_t n, int64_t* off, cudaStream_t st) {
+int64_t scan_counts(const int32_t* count, int64_t n, int64_t* off, int64_t* tsum,
+                    cudaStream_t st) {
   const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  DevMem tsum;
-  tsum.ensure((size_t)std::max<int64_t>(tiles, 1) * 8);
-  scan_tiles_kernel<<<(unsigned)tiles, kScanTile, 0, st>>>(count, n, off, tsum.as<int64_t>());
-  scan_sums_kernel<<<1, kScanTile, 0, st>>>(tsum.as<int64_t>(), tiles, off + n);
-  scan_add_kernel<<<(unsigned)tiles, kScanTile, 0, st>>>(off, n, tsum.as<int64_t>());
+  scan_tiles_kernel<<<(unsigned)tiles, kScanTile, 0, st>>>(count, n, off, tsum);
+  scan_sums_kernel<<<1, kScanTile, 0, st>>>(tsum, tiles, off + n);
+  scan_add_kernel<<<(unsigned)tiles, kScanTile, 0, st>>>(off, n, tsum);
   TBPM_CK(cudaGetLastError());
   int64_t total = 0;
   TBPM_CK(cudaMemcpyAsync(&total, off + n, 8, cudaMemcpyDeviceToHost, st));

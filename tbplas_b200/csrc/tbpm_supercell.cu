@@ -462,11 +462,14 @@ __global__ void __launch_bounds__(256) sc_fill_split_kernel(
 // ---- host side ---------------------------------------------------------------
 
 struct Tables {
-  DevMem frac, pc_eng, sc_eng, hop, fwd_off, fwd_ih, bwd_off, bwd_ih, vac, inv;
+  TempMem frac, pc_eng, sc_eng, hop, fwd_off, fwd_ih, bwd_off, bwd_ih, vac, inv;
+  explicit Tables(Scratch& s)
+      : frac(s), pc_eng(s), sc_eng(s), hop(s), fwd_off(s), fwd_ih(s), bwd_off(s), bwd_ih(s),
+        vac(s), inv(s) {}
 };
 
 template <typename T>
-void upload(DevMem& m, const T* src, size_t count, cudaStream_t st) {
+void upload(TempMem& m, const T* src, size_t count, cudaStream_t st) {
   m.ensure(std::max<size_t>(count, 1) * sizeof(T));
   if (count) TBPM_CK(cudaMemcpyAsync(m.p, src, count * sizeof(T), cudaMemcpyHostToDevice, st));
 }
@@ -484,6 +487,7 @@ struct Prepared {
   Tables tb;
   int maxt = 0;
   double rescale = 1.0;
+  explicit Prepared(Scratch& sc) : tb(sc) {}
 };
 
 void prepare(tbpm_ctx* c, const tbpm_supercell* sc, int layout, double cutoff, Prepared& P) {
@@ -621,7 +625,7 @@ void prepare(tbpm_ctx* c, const tbpm_supercell* sc, int layout, double cutoff, P
     P.rescale = sc->rescale;
   } else {
     const int grid = grid_for(n_rows, 256);
-    DevMem bmax;
+    TempMem bmax(c->scratch);
     bmax.ensure((size_t)grid * 8);
     s.scale = 1.0;
     switch (maxt <= 8 ? 8 : maxt <= 16 ? 16 : maxt <= 32 ? 32 : 64) {
@@ -702,25 +706,26 @@ void fill_split(const Prepared& P, const int64_t* off, Ham& h, bool dxy, bool di
 void drv_supercell_ham(tbpm_ctx* c, const tbpm_supercell* sc, int layout, double cutoff,
                        int64_t* n_rows, int64_t* nnz, double* rescale) {
   Phase phase("tbpm_supercell_ham");
-  Prepared P;
+  ScratchScope scope(c->scratch);
+  Prepared P(c->scratch);
   prepare(c, sc, layout, cutoff, P);
   const bool dxy = layout == TBPM_LAYOUT_DXY;
   P.s.need_dr = dxy ? 1 : 0;
   cudaStream_t st = c->stream;
   const int64_t n = P.s.n_rows;
-  DevMem count, off, nd;
+  TempMem count(c->scratch), off(c->scratch), nd(c->scratch), tsum(c->scratch);
+  tsum.ensure(scan_bytes(n));
   count.ensure((size_t)n * 4);
   off.ensure((size_t)(n + 1) * 8);
   nd.ensure(8);
   TBPM_CK(cudaMemsetAsync(nd.p, 0, 8, st));
   count_rows(P, 1, count.as<int32_t>(), nd.as<unsigned long long>(), st);
-  const int64_t n_off = scan_counts(count.as<int32_t>(), n, off.as<int64_t>(), st);
+  const int64_t n_off = scan_counts(count.as<int32_t>(), n, off.as<int64_t>(), tsum.as<int64_t>(), st);
   unsigned long long n_diag = 0;
   TBPM_CK(cudaMemcpyAsync(&n_diag, nd.p, 8, cudaMemcpyDeviceToHost, st));
   TBPM_CK(cudaStreamSynchronize(st));
   if (n_off > (int64_t)INT32_MAX)
     throw Error{TBPM_ERR_ARG, "supercell: more than 2^31-1 off-diagonal entries"};
-  count.release();
   c->graph.reset();
   c->sess.active = false;
   Ham& h = c->ham;
@@ -759,21 +764,22 @@ void drv_supercell_csr(tbpm_ctx* c, const tbpm_supercell* sc, int layout, double
                        int64_t* n_rows, int64_t* nnz, double* rescale, int64_t* indptr,
                        int32_t* indices, double* hop, double* dx, double* dy) {
   Phase phase("tbpm_supercell_csr");
-  Prepared P;
+  ScratchScope scope(c->scratch);
+  Prepared P(c->scratch);
   prepare(c, sc, layout, cutoff, P);
   const bool dxy = layout == TBPM_LAYOUT_DXY;
   const bool want_dr = dxy && dx && dy;
   P.s.need_dr = want_dr ? 1 : 0;
   cudaStream_t st = c->stream;
   const int64_t n = P.s.n_rows;
-  DevMem count, off, nd;
+  TempMem count(c->scratch), off(c->scratch), nd(c->scratch), tsum(c->scratch);
+  tsum.ensure(scan_bytes(n));
   count.ensure((size_t)n * 4);
   off.ensure((size_t)(n + 1) * 8);
   nd.ensure(8);
   TBPM_CK(cudaMemsetAsync(nd.p, 0, 8, st));
   count_rows(P, 0, count.as<int32_t>(), nd.as<unsigned long long>(), st);
-  const int64_t total = scan_counts(count.as<int32_t>(), n, off.as<int64_t>(), st);
-  count.release();
+  const int64_t total = scan_counts(count.as<int32_t>(), n, off.as<int64_t>(), tsum.as<int64_t>(), st);
   if (n_rows) *n_rows = n;
   if (nnz) *nnz = total;
   if (rescale) *rescale = P.rescale;

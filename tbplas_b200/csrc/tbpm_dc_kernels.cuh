@@ -36,18 +36,10 @@ struct StatePtrs {
 #ifndef TBPM_QE_MINB_A
 #define TBPM_QE_MINB_A 2
 #endif
-#ifndef TBPM_QE_MINB_P
-#define TBPM_QE_MINB_P 2
-#endif
 #ifndef TBPM_QE_ROWS_A
 #define TBPM_QE_ROWS_A 4
 #endif
-// rows per tile of qe_project_kernel, and of qe_accum_kernel (fewer: its tile
-// holds 16 window states)
-template <typename R>
-__host__ __device__ constexpr int qe_tile_rows(int nb) {
-  return nb >= 64 ? 1 : (64 / nb < 8 ? 64 / nb : 8);
-}
+// rows per tile of qe_accum_kernel (its tile holds 16 window states)
 template <typename R>
 __host__ __device__ constexpr int qe_accum_rows(int nb) {
   return nb >= 64 ? 1 : (64 / nb < TBPM_QE_ROWS_A ? 64 / nb : TBPM_QE_ROWS_A);
@@ -77,12 +69,6 @@ constexpr int kQeG = 2;
 __host__ __device__ constexpr int qe_accum_threads(int n_en, int nb) {
   return nb * ((n_en + kQeG - 1) / kQeG < 256 / nb ? (n_en + kQeG - 1) / kQeG : 256 / nb);
 }
-// Threads per block of qe_project_kernel (K threads per element: one per k).
-__host__ __device__ constexpr int qe_project_threads(int n_en, int nb, int K) {
-  return K * nb *
-         ((n_en + kQeG - 1) / kQeG < 256 / (K * nb) ? (n_en + kQeG - 1) / kQeG : 256 / (K * nb));
-}
-
 // Shared memory of qe_accum_kernel.
 template <typename R>
 __host__ __device__ constexpr size_t qe_accum_smem(int n_en, int nb) {
@@ -90,16 +76,6 @@ __host__ __device__ constexpr size_t qe_accum_smem(int n_en, int nb) {
          (size_t)kMaxWindow * kQeG * (size_t)(qe_accum_threads(n_en, nb) / nb) *
              sizeof(double2);                                                       // coefficients
 }
-// Shared memory of qe_project_kernel.
-template <typename R>
-__host__ __device__ constexpr size_t qe_project_smem(int n_en, int nb, int K) {
-  return (sizeof(R) == 4 ? (size_t)qe_tile_rows<R>(nb) * kMaxProject * 2 * nb * sizeof(double2)
-                         : 0) +                                                     // converted u
-         2 * (size_t)qe_tile_rows<R>(nb) * kMaxProject * 2 * nb * 2 * sizeof(R) +   // raw u
-         2 * (size_t)qe_tile_rows<R>(nb) * kQeG * (qe_project_threads(n_en, nb, K) / K) * 2 *
-             sizeof(R);                                                             // raw QE
-}
-
 // QE[r][i][b] (+)= sum_tau c[tau][i] * pos_tau[r][b] + conj(c[tau][i]) * neg_tau[r][b]
 // pos/neg columns of a window state: b and nb + b (ld = 2 nb).  init: start
 // from wf0[r][b] (tbpm.f90:600-603).
@@ -368,147 +344,185 @@ __global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_accum_mma_kernel(
   }
 }
 
-// Tall-skinny reductions over orbitals: block partial sums of
-// conj(u_tau[r][k*nb + b]) * QE[r][i][b] for tau < T, k in {0, 1} (mode 0), or
-// of conj(wf0[r][b]) * QE[r][i][b] (mode 1, T = 1, k = 0).
-// partials[((tau*K + k) * n_en*nb + ib) * 2 + {re,im}][block x].
-// Block: qe_project_threads(n_en, nb, K) threads; thread t has k = t % K and
-// owns the elements ib_lo + t / K + g * (blockDim.x / K), g < kQeG (one state
-// b, kQeG energies); its T x kQeG accumulators stay in registers.
-// Grid: x over row ranges of rows_per_tile, y over chunks of elements.  Each
-// thread sums its rows in order.
+// ---- projections on the quasi-eigenstates (mma.sync) --------------------------
+//
+// sum_r conj(u_tau[r][k*nb + b]) QE[r][i][b] for the M = T*K <= 16 vectors
+// m = tau*K + k, every energy i and state b: per state a product A (vectors x 2N)
+// . B (2N x energies) over the rows' real and imaginary parts,
+//   Re = sum u.re q.re + u.im q.im,  Im = sum u.re q.im - u.im q.re,
+// on mma.sync m8n8k4 f64 (a k-step is two rows x {re, im}; the B fragment of Im is
+// the neighbouring number with a sign).  A block stages tiles of kProjRows rows
+// (cp.async, double-buffered, raw values): the vectors and up to 8 states'
+// elements of up to 256 energies, transposed to [row][state][vector] and
+// [row][state][energy], rows padded by 64 bytes, so that fragment loads touch
+// every bank once.  A warp owns one state and 32 energies (64 accumulator
+// registers) for the block's whole row range; with few states and energies the
+// left-over warps split the rows.  (The FMA kernel before held 2 energies x 8
+// steps per thread and was bound by its shared-memory reads: 8 states' vectors x 57
+// energies x 4 FP32 states of 307,200 rows took 1.18 ms.)
+constexpr int kProjWarps = 8;
+constexpr int kProjNT = 4;  // energy tiles (of 8) per warp
 template <typename R>
-__global__ void __launch_bounds__(256, TBPM_QE_MINB_P) qe_project_kernel(
-    const typename Cx<R>::t* qe, int64_t n_rows, int64_t rows_per_tile, int n_en, int nb,
-    StatePtrs<R> u, int T, int mode, const typename Cx<R>::t* wf0, double* partials) {
+constexpr int kProjRows = sizeof(R) == 8 ? 8 : 16;
+template <typename R>
+constexpr int kProjPad = sizeof(R) == 8 ? 4 : 8;
+
+struct ProjShape {
+  int bb;      // states per block
+  int ge;      // groups of 32 energies per block
+  int ws;      // row splits
+  int n_bc;    // state chunks
+  int n_ec;    // energy chunks
+};
+__host__ __device__ inline ProjShape proj_shape(int n_en, int nb) {
+  ProjShape s;
+  s.bb = nb < kProjWarps ? nb : kProjWarps;
+  const int need = (n_en + 8 * kProjNT - 1) / (8 * kProjNT);
+  s.ge = kProjWarps / s.bb;
+  if (s.ge > need) s.ge = need;
+  s.ws = kProjWarps / (s.bb * s.ge);
+  s.n_bc = (nb + s.bb - 1) / s.bb;
+  s.n_ec = (need + s.ge - 1) / s.ge;
+  return s;
+}
+// complex values of one row of the staged vectors and of the staged QE
+template <typename R>
+__host__ __device__ constexpr int proj_urow(const ProjShape& s) {
+  return s.bb * 16 + kProjPad<R>;
+}
+template <typename R>
+__host__ __device__ constexpr int proj_qrow(const ProjShape& s) {
+  return s.bb * s.ge * 8 * kProjNT + kProjPad<R>;
+}
+template <typename R>
+inline size_t proj_smem(const ProjShape& s) {
+  return 2 * (size_t)kProjRows<R> * (proj_urow<R>(s) + proj_qrow<R>(s)) * 2 * sizeof(R);
+}
+
+// qe_cp_async that writes zeros when !in
+template <typename C>
+__device__ __forceinline__ void qe_cp_async_z(C* dst, const C* src, bool in) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = in ? (int)sizeof(C) : 0;
+  if constexpr (sizeof(C) == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n)
+                 : "memory");
+}
+
+// u.p[tau] has K*nb columns.  partials[((m*n_en + i)*nb + b)*2 + {re,im}][part], part
+// = blockIdx.x * ws + row split, gridDim.x * ws parts.  Grid: x over row ranges of
+// rows_per_block, y over energy and state chunks.
+template <typename R>
+__global__ void __launch_bounds__(kProjWarps * 32, 2) qe_project_kernel(
+    const typename Cx<R>::t* qe, int64_t n_rows, int64_t rows_per_block, int n_en, int nb,
+    const __grid_constant__ StatePtrs<R> u, int T, int K, double* partials) {
   using C = typename Cx<R>::t;
   extern __shared__ double2 qsm[];
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_tile;
-  const int64_t r1 = min(r0 + rows_per_tile, n_rows);
-  const int n_ib = n_en * nb;
-  const int K = mode == 0 ? 2 : 1;
-  const int ld = 2 * nb;
-  const int RS = qe_tile_rows<R>(nb);
-  const int NE = blockDim.x / K;  // threads per k, a multiple of nb
-  const int EBE = kQeG * NE;      // elements of a row the block covers
-  const int ib_lo = blockIdx.y * EBE;
-  const int eb = min(EBE, n_ib - ib_lo);
-  const int k = threadIdx.x % K;
-  const int e = threadIdx.x / K;
-  const int b = e % nb;
-  bool act[kQeG];
-#pragma unroll
-  for (int g = 0; g < kQeG; ++g) act[g] = e + g * NE < eb;
-  const int UW = kMaxProject * ld;  // staged values of one row
-  constexpr bool conv = sizeof(R) == 4;
-  double2* dbl = qsm;                                               // [RS][UW] (FP32 only)
-  C* raw_u = reinterpret_cast<C*>(qsm + (conv ? RS * UW : 0));      // [2][RS][UW]
-  C* raw_q = raw_u + 2 * RS * UW;                                   // [2][RS][EBE]
-  auto issue = [&](int64_t rb, int buf) {
-    const int nr = (int)min((int64_t)RS, r1 - rb);
-    C* du = raw_u + buf * RS * UW;
-    if (mode == 0) {
-#pragma unroll
-      for (int tau = 0; tau < kMaxProject; ++tau) {
-        if (tau < T) {
-          const C* src = u.p[tau] + rb * ld;
-          for (int q = threadIdx.x; q < nr * ld; q += blockDim.x) {
-            const int rr = q / ld;
-            qe_cp_async(du + rr * UW + tau * ld + (q - rr * ld), src + q);
-          }
+  constexpr int RS = kProjRows<R>;
+  const ProjShape sh = proj_shape(n_en, nb);
+  const int UR = proj_urow<R>(sh), QR = proj_qrow<R>(sh);
+  const int BB = sh.bb, EC = sh.ge * 8 * kProjNT;
+  const int b0 = (blockIdx.y % sh.n_bc) * BB, i0 = (blockIdx.y / sh.n_bc) * EC;
+  const int nbb = min(BB, nb - b0), nee = min(EC, n_en - i0);
+  const int M = T * K, ldu = K * nb;
+  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
+  const int64_t r1 = min(r0 + rows_per_block, n_rows);
+  C* buf = reinterpret_cast<C*>(qsm);
+  const int BUF = RS * (UR + QR);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int wb = warp % BB, we = (warp / BB) % sh.ge, wr = warp / (BB * sh.ge);
+  // vectors m >= M and energies past the chunk are never copied: zero them once
+  for (int q = tid; q < 2 * BUF; q += kProjWarps * 32) {
+    C z;
+    z.x = z.y = (R)0;
+    buf[q] = z;
+  }
+  __syncthreads();
+  // a warp copies whole rows; lane l starts at value l of the row and steps by 32
+  const int d_hi = 32 / nbb, d_lo = 32 % nbb, l_hi = lane / nbb, l_lo = lane % nbb;
+  auto issue = [&](int64_t rb, C* dst) {
+    for (int rr = warp; rr < RS && rb < r1; rr += kProjWarps) {
+      const bool in = rb + rr < r1;  // rows past the range become zeros
+      const int64_t row = in ? rb + rr : rb;
+      C* du = dst + rr * UR;
+      for (int m = l_hi, b = l_lo; m < M;) {
+        const int tau = K == 2 ? m >> 1 : m, k = K == 2 ? m & 1 : 0;
+        qe_cp_async_z(du + b * 16 + m, u.p[tau] + row * ldu + k * nb + b0 + b, in);
+        m += d_hi;
+        b += d_lo;
+        if (b >= nbb) {
+          b -= nbb;
+          ++m;
         }
       }
-    } else {
-      for (int q = threadIdx.x; q < nr * nb; q += blockDim.x) {
-        const int rr = q / nb;
-        qe_cp_async(du + rr * UW + (q - rr * nb), wf0 + rb * nb + q);
+      C* dq = dst + RS * UR + rr * QR;
+      const C* sq = qe + (row * n_en + i0) * nb + b0;
+      for (int i = l_hi, b = l_lo; i < nee;) {
+        qe_cp_async_z(dq + b * EC + i, sq + i * nb + b, in);
+        i += d_hi;
+        b += d_lo;
+        if (b >= nbb) {
+          b -= nbb;
+          ++i;
+        }
       }
     }
-    C* dq = raw_q + buf * RS * EBE;
-    for (int q = threadIdx.x; q < nr * eb; q += blockDim.x) {
-      const int rr = q / eb;
-      const int ee = q - rr * eb;
-      qe_cp_async(dq + rr * EBE + ee, qe + (rb + rr) * n_ib + ib_lo + ee);
-    }
-  };
-  double ar[kMaxProject][kQeG], ai[kMaxProject][kQeG];
-#pragma unroll
-  for (int q = 0; q < kMaxProject; ++q)
-#pragma unroll
-    for (int g = 0; g < kQeG; ++g) ar[q][g] = ai[q][g] = 0.0;
-  if (r0 < r1) issue(r0, 0);
-  qe_cp_commit();
-  int j = 0;
-  for (int64_t rb = r0; rb < r1; rb += RS, ++j) {
-    const int nr = (int)min((int64_t)RS, r1 - rb);
-    qe_cp_wait_all();
-    __syncthreads();  // tile j is in shared memory; tile j-1 is consumed
-    if (rb + RS < r1) issue(rb + RS, (j + 1) & 1);
     qe_cp_commit();
-    const C* tu = raw_u + (j & 1) * RS * UW;
-    const C* tq = raw_q + (j & 1) * RS * EBE;
-    if constexpr (conv) {
-      const int per_row = mode == 0 ? T * ld : nb;
-      for (int q = threadIdx.x; q < nr * per_row; q += blockDim.x) {
-        const int rr = q / per_row;
-        const int w = q - rr * per_row;
-        const C v = tu[rr * UW + w];
-        dbl[rr * UW + w] = make_double2((double)v.x, (double)v.y);
-      }
-      __syncthreads();
-    }
-    if (!act[0]) continue;
-    for (int rr = 0; rr < nr; ++rr) {
-      double qr[kQeG], qi[kQeG];
+  };
+  double re[2][kProjNT][2], im[2][kProjNT][2];
 #pragma unroll
-      for (int g = 0; g < kQeG; ++g) {
-        const C qv = act[g] ? tq[rr * EBE + e + g * NE] : C{};
-        qr[g] = (double)qv.x;
-        qi[g] = (double)qv.y;
-      }
-      if (mode == 1) {
-        double2 w;
-        if constexpr (conv)
-          w = dbl[rr * UW + b];
-        else
-          w = make_double2((double)tu[rr * UW + b].x, (double)tu[rr * UW + b].y);
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int g = 0; g < kQeG; ++g) {
-          ar[0][g] += w.x * qr[g] + w.y * qi[g];
-          ai[0][g] += w.x * qi[g] - w.y * qr[g];
-        }
-      } else {
+    for (int n = 0; n < kProjNT; ++n) re[a][n][0] = re[a][n][1] = im[a][n][0] = im[a][n][1] = 0.0;
+  issue(r0, buf);
+  int cur = 0;
+  for (int64_t rb = r0; rb < r1; rb += RS, cur ^= 1) {
+    qe_cp_wait_all();
+    __syncthreads();  // this tile has landed; the other buffer is consumed
+    issue(rb + RS, buf + (cur ^ 1) * BUF);
+    if (wr >= sh.ws || wb >= nbb) continue;
+    const R* tu = reinterpret_cast<const R*>(buf + cur * BUF);
+    const R* tq = reinterpret_cast<const R*>(buf + cur * BUF + RS * UR);
+#pragma unroll 2
+    for (int s = wr; s < RS / 2; s += sh.ws) {
+      const int row = 2 * s + (t >> 1);
+      const R* pu = tu + 2 * (row * UR + wb * 16 + g) + (t & 1);
+      const double fa0 = (double)pu[0], fa1 = (double)pu[16];
+      const R* pq = tq + 2 * (row * QR + wb * EC + we * 8 * kProjNT + g);
 #pragma unroll
-        for (int tau = 0; tau < kMaxProject; ++tau) {
-          if (tau < T) {
-            const int o = rr * UW + tau * ld + k * nb + b;
-            double2 w;
-            if constexpr (conv)
-              w = dbl[o];
-            else
-              w = make_double2((double)tu[o].x, (double)tu[o].y);
-#pragma unroll
-            for (int g = 0; g < kQeG; ++g) {
-              ar[tau][g] += w.x * qr[g] + w.y * qi[g];
-              ai[tau][g] += w.x * qi[g] - w.y * qr[g];
-            }
-          }
-        }
+      for (int n = 0; n < kProjNT; ++n) {
+        const double q0 = (double)pq[16 * n + (t & 1)];
+        const double q1 = (double)pq[16 * n + ((t & 1) ^ 1)];
+        const double qx = (t & 1) ? -q1 : q1;
+        dmma_8x8x4(re[0][n][0], re[0][n][1], fa0, q0);
+        dmma_8x8x4(im[0][n][0], im[0][n][1], fa0, qx);
+        dmma_8x8x4(re[1][n][0], re[1][n][1], fa1, q0);
+        dmma_8x8x4(im[1][n][0], im[1][n][1], fa1, qx);
       }
     }
   }
+  qe_cp_wait_all();
+  if (wr >= sh.ws || wb >= nbb) return;
+  const int64_t parts = (int64_t)gridDim.x * sh.ws;
+  const int64_t part = (int64_t)blockIdx.x * sh.ws + wr;
 #pragma unroll
-  for (int g = 0; g < kQeG; ++g) {
-    if (!act[g]) continue;
-    const int ib = ib_lo + e + g * NE;
+  for (int a = 0; a < 2; ++a) {
+    const int m = 8 * a + g;
+    if (m >= M) continue;
 #pragma unroll
-    for (int tau = 0; tau < kMaxProject; ++tau) {
-      if (tau < (mode == 0 ? T : 1)) {
-        const int64_t o = (int64_t)(tau * K + k) * n_ib + ib;
-        partials[(o * 2 + 0) * gridDim.x + blockIdx.x] = ar[tau][g];
-        partials[(o * 2 + 1) * gridDim.x + blockIdx.x] = ai[tau][g];
+    for (int n = 0; n < kProjNT; ++n)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = we * 8 * kProjNT + 8 * n + 2 * t + q;
+        if (i >= nee) continue;
+        const int64_t o = ((int64_t)m * n_en + i0 + i) * nb + b0 + wb;
+        partials[(o * 2 + 0) * parts + part] = re[a][n][q];
+        partials[(o * 2 + 1) * parts + part] = im[a][n][q];
       }
-    }
   }
 }
 

@@ -2065,16 +2065,13 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
 #endif
 template <class K>
 void qe_smem_attr(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
+  // (a kernel's static shared memory counts towards the default 48 KB too)
+  if (bytes <= 40 * 1024) return;
   TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 template <typename R>
 void qe_accum_attr(size_t bytes) {
   qe_smem_attr(qe_accum_kernel<R>, bytes);
-}
-template <typename R>
-void qe_project_attr(size_t bytes) {
-  qe_smem_attr(qe_project_kernel<R>, bytes);
 }
 
 // Phase 1 on the polynomial route: QE_i = f_i(H) wf0 by the energies' filters
@@ -2373,29 +2370,34 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   // ---- phase 2 ----
   phase.emplace("tbpm_dccond: current correlations");
   const int n_ib = n_en * nb;
-  int64_t rows_per_tile = std::max<int64_t>(64, n / ((int64_t)kSMs * 8));
-  const int pgrid = (int)((n + rows_per_tile - 1) / rows_per_tile);
-  // mode 1 (one projection): one thread per kQeG elements; mode 0: a pair
-  const int pthreads1 = qe_project_threads(n_en, nb, 1);
-  const dim3 pgrid1((unsigned)pgrid,
-                    (unsigned)((n_ib + kQeG * pthreads1 - 1) / (kQeG * pthreads1)));
-  const int pthreads = qe_project_threads(n_en, nb, 2);
-  const dim3 pgrid2((unsigned)pgrid,
-                    (unsigned)((n_ib + kQeG * (pthreads / 2) - 1) / (kQeG * (pthreads / 2))));
-  const size_t psmem1 = qe_project_smem<R>(n_en, nb, 1);
-  const size_t psmem = qe_project_smem<R>(n_en, nb, 2);
-  qe_project_attr<R>(std::max(psmem1, psmem));
-  // |<wf0|QE_i>| per (energy, state)
-  ensure_partials(c, (size_t)2 * n_ib * pgrid);
+  // about four blocks per SM over the row ranges and the chunks
+  const ProjShape psh = proj_shape(n_en, nb);
+  const int64_t chunks = (int64_t)psh.n_bc * psh.n_ec;
+  const int64_t want = std::max<int64_t>(1, 4 * (int64_t)num_sms(c->device) / chunks);
+  const int64_t rows_per_block = std::max<int64_t>(64, (n + want - 1) / want);
+  const int pgrid = (int)((n + rows_per_block - 1) / rows_per_block);
+  const int parts = pgrid * psh.ws;
+  const size_t psmem = proj_smem<R>(psh);
+  qe_smem_attr(qe_project_kernel<R>, psmem);
+  auto project = [&](const StatePtrs<R>& u, int len, int K) {
+    qe_project_kernel<R><<<dim3((unsigned)pgrid, (unsigned)chunks), kProjWarps * 32, psmem,
+                           c->stream>>>(qe, n, rows_per_block, n_en, nb, u, len, K,
+                                        c->partials.as<double>());
+    TBPM_CK(cudaGetLastError());
+    const int64_t n_vals = (int64_t)2 * len * K * n_ib;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), parts, n_vals, c->small.as<double>());
+    TBPM_CK(cudaGetLastError());
+    c->launches += 2;
+  };
+  ensure_partials(c, (size_t)2 * 2 * T2 * n_ib * parts);
   c->small.ensure(sizeof(double) * std::max<size_t>((size_t)2 * T2 * 2 * n_ib, 64));
-  qe_project_kernel<R><<<pgrid1, pthreads1, psmem1, c->stream>>>(
-      qe, n, rows_per_tile, n_en, nb, StatePtrs<R>{}, 1, 1, reinterpret_cast<const C*>(W),
-      c->partials.as<double>());
-  TBPM_CK(cudaGetLastError());
-  reduce_rows_kernel<<<(int)std::min<int64_t>(2 * n_ib, 65535), 256, 0, c->stream>>>(
-      c->partials.as<double>(), pgrid, 2 * n_ib, c->small.as<double>());
-  TBPM_CK(cudaGetLastError());
-  c->launches += 2;
+  // |<wf0|QE_i>| per (energy, state)
+  {
+    StatePtrs<R> w{};
+    w.p[0] = reinterpret_cast<const C*>(W);
+    project(w, 1, 1);
+  }
   std::vector<double> proj(2 * n_ib);
   TBPM_CK(cudaMemcpyAsync(proj.data(), c->small.p, proj.size() * sizeof(double),
                           cudaMemcpyDeviceToHost, c->stream));
@@ -2432,7 +2434,6 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
       h.rescale, n, nb, reinterpret_cast<const C*>(W), nb, 0, 0, reinterpret_cast<C*>(wj));
   TBPM_CK(cudaGetLastError());
   c->launches++;
-  ensure_partials(c, (size_t)2 * 2 * T2 * n_ib * pgrid);
   std::vector<double> vals;
   for (t = 1; t <= n_timestep; t += T2) {
     const int len = std::min(T2, n_timestep - t + 1);
@@ -2458,14 +2459,8 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
       c->launches++;
       u.p[tau] = uq;
     }
-    qe_project_kernel<R><<<pgrid2, pthreads, psmem, c->stream>>>(
-        qe, n, rows_per_tile, n_en, nb, u, len, 0, nullptr, c->partials.as<double>());
-    TBPM_CK(cudaGetLastError());
+    project(u, len, 2);
     const int64_t n_vals = (int64_t)2 * len * 2 * n_ib;
-    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), pgrid, n_vals, c->small.as<double>());
-    TBPM_CK(cudaGetLastError());
-    c->launches += 2;
     c->model_bytes += (double)n * n_ib * 2 * sizeof(R) + (double)len * n * ld * 2 * sizeof(R);
     vals.resize(n_vals);
     TBPM_CK(cudaMemcpyAsync(vals.data(), c->small.p, n_vals * sizeof(double),

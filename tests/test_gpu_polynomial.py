@@ -319,3 +319,24 @@ def test_steps_per_expansion_follow_the_free_memory():
             assert rel_err(got, want) < 1e-12
     finally:
         nat._contexts = kept
+
+
+@pytest.mark.parametrize("ns,n_lim", [(1, 8.5), (2, 8.5), (7, 3.0), (9, 1.0), (16, 2.0)])
+def test_dc_projection_shapes(sample, ns, n_lim):
+    """States and energies around the chunks of the projection kernel (8 states,
+    32 energies per warp, warps left over for row splits), in one batch."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf0 = unit_states(ns, ip.size - 1, seed=31)
+    energies, sel = _energies(sample, 64, (-n_lim, n_lim))
+    bes = bessel_series(math.pi)
+    t_step = 2 * math.pi / sample.energy_range
+    args = (ip, ix, hv, sample.rescale, dx, dy)
+    got = f2py.tbpm_dccond_states(bes, *args, wf0, 64, t_step, energies, sel, 60, 1e-9)
+    ref = oracle.tbpm_dccond(bes, *args, 64, t_step, energies, sel, wf0=wf0)
+    again = oracle.tbpm_dccond(bes, *args, 64, t_step, energies, sel,
+                               wf0=wf0 * (1 + 1e-16 * np.random.default_rng(0).standard_normal(
+                                   wf0.shape)))
+    # wide windows reach energies with hardly any states (test_gpu_dc_shapes.py):
+    # there the oracle's own sensitivity to rounding is the bar
+    assert rel_err(got[0], ref[0]) < 1e-10
+    assert rel_err(got[1], ref[1]) < max(1e-10, 8 * rel_err(again[1], ref[1]))

@@ -181,6 +181,46 @@ __device__ __forceinline__ Pack<float, 4> ldcg_pack(const Pack<float, 4>* p) {
   return r;
 }
 
+// The same through L1, for values made visible by an acquire at GPU scope after
+// which no other SM writes them while they are read.
+__device__ __forceinline__ Pack<double, 1> ld_pack(const Pack<double, 1>* p) {
+  Pack<double, 1> r;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.v[0]), "=d"(r.v[1]) : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ Pack<double, 2> ld_pack(const Pack<double, 2>* p) {
+  Pack<double, 2> r;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ Pack<float, 1> ld_pack(const Pack<float, 1>* p) {
+  Pack<float, 1> r;
+  asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ Pack<float, 2> ld_pack(const Pack<float, 2>* p) {
+  Pack<float, 2> r;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+__device__ __forceinline__ Pack<float, 4> ld_pack(const Pack<float, 4>* p) {
+  Pack<float, 4> r;
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]),
+                 "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
 // Stores with the default (write-back, evict-normal) policy, for values that
 // are read again from L2 shortly after, within the same launch.
 __device__ __forceinline__ void stwb_pack(Pack<double, 1>* p, const Pack<double, 1>& v) {

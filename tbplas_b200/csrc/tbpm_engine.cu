@@ -257,16 +257,27 @@ struct TermTiles {
   const int* win = nullptr;  // window records (ring_window_kernel); null: no windows
 };
 
+// Consumer threads of the ring kernel of a mode.
+template <typename R, int V>
+int ring_items(int mode, bool win) {
+  if (mode == 0) return win ? kRingItems<R, V, 0, true> : kRingItems<R, V, 0, false>;
+  if (mode == 1) return win ? kRingItems<R, V, 1, true> : kRingItems<R, V, 1, false>;
+  if (mode == 2) return win ? kRingItems<R, V, 2, true> : kRingItems<R, V, 2, false>;
+  return kRingItems<R, V, 3, false>;
+}
+
 // Ring layout for rows of tpr packs in kernel mode `mode` (ref_tpr: packs per
 // row of the MODE 2 correlation reference, 0 for none); stages == 0 when the
 // ring does not apply (rows that are not a multiple of 16 bytes, or fewer than
 // two stages fit into the shared memory of one of kRingMinBlocks blocks per SM).
 template <typename R, int V>
-RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win = false) {
+RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win = false,
+                     int items = 0) {
   RingShape s{};
+  if (items == 0) items = ring_items<R, V>(mode, win);
   const size_t row_bytes = (size_t)tpr * sizeof(Pack<R, V>);
-  if (row_bytes % 16 != 0 || tpr < 1 || tpr > kRingConsumers) return s;
-  const int TR = kRingConsumers / tpr;
+  if (row_bytes % 16 != 0 || tpr < 1 || tpr > items) return s;
+  const int TR = items / tpr;
   const Ham& h = c->ham;
   const size_t cs = sizeof(typename Cx<R>::t);
   // CSR entries one stage holds: the mean row length of O over a tile with 25%
@@ -329,7 +340,7 @@ RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win
   s.bar_off = S * off;
   s.smem_bytes = s.bar_off + 2 * S * 8;
   // MODE 2 and 3 reduce their partials in the stage buffers
-  if ((size_t)s.bar_off < (size_t)kRingConsumers * V * 3 * sizeof(double)) return RingShape{};
+  if ((size_t)s.bar_off < (size_t)items * V * 3 * sizeof(double)) return RingShape{};
   return s;
 }
 
@@ -342,7 +353,7 @@ int ring_blocks_per_sm(const tbpm_ctx* c, const RingShape& rs) {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     attr_set[dev] = true;
   }
-  return resident_per_sm(cheb_ring_kernel<R, V, MODE, WIN>, kRingThreads, (size_t)rs.smem_bytes);
+  return resident_per_sm(cheb_ring_kernel<R, V, MODE, WIN>, kRingItems<R, V, MODE, WIN> + 32, (size_t)rs.smem_bytes);
 }
 
 // The window records for tiles of `rows` rows on the current Hamiltonian,
@@ -406,7 +417,7 @@ TermTiles term_tiles(tbpm_ctx* c, int64_t n_rows, int tpr, int ref_tpr = 0) {
     win = true;
     for (int m = 0; m < 3; ++m) win = win && ring_shape<R, V>(c, tpr, m, ref_tpr, true).stages >= 2;
     if (win) {
-      tt.win = window_plan(c, kRingConsumers / tpr);
+      tt.win = window_plan(c, ring_items<R, V>(0, true) / tpr);
       win = tt.win != nullptr;
     }
   }
@@ -431,7 +442,7 @@ TermTiles term_tiles(tbpm_ctx* c, int64_t n_rows, int tpr, int ref_tpr = 0) {
                                          : ring_blocks_per_sm<R, V, 2, false>(c, rs));
       const int64_t tiles = (n_rows + rs.rows - 1) / rs.rows;
       Tile t;
-      t.threads = kRingThreads;
+      t.threads = ring_items<R, V>(m, win && m < 3) + 32;
       t.rpp = rs.rows;
       t.rows_per_tile = rs.rows;
       t.grid = (int)std::max<int64_t>(
@@ -457,20 +468,20 @@ int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
     ra.win = tt.win;
     const size_t smem = (size_t)ra.s.smem_bytes;
     if (mode == 3) {
-      cheb_ring_kernel<R, V, 3, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+      cheb_ring_kernel<R, V, 3, false><<<t.grid, t.threads, smem, c->stream>>>(ra);
     } else if (tt.win) {
       if (mode == 2)
-        cheb_ring_kernel<R, V, 2, true><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+        cheb_ring_kernel<R, V, 2, true><<<t.grid, t.threads, smem, c->stream>>>(ra);
       else if (mode == 1)
-        cheb_ring_kernel<R, V, 1, true><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+        cheb_ring_kernel<R, V, 1, true><<<t.grid, t.threads, smem, c->stream>>>(ra);
       else
-        cheb_ring_kernel<R, V, 0, true><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+        cheb_ring_kernel<R, V, 0, true><<<t.grid, t.threads, smem, c->stream>>>(ra);
     } else if (mode == 2) {
-      cheb_ring_kernel<R, V, 2, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+      cheb_ring_kernel<R, V, 2, false><<<t.grid, t.threads, smem, c->stream>>>(ra);
     } else if (mode == 1) {
-      cheb_ring_kernel<R, V, 1, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+      cheb_ring_kernel<R, V, 1, false><<<t.grid, t.threads, smem, c->stream>>>(ra);
     } else {
-      cheb_ring_kernel<R, V, 0, false><<<t.grid, kRingThreads, smem, c->stream>>>(ra);
+      cheb_ring_kernel<R, V, 0, false><<<t.grid, t.threads, smem, c->stream>>>(ra);
     }
   } else if (mode == 3) {
     const size_t smem = (size_t)t.threads * V * 2 * sizeof(double);
@@ -628,6 +639,177 @@ void launch_pair(tbpm_ctx* c, const PairPlan& pp, const RingShape& rs, const Ter
   c->launches++;
 }
 
+double matrix_bytes(const Ham& h) {
+  const double s = h.prec == TBPM_PREC_FP64 ? 16 : 8;
+  return (double)(h.n + 1) * 4 + (double)h.nnz * (4 + s) + (h.has_diag ? (double)h.n * s : 0.0);
+}
+
+template <class K>
+void qe_smem_attr(K kernel, size_t bytes) {
+  // (a kernel's static shared memory counts towards the default 48 KB too)
+  if (bytes <= 40 * 1024) return;
+  TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
+// Launch of a kernel with a grid barrier: every block is resident at once, so the
+// barrier cannot wait on a block that has not started.
+template <class K, class Args>
+void launch_cooperative(tbpm_ctx* c, K kernel, int grid, int threads, size_t smem,
+                        const Args& args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TBPM_CK(cudaLaunchKernelEx(&cfg, kernel, args));
+}
+
+// Matrix and two vectors up to which one launch beats a launch per term (measured
+// on B200, us per term of the DOS moments, one launch / ring):
+//   FP64  131,072 orbitals x  8 states,  44 MB: 10.6 / 17.3
+//         720,000           x  1,        83 MB: 11.6 / 17.2
+//         320,000           x  5,        78 MB: 23.1 / 28.1
+//        1,280,000          x  1,       148 MB: 34.9 / 35.4
+//         720,000           x  4,       152 MB: 44.7 / 40.9
+//         320,000           x 16,       191 MB: 72.4 / 56.4
+//   FP32  720,000           x  4,        84 MB: 16.9 / 26.1
+//         320,000           x 16,        99 MB: 38.1 / 34.8
+#ifndef TBPM_PERSIST_MB
+#define TBPM_PERSIST_MB 90
+#endif
+// Launch shape of cheb_persist_kernel: for problems whose vectors and matrix stay
+// in L2; grid == 0 when it does not apply.
+struct PersistShape {
+  int grid = 0, threads = 0;
+};
+
+template <typename R, int V>
+PersistShape persist_shape(const tbpm_ctx* c, int ld) {
+  PersistShape s;
+  const tbpm_options& o = c->opts;
+  if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return s;
+  const Ham& h = c->ham;
+  const int tpr = ld / V;
+  constexpr int TMAX = kPersistThreads<R, V>;
+  if (tpr > TMAX) return s;
+  const double bytes = matrix_bytes(h) + 2.0 * (double)h.n * ld * 2 * sizeof(R);
+  const int sms = num_sms(c->device);
+  if (bytes > TBPM_PERSIST_MB * 1e6) return s;
+  const int64_t per_sm = (h.n + sms - 1) / sms;
+  const int rpp = (int)std::min<int64_t>(std::max<int64_t>(per_sm, (128 + tpr - 1) / tpr),
+                                         TMAX / tpr);
+  s.threads = rpp * tpr;
+  s.grid = (int)std::min<int64_t>(sms, (h.n + rpp - 1) / rpp);
+  return s;
+}
+
+// The arguments that every use of cheb_persist_kernel shares: terms k0..k1 with
+// p_k = alpha H p_{k-1} - p_{k-2} (turn: times (-i)^k) on a ring of vectors.
+template <typename R, int V>
+PersistArgs<R, V> persist_args(const tbpm_ctx* c, double alpha, int k0, int k1, int ld,
+                               const Pack<R, V>* p0, Pack<R, V>* const* ring, int slots,
+                               bool turn) {
+  const Ham& h = c->ham;
+  PersistArgs<R, V> a{};
+  a.indptr = h.indptr.as<int32_t>();
+  a.indices = h.indices.as<int32_t>();
+  a.hop = h.hop.as<typename Cx<R>::t>();
+  a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
+  a.n_rows = h.n;
+  a.tpr = ld / V;
+  a.p0 = p0;
+  for (int q = 0; q < slots; ++q) a.ring[q] = ring[q];
+  a.slots = slots;
+  a.alpha = alpha;
+  a.turn = turn ? 1 : 0;
+  a.k0 = k0;
+  a.k1 = k1;
+  a.bar = c->ctr.as<unsigned int>() + 12;
+  a.status = c->status.as<unsigned int>();
+  return a;
+}
+
+template <bool ACC, typename R, int V>
+void launch_persist(tbpm_ctx* c, const PersistShape& s, const PersistArgs<R, V>& a) {
+  const size_t smem = !ACC && a.k_dots >= a.k0
+                          ? (size_t)kPersistBatch * s.threads * V * 2 * sizeof(double)
+                          : 0;
+  qe_smem_attr(cheb_persist_kernel<R, V, ACC>, smem);
+  TBPM_CK(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), c->stream));
+  launch_cooperative(c, cheb_persist_kernel<R, V, ACC>, s.grid, s.threads, smem, a);
+  c->launches++;
+}
+
+#ifndef TBPM_CLUSTER_ITEMS
+#define TBPM_CLUSTER_ITEMS kClusterItems  // (0: off)
+#endif
+// The moments' terms 1..K of a tiny problem by cheb_cluster_kernel: block partials
+// to c->partials, the number of blocks returned (0: it does not apply).
+template <typename R, int V>
+int launch_cluster(tbpm_ctx* c, double alpha, int K, int ld, const Pack<R, V>* p0) {
+  const tbpm_options& o = c->opts;
+  if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return 0;
+  const Ham& h = c->ham;
+  const int tpr = ld / V;
+  constexpr int TMAX = kClusterThreads<R, V>;
+  if (h.n > (1 << 20) || tpr > TMAX) return 0;
+  // at least two rows: the quotient's multiplier 2^32 / rows has 32 bits
+  const int rows = std::max(2, (int)((h.n + kClusterBlocks - 1) / kClusterBlocks));
+  const int rpp = std::max(std::min(rows, TMAX / tpr), (128 + tpr - 1) / tpr);
+  const int threads = rpp * tpr;
+  if (rows > TBPM_CLUSTER_ITEMS * rpp) return 0;
+  const size_t smem = 2 * (size_t)rows * tpr * sizeof(Pack<R, V>) +
+                      (size_t)kPersistBatch * threads * V * 2 * sizeof(double);
+  // (the products' slots start at a multiple of 8 bytes: packs are that or more)
+  if (smem > 200 * 1024 || threads > TMAX) return 0;
+  auto kernel = cheb_cluster_kernel<R, V>;
+  TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  qe_smem_attr(kernel, smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kClusterBlocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kClusterBlocks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n_clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&n_clusters, kernel, &cfg) != cudaSuccess ||
+      n_clusters < 1) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  ensure_partials(c, (size_t)K * ld * 2 * kClusterBlocks);
+  ClusterArgs<R, V> a;
+  a.indptr = h.indptr.as<int32_t>();
+  a.indices = h.indices.as<int32_t>();
+  a.hop = h.hop.as<typename Cx<R>::t>();
+  a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
+  a.n_rows = (int)h.n;
+  a.tpr = tpr;
+  a.p0 = p0;
+  a.alpha = alpha;
+  a.n_terms = K;
+  a.rows = rows;
+  a.magic = (unsigned)(((1ull << 32) + rows - 1) / rows);
+  a.partials = c->partials.as<double>();
+  TBPM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
+  c->launches++;
+  return kClusterBlocks;
+}
+
+// Expansions of this many terms or more run in one launch on small problems (a
+// time step's 16 to 20 stay single launches, which CUDA graphs replay).
+constexpr int kPersistMinTerms = 64;
+
 // Enqueue one expansion (one time step, or one Fermi operator) on the block A.
 // When `partials_out` is set the last term also produces <ref|psi>, <psi|psi>
 // block partials and a finalize launch stores them in out[*step].
@@ -714,8 +896,9 @@ void enqueue_expansion(tbpm_ctx* c, const Expansion& ex, int ld, Pack<R, V>* A, 
   PairPlan* pp = nullptr;
   RingShape prs{};
   const int tk = c->opts.term_kernel;
-  if (n >= 3 && tk == 3 && tt.ring[1]) {
-    prs = tt.rs[1];
+  if (n >= 3 && tk == 3 && tt.ring[1])
+    prs = ring_shape<R, V>(c, tpr, 1, 0, false, kRingConsumers);
+  if (prs.stages >= 2) {
     const size_t smem = (size_t)prs.smem_bytes + pair_extra_smem<R, V>();
     if (smem <= 227 * 1024) {
       const int per_sm = pair_blocks_per_sm<R, V>(c, smem);
@@ -730,7 +913,36 @@ void enqueue_expansion(tbpm_ctx* c, const Expansion& ex, int ld, Pack<R, V>* A, 
       pp = pair_plan(c, q);
     }
   }
-  for (int k = 1; k < n;) {
+  int k_first = 1;
+  const PersistShape ps = n >= kPersistMinTerms && ex.neg_mask == 0
+                              ? persist_shape<R, V>(c, ld)
+                              : PersistShape{};
+  const double alpha = ex.alpha_re != 0.0 ? ex.alpha_re : -ex.alpha_im;
+  const bool turn = ex.alpha_re == 0.0;
+  // the recurrences of the one-launch kernel: real alpha with beta = -1, or -i
+  // times it with beta = 1, and half of alpha in the first term
+  const bool fits = (turn ? ex.beta == 1.0 : ex.alpha_im == 0.0 && ex.beta == -1.0) &&
+                    2 * ex.alpha1_re == ex.alpha_re && 2 * ex.alpha1_im == ex.alpha_im;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (ps.grid > 0) TBPM_CK(cudaStreamIsCapturing(c->stream, &capturing));
+  if (ps.grid > 0 && fits && capturing == cudaStreamCaptureStatusNone) {
+    // all but the last term, which also carries the products with `ref`
+    std::vector<double> w(ex.w[0]);
+    w.insert(w.end(), ex.w[1].begin(), ex.w[1].end());
+    c->wts.ensure(w.size() * sizeof(double));
+    TBPM_CK(cudaMemcpyAsync(c->wts.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice,
+                            c->stream));
+    Pack<R, V>* ring[2] = {Y, X};
+    PersistArgs<R, V> a = persist_args<R, V>(c, alpha, 1, n - 2, ld, A, ring, 2, turn);
+    a.acc = A_out;
+    a.w = c->wts.as<double>();
+    a.n_w = n;
+    a.set_mask = ex.set_mask;
+    launch_persist<true>(c, ps, a);
+    for (int k = 1; k < n - 1; ++k) c->model_bytes += term_bytes[k];
+    k_first = n - 1;
+  }
+  for (int k = k_first; k < n;) {
     const bool pair = pp && k + 1 < n && !(want && k + 1 == n - 1) &&
                       !(terms[k].c.nflush > 0 && terms[k + 1].c.nflush > 0);
     if (pair) {
@@ -1269,97 +1481,37 @@ TermArgs<R, V> poly_term2(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr,
   return poly_term<R, V>(c, pp, k, tpr, (k & 1) ? A : X, dst, dst);
 }
 
-double matrix_bytes(const Ham& h) {
-  const double s = h.prec == TBPM_PREC_FP64 ? 16 : 8;
-  return (double)(h.n + 1) * 4 + (double)h.nnz * (4 + s) + (h.has_diag ? (double)h.n * s : 0.0);
-}
-
-// Launch of a kernel with a grid barrier: every block is resident at once, so the
-// barrier cannot wait on a block that has not started.
-template <class K, class Args>
-void launch_cooperative(tbpm_ctx* c, K kernel, int grid, int threads, size_t smem,
-                        const Args& args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TBPM_CK(cudaLaunchKernelEx(&cfg, kernel, args));
-}
-
-#ifndef TBPM_PERSIST_MB
-#define TBPM_PERSIST_MB 48
-#endif
-#ifndef TBPM_PERSIST_ITEMS
-#define TBPM_PERSIST_ITEMS 8
-#endif
-// All K terms in one cooperative launch (cheb_persist_kernel) when the vectors
-// and the matrix stay in L2 and a thread has few items; false when it does not apply.
-template <typename R, int V>
-bool launch_persist(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A, Pack<R, V>* X,
-                    double* sums) {
-  const tbpm_options& o = c->opts;
-  if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return false;
-  const Ham& h = c->ham;
-  const int tpr = ld / V;
-  constexpr int TMAX = kPersistThreads<R, V>;
-  if (tpr > TMAX) return false;
-  const double bytes = matrix_bytes(h) + 2.0 * (double)h.n * ld * 2 * sizeof(R);
-  const int sms = num_sms(c->device);
-  if (bytes > TBPM_PERSIST_MB * 1e6 || h.n * tpr > (int64_t)TBPM_PERSIST_ITEMS * sms * TMAX)
-    return false;
-  const int64_t per_sm = (h.n + sms - 1) / sms;
-  const int rpp = (int)std::min<int64_t>(std::max<int64_t>(per_sm, (128 + tpr - 1) / tpr),
-                                         TMAX / tpr);
-  const int threads = rpp * tpr;
-  const int grid = (int)std::min<int64_t>(sms, (h.n + rpp - 1) / rpp);
-  const size_t smem = (size_t)threads * V * 2 * sizeof(double);
-  static bool attr_set[64] = {false};
-  const int dev = c->device;
-  if (dev < 0 || dev >= 64) return false;
-  if (!attr_set[dev]) {
-    TBPM_CK(cudaFuncSetAttribute(cheb_persist_kernel<R, V>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-    attr_set[dev] = true;
-  }
-  const int64_t n_vals = (int64_t)K * ld * 2;
-  ensure_partials(c, (size_t)n_vals * grid);
-  unsigned int* bar = c->ctr.as<unsigned int>() + 12;
-  TBPM_CK(cudaMemsetAsync(bar, 0, sizeof(unsigned int), c->stream));
-  PersistArgs<R, V> a;
-  a.indptr = h.indptr.as<int32_t>();
-  a.indices = h.indices.as<int32_t>();
-  a.hop = h.hop.as<typename Cx<R>::t>();
-  a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
-  a.n_rows = h.n;
-  a.tpr = tpr;
-  a.p0 = A;
-  a.p1 = X;
-  a.alpha = pp.alpha;
-  a.n_terms = K;
-  a.partials = c->partials.as<double>();
-  a.bar = bar;
-  a.status = c->status.as<unsigned int>();
-  launch_cooperative(c, cheb_persist_kernel<R, V>, grid, threads, smem, a);
-  reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-      c->partials.as<double>(), grid, n_vals, sums);
-  TBPM_CK(cudaGetLastError());
-  c->launches += 2;
-  c->model_bytes += K * (matrix_bytes(h) + 3.0 * (double)h.n * ld * 2 * sizeof(R));
-  return true;
-}
-
 // Terms 1..K with the products of every term: sums[((k-1)*ld + col)*2 + q],
 // q = 0: <p_k|p_k>, 1: Re <p_k|p_{k-1}>.  p_0 is in A, X is scratch.
 template <typename R, int V>
 void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A,
                           Pack<R, V>* X, double* sums) {
-  if (launch_persist<R, V>(c, pp, K, ld, A, X, sums)) return;
+  const PersistShape ps = persist_shape<R, V>(c, ld);
+  const int64_t n_vals = (int64_t)K * ld * 2;
+  const double all_bytes =
+      K * (matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R));
+  if (const int blocks = launch_cluster<R, V>(c, pp.alpha, K, ld, A)) {
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), blocks, n_vals, sums);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    c->model_bytes += all_bytes;
+    return;
+  }
+  if (ps.grid > 0) {
+    ensure_partials(c, (size_t)n_vals * ps.grid);
+    Pack<R, V>* ring[2] = {A, X};
+    PersistArgs<R, V> a = persist_args<R, V>(c, pp.alpha, 1, K, ld, A, ring, 2, false);
+    a.k_dots = K;
+    a.partials = c->partials.as<double>();
+    launch_persist<false>(c, ps, a);
+    c->model_bytes += all_bytes;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), ps.grid, n_vals, sums);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    return;
+  }
   const int tpr = ld / V;
   const TermTiles tt = term_tiles<R, V>(c, c->ham.n, tpr);
   const int grid = tt.t[3].grid;
@@ -1726,10 +1878,14 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
     return false;
   int64_t max_len = 0;
   for (int k = 0; k < n_seg; ++k) max_len = std::max<int64_t>(max_len, off[k + 1] - off[k]);
+  // the states' chunks set the order of their normalisation sums, as in
+  // dos_segmented_run; the products take about 16 blocks per SM
   const int64_t rows_per_chunk = 4096;
   const int n_chunks = (int)std::max<int64_t>(1, (max_len + rows_per_chunk - 1) / rows_per_chunk);
   const int rpp = std::max(1, 256 / ns);
   const int threads = rpp * ns;
+  const int64_t dot_rows = std::max<int64_t>(4 * rpp, n / (16 * (int64_t)num_sms(c->device)) + 1);
+  const int dot_chunks = (int)std::max<int64_t>(1, (max_len + dot_rows - 1) / dot_rows);
   c->graph.reset();
   c->sess.active = false;
   const size_t vb = (size_t)n * ns * sizeof(C);
@@ -1739,10 +1895,10 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
   c->seg.ensure(sizeof(int64_t) * off.size());
   TBPM_CK(cudaMemcpyAsync(c->seg.p, off.data(), sizeof(int64_t) * off.size(),
                           cudaMemcpyHostToDevice, c->stream));
-  const int64_t per_term = (int64_t)n_cols * 2 * n_chunks;
+  const int64_t per_term = (int64_t)n_cols * 2 * dot_chunks;
   const int chunk =
       (int)std::max<int64_t>(1, std::min<int64_t>(K + 1, (64ll << 20) / (per_term * 8)));
-  ensure_partials(c, (size_t)chunk * per_term);
+  ensure_partials(c, std::max<size_t>((size_t)chunk * per_term, (size_t)n_cols * n_chunks));
   c->small.ensure(sizeof(double) * std::max<size_t>((size_t)n_cols, kMaxCols * 2));
   c->out.ensure((size_t)(T + 3) * n_cols * 2 * sizeof(double));
   const size_t n_sums = (size_t)(K + 1) * n_cols * 2, n_mu = (size_t)n_cols * M;
@@ -1775,8 +1931,8 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
       Pack<R, V>* x = (k & 1) ? X : A;
       Pack<R, V>* y = (k & 1) || k == 0 ? A : X;
       if (k >= 1) launch_term<R, V>(c, tt, poly_term2<R, V>(c, pp, k, tpr, A, X));
-      seg_dots_kernel<R><<<grid, threads, 0, c->stream>>>(
-          c->seg.as<int64_t>(), ns, rows_per_chunk, reinterpret_cast<const C*>(x),
+      seg_dots_kernel<R><<<dim3(dot_chunks, n_seg), threads, 0, c->stream>>>(
+          c->seg.as<int64_t>(), ns, dot_rows, reinterpret_cast<const C*>(x),
           reinterpret_cast<const C*>(y), c->partials.as<double>() + (int64_t)i * per_term);
       TBPM_CK(cudaGetLastError());
       c->launches++;
@@ -1784,7 +1940,7 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
     }
     const int64_t n_vals = (int64_t)m * n_cols * 2;
     reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), n_chunks, n_vals, sums + (int64_t)k0 * n_cols * 2);
+        c->partials.as<double>(), dot_chunks, n_vals, sums + (int64_t)k0 * n_cols * 2);
     TBPM_CK(cudaGetLastError());
     c->launches++;
   }
@@ -1853,12 +2009,21 @@ void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, 
   a.total = n * ld;
   a.m = m;
   for (int j = 0; j < m; ++j) a.out[j] = reinterpret_cast<C*>(states[j]);
-  const int grid = blocks_for(a.total, 256);
+  const int grid = sizeof(R) == 8 ? blocks_for(a.total, 256)
+                                  : (int)std::min<int64_t>(blocks_for((a.total + 7) / 8, 8),
+                                                           (int64_t)num_sms(c->device) * 6);
+  const PersistShape ps = persist_shape<R, V>(c, ld);
   for (int k0 = 0; k0 < n_vec; k0 += window) {
     const int len = std::min(window, n_vec - k0);
+    if (ps.grid > 0 && k0 + len > 1) {
+      launch_persist<false>(c, ps,
+                            persist_args<R, V>(c, pp.alpha, std::max(k0, 1), k0 + len - 1, ld, psi,
+                                               ring.data(), (int)ring.size(), true));
+      c->model_bytes += (k0 + len - std::max(k0, 1)) * term_bytes;
+    }
     for (int q = 0; q < len; ++q) {
       const int k = k0 + q;
-      if (k >= 1) {
+      if (k >= 1 && ps.grid == 0) {
         launch_term<R, V>(c, tt,
                           poly_term<R, V>(c, pp, k, tpr, vec(k - 1), k >= 2 ? vec(k - 2) : nullptr,
                                           vec(k), true));
@@ -1870,21 +2035,30 @@ void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, 
     // outputs are ordered by degree: those that end before this window are done
     a.j0 = 0;
     while (a.j0 < m - 1 && (int)sp.w[a.j0].size() <= k0) ++a.j0;
-    a.init = k0 == 0 ? 0xffffffffu : 0u;
+    a.init = k0 == 0 ? 1 : 0;
     for (int j = 0; j < m; ++j)
       for (int q = 0; q < kCombineWindow; ++q)
         a.w[j][q] = q < len && k0 + q < (int)sp.w[j].size() ? sp.w[j][k0 + q] : 0.0;
-    if (m <= 4)
-      combine_kernel<R, 4><<<grid, 256, 0, c->stream>>>(a);
-    else if (m <= 8)
-      combine_kernel<R, 8><<<grid, 256, 0, c->stream>>>(a);
-    else
-      combine_kernel<R, 16><<<grid, 256, 0, c->stream>>>(a);
+    if constexpr (sizeof(R) == 8) {
+      if (m <= 4)
+        combine_kernel<R, 4><<<grid, 256, 0, c->stream>>>(a);
+      else if (m <= 8)
+        combine_kernel<R, 8><<<grid, 256, 0, c->stream>>>(a);
+      else
+        combine_kernel<R, 16><<<grid, 256, 0, c->stream>>>(a);
+    } else if (m <= 8) {
+      combine_mma_kernel<1><<<grid, 256, 0, c->stream>>>(a);
+    } else {
+      combine_mma_kernel<2><<<grid, 256, 0, c->stream>>>(a);
+    }
     TBPM_CK(cudaGetLastError());
     c->launches++;
     c->model_bytes += vb * (len + (m - a.j0) * (k0 == 0 ? 1 : 2));
   }
 }
+
+template <typename R>
+constexpr int most_steps = sizeof(R) == 8 ? 16 : 8;
 
 // Time steps per expansion and vectors per update for blocks of vb bytes.
 struct StepsShape {
@@ -1895,8 +2069,10 @@ struct StepsShape {
 // The largest shape whose states and ring, beside `other` bytes, fit the memory
 // that is free or held by the buffers they go into.  Model of a step of phase
 // pi/2 in passes over the block (time stepping: 57): 20 at (16, 16), 24 at
-// (8, 16), 27 at (8, 8), 36 at (4, 8).
-StepsShape steps_that_fit(size_t vb, size_t other, size_t held) {
+// (8, 16), 27 at (8, 8), 36 at (4, 8).  FP32 states take 8 at most: the 16 outputs'
+// FP64 products (with the conversions) then cost more than the terms they save
+// (57 energies' DC run: 162 us per step at 16).
+StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -1905,7 +2081,7 @@ StepsShape steps_that_fit(size_t vb, size_t other, size_t held) {
   const size_t reserve = (size_t)2 << 30;
   for (const StepsShape s : {StepsShape{16, 16}, StepsShape{8, 16}, StepsShape{8, 8},
                              StepsShape{4, 8}})
-    if (vb * (size_t)(s.m + s.window + 2) + other + reserve <= free_b + held) return s;
+    if (s.m <= m_max && vb * (size_t)(s.m + s.window + 2) + other + reserve <= free_b + held) return s;
   return StepsShape{};
 }
 
@@ -1924,7 +2100,8 @@ StepsShape steps_room(tbpm_ctx* c, const PolyPlan* pp, int ld, int ref_ld) {
   const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
   const size_t ref = (size_t)c->ham.n * ref_ld * 2 * sizeof(R);
   const StepsShape s =
-      steps_that_fit(vb, vb + ref, c->A.bytes + c->X.bytes + c->Y.bytes + c->wf0.bytes);
+      steps_that_fit(vb, vb + ref, c->A.bytes + c->X.bytes + c->Y.bytes + c->wf0.bytes,
+                     most_steps<R>);
   if (s.m > 0) c->A.ensure(vb * (size_t)(1 + s.window + s.m));
   return s;
 }
@@ -2063,12 +2240,6 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
 #ifndef TBPM_QE_MMA
 #define TBPM_QE_MMA 1  // quasi-eigenstate accumulation on mma.sync f64 (0: FMA kernel)
 #endif
-template <class K>
-void qe_smem_attr(K kernel, size_t bytes) {
-  // (a kernel's static shared memory counts towards the default 48 KB too)
-  if (bytes <= 40 * 1024) return;
-  TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-}
 template <typename R>
 void qe_accum_attr(size_t bytes) {
   qe_smem_attr(qe_accum_kernel<R>, bytes);
@@ -2140,43 +2311,58 @@ void dc_filter(tbpm_ctx* c, const PolyPlan& pp, int nb, const Pack<R, V>* W, int
   };
   const double term_bytes = matrix_bytes(c->ham) + 3.0 * (double)vb;
   C* qe = c->qe.as<C>();
-  const int rt = qe_mma_rows(nb);
+  const int rt = qe_filter_rows<R>(nb);
   const int64_t tiles = (n + rt - 1) / rt;
   const int groups = ((n_en + 7) / 8 + kQeMmaWarps * kQeMmaMT - 1) / (kQeMmaWarps * kQeMmaMT);
-  const dim3 qgrid((unsigned)std::min<int64_t>(tiles, (int64_t)num_sms(c->device) * 4),
+  const dim3 qgrid((unsigned)std::min<int64_t>(tiles, (int64_t)num_sms(c->device) * 2),
                    (unsigned)std::max(groups, 1));
-  const size_t qsmem = qe_filter_smem(nb);
+  const size_t qsmem = qe_filter_smem<R>(nb);
   qe_smem_attr(qe_filter_mma_kernel<R>, qsmem);
+  const PersistShape ps = persist_shape<R, V>(c, nb);
+  std::vector<Pack<R, V>*> ring(slots);
+  for (int q = 0; q < slots; ++q)
+    ring[q] = reinterpret_cast<Pack<R, V>*>(c->A.as<char>() + vb * q);
+  auto reduce_terms = [&](int k, int count, int grid) {  // terms k .. k + count - 1
+    const int64_t n_vals = (int64_t)count * nb * 2;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), grid, n_vals, sums + (int64_t)(k - 1) * nb * 2);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+  };
   int pend = 0;  // terms whose block partials wait for their reduction
-  FilterPtrs<R> win{};
-  int w0 = 0;  // first vector of the window
-  for (int k = 0; k <= last; ++k) {
-    if (k >= 1) {
+  for (int w0 = 0; w0 <= last; w0 += kFilterWindow) {
+    const int w1 = std::min(w0 + kFilterWindow - 1, last);
+    const int k_lo = std::max(w0, 1);
+    if (ps.grid > 0 && k_lo <= w1) {
+      ensure_partials(c, (size_t)kFilterWindow * nb * 2 * ps.grid);
+      PersistArgs<R, V> a =
+          persist_args<R, V>(c, pp.alpha, k_lo, w1, nb, W, ring.data(), slots, false);
+      a.k_dots = K;
+      a.partials = c->partials.as<double>();
+      launch_persist<false>(c, ps, a);
+      c->model_bytes += (w1 - k_lo + 1) * term_bytes;
+      if (k_lo <= K) reduce_terms(k_lo, std::min(w1, K) - k_lo + 1, ps.grid);
+    }
+    for (int k = k_lo; ps.grid == 0 && k <= w1; ++k) {
       TermArgs<R, V> a = poly_term<R, V>(c, pp, k, tpr, vec(k - 1), k >= 2 ? vec(k - 2) : nullptr,
                                          vec(k));
       if (k <= K) a.partials = c->partials.as<double>() + (int64_t)pend * per_term;
       launch_term<R, V>(c, tt, a);
       c->model_bytes += term_bytes;
       if (k <= K && (++pend == chunk || k == K)) {
-        const int64_t n_vals = (int64_t)pend * nb * 2;
-        reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-            c->partials.as<double>(), grid3, n_vals, sums + (int64_t)(k - pend) * nb * 2);
-        TBPM_CK(cudaGetLastError());
-        c->launches++;
+        reduce_terms(k - pend + 1, pend, grid3);
         pend = 0;
       }
     }
     if (n_en == 0) continue;
-    win.p[k - w0] = reinterpret_cast<const C*>(vec(k));
-    if (k - w0 + 1 == kFilterWindow || k == last) {
-      qe_filter_mma_kernel<R><<<qgrid, kQeMmaWarps * 32, qsmem, c->stream>>>(
-          qe, n, n_en, nb, win, k - w0 + 1, coef + (int64_t)w0 * n_en, w0 == 0 ? 1 : 0);
-      TBPM_CK(cudaGetLastError());
-      c->launches++;
-      c->model_bytes += (double)n * n_en * nb * sizeof(C) * (w0 == 0 ? 1 : 2) +
-                        (double)(k - w0 + 1) * (double)vb;
-      w0 = k + 1;
-    }
+    FilterPtrs<R> win{};
+    for (int k = w0; k <= w1; ++k) win.p[k - w0] = reinterpret_cast<const C*>(vec(k));
+    qe_filter_mma_kernel<R><<<qgrid, kQeMmaWarps * 32, qsmem, c->stream>>>(
+        qe, n, n_en, nb, win, w1 - w0 + 1, coef + (int64_t)w0 * n_en, w0 == 0 ? 1 : 0);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    c->model_bytes += (double)n * n_en * nb * sizeof(C) * (w0 == 0 ? 1 : 2) +
+                      (double)(w1 - w0 + 1) * (double)vb;
   }
   const bool check = chk_step >= 2 && chk_step <= T;
   if (!dos && !check) return;
@@ -2408,7 +2594,8 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   // several steps per expansion where their blocks fit beside QE
   StepsShape shape;
   if (pp) {
-    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes);
+    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes,
+                           most_steps<R>);
     if (shape.m > 0) {
       c->A.ensure(vb * (size_t)(shape.m + shape.window + 2 + T2));
     } else {
@@ -2585,8 +2772,10 @@ __global__ void scatter_sites_kernel(const int32_t* sites, const double2* vals, 
   v[sites[i]] = o;
 }
 
-// Slices of the N rows for the split-K contraction: enough blocks for about
-// four per SM, slices a multiple of the 16-row step.
+// Slices of the N rows for the split-K contraction: at most four blocks per SM
+// (two waves of the two that are resident; one block more would start a third:
+// 25 slices of 24 tiles took 2.5 ms where 24 take 1.75 ms), slices a multiple of the
+// 16-row step.
 struct PqSplit {
   int slices;
   int64_t rows;
@@ -2594,7 +2783,7 @@ struct PqSplit {
 
 PqSplit pq_split(const tbpm_ctx* c, int64_t n, int m, int nk) {
   const int64_t tiles = (int64_t)((m + kPqTile - 1) / kPqTile) * ((nk + kPqTile - 1) / kPqTile);
-  const int64_t want = std::max<int64_t>(1, (4 * (int64_t)num_sms(c->device) + tiles - 1) / tiles);
+  const int64_t want = std::max<int64_t>(1, 4 * (int64_t)num_sms(c->device) / tiles);
   const int64_t max_slices = std::max<int64_t>(1, n / (16 * kPqK));
   const int64_t sl = std::min(want, max_slices);
   int64_t rows = (n + sl - 1) / sl;
@@ -2738,6 +2927,51 @@ void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
 
 // ---- psi(t) -------------------------------------------------------------------
 
+// Two staging buffers of a call and the stream their copies run on.
+struct FrameCopies {
+  tbpm_ctx* c;
+  size_t bytes;
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ready = nullptr;
+  int slot = 0;
+  double* host = nullptr;  // destination of the staged frame, null: none
+
+  FrameCopies(tbpm_ctx* ctx, size_t n) : c(ctx), bytes((n + 255) & ~(size_t)255) {
+    c->stage.ensure(2 * bytes);
+    TBPM_CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    const cudaError_t e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      cudaStreamDestroy(stream);
+      throw_cuda(e, "cudaEventCreateWithFlags");
+    }
+  }
+  ~FrameCopies() {
+    cudaStreamSynchronize(stream);
+    cudaEventDestroy(ready);
+    cudaStreamDestroy(stream);
+  }
+  FrameCopies(const FrameCopies&) = delete;
+  FrameCopies& operator=(const FrameCopies&) = delete;
+
+  double2* next() { return reinterpret_cast<double2*>(c->stage.as<char>() + slot * bytes); }
+  // next() has been filled on the context stream; its copy goes to dst at flush()
+  void stage(double* dst) {
+    TBPM_CK(cudaEventRecord(ready, c->stream));
+    host = dst;
+  }
+  // Copies the staged frame, complete when this returns (the other buffer is
+  // then free for the next frame).
+  void flush() {
+    if (!host) return;
+    double* dst = host;
+    host = nullptr;
+    TBPM_CK(cudaStreamWaitEvent(stream, ready, 0));
+    TBPM_CK(cudaMemcpyAsync(dst, next(), (size_t)c->ham.n * 16, cudaMemcpyDeviceToHost, stream));
+    TBPM_CK(cudaStreamSynchronize(stream));
+    slot ^= 1;
+  }
+};
+
 template <typename R>
 void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, const double* psi0, const int32_t* time_log,
                int n_log, int n_timestep, int chk_step, double chk_thr, double* psi_t) {
@@ -2786,10 +3020,20 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, c
     }
     done = target;
   };
+  // A logged state is converted into one of two staging buffers; its copy to the
+  // host (which blocks the calling thread) is issued on a second stream after
+  // the next propagation has been enqueued, so that both run at the same time.
+  // (Five frames of 8 MB: 25 ms of which 15 were on the device.)
+  FrameCopies frames(c, (size_t)n * 16);
   for (int t = 1; t <= n_timestep; ++t) {
     if (ptr < n_log && time_log[ptr] == t - 1) {
       advance_to(t - 1);
-      download_states<R>(c, A, 1, 1, 0, psi_t + 2 * (size_t)ptr * n);
+      frames.flush();
+      deinterleave_kernel<R><<<blocks_for(n, 256), 256, 0, c->stream>>>(
+          reinterpret_cast<const typename Cx<R>::t*>(A), 1, n, 1, 0, frames.next());
+      TBPM_CK(cudaGetLastError());
+      c->launches++;
+      frames.stage(psi_t + 2 * (size_t)ptr * n);
       if (ptr < n_log - 1) ++ptr;
       else ptr = n_log;  // further matches impossible (sorted, unique)
     }
@@ -2802,9 +3046,16 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, c
   }
   if (ptr < n_log && time_log[ptr] == n_timestep) {
     advance_to(n_timestep);
-    download_states<R>(c, A, 1, 1, 0, psi_t + 2 * (size_t)ptr * n);
+    frames.flush();
+    deinterleave_kernel<R><<<blocks_for(n, 256), 256, 0, c->stream>>>(
+        reinterpret_cast<const typename Cx<R>::t*>(A), 1, n, 1, 0, frames.next());
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+    frames.stage(psi_t + 2 * (size_t)ptr * n);
   }
+  frames.flush();
   TBPM_CK(cudaStreamSynchronize(c->stream));
+  check_status(c);
 }
 
 // ---- Fermi coefficients (funcs.f90:60-123) --------------------------------------

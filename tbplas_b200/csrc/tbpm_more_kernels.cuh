@@ -318,8 +318,17 @@ __device__ __forceinline__ double haydock_grid_sum(const double* p, int n, doubl
   return t;
 }
 
-__device__ __forceinline__ double2 ldcg_c(const double2* p) { return __ldcg(p); }
-__device__ __forceinline__ float2 ldcg_c(const float2* p) { return __ldcg(p); }
+// Ordinary loads of vectors that other SMs wrote before the last grid barrier
+// (volatile: not moved across it, and not through the read-only path); rows that
+// neighbours share hit L1.
+__device__ __forceinline__ double2 ld_c(const double2* p) {
+  const Pack<double, 1> v = ld_pack(reinterpret_cast<const Pack<double, 1>*>(p));
+  return make_double2(v.v[0], v.v[1]);
+}
+__device__ __forceinline__ float2 ld_c(const float2* p) {
+  const Pack<float, 1> v = ld_pack(reinterpret_cast<const Pack<float, 1>*>(p));
+  return make_float2(v.v[0], v.v[1]);
+}
 
 // The whole recursion (propagation.f90:85-155) in one cooperative launch.  With
 // w the unnormalised vector and v = w / b_{d-1}:
@@ -348,7 +357,7 @@ __global__ void __launch_bounds__(kHaydockThreads, 1)
     double cr = 0.0, ci = 0.0;
     for (int64_t r = r0; r < k.n_rows; r += stride) {
       const int j0 = __ldg(k.indptr + r), j1 = __ldg(k.indptr + r + 1);
-      const C own = ldcg_c(w + r);
+      const C own = ld_c(w + r);
       double vr = 0.0, vi = 0.0;
       if (k.diag) {
         const C g = ldg_c(k.diag + r);
@@ -358,7 +367,7 @@ __global__ void __launch_bounds__(kHaydockThreads, 1)
 #pragma unroll 4
       for (int j = j0; j < j1; ++j) {
         const C h = ldg_c(k.hop + j);
-        const C x = ldcg_c(w + __ldg(k.indices + j));
+        const C x = ld_c(w + __ldg(k.indices + j));
         vr += (double)h.x * (double)x.x - (double)h.y * (double)x.y;
         vi += (double)h.x * (double)x.y + (double)h.y * (double)x.x;
       }
@@ -382,12 +391,12 @@ __global__ void __launch_bounds__(kHaydockThreads, 1)
     const double ai = haydock_grid_sum(k.partials + gridDim.x, gridDim.x, &bcast);
     double nn = 0.0;
     for (int64_t r = r0; r < k.n_rows; r += stride) {
-      const C x = ldcg_c(w + r), z = ldcg_c(k.y + r);
+      const C x = ld_c(w + r), z = ld_c(k.y + r);
       const double xr = s * (double)x.x, xi = s * (double)x.y;
       double vr = (double)z.x - (ar * xr - ai * xi);
       double vi = (double)z.y - (ar * xi + ai * xr);
       if (d > 0) {
-        const C p = ldcg_c(w_prev + r);
+        const C p = ld_c(w_prev + r);
         vr -= b_prev * (s_prev * (double)p.x);
         vi -= b_prev * (s_prev * (double)p.y);
       }

@@ -19,6 +19,8 @@
 //  moment_density_kernel  moments -> weights rho_j of Gauss-Chebyshev nodes.
 //  moment_curve_kernel    C(t) = sum_j P(x_j)^t rho_j, and the norms.
 //  cheb_persist_kernel    all terms of a small problem in one launch.
+//  cheb_cluster_kernel    the same for a tiny one, in the shared memory of one
+//                         cluster.
 //  seg_dots_kernel        the two products per (segment, state) of packed samples.
 //  filter_values_kernel,  the quasi-eigenstates' energy filters on the nodes and
 //  filter_coef_kernel     their Chebyshev coefficients.
@@ -237,6 +239,8 @@ static __global__ void __launch_bounds__(128) moment_curve_kernel(const PolyNode
 
 // ---- all terms of a small problem in one launch -----------------------------
 
+constexpr int kPersistRing = 34;  // most vectors kept
+
 template <typename R, int V>
 struct PersistArgs {
   const int32_t* indptr;
@@ -245,32 +249,53 @@ struct PersistArgs {
   const typename Cx<R>::t* diag;
   int64_t n_rows;
   int tpr;
-  Pack<R, V>* p0;    // p_0 on entry; overwritten by p_2, p_4, ...
-  Pack<R, V>* p1;    // receives p_1, p_3, ...
-  double alpha;      // 2 / a
-  int n_terms;       // K
-  double* partials;  // [((k-1)*ld*2 + col*2 + q) * gridDim.x + block]
-  unsigned int* bar;     // grid barrier, zero on entry
+  const Pack<R, V>* p0;          // p_0
+  Pack<R, V>* ring[kPersistRing];  // p_k, k >= 1, is ring[k % slots]
+  int slots;
+  double alpha;       // 2 / a
+  int turn;           // 1: the vectors times (-i)^k
+  int k0, k1;         // terms k0 <= k <= k1 of this launch
+  // ACC kernels: the weighted sum of the vectors is folded into acc every third
+  // term (k = 2, 5, 8, ...; k0 is 1), weights w[set*n_w + k]
+  Pack<R, V>* acc;
+  const double* w;
+  int n_w;
+  unsigned long long set_mask;  // columns that use set 1
+  int k_dots;         // products are formed for k <= k_dots
+  double* partials;   // [((k-k0)*ld*2 + col*2 + q) * gridDim.x + block]
+  unsigned int* bar;      // grid barrier, zero on entry
   unsigned int* status;  // bit 0: a bounded wait ran out
 };
 
 // most threads of a block: 128 registers a thread for 32-byte packs, 102 for
 // 16-byte ones, 64 for 8-byte ones
+#ifndef TBPM_PERSIST_T16
+#define TBPM_PERSIST_T16 768
+#endif
 template <typename R, int V>
-constexpr int kPersistThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? 640 : 1024);
-constexpr int kPersistDeg = 4;  // row entries whose gathers are issued together
+constexpr int kPersistThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? TBPM_PERSIST_T16 : 1024);
+// the same of the cluster kernel, whose items take more registers
+template <typename R, int V>
+constexpr int kClusterThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? 640 : 768);
+constexpr int kPersistDeg = 3;  // row entries whose gathers are issued together
+constexpr int kPersistBatch = 4;  // terms whose products are reduced together
 constexpr unsigned long long kPersistWaitNs = 2000000000ull;  // 2 s per wait
 
-// The moments' terms p_k = (2/a) H p_{k-1} - p_{k-2}, k = 1..K, of a problem
-// whose vectors stay in L2, under one cooperative launch: a grid barrier per
+// The terms p_k = (2/a) H p_{k-1} - p_{k-2}, k0 <= k <= k1, of a problem whose
+// vectors stay in L2, under one cooperative launch: a grid barrier per
 // term instead of a launch per term.  What bounds it is latency, not bytes: a
 // barrier round trip and one gather.  The matrix entries of a thread's next
 // item (a row's pack of V columns; up to kPersistDeg entries) are loaded as soon
 // as those of the current item are used, so the first item's are in registers
-// when the barrier opens.  p_k is read with L2-only loads, as other SMs wrote it
-// in this launch.  The block's two products per column are reduced after its
-// arrival on the barrier, while the other blocks arrive.
-template <typename R, int V>
+// when the barrier opens.  p_k, which other SMs wrote in this launch, is read by
+// ordinary loads: the acquire and the fence after the barrier make the writes
+// visible, and neighbouring rows of a tile then hit L1.  A term's two products per
+// column stay in shared memory per thread and are reduced every kPersistBatch terms, one
+// warp per product: the reduction's barriers were as long as the grid's.
+//
+// ACC: expansions (Fermi operators, psi_t's jumps) instead of moments; the sums
+// are formed in FP64 as in the launched terms, so states are bit-identical.
+template <typename R, int V, bool ACC>
 __global__ void __launch_bounds__((kPersistThreads<R, V>), 1)
     cheb_persist_kernel(const __grid_constant__ PersistArgs<R, V> a) {
   using C = typename Cx<R>::t;
@@ -310,9 +335,21 @@ __global__ void __launch_bounds__((kPersistThreads<R, V>), 1)
   if (any) load(r_first);
   __syncthreads();
   const R alpha2 = (R)a.alpha, alpha1 = (R)(0.5 * a.alpha);
-  for (int k = 1; k <= a.n_terms; ++k) {
-    const Pack<R, V>* src = (k & 1) ? a.p0 : a.p1;
-    Pack<R, V>* dst = (k & 1) ? a.p1 : a.p0;
+  const R sgn = a.turn ? (R)1 : (R)-1;  // of p_{k-2}
+  for (int k = a.k0; k <= a.k1; ++k) {
+    const Pack<R, V>* src = k == 1 ? a.p0 : a.ring[(k - 1) % a.slots];
+    const Pack<R, V>* prv = k == 2 ? a.p0 : a.ring[(k + a.slots - 2) % a.slots];
+    Pack<R, V>* dst = a.ring[k % a.slots];
+    const bool dots = !ACC && k <= a.k_dots;
+    const bool flush = ACC && k % 3 == 2;
+    double fw[2][3];
+    if (flush) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        fw[0][q] = __ldg(a.w + k - 2 + q);
+        fw[1][q] = __ldg(a.w + a.n_w + k - 2 + q);
+      }
+    }
     const R al = k == 1 ? alpha1 : alpha2;
     double nrm[V], cre[V];
 #pragma unroll
@@ -323,11 +360,11 @@ __global__ void __launch_bounds__((kPersistThreads<R, V>), 1)
         Pack<R, V> x[kPersistDeg];
 #pragma unroll
         for (int u = 0; u < kPersistDeg; ++u)
-          if (c[u] >= 0) x[u] = ldcg_pack(src + (int64_t)c[u] * tpr + lane);
-        const Pack<R, V> own = ldcg_pack(src + e);
+          if (c[u] >= 0) x[u] = ld_pack(src + (int64_t)c[u] * tpr + lane);
+        const Pack<R, V> own = ld_pack(src + e);
         Pack<R, V> pm2;
         if (k >= 2) {
-          pm2 = ldcg_pack(dst + e);
+          pm2 = ld_pack(prv + e);
         } else {
 #pragma unroll
           for (int q = 0; q < 2 * V; ++q) pm2.v[q] = (R)0;
@@ -347,46 +384,85 @@ __global__ void __launch_bounds__((kPersistThreads<R, V>), 1)
               sim[v] = fma(h[u].x, x[u].v[2 * v + 1], fma(h[u].y, x[u].v[2 * v], sim[v]));
             }
           }
-        for (int j = j0 + kPersistDeg; j < j1; ++j) {
-          const C hj = ldg_c(a.hop + j);
-          const Pack<R, V> xj = ldcg_pack(src + (int64_t)__ldg(a.indices + j) * tpr + lane);
+        for (int jb = j0 + kPersistDeg; jb < j1; jb += kPersistDeg) {  // longer rows
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            sre[v] = fma(hj.x, xj.v[2 * v], fma(-hj.y, xj.v[2 * v + 1], sre[v]));
-            sim[v] = fma(hj.x, xj.v[2 * v + 1], fma(hj.y, xj.v[2 * v], sim[v]));
-          }
+          for (int u = 0; u < kPersistDeg; ++u)
+            if (jb + u < j1) {
+              h[u] = ldg_c(a.hop + jb + u);
+              x[u] = ld_pack(src + (int64_t)__ldg(a.indices + jb + u) * tpr + lane);
+            }
+#pragma unroll
+          for (int u = 0; u < kPersistDeg; ++u)
+            if (jb + u < j1) {
+#pragma unroll
+              for (int v = 0; v < V; ++v) {
+                sre[v] = fma(h[u].x, x[u].v[2 * v], fma(-h[u].y, x[u].v[2 * v + 1], sre[v]));
+                sim[v] = fma(h[u].x, x[u].v[2 * v + 1], fma(h[u].y, x[u].v[2 * v], sim[v]));
+              }
+            }
         }
         load(r + stride < n ? r + stride : r_first);
         Pack<R, V> pk;
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          pk.v[2 * v] = fma(al, sre[v], -pm2.v[2 * v]);
-          pk.v[2 * v + 1] = fma(al, sim[v], -pm2.v[2 * v + 1]);
-          const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
-          nrm[v] += xr * xr + xi * xi;
-          cre[v] += xr * (double)own.v[2 * v] + xi * (double)own.v[2 * v + 1];
+          const R br = a.turn ? sim[v] : sre[v], bi = a.turn ? -sre[v] : sim[v];
+          pk.v[2 * v] = fma(al, br, sgn * pm2.v[2 * v]);
+          pk.v[2 * v + 1] = fma(al, bi, sgn * pm2.v[2 * v + 1]);
+          if (!ACC) {
+            const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
+            nrm[v] += xr * xr + xi * xi;
+            cre[v] += xr * (double)own.v[2 * v] + xi * (double)own.v[2 * v + 1];
+          }
+        }
+        if (flush) {
+          Pack<R, V> acc;
+          if (k > 2) acc = ld_pack(a.acc + e);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const int set = (int)(a.set_mask >> (lane * V + v)) & 1;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const int i = 2 * v + q;
+              double sum = k > 2 ? (double)acc.v[i] : 0.0;
+              sum += (set ? fw[1][0] : fw[0][0]) * (double)pm2.v[i];
+              sum += (set ? fw[1][1] : fw[0][1]) * (double)own.v[i];
+              sum += (set ? fw[1][2] : fw[0][2]) * (double)pk.v[i];
+              acc.v[i] = (R)sum;
+            }
+          }
+          stwb_pack(a.acc + e, acc);
         }
         stwb_pack(dst + e, pk);
       }
     }
-    // arrive, reduce this block's products, then wait for the others
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0 && k < a.n_terms) atomicAdd(a.bar, 1u);
-    if (in) {
+    // the products of this term: psm[slot of the batch][column value][thread row]
+    const int bs = (k - a.k0) % kPersistBatch;
+    if (dots && in) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        psm[slot * width + (lane * V + v) * 2] = nrm[v];
-        psm[slot * width + (lane * V + v) * 2 + 1] = cre[v];
+        psm[(bs * width + (lane * V + v) * 2) * rpp + slot] = nrm[v];
+        psm[(bs * width + (lane * V + v) * 2 + 1) * rpp + slot] = cre[v];
       }
     }
+    // arrive, then reduce a full batch of products while the others arrive
+    __threadfence();
     __syncthreads();
-    tree_reduce_slots(psm, rpp, width, slot, lane, tpr);
-    for (int q = threadIdx.x; q < width; q += blockDim.x)
-      a.partials[((int64_t)(k - 1) * ld2 + q) * gridDim.x + blockIdx.x] = psm[q];
-    if (k == a.n_terms) break;
+    if (threadIdx.x == 0 && k < a.k1) atomicAdd(a.bar, 1u);
+    const int k_end = min(a.k1, a.k_dots);  // last term with products
+    if (dots && (bs == kPersistBatch - 1 || k == k_end)) {
+      const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
+      const int full = blockDim.x >> 5;  // a partial last warp takes no part
+      const int64_t k_first = k - bs - a.k0;
+      for (int q = warp < full ? warp : (bs + 1) * width; q < (bs + 1) * width; q += full) {
+        double t = 0.0;
+        for (int i = wl; i < rpp; i += 32) t += psm[q * rpp + i];
+        for (int sft = 16; sft > 0; sft >>= 1) t += __shfl_xor_sync(0xffffffffu, t, sft);
+        if (wl == 0) a.partials[(k_first * ld2 + q) * gridDim.x + blockIdx.x] = t;
+      }
+    }
+    if (k == a.k1) break;
     if (threadIdx.x == 0) {
-      const unsigned int want = (unsigned int)k * gridDim.x;
+      const unsigned int want = (unsigned int)(k - a.k0 + 1) * gridDim.x;
       unsigned long long t0 = 0;
       for (unsigned int spin = 0;; ++spin) {
         unsigned int seen;
@@ -407,6 +483,206 @@ __global__ void __launch_bounds__((kPersistThreads<R, V>), 1)
     }
     __syncthreads();
     if (stop) break;
+  }
+}
+
+// ---- tiny problems in the shared memory of one cluster -------------------------
+
+template <typename R, int V>
+struct ClusterArgs {
+  const int32_t* indptr;
+  const int32_t* indices;
+  const typename Cx<R>::t* hop;
+  const typename Cx<R>::t* diag;
+  int n_rows;
+  int tpr;
+  const Pack<R, V>* p0;
+  double alpha;        // 2 / a
+  int n_terms;
+  int rows;            // rows per block: block q owns rows [q*rows, (q+1)*rows)
+  unsigned int magic;  // ceil(2^32 / rows): c / rows = umulhi(c, magic) for c*rows < 2^32
+  double* partials;    // [((k-1)*ld*2 + col*2 + q) * gridDim.x + block]
+};
+
+constexpr int kClusterBlocks = 16;
+constexpr int kClusterItems = 2;  // most items of a thread (their matrix rows stay in registers)
+
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Arrival and wait of every thread of the cluster, releasing its writes.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// 16 bytes (8 for one complex64) of a block of the cluster
+__device__ __forceinline__ void cluster_ld(uint32_t a, double* v) {
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_ld(uint32_t a, float* v) {
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_ld4(uint32_t a, float* v) {
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+               : "r"(a)
+               : "memory");
+}
+template <typename R, int V>
+__device__ __forceinline__ Pack<R, V> cluster_ld_pack(uint32_t a) {
+  Pack<R, V> p;
+  if constexpr (sizeof(R) == 4 && V >= 2) {
+#pragma unroll
+    for (int q = 0; q < V / 2; ++q) cluster_ld4(a + 16 * q, p.v + 4 * q);
+  } else {
+#pragma unroll
+    for (int q = 0; q < V; ++q) cluster_ld(a + 2 * sizeof(R) * q, p.v + 2 * q);
+  }
+  return p;
+}
+
+// The moments' terms of a problem whose two vectors fit the shared memory of one
+// cluster of 16 blocks.  A term of cheb_persist_kernel is a grid barrier through L2
+// and a gather from L2; here it is the hardware barrier of the cluster and a
+// gather from distributed shared memory, on 16 SMs instead of 148, so it is
+// the better one while a thread has few items: their matrix rows then stay in
+// registers.
+template <typename R, int V>
+__global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
+    cheb_cluster_kernel(const __grid_constant__ ClusterArgs<R, V> a) {
+  using C = typename Cx<R>::t;
+  extern __shared__ __align__(128) char csm[];
+  const int tpr = a.tpr, rows = a.rows;
+  const int slot = threadIdx.x / tpr;
+  const int lane = threadIdx.x - slot * tpr;
+  const int rpp = blockDim.x / tpr;
+  const int r_base = blockIdx.x * rows;
+  const int n_own = max(0, min(rows, a.n_rows - r_base));
+  const int vec = rows * tpr;  // packs of a vector per block
+  Pack<R, V>* buf = reinterpret_cast<Pack<R, V>*>(csm);  // p_even | p_odd
+  double* psm = reinterpret_cast<double*>(csm + 2 * (size_t)vec * sizeof(Pack<R, V>));
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(csm);
+  const uint32_t odd = (uint32_t)(vec * sizeof(Pack<R, V>));
+  const int width = tpr * V * 2;
+  const bool any = slot < rpp && slot < n_own;
+  for (int q = threadIdx.x; q < n_own * tpr; q += blockDim.x)
+    buf[q] = a.p0[(int64_t)r_base * tpr + q];
+  // matrix entries of the thread's items; ca: address of a neighbour in p_even
+  constexpr int NI = kClusterItems;
+  int j0[NI], j1[NI];
+  uint32_t ca[NI][kPersistDeg];
+  C h[NI][kPersistDeg], d[NI];
+  auto neighbour = [&](int c) {
+    const uint32_t q = __umulhi((uint32_t)c, a.magic);
+    const uint32_t l = (uint32_t)c - q * (uint32_t)rows;
+    return cluster_map(base + (l * (uint32_t)tpr + (uint32_t)lane) * (uint32_t)sizeof(Pack<R, V>),
+                       q);
+  };
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int r = slot + i * rpp;
+    j0[i] = j1[i] = 0;
+    d[i].x = d[i].y = (R)0;
+    if (any && r < n_own) {
+      j0[i] = __ldg(a.indptr + r_base + r);
+      j1[i] = __ldg(a.indptr + r_base + r + 1);
+      if (a.diag) d[i] = ldg_c(a.diag + r_base + r);
+    }
+#pragma unroll
+    for (int u = 0; u < kPersistDeg; ++u)
+      if (j0[i] + u < j1[i]) {
+        ca[i][u] = neighbour(__ldg(a.indices + j0[i] + u));
+        h[i][u] = ldg_c(a.hop + j0[i] + u);
+      }
+  }
+  cluster_sync();
+  const R alpha2 = (R)a.alpha, alpha1 = (R)(0.5 * a.alpha);
+  for (int k = 1; k <= a.n_terms; ++k) {
+    const uint32_t so = (k & 1) ? 0u : odd;  // p_{k-1}
+    const Pack<R, V>* src = buf + ((k & 1) ? 0 : vec);
+    Pack<R, V>* dst = buf + ((k & 1) ? vec : 0);
+    const R al = k == 1 ? alpha1 : alpha2;
+    double nrm[V], cre[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) nrm[v] = cre[v] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int r = slot + i * rpp;
+      if (any && r < n_own) {
+        const int e = r * tpr + lane;
+        Pack<R, V> x[kPersistDeg];
+#pragma unroll
+        for (int u = 0; u < kPersistDeg; ++u)
+          if (j0[i] + u < j1[i]) x[u] = cluster_ld_pack<R, V>(ca[i][u] + so);
+        const Pack<R, V> own = src[e];
+        Pack<R, V> pm2;
+        if (k >= 2) {
+          pm2 = dst[e];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 2 * V; ++q) pm2.v[q] = (R)0;
+        }
+        R sre[V], sim[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          sre[v] = d[i].x * own.v[2 * v] - d[i].y * own.v[2 * v + 1];
+          sim[v] = d[i].x * own.v[2 * v + 1] + d[i].y * own.v[2 * v];
+        }
+#pragma unroll
+        for (int u = 0; u < kPersistDeg; ++u)
+          if (j0[i] + u < j1[i]) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              sre[v] = fma(h[i][u].x, x[u].v[2 * v], fma(-h[i][u].y, x[u].v[2 * v + 1], sre[v]));
+              sim[v] = fma(h[i][u].x, x[u].v[2 * v + 1], fma(h[i][u].y, x[u].v[2 * v], sim[v]));
+            }
+          }
+        for (int j = j0[i] + kPersistDeg; j < j1[i]; ++j) {
+          const C hj = ldg_c(a.hop + j);
+          const Pack<R, V> xj = cluster_ld_pack<R, V>(neighbour(__ldg(a.indices + j)) + so);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            sre[v] = fma(hj.x, xj.v[2 * v], fma(-hj.y, xj.v[2 * v + 1], sre[v]));
+            sim[v] = fma(hj.x, xj.v[2 * v + 1], fma(hj.y, xj.v[2 * v], sim[v]));
+          }
+        }
+        Pack<R, V> pk;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          pk.v[2 * v] = fma(al, sre[v], -pm2.v[2 * v]);
+          pk.v[2 * v + 1] = fma(al, sim[v], -pm2.v[2 * v + 1]);
+          const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
+          nrm[v] += xr * xr + xi * xi;
+          cre[v] += xr * (double)own.v[2 * v] + xi * (double)own.v[2 * v + 1];
+        }
+        dst[e] = pk;
+      }
+    }
+    // products per thread, reduced in batches as in cheb_persist_kernel
+    const int bs = (k - 1) % kPersistBatch;
+    if (slot < rpp) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        psm[(bs * width + (lane * V + v) * 2) * rpp + slot] = nrm[v];
+        psm[(bs * width + (lane * V + v) * 2 + 1) * rpp + slot] = cre[v];
+      }
+    }
+    cluster_sync();
+    if (bs == kPersistBatch - 1 || k == a.n_terms) {
+      const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
+      const int full = blockDim.x >> 5;  // a partial last warp takes no part
+      const int64_t k_first = k - 1 - bs;
+      for (int q = warp < full ? warp : (bs + 1) * width; q < (bs + 1) * width; q += full) {
+        double t = 0.0;
+        for (int i = wl; i < rpp; i += 32) t += psm[q * rpp + i];
+        for (int sft = 16; sft > 0; sft >>= 1) t += __shfl_xor_sync(0xffffffffu, t, sft);
+        if (wl == 0) a.partials[(k_first * width + q) * gridDim.x + blockIdx.x] = t;
+      }
+      __syncthreads();  // the batch's slots are free again
+    }
   }
 }
 
@@ -549,12 +825,24 @@ struct FilterPtrs {
   const typename Cx<R>::t* p[kFilterWindow];
 };
 
-// Shared memory of qe_filter_mma_kernel: the window's values of a tile,
-// [tau][pair], rows padded by 4 pairs (64 bytes), so that the four tau of a
-// fragment load lie in different banks.
-constexpr int kFilterPad = 4;
+// (row, state) pairs per staged tile of qe_filter_mma_kernel: 32 KB a buffer
+template <typename R>
+constexpr int kFilterPairs = sizeof(R) == 8 ? 64 : 128;
+// Rows per tile: about that many pairs, rows * nb a multiple of 4.
+template <typename R>
+__host__ __device__ constexpr int qe_filter_rows(int nb) {
+  const int q = nb % 4 == 0 ? 1 : (nb % 2 == 0 ? 2 : 4);  // rows that make whole 8-column tiles
+  const int r = (kFilterPairs<R> + nb - 1) / nb;
+  return (r + q - 1) / q * q;
+}
+// Shared memory: two buffers of the window's values of a tile, [tau][pair], the
+// pairs padded by 64 bytes, so that the four tau of a fragment load lie in
+// different banks.
+template <typename R>
+constexpr int kFilterPad = sizeof(R) == 8 ? 4 : 8;
+template <typename R>
 __host__ __device__ constexpr size_t qe_filter_smem(int nb) {
-  return (size_t)kFilterWindow * (qe_mma_rows(nb) * nb + kFilterPad) * sizeof(double2);
+  return 2 * (size_t)kFilterWindow * (qe_filter_rows<R>(nb) * nb + kFilterPad<R>) * 2 * sizeof(R);
 }
 
 // QE[r][i][b] (+)= sum_{tau < T} c[tau][i] p_tau[r][b], c real: per tile of
@@ -562,17 +850,22 @@ __host__ __device__ constexpr size_t qe_filter_smem(int nb) {
 // with the fragments and the split over warps of qe_accum_mma_kernel (whose
 // +/- windows need 2 x 16 coefficients for 16 steps).  A window of 32 vectors
 // per pass over QE: at 16 the pass over QE (32 bytes a complex128 element
-// against 32 FMAs) was the longer side.  A warp's QE elements of the next
-// column tile are loaded before the products of the current one.
+// against 32 FMAs) was the longer side.  The next tile's values are on their
+// way into the other buffer (cp.async) during the products, and a warp's QE
+// elements of the next column tile are loaded before the products of the
+// current one: one barrier per tile.  (Staged by plain loads in tiles of 32
+// pairs: 57 energies x 4 FP32 states of 307,200 rows took 843 us per pass, 1.3
+// TB/s; 7 energies x 2 FP64 states of 192,640 rows 189 us.)
 template <typename R>
 __global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_filter_mma_kernel(
     typename Cx<R>::t* qe, int64_t n_rows, int n_en, int nb,
     const __grid_constant__ FilterPtrs<R> win, int T, const double* coef, int init) {
   using C = typename Cx<R>::t;
   extern __shared__ double2 qsm[];
-  const int RT = qe_mma_rows(nb);
+  const int RT = qe_filter_rows<R>(nb);
   const int P = RT * nb;  // pairs of a tile; P % 4 == 0
-  const int PS = P + kFilterPad;
+  const int PS = P + kFilterPad<R>;
+  C* buf[2] = {reinterpret_cast<C*>(qsm), reinterpret_cast<C*>(qsm) + kFilterWindow * PS};
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int n_mt = (n_en + 7) / 8;
@@ -593,47 +886,68 @@ __global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_filter_mma_kernel(
       afr[m][st] = i < n_en && tau < T ? coef[(int64_t)tau * n_en + i] : 0.0;
     }
   }
-  for (int64_t r0 = (int64_t)blockIdx.x * RT; r0 < n_rows; r0 += (int64_t)gridDim.x * RT) {
+  // vectors past the window (tau >= T) are zeroed once; their coefficients are
+  // zero too, but what lies in shared memory need not be finite
+  for (int q = threadIdx.x; q < 2 * kFilterWindow * PS; q += blockDim.x) {
+    C z;
+    z.x = z.y = (R)0;
+    buf[0][q] = z;
+  }
+  __syncthreads();
+  auto issue = [&](int64_t r0, C* dst) {
+    if (r0 < n_rows) {
+      const int np = (int)min((int64_t)RT, n_rows - r0) * nb;
+      // a warp per vector: consecutive lanes copy consecutive pairs
+      for (int tau = warp; tau < T; tau += kQeMmaWarps) {
+        const C* src = win.p[tau] + r0 * nb;
+        for (int q = lane; q < np; q += 32) qe_cp_async(dst + tau * PS + q, src + q);
+      }
+    }
+    qe_cp_commit();
+  };
+  const int64_t r_first = (int64_t)blockIdx.x * RT, r_step = (int64_t)gridDim.x * RT;
+  issue(r_first, buf[0]);
+  int cur = 0;
+  for (int64_t r0 = r_first; r0 < n_rows; r0 += r_step, cur ^= 1) {
     const int nr = (int)min((int64_t)RT, n_rows - r0);
     const int np = nr * nb;  // pairs in range
+    C* base = qe + r0 * n_en * nb;
+    // offset of the lane's element of energy tile 0 in the rows of this tile
+    auto at = [&](int pc) {
+      const int rr = pc / nb;
+      return (rr * n_en + mt0 * 8 + g) * nb + (pc - rr * nb);
+    };
     auto load_c = [&](int nt, C* v) {
       const int pc = 4 * nt + t;
-      const int rr = pc / nb, bb = pc - rr * nb;
+      const int o = at(pc);
 #pragma unroll
       for (int m = 0; m < kQeMmaMT; ++m) {
-        const int i = (mt0 + m) * 8 + g;
         v[m].x = v[m].y = (R)0;
-        if (!init && nt < P / 4 && pc < np && i < n_en)
-          v[m] = qe[((r0 + rr) * n_en + i) * nb + bb];
+        if (!init && pc < np && (mt0 + m) * 8 + g < n_en) v[m] = base[o + 8 * m * nb];
       }
     };
+    // (FP64 elements are loaded at their use: a second set spilled)
+    constexpr bool ahead = sizeof(R) == 4;
     C cv[kQeMmaMT];
-    load_c(nt_first, cv);
-    __syncthreads();  // the previous tile's values are consumed
-    for (int q = threadIdx.x; q < kFilterWindow * P; q += blockDim.x) {
-      const int tau = q / P;
-      const int pr = q - tau * P;
-      double2 v = make_double2(0.0, 0.0);
-      if (tau < T && pr < np) {
-        const C x = ldg_c(win.p[tau] + r0 * nb + pr);
-        v = make_double2((double)x.x, (double)x.y);
-      }
-      qsm[tau * PS + pr] = v;
-    }
-    __syncthreads();
-    for (int nt = nt_first; nt < P / 4; nt += nt_step) {
+    if (ahead) load_c(nt_first, cv);
+    qe_cp_wait_all();
+    __syncthreads();  // this tile has landed; the other buffer is consumed
+    issue(r0 + r_step, buf[cur ^ 1]);
+    const R* tile = reinterpret_cast<const R*>(buf[cur]);
+    for (int nt = nt_first; 4 * nt < np; nt += nt_step) {
       // B fragment: B[k = 4*s + t][n = g]; column g is pair 4*nt + g/2, part g&1
-      const double* b = reinterpret_cast<const double*>(qsm + 4 * nt) + g;
+      const R* b = tile + 8 * nt + g;
       double bfr[kFilterWindow / 4];
 #pragma unroll
-      for (int st = 0; st < kFilterWindow / 4; ++st) bfr[st] = b[(4 * st + t) * 2 * PS];
+      for (int st = 0; st < kFilterWindow / 4; ++st) bfr[st] = (double)b[(4 * st + t) * 2 * PS];
       double c0[kQeMmaMT], c1[kQeMmaMT];
+      if (!ahead) load_c(nt, cv);
 #pragma unroll
       for (int m = 0; m < kQeMmaMT; ++m) {
         c0[m] = (double)cv[m].x;
         c1[m] = (double)cv[m].y;
       }
-      load_c(nt + nt_step, cv);
+      if (ahead) load_c(nt + nt_step, cv);
 #pragma unroll
       for (int m = 0; m < kQeMmaMT; ++m) {
         if (mt0 + m < n_mt) {
@@ -643,26 +957,25 @@ __global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_filter_mma_kernel(
         }
       }
       const int pc = 4 * nt + t;
-      const int rr = pc / nb, bb = pc - rr * nb;
+      const int o = at(pc);
 #pragma unroll
       for (int m = 0; m < kQeMmaMT; ++m) {
-        const int i = (mt0 + m) * 8 + g;
-        if (pc < np && i < n_en) {
-          C o;
-          o.x = (R)c0[m];
-          o.y = (R)c1[m];
-          qe[((r0 + rr) * n_en + i) * nb + bb] = o;
+        if (pc < np && (mt0 + m) * 8 + g < n_en) {
+          C v;
+          v.x = (R)c0[m];
+          v.y = (R)c1[m];
+          base[o + 8 * m * nb] = v;
         }
       }
     }
   }
+  qe_cp_wait_all();
 }
 
 // ---- several time steps from one expansion ----------------------------------------
 
 constexpr int kCombineWindow = 16;  // Chebyshev vectors per pass
 constexpr int kCombineSteps = 16;   // most time steps per expansion
-constexpr int kCombineBatch = 8;    // vectors loaded together
 
 template <typename R>
 struct CombineArgs {
@@ -672,16 +985,20 @@ struct CombineArgs {
   int64_t total;                            // values of a block
   int np;                                   // vectors of this pass
   int j0, m;                                // outputs j0 <= j < m take part
-  unsigned int init;                        // bit j: out_j starts here (is not read)
+  int init;                                 // 1: the outputs start here (are not read)
 };
 
 // out_j[e] (+)= sum_tau w[j][tau] p_tau[e] for up to 16 outputs: the states
 // after 1..m time steps all come from the same Chebyshev vectors, so m steps of
 // phase tau take n(m tau) products with H instead of m n(tau) (AC: 57 instead of
-// 240 for 16 steps).  One complex value per thread; the weights are
-// compile-time offsets into the parameter bank.  Sums in FP64.  Bound by memory: 16
-// values read for 32 FMAs each, 9 TB/s of reads at the FP64 peak.
-// p_0 may be out_{m-1}: a thread reads every p of its value before it writes.
+// 240 for 16 steps).  Sums in FP64; both kernels are bound by memory when their
+// loads are in flight early enough:
+//  combine_kernel (FP64): one value per thread, 16 accumulators, the weights
+//    compile-time offsets into the parameter bank.  Blocks of 196 MB: 1.04 ms a
+//    pass, 6.3 TB/s; the product on mma.sync took 1.30 ms.
+//  combine_mma_kernel (FP32): the same on 20 MB blocks took 329 us a pass, 1.9 TB/s, 8
+//    bytes a load and a conversion for every 32 FMAs; mma.sync takes 235 us.
+// p_0 may be an output: every p of a value is read before the value is written.
 template <typename R, int M>
 __global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__ CombineArgs<R> a) {
   using C = typename Cx<R>::t;
@@ -691,23 +1008,23 @@ __global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__
 #pragma unroll
   for (int j = 0; j < M; ++j) {
     re[j] = im[j] = 0.0;
-    if (j >= a.j0 && j < a.m && !((a.init >> j) & 1u)) {
+    if (!a.init && j >= a.j0 && j < a.m) {
       const C o = a.out[j][e];
       re[j] = (double)o.x;
       im[j] = (double)o.y;
     }
   }
 #pragma unroll
-  for (int q0 = 0; q0 < kCombineWindow; q0 += kCombineBatch) {
+  for (int q0 = 0; q0 < kCombineWindow; q0 += 8) {
     if (q0 < a.np) {
-      C p[kCombineBatch];
+      C p[8];
 #pragma unroll
-      for (int q = 0; q < kCombineBatch; ++q) {
+      for (int q = 0; q < 8; ++q) {
         p[q].x = p[q].y = (R)0;
         if (q0 + q < a.np) p[q] = a.p[q0 + q][e];
       }
 #pragma unroll
-      for (int q = 0; q < kCombineBatch; ++q) {
+      for (int q = 0; q < 8; ++q) {
         const double x = (double)p[q].x, y = (double)p[q].y;
 #pragma unroll
         for (int j = 0; j < M; ++j) {
@@ -725,6 +1042,63 @@ __global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__
       o.y = (R)im[j];
       a.out[j][e] = o;
     }
+}
+
+// W (16 x 16) . P (16 x values) on mma.sync m8n8k4 f64: a warp takes 8 values e at
+// a time, lane (g, t) loads p_tau of value g for tau = 4s + t; their real parts
+// are the 8 columns of one product, the imaginary parts those of another, so a
+// lane's accumulators are the real and imaginary parts of values 2t and 2t + 1
+// of output g.  W stays in registers.
+template <int MT>
+__global__ void __launch_bounds__(256, 3)
+    combine_mma_kernel(const __grid_constant__ CombineArgs<float> a) {
+  const int lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  constexpr int NS = kCombineWindow / 4;
+  double w[MT][NS];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) w[m][s] = a.w[8 * m + g][4 * s + t];
+  const int64_t step = 8 * (int64_t)gridDim.x * (blockDim.x >> 5);
+  const float2 zero = make_float2(0.0f, 0.0f);
+  for (int64_t e0 = 8 * ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+       e0 < a.total; e0 += step) {
+    float2 x[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+      x[s] = e0 + g < a.total && 4 * s + t < a.np ? a.p[4 * s + t][e0 + g] : zero;
+    const int64_t e = e0 + 2 * t;
+    double re[MT][2], im[MT][2];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int j = 8 * m + g;
+      const bool in = !a.init && j >= a.j0 && j < a.m;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float2 o = in && e + q < a.total ? a.out[j][e + q] : zero;
+        re[m][q] = (double)o.x;
+        im[m][q] = (double)o.y;
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        dmma_8x8x4(re[m][0], re[m][1], w[m][s], (double)x[s].x);
+        dmma_8x8x4(im[m][0], im[m][1], w[m][s], (double)x[s].y);
+      }
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const int j = 8 * m + g;
+      if (j >= a.j0 && j < a.m) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          if (e + q < a.total)
+            a.out[j][e + q] = make_float2((float)re[m][q], (float)im[m][q]);
+      }
+    }
+  }
 }
 
 }  // namespace tbpm

@@ -8,7 +8,7 @@
 // 3 those of <p_k|p_k> and Re <p_k|p_{k-1}>.  Only the way the operands reach
 // the threads differs.
 //
-// A block is one producer warp and kRingConsumerWarps consumer warps.  The
+// A block is one producer warp and kRingWarps consumer warps.  The
 // persistent grid walks row tiles grid-stride; tile i of a block goes to stage
 // i % S of a ring of S shared-memory stages.  For each tile the producer warp
 // issues 1-D bulk copies (cp.async.bulk global -> shared, completion counted in
@@ -50,6 +50,12 @@ namespace tbpm {
 #ifndef TBPM_RING_WARPS
 #define TBPM_RING_WARPS 15  // consumer warps per block
 #endif
+#ifndef TBPM_RING_WARPS_SMALL
+#define TBPM_RING_WARPS_SMALL 22  // the same for packs of 16 or 8 bytes
+#endif
+#ifndef TBPM_RING_WARPS_PLAIN
+#define TBPM_RING_WARPS_PLAIN 19  // consumer warps of the modes without an accumulator
+#endif
 #ifndef TBPM_RING_MINB
 #define TBPM_RING_MINB 1  // resident blocks per SM the stages are sized for
 #endif
@@ -71,6 +77,16 @@ constexpr unsigned long long kRingWaitNs = 2000000000ull;  // 2 s per wait
 #ifndef TBPM_RING_GATHER
 #define TBPM_RING_GATHER 3  // neighbour gathers issued together (measured: 3 beats 4)
 #endif
+
+// Consumer warps per block by the size of a thread's pack and the kernel mode: a
+// thread holds one item's gathers, so more threads are more gathers in flight, as
+// far as the registers go.
+template <typename R, int V, int MODE, bool WIN>
+constexpr int kRingWarps =
+    sizeof(R) * V == 16 ? ((MODE == 0 || MODE == 3) && !WIN ? TBPM_RING_WARPS_PLAIN : kRingConsumerWarps)
+                        : TBPM_RING_WARPS_SMALL;
+template <typename R, int V, int MODE, bool WIN>
+constexpr int kRingItems = kRingWarps<R, V, MODE, WIN> * 32;
 
 // Shared-memory layout of one stage (byte offsets, 128-byte aligned parts)
 // and the ring.  Offsets of absent parts are -1.
@@ -182,7 +198,7 @@ __device__ __forceinline__ Pack<R, V> lds_pack(const char* p) {
 }
 
 template <typename R, int V, int MODE, bool WIN>
-__global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
+__global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBlocks)
     cheb_ring_kernel(const __grid_constant__ RingArgs<R, V> ra) {
   using C = typename Cx<R>::t;
   extern __shared__ __align__(128) char rsm[];
@@ -204,7 +220,7 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
       ring_bar_init(full0 + 8u * s, 1);
-      ring_bar_init(empty0 + 8u * s, kRingConsumerWarps);
+      ring_bar_init(empty0 + 8u * s, (kRingWarps<R, V, MODE, WIN>));
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
   const int slot = tid / tpr;
   const int lane = tid - slot * tpr;
 
-  if (tid >= kRingConsumers) {
+  if (tid >= kRingItems<R, V, MODE, WIN>) {
     // ---------------- producer warp ----------------
     const int wl = tid & 31;
     int64_t issued = 0;
@@ -553,7 +569,7 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
     __syncthreads();
     double* red = reinterpret_cast<double*>(rsm);
     const int width = tpr * V * NV;
-    if (tid < kRingConsumers && slot < TR) {
+    if (tid < kRingItems<R, V, MODE, WIN> && slot < TR) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         double* p = red + slot * width + (lane * V + v) * NV;
@@ -564,7 +580,7 @@ __global__ void __launch_bounds__(kRingThreads, kRingMinBlocks)
     }
     __syncthreads();
     tree_reduce_slots(red, TR, width, slot, lane, tpr);
-    if (tid < kRingConsumers && slot == 0) {
+    if (tid < kRingItems<R, V, MODE, WIN> && slot == 0) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         const int col = lane * V + v;

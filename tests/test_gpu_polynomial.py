@@ -95,15 +95,18 @@ def test_dos_long_run_of_general_matrices(n, degree, width):
         assert rel_err(got, ref) < 1e-10
 
 
-def test_dos_long_run_several_items_per_thread():
-    """32,768 orbitals x 16 states: several items per thread of the one-launch
-    kernel, device-generated states."""
-    s = tb.make_graphene_sample(128, 128, disorder=1.0, rescale=9.0, seed=11)
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,ns", [(101, 1), (128, 2), (128, 16), (256, 1), (300, 3)])
+def test_dos_long_run_block_shapes(prec, nx, ns):
+    """From the last size of the cluster kernel to several items per thread of
+    the largest blocks of the one-launch kernel, device-generated states."""
+    s = tb.make_graphene_sample(nx, nx, disorder=1.0, rescale=9.0, seed=11)
     h = s.build_ham_csr()
     bes = bessel_series(math.pi)
-    got = f2py.tbpm_dos(bes, h.indptr, h.indices, h.data, 7, 64, 16, "", 0, 128, 1e-9)
-    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 64, seed=7, n_samples=16)
-    assert rel_err(got, ref) < 1e-10
+    f2py.set_backend(precision=prec)
+    got = f2py.tbpm_dos(bes, h.indptr, h.indices, h.data, 7, 64, ns, "", 0, 128, 1e-9)
+    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 64, seed=7, n_samples=ns)
+    assert rel_err(got, ref) < TOL[prec]
 
 
 def test_dos_other_time_steps(flake):

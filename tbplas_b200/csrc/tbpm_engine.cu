@@ -263,6 +263,7 @@ int ring_items(int mode, bool win) {
   if (mode == 0) return win ? kRingItems<R, V, 0, true> : kRingItems<R, V, 0, false>;
   if (mode == 1) return win ? kRingItems<R, V, 1, true> : kRingItems<R, V, 1, false>;
   if (mode == 2) return win ? kRingItems<R, V, 2, true> : kRingItems<R, V, 2, false>;
+  if (mode == 4) return kRingItems<R, V, 4, false>;
   return kRingItems<R, V, 3, false>;
 }
 
@@ -466,6 +467,8 @@ int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
     ra.s = tt.rs[mode];
     ra.status = c->status.as<unsigned int>();
     ra.win = tt.win;
+    ra.tiles = nullptr;
+    ra.n_tiles = 0;
     const size_t smem = (size_t)ra.s.smem_bytes;
     if (mode == 3) {
       cheb_ring_kernel<R, V, 3, false><<<t.grid, t.threads, smem, c->stream>>>(ra);
@@ -497,6 +500,54 @@ int launch_term(tbpm_ctx* c, const TermTiles& tt, const TermArgs<R, V>& a) {
   TBPM_CK(cudaGetLastError());
   c->launches++;
   return t.grid;
+}
+
+// Tiles of packed realisations for the ring kernel's mode 4: none crosses a
+// realisation.  rows == 0: the mode does not apply (no ring, or a row's packs
+// are no power of two, so that a warp does not hold whole rows).
+struct SegTiles {
+  RingShape rs{};
+  int grid = 0;
+  int n_tiles = 0;
+  int warps = 0;
+  std::vector<int2> tiles;
+  std::vector<int> first;  // first tile of every realisation, and the end
+};
+
+template <typename R, int V>
+SegTiles seg_tiles(const tbpm_ctx* c, const std::vector<int64_t>& off, int tpr) {
+  SegTiles t;
+  if (c->opts.term_kernel == 1 || c->opts.rows_per_tile > 0 || tpr > 32 || (tpr & (tpr - 1)))
+    return t;
+  t.rs = ring_shape<R, V>(c, tpr, 4, 0);
+  if (t.rs.stages == 0) return t;
+  t.warps = ring_items<R, V>(4, false) / 32;
+  for (size_t k = 0; k + 1 < off.size(); ++k) {
+    t.first.push_back((int)t.tiles.size());
+    for (int64_t r = off[k]; r < off[k + 1]; r += t.rs.rows)
+      t.tiles.push_back(make_int2((int)r, (int)std::min<int64_t>(t.rs.rows, off[k + 1] - r)));
+  }
+  t.first.push_back((int)t.tiles.size());
+  t.n_tiles = (int)t.tiles.size();
+  const int per_sm = ring_blocks_per_sm<R, V, 4, false>(c, t.rs);
+  t.grid = std::max(1, std::min(per_sm * num_sms(c->device), t.n_tiles));
+  return t;
+}
+
+template <typename R, int V>
+void launch_seg_term(tbpm_ctx* c, const SegTiles& t, const int2* tiles,
+                     const TermArgs<R, V>& a) {
+  RingArgs<R, V> ra;
+  ra.t = a;
+  ra.s = t.rs;
+  ra.status = c->status.as<unsigned int>();
+  ra.win = nullptr;
+  ra.tiles = tiles;
+  ra.n_tiles = t.n_tiles;
+  cheb_ring_kernel<R, V, 4, false>
+      <<<t.grid, t.warps * 32 + 32, (size_t)t.rs.smem_bytes, c->stream>>>(ra);
+  TBPM_CK(cudaGetLastError());
+  c->launches++;
 }
 
 // ---- paired terms (tbpm_pair_kernels.cuh) --------------------------------
@@ -1264,6 +1315,9 @@ void read_out(tbpm_ctx* c, std::vector<double>& host, size_t n_doubles) {
 // milliseconds to a second, and time stepping keeps its results bit for bit
 // equal to those of sessions (checkpoints) and of the other term kernels.
 constexpr int kPolyMinSteps = 64;
+// The transforms between moments and curves grow with the square of the run, the
+// terms only linearly; beyond this length they would be the longer part.
+constexpr int kPolyMaxSteps = 65536;
 // Largest deviation |P(x) - exp(-i tau x)| over the spectrum for which powers
 // of P count as unitary (the default Bessel precision leaves 1e-14).
 constexpr double kPolyUnitary = 1e-12;
@@ -1339,7 +1393,7 @@ void step_polynomial(const PolyPlan& pp, long double x, long double* re, long do
 // factor below the spectral radius, a non-Hermitian H) is time-stepped as before.
 bool poly_route(tbpm_ctx* c, const double* bes, int n_bes, int n_timestep, int chk_step,
                 double chk_thr, PolyPlan* pp) {
-  if (n_timestep < kPolyMinSteps) return false;
+  if (n_timestep < kPolyMinSteps || n_timestep > kPolyMaxSteps) return false;
   const bool check = chk_step >= 2 && chk_step <= n_timestep;
   if (check && !(effective_thr(c, chk_thr) >= kPolyMinThr)) return false;
   const Spectrum& sp = ham_spectrum(c);
@@ -1423,8 +1477,11 @@ std::vector<double> power_weights(const PolyPlan& pp, int m) {
   for (int k = 0; k < M; ++k) {
     const std::vector<double>& f = (k & 1) ? im : re;
     double s = 0.0;
-    for (int j = 0; j < M / 2; ++j)
-      s += f[j] * tab[(size_t)((int64_t)k * (2 * j + 1) % (4 * M))];
+    for (int j = 0, q = k; j < M / 2; ++j) {  // q = k (2j + 1) mod 4M
+      s += f[j] * tab[q];
+      q += 2 * k;
+      if (q >= 4 * M) q -= 4 * M;
+    }
     s *= 2.0;
     if (M & 1) s += f[M / 2] * tab[(size_t)((int64_t)k * M % (4 * M))];
     s *= (k ? 2.0 : 1.0) / M;
@@ -1895,7 +1952,10 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
   c->seg.ensure(sizeof(int64_t) * off.size());
   TBPM_CK(cudaMemcpyAsync(c->seg.p, off.data(), sizeof(int64_t) * off.size(),
                           cudaMemcpyHostToDevice, c->stream));
-  const int64_t per_term = (int64_t)n_cols * 2 * dot_chunks;
+  const int tpr = ns / V;
+  const SegTiles st = seg_tiles<R, V>(c, off, tpr);
+  const int64_t seg_stride = (int64_t)st.n_tiles * st.warps * ns * 2;
+  const int64_t per_term = std::max<int64_t>((int64_t)n_cols * 2 * dot_chunks, seg_stride);
   const int chunk =
       (int)std::max<int64_t>(1, std::min<int64_t>(K + 1, (64ll << 20) / (per_term * 8)));
   ensure_partials(c, std::max<size_t>((size_t)chunk * per_term, (size_t)n_cols * n_chunks));
@@ -1921,28 +1981,64 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
       c->small.as<double>(), reinterpret_cast<C*>(A), nullptr);
   TBPM_CK(cudaGetLastError());
   c->launches += 2;
-  const int tpr = ns / V;
   const TermTiles tt = term_tiles<R, V>(c, n, tpr);
-  const double bytes = matrix_bytes(c->ham) + 5.0 * (double)vb;
-  for (int k0 = 0; k0 <= K; k0 += chunk) {  // row 0 of the sums: <p_0|p_0>
+  const double bytes = matrix_bytes(c->ham) + (st.grid > 0 ? 3.0 : 5.0) * (double)vb;
+  auto dots = [&](const Pack<R, V>* x, const Pack<R, V>* y, double* out) {
+    seg_dots_kernel<R><<<dim3(dot_chunks, n_seg), threads, 0, c->stream>>>(
+        c->seg.as<int64_t>(), ns, dot_rows, reinterpret_cast<const C*>(x),
+        reinterpret_cast<const C*>(y), out);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+  };
+  auto reduce_dots = [&](int k, int count) {  // rows k .. k + count - 1 of the sums
+    const int64_t n_vals = (int64_t)count * n_cols * 2;
+    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
+        c->partials.as<double>(), dot_chunks, n_vals, sums + (int64_t)k * n_cols * 2);
+    TBPM_CK(cudaGetLastError());
+    c->launches++;
+  };
+  int k0 = 0;
+  if (st.grid > 0) {
+    // the products come out of the terms (20 samples, 1.4M rows, 4 FP64 states, 128
+    // steps: 32.8 ms with a separate pass over both vectors per term, 50 us and 39 us;
+    // 27.6 ms with them here)
+    ScratchScope scope(c->scratch);
+    TempMem tiles(c->scratch), first(c->scratch);
+    tiles.ensure(st.tiles.size() * sizeof(int2));
+    first.ensure(st.first.size() * sizeof(int));
+    TBPM_CK(cudaMemcpyAsync(tiles.p, st.tiles.data(), st.tiles.size() * sizeof(int2),
+                            cudaMemcpyHostToDevice, c->stream));
+    TBPM_CK(cudaMemcpyAsync(first.p, st.first.data(), st.first.size() * sizeof(int),
+                            cudaMemcpyHostToDevice, c->stream));
+    dots(A, A, c->partials.as<double>());
+    reduce_dots(0, 1);
+    for (k0 = 1; k0 <= K; k0 += chunk) {
+      const int m = std::min(chunk, K + 1 - k0);
+      for (int i = 0; i < m; ++i) {
+        TermArgs<R, V> a = poly_term2<R, V>(c, pp, k0 + i, tpr, A, X);
+        a.partials = c->partials.as<double>() + (int64_t)i * seg_stride;
+        launch_seg_term<R, V>(c, st, tiles.as<int2>(), a);
+        c->model_bytes += bytes;
+      }
+      seg_tile_reduce_kernel<<<dim3((unsigned)n_seg, (unsigned)m), 256, 0, c->stream>>>(
+          c->partials.as<double>(), seg_stride, first.as<int>(), st.warps, ns * 2,
+          sums + (int64_t)k0 * n_cols * 2);
+      TBPM_CK(cudaGetLastError());
+      c->launches++;
+    }
+    TBPM_CK(cudaStreamSynchronize(c->stream));  // the tables go out of scope
+  }
+  for (; k0 <= K; k0 += chunk) {  // row 0 of the sums: <p_0|p_0>
     const int m = std::min(chunk, K + 1 - k0);
     for (int i = 0; i < m; ++i) {
       const int k = k0 + i;
       Pack<R, V>* x = (k & 1) ? X : A;
       Pack<R, V>* y = (k & 1) || k == 0 ? A : X;
       if (k >= 1) launch_term<R, V>(c, tt, poly_term2<R, V>(c, pp, k, tpr, A, X));
-      seg_dots_kernel<R><<<dim3(dot_chunks, n_seg), threads, 0, c->stream>>>(
-          c->seg.as<int64_t>(), ns, dot_rows, reinterpret_cast<const C*>(x),
-          reinterpret_cast<const C*>(y), c->partials.as<double>() + (int64_t)i * per_term);
-      TBPM_CK(cudaGetLastError());
-      c->launches++;
+      dots(x, y, c->partials.as<double>() + (int64_t)i * n_cols * 2 * dot_chunks);
       c->model_bytes += bytes;
     }
-    const int64_t n_vals = (int64_t)m * n_cols * 2;
-    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), dot_chunks, n_vals, sums + (int64_t)k0 * n_cols * 2);
-    TBPM_CK(cudaGetLastError());
-    c->launches++;
+    reduce_dots(k0, m);
   }
   enqueue_moment_curves(c, pp, M, T, n_cols, sums + (int64_t)n_cols * 2, (int64_t)n_cols * 2,
                         sums, 2, mu, rho, nodes, chk_step);
@@ -2072,7 +2168,8 @@ struct StepsShape {
 // (8, 16), 27 at (8, 8), 36 at (4, 8).  FP32 states take 8 at most: the 16 outputs'
 // FP64 products (with the conversions) then cost more than the terms they save
 // (57 energies' DC run: 162 us per step at 16).
-StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max) {
+StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max,
+                          size_t cap = SIZE_MAX) {
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -2081,7 +2178,9 @@ StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max) {
   const size_t reserve = (size_t)2 << 30;
   for (const StepsShape s : {StepsShape{16, 16}, StepsShape{8, 16}, StepsShape{8, 8},
                              StepsShape{4, 8}})
-    if (s.m <= m_max && vb * (size_t)(s.m + s.window + 2) + other + reserve <= free_b + held) return s;
+    if (const size_t need = vb * (size_t)(s.m + s.window + 2) + other;
+        s.m <= m_max && need <= cap && need + reserve <= free_b + held)
+      return s;
   return StepsShape{};
 }
 
@@ -2098,7 +2197,8 @@ template <typename R>
 StepsShape steps_room(tbpm_ctx* c, const PolyPlan* pp, int ld, int ref_ld) {
   if (!pp) return StepsShape{};
   const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
-  const size_t ref = (size_t)c->ham.n * ref_ld * 2 * sizeof(R);
+  // the reference block, and the staging of states that come from the host
+  const size_t ref = (size_t)c->ham.n * ref_ld * (2 * sizeof(R) + 16);
   const StepsShape s =
       steps_that_fit(vb, vb + ref, c->A.bytes + c->X.bytes + c->Y.bytes + c->wf0.bytes,
                      most_steps<R>);
@@ -2243,6 +2343,13 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
 template <typename R>
 void qe_accum_attr(size_t bytes) {
   qe_smem_attr(qe_accum_kernel<R>, bytes);
+}
+
+// The tables of n_en energies' filters for T steps (values on the nodes,
+// coefficients, window factors) have to stay small beside QE.
+bool filters_fit(const PolyPlan& pp, int T, int n_en) {
+  const double M = bessel_degree(pp.tau * (double)pp.a * T);
+  return 16.0 * n_en * (M + T) < 1e9;
 }
 
 // Phase 1 on the polynomial route: QE_i = f_i(H) wf0 by the energies' filters
@@ -2594,8 +2701,14 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   // several steps per expansion where their blocks fit beside QE
   StepsShape shape;
   if (pp) {
-    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes,
-                           most_steps<R>);
+    // a memory budget covers QE and these blocks together
+    size_t cap = SIZE_MAX;
+    if (c->opts.dc_budget_gb > 0) {
+      const size_t budget = (size_t)(c->opts.dc_budget_gb * 1073741824.0);
+      cap = budget > qe_bytes ? budget - qe_bytes : 0;
+    }
+    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes, most_steps<R>,
+                           cap);
     if (shape.m > 0) {
       c->A.ensure(vb * (size_t)(shape.m + shape.window + 2 + T2));
     } else {
@@ -3004,21 +3117,26 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, c
   // times the state is not needed: on the polynomial route the m steps are one
   // expansion of about tau*a*m terms (512 x 480 graphene, one state, 64 steps
   // between frames: 260 terms instead of 1216).
+  // Long intervals are taken in pieces: the weights of a piece cost the host the
+  // square of its length (512 steps: about 2 ms, beside 1700 terms on the device).
+  constexpr int kMaxJump = 512;
   auto advance_to = [&](int target) {
-    if (target <= done) return;
-    if (poly) {
-      if (target - done != jump_m) {
-        jump_m = target - done;
-        jump = power_expansion(pp, jump_m);
+    while (poly && target > done) {
+      const int m = std::min(target - done, kMaxJump);
+      if (m != jump_m) {
+        jump_m = m;
+        jump = power_expansion(pp, m);
       }
       enqueue_expansion<R, V>(c, jump, 1, A, X, Y, nullptr, 0, c->out.as<double>(),
                               counters(c, 0));
       ++rows;
-    } else {
+      done += m;
+    }
+    if (target > done) {
       run_steps(c, target - done, key, step);
       rows += target - done;
+      done = target;
     }
-    done = target;
   };
   // A logged state is converted into one of two staging buffers; its copy to the
   // host (which blocks the calling thread) is issued on a second stream after
@@ -3454,7 +3572,8 @@ void drv_dc_part(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, i
     (void)cudaGetLastError();
   }
   PolyPlan pp;
-  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
+                    filters_fit(pp, n_timestep, en_chunk);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;
@@ -3591,7 +3710,8 @@ void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf
     (void)cudaGetLastError();
   }
   PolyPlan pp;
-  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
+                    filters_fit(pp, n_timestep, n_energies);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;

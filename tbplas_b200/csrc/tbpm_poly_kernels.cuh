@@ -722,6 +722,32 @@ __global__ void __launch_bounds__(256) seg_dots_kernel(const int64_t* seg_off, i
   }
 }
 
+// out[(seg*ns2 + v)] = sum of the entries [first[seg], first[seg+1]) x per_tile of one
+// term, entries of ns2 values; block (seg, term), fixed order.  Terms follow
+// each other at `stride` doubles in `partials`, n_seg*ns2 doubles in `out`.
+static __global__ void __launch_bounds__(256) seg_tile_reduce_kernel(const double* partials,
+                                                                     int64_t stride,
+                                                                     const int* first, int per_tile,
+                                                                     int ns2, double* out) {
+  __shared__ double red[256];
+  const int seg = blockIdx.x;
+  const int groups = 256 / ns2;
+  const int grp = threadIdx.x / ns2;
+  const int v = threadIdx.x - grp * ns2;
+  const double* p = partials + blockIdx.y * stride;
+  const int64_t e0 = (int64_t)first[seg] * per_tile, e1 = (int64_t)first[seg + 1] * per_tile;
+  double s = 0.0;
+  if (grp < groups)
+    for (int64_t e = e0 + grp; e < e1; e += groups) s += p[e * ns2 + v];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < ns2) {
+    double t = 0.0;
+    for (int g = 0; g < groups; ++g) t += red[g * ns2 + threadIdx.x];
+    out[((int64_t)blockIdx.y * gridDim.x + seg) * ns2 + threadIdx.x] = t;
+  }
+}
+
 // ---- quasi-eigenstates as energy filters ---------------------------------------
 
 // Phase 1 of tbpm_dccond (tbpm.f90:600-638) accumulates

@@ -6,7 +6,9 @@
 // deferred Bessel/Fermi-weighted flush of up to three pending terms into the
 // accumulator and, in MODE 2, the <ref|psi> / <psi|psi> block partials, in MODE
 // 3 those of <p_k|p_k> and Re <p_k|p_{k-1}>.  Only the way the operands reach
-// the threads differs.
+// the threads differs.  MODE 4 is mode 3 for packed realisations: the tiles come
+// from a table in which none crosses a realisation, and every consumer warp
+// writes its rows' products per tile, so that they can be summed per realisation.
 //
 // A block is one producer warp and kRingWarps consumer warps.  The
 // persistent grid walks row tiles grid-stride; tile i of a block goes to stage
@@ -83,7 +85,7 @@ constexpr unsigned long long kRingWaitNs = 2000000000ull;  // 2 s per wait
 // far as the registers go.
 template <typename R, int V, int MODE, bool WIN>
 constexpr int kRingWarps =
-    sizeof(R) * V == 16 ? ((MODE == 0 || MODE == 3) && !WIN ? TBPM_RING_WARPS_PLAIN : kRingConsumerWarps)
+    sizeof(R) * V == 16 ? (MODE == 0 && !WIN ? TBPM_RING_WARPS_PLAIN : kRingConsumerWarps)
                         : TBPM_RING_WARPS_SMALL;
 template <typename R, int V, int MODE, bool WIN>
 constexpr int kRingItems = kRingWarps<R, V, MODE, WIN> * 32;
@@ -110,6 +112,8 @@ struct RingArgs {
   RingShape s;
   unsigned int* status;  // bit 0: a bounded wait ran out
   const int* win;        // WIN kernels: per tile kRingWinInts ints (ring_window_kernel)
+  const int2* tiles;     // MODE 4: (first row, rows) of every tile
+  int n_tiles;
 };
 
 // Row windows (the WIN kernels): a tile's off-diagonal columns and its own
@@ -212,7 +216,7 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
   const uint32_t full0 = ring_smem(rsm + sh.bar_off);
   const uint32_t empty0 = full0 + 8u * (uint32_t)S;
   const int nflush = MODE == 1 || MODE == 2 ? a.c.nflush : 0;
-  const bool need_own = MODE == 3 || a.diag != nullptr || nflush >= 2;
+  const bool need_own = MODE >= 3 || a.diag != nullptr || nflush >= 2;
   const bool add_acc = nflush > 0 && !a.c.acc_init;
   const int64_t row_bytes = (int64_t)tpr * sizeof(Pack<R, V>);
   const bool ref_staged = MODE == 2 && a.ref != nullptr && sh.ref_off >= 0;
@@ -231,6 +235,21 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
   for (int v = 0; v < V; ++v) cre[v] = cim[v] = nrm[v] = 0.0;
   const int slot = tid / tpr;
   const int lane = tid - slot * tpr;
+  // the block's i-th tile: first row and rows; false past the last one
+  auto tile_of = [&](int64_t i, int64_t* r0, int* nr) -> bool {
+    const int64_t t = (int64_t)blockIdx.x + i * gridDim.x;
+    if constexpr (MODE == 4) {
+      if (t >= ra.n_tiles) return false;
+      const int2 v = __ldg(ra.tiles + t);
+      *r0 = v.x;
+      *nr = v.y;
+    } else {
+      *r0 = t * TR;
+      if (*r0 >= n) return false;
+      *nr = (int)(n - *r0 < TR ? n - *r0 : TR);
+    }
+    return true;
+  };
 
   if (tid >= kRingItems<R, V, MODE, WIN>) {
     // ---------------- producer warp ----------------
@@ -239,11 +258,11 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
     bool ok = true;
     // CSR bounds of the next 32 tiles, one tile per lane, loaded a batch ahead
     auto bounds = [&](int64_t i, int* b0, int* b1) {
-      const int64_t r0 = ((int64_t)blockIdx.x + i * gridDim.x) * TR;
-      if (r0 < n) {
-        const int64_t r1 = r0 + TR < n ? r0 + TR : n;
+      int64_t r0;
+      int nr;
+      if (tile_of(i, &r0, &nr)) {
         *b0 = __ldg(a.indptr + r0);
-        *b1 = __ldg(a.indptr + r1);
+        *b1 = __ldg(a.indptr + r0 + nr);
       } else {
         *b0 = *b1 = 0;
       }
@@ -269,8 +288,9 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       record(32 + wl, wnxt);
     }
     for (int64_t i = 0;; ++i) {
-      const int64_t r0 = ((int64_t)blockIdx.x + i * gridDim.x) * TR;
-      if (r0 >= n) break;
+      int64_t r0;
+      int nr;
+      if (!tile_of(i, &r0, &nr)) break;
       if (i > 0 && (i & 31) == 0) {
         cur0 = nxt0;
         cur1 = nxt1;
@@ -308,7 +328,6 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       if (wl == 0) {
         char* st = rsm + (size_t)s * sh.stage_bytes;
         const uint32_t bar = full0 + 8u * s;
-        const int nr = (int)(n - r0 < TR ? n - r0 : TR);
         // indptr[r0 .. r0+nr] from the 16-byte boundary at or below r0
         const int64_t r0a = r0 & ~(int64_t)3;
         const uint32_t ip_bytes = (uint32_t)(((r0 + nr + 1 - r0a + 3) & ~(int64_t)3) * 4);
@@ -403,8 +422,9 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
     const bool ref_lane = do_corr && a.ref != nullptr && lane < a.ref_tpr;
     constexpr int GB = TBPM_RING_GATHER;
     for (int64_t i = 0;; ++i) {
-      const int64_t r0 = ((int64_t)blockIdx.x + i * gridDim.x) * TR;
-      if (r0 >= n) break;
+      int64_t r0;
+      int nr;
+      if (!tile_of(i, &r0, &nr)) break;
       const int s = (int)(i % S);
       if (!__all_sync(0xffffffffu, ring_wait(full0 + 8u * s, (uint32_t)((i / S) & 1)))) {
         if ((tid & 31) == 0) atomicOr(ra.status, 1u);
@@ -412,8 +432,7 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       }
       const char* st = rsm + (size_t)s * sh.stage_bytes;
       const int64_t r = r0 + slot;
-      if (active && r < n) {
-        const int nr = (int)(n - r0 < TR ? n - r0 : TR);
+      if (active && slot < nr) {
         const int32_t* ip = reinterpret_cast<const int32_t*>(st + sh.ip_off) + (r0 & 3);
         const int j0 = ip[slot], j1 = ip[slot + 1];
         const int ja = ip[0] & ~3;
@@ -508,7 +527,7 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
           pk.v[2 * v] = fma(ar, sre[v], fma(-ai, sim[v], beta * pm2.v[2 * v]));
           pk.v[2 * v + 1] = fma(ar, sim[v], fma(ai, sre[v], beta * pm2.v[2 * v + 1]));
         }
-        if (MODE == 3) {
+        if (MODE >= 3) {
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             const double xr = (double)pk.v[2 * v], xi = (double)pk.v[2 * v + 1];
@@ -559,10 +578,31 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       }
       __syncwarp();
       if ((tid & 31) == 0) ring_arrive(empty0 + 8u * s);
+      if constexpr (MODE == 4) {
+        // sums over the warp's rows (tpr is a power of two), one entry per
+        // (tile, warp): partials[((tile*warps + warp)*ld + col)*2 + q]
+        for (int w = 16; w >= tpr; w >>= 1)
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            nrm[v] += __shfl_xor_sync(0xffffffffu, nrm[v], w);
+            cre[v] += __shfl_xor_sync(0xffffffffu, cre[v], w);
+          }
+        const int64_t t = (int64_t)blockIdx.x + i * gridDim.x;
+        double* out = a.partials + ((t * kRingWarps<R, V, MODE, WIN> + (tid >> 5)) * tpr + lane) *
+                                       (2 * V);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          if ((tid & 31) < tpr) {
+            out[2 * v] = nrm[v];
+            out[2 * v + 1] = cre[v];
+          }
+          nrm[v] = cre[v] = 0.0;
+        }
+      }
     }
   }
 
-  if constexpr (MODE >= 2) {
+  if constexpr (MODE == 2 || MODE == 3) {
     // block partials of the products, reduced in a fixed order over the rows
     // of a tile; the stage buffers are free (every copy was consumed)
     constexpr int NV = MODE == 3 ? 2 : 3;

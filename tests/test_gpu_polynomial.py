@@ -165,7 +165,7 @@ def test_norm_errors_of_long_runs(flake):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-@pytest.mark.parametrize("ns", [1, 4])
+@pytest.mark.parametrize("ns", [1, 3, 4, 16])
 def test_packed_realisations_long_run(prec, ns):
     samples = [tb.make_graphene_sample(nx, ny, disorder=w, vacancy_rate=v, rescale=10.0, seed=i)
                for i, (nx, ny, w, v) in enumerate([(6, 5, 0.0, 0.0), (9, 7, 1.5, 0.02),
@@ -192,7 +192,8 @@ def sample():
 
 
 @pytest.mark.parametrize("n_t,log", [(64, [0, 64]), (150, [0, 1, 2, 17, 90, 149]),
-                                     (80, [79, 80]), (300, [7, 299])])
+                                     (80, [79, 80]), (300, [7, 299]),
+                                     (1100, [3, 1100])])
 def test_psi_t_jumps(sample, n_t, log):
     """One expansion per logged interval, with and without the norm check."""
     h = sample.build_ham_csr()

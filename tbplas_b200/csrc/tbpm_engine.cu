@@ -3008,11 +3008,17 @@ template <typename R>
 void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
   using C = typename Cx<R>::t;
   const Ham& h = c->ham;
-  // enough threads for one row each, spread over the SMs
+  // Enough threads for one row each, spread over the SMs.  Blocks of 768 have the
+  // registers to load a row ahead; past five rows a thread (their own rows no longer
+  // fit the shared memory in FP64) the more loads in flight of 1024 win.  Measured on
+  // B200, us per depth, 768 / 1024: FP64 320,000 orbitals 10.5 / 11.8, 524,288 12.6 /
+  // 14.0, 980,000 28.3 / 25.8; FP32 320,000 11.0 / 12.0, 980,000 19.4 / 18.7.
   const int sms = num_sms(c->device);
   const int64_t per_sm = (h.n + sms - 1) / sms;
-  const int threads =
-      (int)std::min<int64_t>(kHaydockThreads, std::max<int64_t>(128, (per_sm + 31) / 32 * 32));
+  const bool large = h.n > 5 * (int64_t)sms * 768;
+  auto kernel = large ? haydock_kernel<R, 1024> : haydock_kernel<R, 768>;
+  const int threads = (int)std::min<int64_t>(
+      large ? 1024 : 768, std::max<int64_t>(128, (per_sm + 31) / 32 * 32));
   const int grid = (int)std::min<int64_t>(sms, (h.n + threads - 1) / threads);
   ensure_partials(c, (size_t)3 * grid);
   c->ctr.ensure(16 * sizeof(int));
@@ -3030,10 +3036,14 @@ void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
   a.a = sc;
   a.b = sc + 2 * n_depth;
   a.partials = c->partials.as<double>();
+  const int64_t items = (h.n + (int64_t)grid * threads - 1) / ((int64_t)grid * threads);
+  const size_t item_bytes = 3 * (size_t)threads * sizeof(C);
+  a.cap = (int)std::min<int64_t>(items, (int64_t)(kHaydockSmem / item_bytes));
   a.bar = c->ctr.as<unsigned int>() + 12;
   a.status = c->status.as<unsigned int>();
   TBPM_CK(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), c->stream));
-  launch_cooperative(c, haydock_kernel<R>, grid, threads, 0, a);
+  qe_smem_attr(kernel, a.cap * item_bytes);
+  launch_cooperative(c, kernel, grid, threads, a.cap * item_bytes, a);
   c->launches++;
   c->model_bytes += (double)n_depth * (matrix_bytes(h) + 6.0 * h.n * sizeof(C));
 }

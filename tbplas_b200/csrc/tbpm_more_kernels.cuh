@@ -252,11 +252,13 @@ struct HaydockArgs {
   double* a;         // [2 * n_depth]
   double* b;         // [n_depth]
   double* partials;  // [3 * gridDim.x]: <v|y> (re, im), <w|w>
+  int cap;               // own rows of w, w_prev and y a thread keeps in shared memory
   unsigned int* bar;     // grid barrier, zero on entry
   unsigned int* status;  // bit 0: a bounded wait ran out
 };
 
-constexpr int kHaydockThreads = 1024;
+constexpr int kHaydockDeg = 3;  // row entries whose gathers are issued together
+constexpr size_t kHaydockSmem = 192 * 1024;  // for the threads' own rows
 constexpr unsigned long long kHaydockWaitNs = 2000000000ull;  // 2 s per wait
 
 // Arrival of the block on the grid barrier and bounded wait for `want` arrivals;
@@ -289,33 +291,39 @@ __device__ __forceinline__ bool haydock_barrier(unsigned int* bar, unsigned int 
   return *stop == 0;
 }
 
-// Sum of a block's per-thread values (in every thread of warp 0), fixed order.
-__device__ __forceinline__ double haydock_block_sum(double v, double* red) {
-  for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+// Sums of a block's N per-thread values, fixed order: value i to out[i * stride].
+template <int N>
+__device__ __forceinline__ void haydock_block_sums(double (&v)[N], double (*red)[32], double* out,
+                                                   int stride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    for (int s = 16; s > 0; s >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], s);
+    if (lane == 0) red[i][warp] = v[i];
   }
   __syncthreads();
-  return t;
+  if (warp < N) {  // one warp per value (a block has four warps or more)
+    double t = lane < (blockDim.x >> 5) ? red[warp][lane] : 0.0;
+    for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
+    if (lane == 0) out[warp * stride] = t;
+  }
 }
 
-// Sum over the grid's partials, read past L1 (other blocks wrote them in this
-// launch), in the same order in every block; in every thread.
-__device__ __forceinline__ double haydock_grid_sum(const double* p, int n, double* bcast) {
-  if (threadIdx.x < 32) {
+// Sums over the grid's partials of N values, read past L1 (other blocks wrote them in
+// this launch), in the same order in every block; to every thread.
+template <int N>
+__device__ __forceinline__ void haydock_grid_sums(const double* p, int n, double* bcast,
+                                                  double (&sum)[N]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < N) {
     double t = 0.0;
-    for (int i = threadIdx.x; i < n; i += 32) t += __ldcg(p + i);
+    for (int i = lane; i < n; i += 32) t += __ldcg(p + warp * n + i);
     for (int s = 16; s > 0; s >>= 1) t += __shfl_xor_sync(0xffffffffu, t, s);
-    if (threadIdx.x == 0) *bcast = t;
+    if (lane == 0) bcast[warp] = t;
   }
   __syncthreads();
-  const double t = *bcast;
-  __syncthreads();
-  return t;
+#pragma unroll
+  for (int i = 0; i < N; ++i) sum[i] = bcast[i];
 }
 
 // Ordinary loads of vectors that other SMs wrote before the last grid barrier
@@ -334,69 +342,122 @@ __device__ __forceinline__ float2 ld_c(const float2* p) {
 // w the unnormalised vector and v = w / b_{d-1}:
 //   y = rescale H v, a_d = <v|y>;  w' = y - a_d v - b_{d-1} v_prev, b_d = |w'|.
 // Two grid barriers per depth (one per inner product) replace five launches, and
-// the division by b_d is folded into the next depth instead of taking a pass:
-// the matrix and 6 vector passes instead of 9.  512 x 512 graphene fits L2, so a
-// depth is bound by the two barrier round trips and L2: 16.5 us (measured; the
-// five launches took 35 us).
-template <typename R>
-__global__ void __launch_bounds__(kHaydockThreads, 1)
+// the division by b_d is folded into the next depth instead of taking a pass.
+// The matrix and w stay in L2 for some hundred thousand orbitals; what a depth
+// then costs is latency: the barriers and the chain from a row's entries to the
+// gathered values.  So a row's entries are loaded one item ahead (the first row's
+// before the barrier), its gathers are issued together, and a thread's own rows of
+// w, w_prev and y (as many as fit the shared memory: `cap` per thread) never leave
+// the SM: the second half of a depth then reads nothing from L2.  524,288
+// orbitals, per depth: 12.5 us, 16.5 us with the entries in the loop and all
+// vectors in L2, 35 us as five launches.
+template <typename R, int T_MAX>
+__global__ void __launch_bounds__(T_MAX, 1)
     haydock_kernel(const __grid_constant__ HaydockArgs<R> k) {
   using C = typename Cx<R>::t;
-  __shared__ double red[32];
-  __shared__ double bcast;
+  extern __shared__ __align__(16) char hsm[];
+  __shared__ double red[2][32];
+  __shared__ double bcast[3];
   __shared__ int stop;
   if (threadIdx.x == 0) stop = 0;
-  __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t r0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int T = blockDim.x, cap = k.cap;
+  // own rows: item i of the thread at [i * T]
+  C* sw = reinterpret_cast<C*>(hsm) + threadIdx.x;
+  C* sp = sw + (size_t)cap * T;
+  C* const sy = sp + (size_t)cap * T;
   unsigned int want = 0;
   double s = 1.0, s_prev = 0.0, b_prev = 0.0;  // v = s w, v_prev = s_prev w_prev
   C* w = k.w0;
   C* w_prev = k.w1;
+  {
+    int i = 0;
+    for (int64_t r = r0; r < k.n_rows && i < cap; r += stride, ++i) sw[i * T] = ld_c(w + r);
+  }
+  // matrix entries of the current item
+  int j0 = 0, j1 = 0;
+  int c[kHaydockDeg];
+  C h[kHaydockDeg];
+  C g;
+  g.x = g.y = (R)0;
+  auto load = [&](int64_t r) {
+    j0 = __ldg(k.indptr + r);
+    j1 = __ldg(k.indptr + r + 1);
+#pragma unroll
+    for (int u = 0; u < kHaydockDeg; ++u) {
+      c[u] = -1;
+      if (j0 + u < j1) {
+        c[u] = __ldg(k.indices + j0 + u);
+        h[u] = ldg_c(k.hop + j0 + u);
+      }
+    }
+    if (k.diag) g = ldg_c(k.diag + r);
+  };
+  if (r0 < k.n_rows) load(r0);
+  __syncthreads();
   for (int d = 0; d < k.n_depth; ++d) {
-    double cr = 0.0, ci = 0.0;
-    for (int64_t r = r0; r < k.n_rows; r += stride) {
-      const int j0 = __ldg(k.indptr + r), j1 = __ldg(k.indptr + r + 1);
-      const C own = ld_c(w + r);
+    double cs[2] = {0.0, 0.0};
+    int i = 0;
+    for (int64_t r = r0; r < k.n_rows; r += stride, ++i) {
+      C x[kHaydockDeg];
+#pragma unroll
+      for (int u = 0; u < kHaydockDeg; ++u)
+        if (c[u] >= 0) x[u] = ld_c(w + c[u]);
+      const C own = i < cap ? sw[i * T] : ld_c(w + r);
       double vr = 0.0, vi = 0.0;
       if (k.diag) {
-        const C g = ldg_c(k.diag + r);
         vr = (double)g.x * (double)own.x - (double)g.y * (double)own.y;
         vi = (double)g.x * (double)own.y + (double)g.y * (double)own.x;
       }
-#pragma unroll 4
-      for (int j = j0; j < j1; ++j) {
-        const C h = ldg_c(k.hop + j);
-        const C x = ld_c(w + __ldg(k.indices + j));
-        vr += (double)h.x * (double)x.x - (double)h.y * (double)x.y;
-        vi += (double)h.x * (double)x.y + (double)h.y * (double)x.x;
+#pragma unroll
+      for (int u = 0; u < kHaydockDeg; ++u)
+        if (c[u] >= 0) {
+          vr += (double)h[u].x * (double)x[u].x - (double)h[u].y * (double)x[u].y;
+          vi += (double)h[u].x * (double)x[u].y + (double)h[u].y * (double)x[u].x;
+        }
+      for (int jb = j0 + kHaydockDeg; jb < j1; jb += kHaydockDeg) {  // longer rows
+#pragma unroll
+        for (int u = 0; u < kHaydockDeg; ++u)
+          if (jb + u < j1) {
+            h[u] = ldg_c(k.hop + jb + u);
+            x[u] = ld_c(w + __ldg(k.indices + jb + u));
+          }
+#pragma unroll
+        for (int u = 0; u < kHaydockDeg; ++u)
+          if (jb + u < j1) {
+            vr += (double)h[u].x * (double)x[u].x - (double)h[u].y * (double)x[u].y;
+            vi += (double)h[u].x * (double)x[u].y + (double)h[u].y * (double)x[u].x;
+          }
       }
+      load(r + stride < k.n_rows ? r + stride : r0);
       C o;
       o.x = (R)(vr * s * k.rescale);
       o.y = (R)(vi * s * k.rescale);
-      k.y[r] = o;
+      if (i < cap)
+        sy[i * T] = o;
+      else
+        k.y[r] = o;
       const double xr = s * (double)own.x, xi = s * (double)own.y;
-      cr += xr * (double)o.x + xi * (double)o.y;
-      ci += xr * (double)o.y - xi * (double)o.x;
+      cs[0] += xr * (double)o.x + xi * (double)o.y;
+      cs[1] += xr * (double)o.y - xi * (double)o.x;
     }
-    const double tr = haydock_block_sum(cr, red);
-    const double ti = haydock_block_sum(ci, red);
-    if (threadIdx.x == 0) {
-      k.partials[blockIdx.x] = tr;
-      k.partials[gridDim.x + blockIdx.x] = ti;
-    }
+    haydock_block_sums(cs, red, k.partials + blockIdx.x, (int)gridDim.x);
     want += gridDim.x;
     if (!haydock_barrier(k.bar, want, k.status, &stop)) return;
-    const double ar = haydock_grid_sum(k.partials, gridDim.x, &bcast);
-    const double ai = haydock_grid_sum(k.partials + gridDim.x, gridDim.x, &bcast);
-    double nn = 0.0;
-    for (int64_t r = r0; r < k.n_rows; r += stride) {
-      const C x = ld_c(w + r), z = ld_c(k.y + r);
+    double a[2];
+    haydock_grid_sums(k.partials, (int)gridDim.x, bcast, a);
+    const double ar = a[0], ai = a[1];
+    double nn[1] = {0.0};
+    i = 0;
+    for (int64_t r = r0; r < k.n_rows; r += stride, ++i) {
+      const bool in = i < cap;
+      const C x = in ? sw[i * T] : ld_c(w + r), z = in ? sy[i * T] : ld_c(k.y + r);
       const double xr = s * (double)x.x, xi = s * (double)x.y;
       double vr = (double)z.x - (ar * xr - ai * xi);
       double vi = (double)z.y - (ar * xi + ai * xr);
       if (d > 0) {
-        const C p = ld_c(w_prev + r);
+        const C p = in ? sp[i * T] : ld_c(w_prev + r);
         vr -= b_prev * (s_prev * (double)p.x);
         vi -= b_prev * (s_prev * (double)p.y);
       }
@@ -404,13 +465,15 @@ __global__ void __launch_bounds__(kHaydockThreads, 1)
       o.x = (R)vr;
       o.y = (R)vi;
       w_prev[r] = o;
-      nn += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
+      if (in) sp[i * T] = o;
+      nn[0] += (double)o.x * (double)o.x + (double)o.y * (double)o.y;
     }
-    const double tn = haydock_block_sum(nn, red);
-    if (threadIdx.x == 0) k.partials[2 * gridDim.x + blockIdx.x] = tn;
+    haydock_block_sums(nn, red, k.partials + 2 * gridDim.x + blockIdx.x, (int)gridDim.x);
     want += gridDim.x;
     if (!haydock_barrier(k.bar, want, k.status, &stop)) return;
-    const double b = sqrt(haydock_grid_sum(k.partials + 2 * gridDim.x, gridDim.x, &bcast));
+    double bb[1];
+    haydock_grid_sums(k.partials + 2 * gridDim.x, (int)gridDim.x, bcast + 2, bb);
+    const double b = sqrt(bb[0]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       k.a[2 * d] = ar;
       k.a[2 * d + 1] = ai;
@@ -419,6 +482,9 @@ __global__ void __launch_bounds__(kHaydockThreads, 1)
     C* t = w;
     w = w_prev;
     w_prev = t;
+    t = sw;
+    sw = sp;
+    sp = t;
     s_prev = s;
     s = 1.0 / b;
     b_prev = b;

@@ -285,6 +285,40 @@ def test_haydock_small_samples(nx, ny):
         if n > 1 else rel_err(a[:1], ra[:1]) < FP64_TOL
 
 
+@pytest.mark.parametrize("prec,nx,ny,tol", [("fp64", 380, 400, FP64_TOL),
+                                            ("fp64", 557, 560, FP64_TOL),
+                                            ("fp32", 400, 380, 3e-5), ("fp32", 787, 790, 3e-5)])
+def test_haydock_rows_in_and_past_shared_memory(prec, nx, ny, tol):
+    """Three rows per thread, and more than the shared memory holds of its own rows
+    (four in FP64, eight in FP32)."""
+    s = tb.make_graphene_device_sample(nx, ny, disorder=1.0, rescale=9.0, seed=4)
+    h = s.download_ham_csr()
+    f2py.set_backend(precision=prec)
+    w = unit_states(1, 1, seed=8)
+    a, b = f2py.haydock_coef([77], h.indptr, h.indices, h.data, s.rescale, 7, w)
+    ra, rb = oracle.haydock_coef([77], h.indptr, h.indices, h.data, s.rescale, 7, w)
+    assert rel_err(a, ra) < tol and rel_err(b, rb) < tol
+
+
+@pytest.mark.parametrize("density,depth", [(0.005, 2), (0.02, 6), (0.06, 6)])
+def test_haydock_row_lengths(density, depth):
+    """Rows of no entry, of fewer and of more than the gathers issued together."""
+    rng = np.random.default_rng(int(1000 * density))
+    n = 300
+    m = np.triu(rng.random((n, n)) < density, 1) * (rng.standard_normal((n, n))
+                                                    + 1j * rng.standard_normal((n, n)))
+    m = m + m.conj().T + np.diag(rng.standard_normal(n) * (rng.random(n) < 0.5))
+    m[0, 1] = 0.3 - 0.2j  # the first site is connected
+    m[1, 0] = np.conj(m[0, 1])
+    ip = np.concatenate([[0], np.cumsum((m != 0).sum(1))]).astype(np.int32)
+    ix = np.concatenate([np.flatnonzero(row) for row in m]).astype(np.int32)
+    hv = m[m != 0]
+    w = unit_states(1, 1, seed=8)
+    a, b = f2py.haydock_coef([0], ip, ix, hv, 3.0, depth, w)
+    ra, rb = oracle.haydock_coef([0], ip, ix, hv, 3.0, depth, w)
+    assert rel_err(a, ra) < FP64_TOL and rel_err(b, rb) < FP64_TOL
+
+
 @pytest.mark.parametrize("nk", [2, 63, 64, 65, 129, 200])
 @pytest.mark.parametrize("nx,ny", [(2, 2), (13, 17), (60, 57)])
 def test_kbdc_tile_edges(nk, nx, ny):

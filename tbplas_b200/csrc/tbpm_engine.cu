@@ -2106,8 +2106,8 @@ void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, 
   a.m = m;
   for (int j = 0; j < m; ++j) a.out[j] = reinterpret_cast<C*>(states[j]);
   const int grid = sizeof(R) == 8 ? blocks_for(a.total, 256)
-                                  : (int)std::min<int64_t>(blocks_for((a.total + 7) / 8, 8),
-                                                           (int64_t)num_sms(c->device) * 6);
+                                  : (int)std::min<int64_t>(blocks_for((a.total + 15) / 16, 8),
+                                                           (int64_t)num_sms(c->device) * 4);
   const PersistShape ps = persist_shape<R, V>(c, ld);
   for (int k0 = 0; k0 < n_vec; k0 += window) {
     const int len = std::min(window, n_vec - k0);
@@ -2142,10 +2142,13 @@ void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, 
         combine_kernel<R, 8><<<grid, 256, 0, c->stream>>>(a);
       else
         combine_kernel<R, 16><<<grid, 256, 0, c->stream>>>(a);
-    } else if (m <= 8) {
-      combine_mma_kernel<1><<<grid, 256, 0, c->stream>>>(a);
     } else {
-      combine_mma_kernel<2><<<grid, 256, 0, c->stream>>>(a);
+      // blocks of a multiple of four values keep their 16-byte boundaries
+      bool wide = a.total % 4 == 0;
+      for (int q = 0; q < len; ++q) wide = wide && reinterpret_cast<uintptr_t>(a.p[q]) % 16 == 0;
+      for (int j = 0; j < m; ++j) wide = wide && reinterpret_cast<uintptr_t>(a.out[j]) % 16 == 0;
+      if (wide) combine_mma_kernel<true><<<grid, 256, 0, c->stream>>>(a);
+      else combine_mma_kernel<false><<<grid, 256, 0, c->stream>>>(a);
     }
     TBPM_CK(cudaGetLastError());
     c->launches++;
@@ -2154,7 +2157,7 @@ void enqueue_steps(tbpm_ctx* c, const PolyPlan& pp, const StepsPlan& sp, int m, 
 }
 
 template <typename R>
-constexpr int most_steps = sizeof(R) == 8 ? 16 : 8;
+constexpr int most_steps = sizeof(R) == 8 ? 16 : 8;  // (combine_mma_kernel: 8 outputs)
 
 // Time steps per expansion and vectors per update for blocks of vb bytes.
 struct StepsShape {
@@ -2164,10 +2167,11 @@ struct StepsShape {
 
 // The largest shape whose states and ring, beside `other` bytes, fit the memory
 // that is free or held by the buffers they go into.  Model of a step of phase
-// pi/2 in passes over the block (time stepping: 57): 20 at (16, 16), 24 at
-// (8, 16), 27 at (8, 8), 36 at (4, 8).  FP32 states take 8 at most: the 16 outputs'
-// FP64 products (with the conversions) then cost more than the terms they save
-// (57 energies' DC run: 162 us per step at 16).
+// pi/2 in passes over the block (time stepping: 57): 18 at (16, 32), 20 at (16, 16),
+// 24 at (8, 16), 27 at (8, 8), 36 at (4, 8).  Windows of 32 instead of 16 vectors: AC
+// 561 -> 541 ms (256,000 cells x 8 states), FP32 DC 201 -> 183 ms.  FP32 states take 8
+// steps at most: the 16 outputs' FP64 products cost more than the terms they save
+// (DC 183 ms at 8, 212 ms at 16).
 StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max,
                           size_t cap = SIZE_MAX) {
   size_t free_b = 0, total_b = 0;
@@ -2176,7 +2180,8 @@ StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max,
     return StepsShape{};
   }
   const size_t reserve = (size_t)2 << 30;
-  for (const StepsShape s : {StepsShape{16, 16}, StepsShape{8, 16}, StepsShape{8, 8},
+  for (const StepsShape s : {StepsShape{16, kCombineWindow}, StepsShape{16, 16},
+                             StepsShape{8, kCombineWindow}, StepsShape{8, 16}, StepsShape{8, 8},
                              StepsShape{4, 8}})
     if (const size_t need = vb * (size_t)(s.m + s.window + 2) + other;
         s.m <= m_max && need <= cap && need + reserve <= free_b + held)
@@ -2186,7 +2191,7 @@ StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max,
 
 // Blocks of several steps can fill the device; they are given back after the
 // call when they hold more than this.
-constexpr size_t kKeepBytes = (size_t)8 << 30;
+constexpr size_t kKeepBytes = (size_t)12 << 30;
 void trim(DevMem& m) {
   if (m.bytes > kKeepBytes) m.release();
 }

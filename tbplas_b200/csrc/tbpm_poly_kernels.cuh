@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(kQeMmaWarps * 32, 2) qe_filter_mma_kernel(
 
 // ---- several time steps from one expansion ----------------------------------------
 
-constexpr int kCombineWindow = 16;  // Chebyshev vectors per pass
+constexpr int kCombineWindow = 32;  // Chebyshev vectors per pass
 constexpr int kCombineSteps = 16;   // most time steps per expansion
 
 template <typename R>
@@ -1020,10 +1020,13 @@ struct CombineArgs {
 // 240 for 16 steps).  Sums in FP64; both kernels are bound by memory when their
 // loads are in flight early enough:
 //  combine_kernel (FP64): one value per thread, 16 accumulators, the weights
-//    compile-time offsets into the parameter bank.  Blocks of 196 MB: 1.04 ms a
-//    pass, 6.3 TB/s; the product on mma.sync took 1.30 ms.
-//  combine_mma_kernel (FP32): the same on 20 MB blocks took 329 us a pass, 1.9 TB/s, 8
-//    bytes a load and a conversion for every 32 FMAs; mma.sync takes 235 us.
+//    compile-time offsets into the parameter bank.  Blocks of 196 MB, 16 steps: 3.1 ms
+//    an expansion in windows of 32 vectors, 4.2 ms in windows of 16 (the outputs are
+//    read and written more often), 6.3 TB/s; the product on mma.sync took 25% more.
+//  combine_mma_kernel (FP32): blocks of 20 MB, 8 steps of 42 vectors: 0.61 ms an
+//    expansion; 0.83 ms with 8-byte loads, pointers from the parameter bank in the
+//    loop and windows of 16.  combine_kernel took 1.4 times that, with a conversion
+//    for every 32 FMAs.
 // p_0 may be an output: every p of a value is read before the value is written.
 template <typename R, int M>
 __global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__ CombineArgs<R> a) {
@@ -1070,58 +1073,85 @@ __global__ void __launch_bounds__(256, 2) combine_kernel(const __grid_constant__
     }
 }
 
-// W (16 x 16) . P (16 x values) on mma.sync m8n8k4 f64: a warp takes 8 values e at
-// a time, lane (g, t) loads p_tau of value g for tau = 4s + t; their real parts
-// are the 8 columns of one product, the imaginary parts those of another, so a
-// lane's accumulators are the real and imaginary parts of values 2t and 2t + 1
-// of output g.  W stays in registers.
-template <int MT>
-__global__ void __launch_bounds__(256, 3)
+// W (8 x window) . P (window x values) on mma.sync m8n8k4 f64.  A warp takes 16
+// values at a time: lane (g, t) loads p_tau of values 2g and 2g + 1 for tau = 4s + t;
+// the even and the odd values, real and imaginary parts, are the 8 columns of four
+// products, so that a lane's accumulators are values 4t .. 4t + 3 of output g: 32
+// bytes in a row.  W and the pointers (read by lane, so not from the parameter bank
+// in the loop) stay in registers.  WIDE: whole groups of four values at 16-byte
+// boundaries; else each value is checked and moved by itself.
+template <bool WIDE>
+__global__ void __launch_bounds__(256, 2)
     combine_mma_kernel(const __grid_constant__ CombineArgs<float> a) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   constexpr int NS = kCombineWindow / 4;
-  double w[MT][NS];
+  double w[NS];
+  const float2* p[NS];
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
+  for (int s = 0; s < NS; ++s) p[s] = 4 * s + t < a.np ? a.p[4 * s + t] : nullptr;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) w[m][s] = a.w[8 * m + g][4 * s + t];
-  const int64_t step = 8 * (int64_t)gridDim.x * (blockDim.x >> 5);
-  const float2 zero = make_float2(0.0f, 0.0f);
-  for (int64_t e0 = 8 * ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  for (int s = 0; s < NS; ++s) w[s] = a.w[g][4 * s + t];
+  const bool in = g >= a.j0 && g < a.m;
+  float2* const out = in ? a.out[g] : nullptr;
+  const int64_t step = 16 * (int64_t)gridDim.x * (blockDim.x >> 5);
+  // values e, e + 1
+  auto ld2 = [&](const float2* q, int64_t e) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if constexpr (WIDE) {
+      if (e < a.total) v = *reinterpret_cast<const float4*>(q + e);
+    } else {
+      if (e < a.total) {
+        const float2 u = q[e];
+        v.x = u.x;
+        v.y = u.y;
+      }
+      if (e + 1 < a.total) {
+        const float2 u = q[e + 1];
+        v.z = u.x;
+        v.w = u.y;
+      }
+    }
+    return v;
+  };
+  for (int64_t e0 = 16 * ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
        e0 < a.total; e0 += step) {
-    float2 x[NS];
+    float4 x[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s)
-      x[s] = e0 + g < a.total && 4 * s + t < a.np ? a.p[4 * s + t][e0 + g] : zero;
-    const int64_t e = e0 + 2 * t;
-    double re[MT][2], im[MT][2];
+      x[s] = p[s] ? ld2(p[s], e0 + 2 * g) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int64_t e = e0 + 4 * t;
+    double re[2][2], im[2][2];  // [odd value][column 2t, 2t + 1]
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const int j = 8 * m + g;
-      const bool in = !a.init && j >= a.j0 && j < a.m;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const float2 o = in && e + q < a.total ? a.out[j][e + q] : zero;
-        re[m][q] = (double)o.x;
-        im[m][q] = (double)o.y;
-      }
+    for (int q = 0; q < 2; ++q) {
+      float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (!a.init && in) o = ld2(out, e + 2 * q);
+      re[0][q] = (double)o.x;
+      im[0][q] = (double)o.y;
+      re[1][q] = (double)o.z;
+      im[1][q] = (double)o.w;
     }
 #pragma unroll
     for (int s = 0; s < NS; ++s)
-#pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        dmma_8x8x4(re[m][0], re[m][1], w[m][s], (double)x[s].x);
-        dmma_8x8x4(im[m][0], im[m][1], w[m][s], (double)x[s].y);
+      if (4 * s < a.np) {
+        dmma_8x8x4(re[0][0], re[0][1], w[s], (double)x[s].x);
+        dmma_8x8x4(im[0][0], im[0][1], w[s], (double)x[s].y);
+        dmma_8x8x4(re[1][0], re[1][1], w[s], (double)x[s].z);
+        dmma_8x8x4(im[1][0], im[1][1], w[s], (double)x[s].w);
       }
+    __syncwarp();  // an output may be p_0: the warp has read these values
+    if (in) {
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      const int j = 8 * m + g;
-      if (j >= a.j0 && j < a.m) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          if (e + q < a.total)
-            a.out[j][e + q] = make_float2((float)re[m][q], (float)im[m][q]);
+      for (int q = 0; q < 2; ++q) {
+        const float4 o = make_float4((float)re[0][q], (float)im[0][q], (float)re[1][q],
+                                     (float)im[1][q]);
+        const int64_t f = e + 2 * q;
+        if constexpr (WIDE) {
+          if (f < a.total) *reinterpret_cast<float4*>(out + f) = o;
+        } else {
+          if (f < a.total) out[f] = make_float2(o.x, o.y);
+          if (f + 1 < a.total) out[f + 1] = make_float2(o.z, o.w);
+        }
       }
     }
   }

@@ -293,8 +293,8 @@ def test_dyn_pol_long_run(sample, prec, tol):
 
 
 def test_steps_per_expansion_follow_the_free_memory():
-    """The same AC run with less and less free device memory (16, 8, 8 and 4
-    steps per expansion, then step by step): equal to rounding."""
+    """The same AC run with less and less free device memory (16, 8 and 4 steps per
+    expansion with windows of 32, 16 and 8 vectors, then step by step): equal to rounding."""
     import torch
     s = tb.make_graphene_sample(192, 192, disorder=1.0, rescale=9.0, seed=2)
     ip, ix, hv, dx, dy = s.build_ham_dxy()
@@ -309,7 +309,7 @@ def test_steps_per_expansion_follow_the_free_memory():
     try:
         want = f2py.tbpm_accond_states(*args)
         ctx.close()
-        for blocks in (30, 24, 16, 8):
+        for blocks in (44, 30, 24, 16, 8):
             nat._contexts[0] = ctx = nat.Context(0)
             f2py._ctx()
             torch.cuda.synchronize()

@@ -56,7 +56,7 @@ namespace tbpm {
 #define TBPM_RING_WARPS_SMALL 22  // the same for packs of 16 or 8 bytes
 #endif
 #ifndef TBPM_RING_WARPS_PLAIN
-#define TBPM_RING_WARPS_PLAIN 19  // consumer warps of the modes without an accumulator
+#define TBPM_RING_WARPS_PLAIN 19  // the same for mode 0 (recurrence only)
 #endif
 #ifndef TBPM_RING_MINB
 #define TBPM_RING_MINB 1  // resident blocks per SM the stages are sized for
@@ -81,8 +81,11 @@ constexpr unsigned long long kRingWaitNs = 2000000000ull;  // 2 s per wait
 #endif
 
 // Consumer warps per block by the size of a thread's pack and the kernel mode: a
-// thread holds one item's gathers, so more threads are more gathers in flight, as
-// far as the registers go.
+// thread holds one item's gathers, so more threads are more gathers in flight, but
+// their registers and the larger stages (which leave less L1 for the gathers) bound
+// them.  Measured on B200, 32-byte packs: AC (mostly mode 0, 24 FP64 columns) 552 ms
+// with 15, 559 with 17, 538 with 19, 591 with 20; moments (mode 3, 4.8M orbitals x 16)
+// FP64 100 ms with 15 and 107 with 16, FP32 42.7 with 15 and 44.4 with 19.
 template <typename R, int V, int MODE, bool WIN>
 constexpr int kRingWarps =
     sizeof(R) * V == 16 ? (MODE == 0 && !WIN ? TBPM_RING_WARPS_PLAIN : kRingConsumerWarps)
@@ -178,9 +181,11 @@ __device__ __forceinline__ uint64_t ring_evict_first_policy() {
   return p;
 }
 
-// Wait for the phase of parity `parity` of mbarrier `bar`, at most kRingWaitNs.
+// Wait for the phase of parity `parity` of mbarrier `bar`, at most about kRingWaitNs.
+// The clock is read only once the first tries have failed: a consumer waits once per
+// item, mostly on copies that have landed, and the read is on its critical path.
 __device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
-  const unsigned long long t0 = ring_clock_ns();
+  unsigned long long t0 = 0;
   for (;;) {
     for (int i = 0; i < 64; ++i) {
       uint32_t ok;
@@ -192,7 +197,9 @@ __device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity) {
           : "memory");
       if (ok) return true;
     }
-    if (ring_clock_ns() - t0 > kRingWaitNs) return false;
+    const unsigned long long now = ring_clock_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > kRingWaitNs) return false;
   }
 }
 
@@ -287,6 +294,8 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       record(wl, wcur);
       record(32 + wl, wnxt);
     }
+    int s = 0;          // i % S
+    uint32_t pass = 0;  // (i / S) & 1
     for (int64_t i = 0;; ++i) {
       int64_t r0;
       int nr;
@@ -317,11 +326,10 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       }
       const int j0 = __shfl_sync(0xffffffffu, cur0, (int)(i & 31));
       const int j1 = __shfl_sync(0xffffffffu, cur1, (int)(i & 31));
-      const int s = (int)(i % S);
       // the whole warp takes the same branch (the vote), so the shuffles above
       // stay convergent
       if (i >= S &&
-          !__all_sync(0xffffffffu, ring_wait(empty0 + 8u * s, (uint32_t)(((i / S) + 1) & 1)))) {
+          !__all_sync(0xffffffffu, ring_wait(empty0 + 8u * s, pass ^ 1u))) {
         ok = false;
         break;
       }
@@ -403,6 +411,10 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       }
       __syncwarp();
       ++issued;
+      if (++s == S) {
+        s = 0;
+        pass ^= 1u;
+      }
     }
     if (!ok && wl == 0) atomicOr(ra.status, 1u);
     // the last S tiles' copies must land before the block may end
@@ -417,16 +429,19 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
     const unsigned neg_bits = (unsigned)(a.c.neg_mask >> (lane * V)) & ((1u << V) - 1u);
     const unsigned set_bits = (unsigned)(a.c.set_mask >> (lane * V)) & ((1u << V) - 1u);
     const R beta = (R)a.c.beta;
+    const R alpha_re = (R)a.c.alpha_re, alpha_im = (R)a.c.alpha_im;
     constexpr bool do_corr = MODE == 2;
     const bool active = slot < TR;
     const bool ref_lane = do_corr && a.ref != nullptr && lane < a.ref_tpr;
     constexpr int GB = TBPM_RING_GATHER;
+    // stage and pass run along: as i % S and i / S they took two 64-bit divisions an item
+    int s = 0;
+    uint32_t pass = 0;
     for (int64_t i = 0;; ++i) {
       int64_t r0;
       int nr;
       if (!tile_of(i, &r0, &nr)) break;
-      const int s = (int)(i % S);
-      if (!__all_sync(0xffffffffu, ring_wait(full0 + 8u * s, (uint32_t)((i / S) & 1)))) {
+      if (!__all_sync(0xffffffffu, ring_wait(full0 + 8u * s, pass))) {
         if ((tid & 31) == 0) atomicOr(ra.status, 1u);
         break;
       }
@@ -489,7 +504,7 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
                         : lds_pack<R, V>(st + sh.own_off + te * sizeof(Pack<R, V>));
             if (a.diag) {
               constexpr int al = 16 / (int)sizeof(C);
-              const C d = reinterpret_cast<const C*>(st + sh.diag_off)[r - (r0 - r0 % al)];
+              const C d = reinterpret_cast<const C*>(st + sh.diag_off)[r - (r0 & ~(int64_t)(al - 1))];
 #pragma unroll
               for (int v = 0; v < V; ++v) {
                 sre[v] = d.x * own.v[2 * v] - d.y * own.v[2 * v + 1];
@@ -522,8 +537,8 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
 #pragma unroll
         for (int v = 0; v < V; ++v) {
           const bool neg = (neg_bits >> v) & 1u;
-          const R ar = (R)(neg ? -a.c.alpha_re : a.c.alpha_re);
-          const R ai = (R)(neg ? -a.c.alpha_im : a.c.alpha_im);
+          const R ar = neg ? -alpha_re : alpha_re;
+          const R ai = neg ? -alpha_im : alpha_im;
           pk.v[2 * v] = fma(ar, sre[v], fma(-ai, sim[v], beta * pm2.v[2 * v]));
           pk.v[2 * v + 1] = fma(ar, sim[v], fma(ai, sre[v], beta * pm2.v[2 * v + 1]));
         }
@@ -578,6 +593,10 @@ __global__ void __launch_bounds__((kRingItems<R, V, MODE, WIN> + 32), kRingMinBl
       }
       __syncwarp();
       if ((tid & 31) == 0) ring_arrive(empty0 + 8u * s);
+      if (++s == S) {
+        s = 0;
+        pass ^= 1u;
+      }
       if constexpr (MODE == 4) {
         // sums over the warp's rows (tpr is a power of two), one entry per
         // (tile, warp): partials[((tile*warps + warp)*ld + col)*2 + q]

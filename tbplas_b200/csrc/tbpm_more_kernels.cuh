@@ -375,26 +375,19 @@ __global__ void __launch_bounds__(T_MAX, 1)
     int i = 0;
     for (int64_t r = r0; r < k.n_rows && i < cap; r += stride, ++i) sw[i * T] = ld_c(w + r);
   }
-  // matrix entries of the current item
-  int j0 = 0, j1 = 0;
+  // columns and row bounds of the current item, row bounds of the next one
+  int j0 = 0, j1 = 0, n0 = 0, n1 = 0;
   int c[kHaydockDeg];
-  C h[kHaydockDeg];
-  C g;
-  g.x = g.y = (R)0;
-  auto load = [&](int64_t r) {
-    j0 = __ldg(k.indptr + r);
-    j1 = __ldg(k.indptr + r + 1);
+  auto next_row = [&](int64_t r) { return r + stride < k.n_rows ? r + stride : r0; };
+  if (r0 < k.n_rows) {
+    j0 = __ldg(k.indptr + r0);
+    j1 = __ldg(k.indptr + r0 + 1);
+    n0 = __ldg(k.indptr + next_row(r0));
+    n1 = __ldg(k.indptr + next_row(r0) + 1);
 #pragma unroll
-    for (int u = 0; u < kHaydockDeg; ++u) {
-      c[u] = -1;
-      if (j0 + u < j1) {
-        c[u] = __ldg(k.indices + j0 + u);
-        h[u] = ldg_c(k.hop + j0 + u);
-      }
-    }
-    if (k.diag) g = ldg_c(k.diag + r);
-  };
-  if (r0 < k.n_rows) load(r0);
+    for (int u = 0; u < kHaydockDeg; ++u)
+      c[u] = j0 + u < j1 ? __ldg(k.indices + j0 + u) : -1;
+  }
   __syncthreads();
   for (int d = 0; d < k.n_depth; ++d) {
     double cs[2] = {0.0, 0.0};
@@ -405,6 +398,21 @@ __global__ void __launch_bounds__(T_MAX, 1)
       for (int u = 0; u < kHaydockDeg; ++u)
         if (c[u] >= 0) x[u] = ld_c(w + c[u]);
       const C own = i < cap ? sw[i * T] : ld_c(w + r);
+      // beside the gathers: this item's values, the next one's columns and the
+      // bounds of the one after it
+      C h[kHaydockDeg];
+#pragma unroll
+      for (int u = 0; u < kHaydockDeg; ++u)
+        if (c[u] >= 0) h[u] = ldg_c(k.hop + j0 + u);
+      C g;
+      g.x = g.y = (R)0;
+      if (k.diag) g = ldg_c(k.diag + r);
+      int c_next[kHaydockDeg];
+#pragma unroll
+      for (int u = 0; u < kHaydockDeg; ++u)
+        c_next[u] = n0 + u < n1 ? __ldg(k.indices + n0 + u) : -1;
+      const int64_t r2 = next_row(next_row(r));
+      const int m0 = __ldg(k.indptr + r2), m1 = __ldg(k.indptr + r2 + 1);
       double vr = 0.0, vi = 0.0;
       if (k.diag) {
         vr = (double)g.x * (double)own.x - (double)g.y * (double)own.y;
@@ -430,7 +438,12 @@ __global__ void __launch_bounds__(T_MAX, 1)
             vi += (double)h[u].x * (double)x[u].y + (double)h[u].y * (double)x[u].x;
           }
       }
-      load(r + stride < k.n_rows ? r + stride : r0);
+#pragma unroll
+      for (int u = 0; u < kHaydockDeg; ++u) c[u] = c_next[u];
+      j0 = n0;
+      j1 = n1;
+      n0 = m0;
+      n1 = m1;
       C o;
       o.x = (R)(vr * s * k.rescale);
       o.y = (R)(vi * s * k.rescale);

@@ -2,7 +2,7 @@
 
 The reference's TBPM drivers hold their state inside one Fortran call
 (tbplas/fortran/tbpm.f90:6-93), so a run that is interrupted starts again from
-t = 0.  `dos_checkpointed` runs the same computation as `f2py.tbpm_dos` as a
+t = 0.  `dos_checkpointed` takes the time steps of `f2py.tbpm_dos` in a
 device-resident session and, every `every` time steps, writes what the run
 needs to go on to one .npz file:
 
@@ -14,8 +14,9 @@ needs to go on to one .npz file:
   precision, batch width, state distribution).
 
 Called again with the same inputs and path, it resumes from that file
-(tbpm_session_dos_resume) and returns exactly what an uninterrupted run
-returns.  A file whose fingerprint does not match is ignored.  The file is
+(tbpm_session_dos_resume) and returns exactly what an uninterrupted
+`dos_checkpointed` run returns.  (`f2py.tbpm_dos` computes runs of 64 steps or
+more from Chebyshev moments instead: the same curve to rounding.)  A file whose fingerprint does not match is ignored.  The file is
 written atomically (temporary file + rename) and removed when the run ends.
 
 `dc_checkpointed` does the same for f2py.tbpm_dccond (tbpm.f90:497-718) at the
@@ -91,7 +92,8 @@ def dos_checkpointed(bes, s_indptr, s_indices, s_hop, seed, n_timestep, n_ran_sa
     :param every: time steps between checkpoints
     :param on_checkpoint: called as on_checkpoint(first_state, rows_done)
         after every checkpoint write
-    :return: (n_timestep+1,) complex128 correlation, as f2py.tbpm_dos
+    :return: (n_timestep+1,) complex128 correlation, as f2py.tbpm_dos (bit for
+        bit below 64 steps, to rounding from there)
     """
     if every < 1:
         raise ValueError("every must be >= 1")

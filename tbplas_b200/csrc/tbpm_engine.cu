@@ -722,17 +722,17 @@ void launch_cooperative(tbpm_ctx* c, K kernel, int grid, int threads, size_t sme
 
 // Matrix and two vectors up to which one launch beats a launch per term (measured
 // on B200, us per term of the DOS moments, one launch / ring):
-//   FP64  131,072 orbitals x  8 states,  44 MB: 10.6 / 17.3
-//         720,000           x  1,        83 MB: 11.6 / 17.2
-//         320,000           x  5,        78 MB: 23.1 / 28.1
-//        1,280,000          x  1,       148 MB: 34.9 / 35.4
-//         720,000           x  4,       152 MB: 44.7 / 40.9
-//         320,000           x 16,       191 MB: 72.4 / 56.4
-//   FP32  720,000           x  4,        84 MB: 16.9 / 26.1
-//         320,000           x 16,        99 MB: 38.1 / 34.8
-#ifndef TBPM_PERSIST_MB
-#define TBPM_PERSIST_MB 90
-#endif
+//   FP64  131,072 orbitals x  8 states,  44 MB:  9.2 / 16.5
+//         720,000           x  1,        83 MB:  9.5 / 17.3
+//         320,000           x  5,        78 MB: 17.3 / 26.0
+//        1,280,000          x  1,       148 MB: 27.2 / 35.5
+//         720,000           x  4,       152 MB: 36.7 / 40.3
+//         320,000           x 16,       191 MB: 57.6 / 55.7
+//   FP32  720,000           x  4,        84 MB: 13.7 / 26.0
+//         320,000           x 16,        99 MB: 25.6 / 33.1
+// Moments reuse two vectors; windows of vectors and accumulators leave less of L2 to
+// each, so their line lies lower.
+constexpr double kPersistMoments = 160e6, kPersistOther = 90e6;
 // Launch shape of cheb_persist_kernel: for problems whose vectors and matrix stay
 // in L2; grid == 0 when it does not apply.
 struct PersistShape {
@@ -740,7 +740,7 @@ struct PersistShape {
 };
 
 template <typename R, int V>
-PersistShape persist_shape(const tbpm_ctx* c, int ld) {
+PersistShape persist_shape(const tbpm_ctx* c, int ld, double most = kPersistOther) {
   PersistShape s;
   const tbpm_options& o = c->opts;
   if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return s;
@@ -750,7 +750,7 @@ PersistShape persist_shape(const tbpm_ctx* c, int ld) {
   if (tpr > TMAX) return s;
   const double bytes = matrix_bytes(h) + 2.0 * (double)h.n * ld * 2 * sizeof(R);
   const int sms = num_sms(c->device);
-  if (bytes > TBPM_PERSIST_MB * 1e6) return s;
+  if (bytes > most) return s;
   const int64_t per_sm = (h.n + sms - 1) / sms;
   const int rpp = (int)std::min<int64_t>(std::max<int64_t>(per_sm, (128 + tpr - 1) / tpr),
                                          TMAX / tpr);
@@ -1543,7 +1543,7 @@ TermArgs<R, V> poly_term2(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr,
 template <typename R, int V>
 void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A,
                           Pack<R, V>* X, double* sums) {
-  const PersistShape ps = persist_shape<R, V>(c, ld);
+  const PersistShape ps = persist_shape<R, V>(c, ld, kPersistMoments);
   const int64_t n_vals = (int64_t)K * ld * 2;
   const double all_bytes =
       K * (matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R));
@@ -3101,8 +3101,9 @@ struct FrameCopies {
 };
 
 template <typename R>
-void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes, const double* psi0, const int32_t* time_log,
-               int n_log, int n_timestep, int chk_step, double chk_thr, double* psi_t) {
+void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes,
+               const double* psi0, const int32_t* time_log, int n_log, int n_timestep,
+               int chk_step, double chk_thr, double* psi_t) {
   constexpr int V = 1;
   c->graph.reset();
   ensure_vectors(c, 1, 1);

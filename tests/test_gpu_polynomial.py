@@ -96,7 +96,7 @@ def test_dos_long_run_of_general_matrices(n, degree, width):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
-@pytest.mark.parametrize("nx,ns", [(101, 1), (128, 2), (128, 16), (256, 1), (300, 3)])
+@pytest.mark.parametrize("nx,ns", [(101, 1), (128, 2), (128, 16), (256, 1), (300, 3), (580, 2)])
 def test_dos_long_run_block_shapes(prec, nx, ns):
     """From the last size of the cluster kernel to several items per thread of
     the largest blocks of the one-launch kernel, device-generated states."""

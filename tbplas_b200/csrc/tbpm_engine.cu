@@ -1916,6 +1916,31 @@ void dos_segmented_run(tbpm_ctx* c, const Expansion& ex, const std::vector<int64
     }
 }
 
+// Whether no entry of the resident Hamiltonian couples two realisations.  Moments
+// need that: <p_k|p_k> over a part of the rows is a moment of that part's states only
+// when H maps the part onto itself.
+bool segments_closed(tbpm_ctx* c, const std::vector<int64_t>& off) {
+  const int n_seg = (int)off.size() - 1;
+  int64_t max_len = 0;
+  for (int k = 0; k < n_seg; ++k) max_len = std::max<int64_t>(max_len, off[k + 1] - off[k]);
+  c->seg.ensure(sizeof(int64_t) * off.size());
+  c->poly.ensure(256);
+  TBPM_CK(cudaMemcpyAsync(c->seg.p, off.data(), sizeof(int64_t) * off.size(),
+                          cudaMemcpyHostToDevice, c->stream));
+  TBPM_CK(cudaMemsetAsync(c->poly.p, 0, sizeof(unsigned int), c->stream));
+  const unsigned chunks =
+      (unsigned)std::min<int64_t>(blocks_for(std::max<int64_t>(max_len, 1), 256), 64);
+  seg_closed_kernel<<<dim3(chunks, (unsigned)n_seg), 256, 0, c->stream>>>(
+      c->seg.as<int64_t>(), c->ham.indptr.as<int32_t>(), c->ham.indices.as<int32_t>(),
+      c->poly.as<unsigned int>());
+  TBPM_CK(cudaGetLastError());
+  c->launches++;
+  unsigned int coupled = 0;
+  TBPM_CK(cudaMemcpyAsync(&coupled, c->poly.p, sizeof coupled, cudaMemcpyDeviceToHost, c->stream));
+  TBPM_CK(cudaStreamSynchronize(c->stream));
+  return coupled == 0;
+}
+
 // dos_segmented_run by moments: the terms of all realisations run as one block
 // row-interleaved state block, seg_dots_kernel forms the two products of every
 // term per (segment, state).
@@ -3963,7 +3988,8 @@ void drv_dos_segmented(tbpm_ctx* c, const double* bes, int n_bes, const int64_t*
   c->model_bytes = 0;
   const Expansion ex = time_step_expansion(bes, n_bes);
   PolyPlan pp;
-  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
+                    segments_closed(c, off);
   dispatch(c->ham.prec, pick_V(c->ham.prec, n_states, n_states, c->opts.vector_width),
            [&](auto tag) {
              using P = decltype(tag);

@@ -21,6 +21,7 @@
 //  cheb_persist_kernel    all terms of a small problem in one launch.
 //  cheb_cluster_kernel    the same for a tiny one, in the shared memory of one
 //                         cluster.
+//  seg_closed_kernel      whether packed samples are uncoupled.
 //  seg_dots_kernel        the two products per (segment, state) of packed samples.
 //  filter_values_kernel,  the quasi-eigenstates' energy filters on the nodes and
 //  filter_coef_kernel     their Chebyshev coefficients.
@@ -702,6 +703,20 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
 }
 
 // ---- packed realisations ------------------------------------------------------
+
+// *coupled becomes nonzero when an entry leads from one realisation to another.
+// Block (row chunk, realisation), threads over rows.
+static __global__ void __launch_bounds__(256) seg_closed_kernel(const int64_t* seg_off,
+                                                                const int32_t* indptr,
+                                                                const int32_t* indices,
+                                                                unsigned int* coupled) {
+  const int64_t s0 = seg_off[blockIdx.y], s1 = seg_off[blockIdx.y + 1];
+  bool out = false;
+  for (int64_t r = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < s1;
+       r += (int64_t)gridDim.x * blockDim.x)
+    for (int j = indptr[r]; j < indptr[r + 1]; ++j) out |= indices[j] < s0 || indices[j] >= s1;
+  if (__syncthreads_or(out) && threadIdx.x == 0) atomicOr(coupled, 1u);
+}
 
 // <x|x> and Re <x|y> per (segment, column):
 // partials[((seg*ns + col)*2 + q)*n_chunks + chunk]; launch shape of seg_corr_kernel

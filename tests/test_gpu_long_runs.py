@@ -1,0 +1,48 @@
+"""Long runs at the edges of what their routes accept: packed samples that are not
+uncoupled, matrices that are Hermitian to rounding only, more terms than one launch
+or one buffer takes, memory that other buffers hold, and device waits that run out.
+The oracle and dense diagonalisation are the reference, FP64 to a relative 1e-10.
+"""
+
+import math
+
+import numpy as np
+import pytest
+
+import tbplas_b200 as tb
+from tbplas_b200 import _native as nat
+from tbplas_b200.fortran import f2py
+from oracle import oracle
+
+from conftest import bessel_series, rel_err, unit_states
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _backend():
+    f2py.set_backend(precision="fp64", batch=16, device=0, state_kind="exp", term_kernel=0,
+                     use_graphs=True, vector_width=0, threads_per_block=0, rows_per_tile=0)
+    yield
+    f2py.set_backend(precision="fp64", batch=16, term_kernel=0, vector_width=0)
+
+
+@pytest.mark.parametrize("n_t", [20, 80])
+def test_coupled_realisations(n_t):
+    """A matrix that couples the row ranges: each range's part of <psi(0)|psi(t)> on the
+    time-stepped route below and above 64 steps, and the norm check still refuses it."""
+    s = tb.make_graphene_sample(5, 4, disorder=1.0, rescale=9.0, seed=5)
+    h = s.build_ham_csr()
+    off = [0, 13, h.shape[0]]
+    bes = bessel_series(math.pi)
+    args = (bes, h.indptr, h.indices, h.data, off, 2, 11, n_t)
+    _, per = f2py.tbpm_dos_segmented(*args, 10 ** 6, 1e-9, per_state=True)
+    e, v = np.linalg.eigh(h.toarray())
+    for b in range(2):
+        parts = [oracle.random_state(off[k + 1] - off[k], 11 * (2 * k + b + 1)) for k in range(2)]
+        w = np.concatenate([p / np.linalg.norm(p) for p in parts])
+        wt = np.exp(-1j * math.pi * np.outer(e, np.arange(n_t + 1))) * (v.conj().T @ w)[:, None]
+        terms = w.conj()[:, None] * (v @ wt)
+        assert rel_err(per[:, b], [terms[:13].sum(0), terms[13:].sum(0)]) < 1e-10
+    with pytest.raises(nat.NormError):
+        f2py.tbpm_dos_segmented(*args, 16, 1e-9)

@@ -1328,6 +1328,12 @@ constexpr double kPolyMargin = 1.01;
 // With a norm-check threshold below this the check would see the rounding of
 // the time steps themselves; such a run is time-stepped.
 constexpr double kPolyMinThr = 1e-11;
+// Largest |tau| T |(H - H^+)/2| of a run.  Time stepping lets the states grow or decay
+// with the anti-Hermitian part of H, moments take H as Hermitian: the product bounds what
+// that changes in a curve (FP32: the states' own rounding is above it), and twice the
+// product is the largest drift of the squared norm, of which the norm check has to see
+// anything near its threshold.
+constexpr double kPolySkew64 = 1e-11, kPolySkew32 = 1e-5;
 
 struct PolyPlan {
   float alpha = 0;         // 2/a, a float, so that both precisions run the same y = H/a
@@ -1342,7 +1348,7 @@ const Spectrum& ham_spectrum(tbpm_ctx* c) {
   const Ham& h = c->ham;
   if (sp.gen == h.gen && h.gen != 0) return sp;
   c->poly.ensure(256);
-  TBPM_CK(cudaMemsetAsync(c->poly.p, 0, 16, c->stream));
+  TBPM_CK(cudaMemsetAsync(c->poly.p, 0, 3 * sizeof(unsigned long long), c->stream));
   const int grid = (int)std::min<int64_t>(blocks_for(h.n, 256), (int64_t)num_sms(c->device) * 16);
   auto launch = [&](auto tag) {
     using R = decltype(tag);
@@ -1359,11 +1365,12 @@ const Spectrum& ham_spectrum(tbpm_ctx* c) {
     launch(float{});
   TBPM_CK(cudaGetLastError());
   c->launches++;
-  unsigned long long info[2];
+  unsigned long long info[3];
   TBPM_CK(cudaMemcpyAsync(info, c->poly.p, sizeof info, cudaMemcpyDeviceToHost, c->stream));
   TBPM_CK(cudaStreamSynchronize(c->stream));
   std::memcpy(&sp.bound, &info[0], sizeof(double));
-  sp.hermitian = info[1] == 0;
+  std::memcpy(&sp.skew, &info[1], sizeof(double));
+  sp.hermitian = info[2] == 0;
   sp.gen = h.gen;
   return sp;
 }
@@ -1409,6 +1416,9 @@ bool poly_route(tbpm_ctx* c, const double* bes, int n_bes, int n_timestep, int c
   for (int k = 1; k < n_bes; k += 2) tau += 2.0 * k * bes[k];
   pp->tau = tau;
   if (!(std::fabs(tau) < 1e3)) return false;
+  double drift = c->ham.prec == TBPM_PREC_FP64 ? kPolySkew64 : kPolySkew32;
+  if (check) drift = std::min(drift, 0.25 * effective_thr(c, chk_thr));
+  if (!(std::fabs(tau) * n_timestep * sp.skew <= drift)) return false;
   for (int j = 0; j <= 64; ++j) {
     const long double x = pp->a * (long double)(j - 32) / 32.0L;
     long double re, im;

@@ -189,6 +189,7 @@ struct Spectrum {
   uint64_t gen = 0;
   bool hermitian = false;
   double bound = 0;  // Gershgorin: every eigenvalue lies in [-bound, bound]
+  double skew = 0;   // the same of the anti-Hermitian part
 };
 
 struct Session {

@@ -15,7 +15,7 @@
 // 1.8 ms; 20 packed samples, 4 states, 128 steps: 178 -> 40 ms.  The error against
 // exact propagation stays where it was (1e-15 to 1e-14).
 //
-//  ham_spectrum_kernel    Gershgorin bound of H and whether H is Hermitian.
+//  ham_spectrum_kernel    Gershgorin bounds of H and of its anti-Hermitian part.
 //  moment_density_kernel  moments -> weights rho_j of Gauss-Chebyshev nodes.
 //  moment_curve_kernel    C(t) = sum_j P(x_j)^t rho_j, and the norms.
 //  cheb_persist_kernel    all terms of a small problem in one launch.
@@ -41,8 +41,9 @@ namespace tbpm {
 constexpr int kSpectrumMaxRow = 64;
 
 // info[0]: largest row sum |D_r| + sum_j |O_rj| (the bits of a non-negative
-// double, ordered like it), info[1]: nonzero when H is not Hermitian to `tol`
-// (relative) or a row is longer than kSpectrumMaxRow.  One thread per row; a
+// double, ordered like it), info[1]: the same of the anti-Hermitian part
+// (H - H^+)/2, info[2]: nonzero when an entry is not the conjugate of its transpose
+// to `tol` (relative) or a row is longer than kSpectrumMaxRow.  One thread per row; a
 // row's transposed entries lie in its neighbours' rows, which are near in
 // memory.  Runs once per Hamiltonian.
 template <typename R>
@@ -52,15 +53,16 @@ __global__ void __launch_bounds__(256) ham_spectrum_kernel(const int32_t* indptr
                                                            const typename Cx<R>::t* diag,
                                                            int64_t n, double tol,
                                                            unsigned long long* info) {
-  double bound = 0.0;
+  double bound = 0.0, skew = 0.0;
   bool bad = false;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x) {
     const int j0 = indptr[r], j1 = indptr[r + 1];
-    double s = 0.0;
+    double s = 0.0, sk = 0.0;
     if (diag) {
       const typename Cx<R>::t d = diag[r];
       s = fabs((double)d.x);
+      sk = fabs((double)d.y);
       if (!(fabs((double)d.y) <= tol * fmax(1.0, s))) bad = true;
     }
     if (j1 - j0 > kSpectrumMaxRow) {
@@ -90,15 +92,21 @@ __global__ void __launch_bounds__(256) ham_spectrum_kernel(const int32_t* indptr
         }
       const double lim = tol * (fabs(fr) + fabs(fi));
       if (!(fabs(fr - br) <= lim && fabs(fi + bi) <= lim)) bad = true;
+      sk += 0.5 * hypot(fr - br, fi + bi);
     }
     if (!(s <= 1e300)) bad = true;
     bound = fmax(bound, s);
+    skew = fmax(skew, sk);
   }
-  for (int w = 16; w > 0; w >>= 1) bound = fmax(bound, __shfl_xor_sync(0xffffffffu, bound, w));
+  for (int w = 16; w > 0; w >>= 1) {
+    bound = fmax(bound, __shfl_xor_sync(0xffffffffu, bound, w));
+    skew = fmax(skew, __shfl_xor_sync(0xffffffffu, skew, w));
+  }
   const bool any = __any_sync(0xffffffffu, bad);
   if ((threadIdx.x & 31) == 0) {
     atomicMax(info, (unsigned long long)__double_as_longlong(bound));
-    if (any) atomicOr(info + 1, 1ull);
+    atomicMax(info + 1, (unsigned long long)__double_as_longlong(skew));
+    if (any) atomicOr(info + 2, 1ull);
   }
 }
 

@@ -8,6 +8,7 @@ import math
 
 import numpy as np
 import pytest
+import scipy.sparse as sp
 
 import tbplas_b200 as tb
 from tbplas_b200 import _native as nat
@@ -46,3 +47,32 @@ def test_coupled_realisations(n_t):
         assert rel_err(per[:, b], [terms[:13].sum(0), terms[13:].sum(0)]) < 1e-10
     with pytest.raises(nat.NormError):
         f2py.tbpm_dos_segmented(*args, 16, 1e-9)
+
+
+def _lossy(eps):
+    """A sample with -i eps on every site: the states decay by exp(-eps tau t)."""
+    h = tb.make_graphene_sample(3, 2, disorder=1.0, rescale=9.0, seed=5).build_ham_csr()
+    h = sp.csr_matrix(h - 1j * eps * sp.identity(h.shape[0]))
+    h.sort_indices()
+    return h
+
+
+def test_loss_below_the_hermiticity_tolerance_reaches_the_norm_check():
+    """2 eps tau t = 2.9e-11 at the check, the threshold is 1e-11."""
+    h = _lossy(9e-15)
+    wf0 = unit_states(1, h.shape[0], seed=1)
+    bes = bessel_series(math.pi)
+    with pytest.raises(nat.NormError):
+        f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, 512, 512, 1e-11)
+    f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, 512, 512, 1e-9)
+
+
+@pytest.mark.parametrize("n_t", [300, 16384])
+def test_loss_below_the_hermiticity_tolerance_over_long_runs(n_t):
+    """The decay grows with the run: 8e-12 and 4.6e-10 at its end."""
+    h = _lossy(9e-15)
+    wf0 = unit_states(1, h.shape[0], seed=1)
+    bes = bessel_series(math.pi)
+    got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, n_t, 10 ** 6, 1e-9)
+    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, n_t, wf0=wf0)
+    assert rel_err(got, ref) < 1e-10

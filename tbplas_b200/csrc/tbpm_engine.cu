@@ -1991,8 +1991,9 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
   const SegTiles st = seg_tiles<R, V>(c, off, tpr);
   const int64_t seg_stride = (int64_t)st.n_tiles * st.warps * ns * 2;
   const int64_t per_term = std::max<int64_t>((int64_t)n_cols * 2 * dot_chunks, seg_stride);
-  const int chunk =
-      (int)std::max<int64_t>(1, std::min<int64_t>(K + 1, (64ll << 20) / (per_term * 8)));
+  // (a chunk's terms are the y axis of seg_tile_reduce_kernel's grid: 65,535 at most)
+  const int chunk = (int)std::max<int64_t>(
+      1, std::min<int64_t>({(int64_t)K + 1, (64ll << 20) / (per_term * 8), (int64_t)65535}));
   ensure_partials(c, std::max<size_t>((size_t)chunk * per_term, (size_t)n_cols * n_chunks));
   c->small.ensure(sizeof(double) * std::max<size_t>((size_t)n_cols, kMaxCols * 2));
   c->out.ensure((size_t)(T + 3) * n_cols * 2 * sizeof(double));

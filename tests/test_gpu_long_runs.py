@@ -76,3 +76,17 @@ def test_loss_below_the_hermiticity_tolerance_over_long_runs(n_t):
     got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, n_t, 10 ** 6, 1e-9)
     ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, n_t, wf0=wf0)
     assert rel_err(got, ref) < 1e-10
+
+
+@pytest.mark.parametrize("ns", [1, 2])
+def test_packed_run_of_more_terms_than_a_grid_axis(ns):
+    """50,000 steps of one tiny realisation: 75,000 terms whose sums are reduced
+    together, where a grid has 65,535 blocks on its second axis."""
+    h = tb.make_graphene_sample(2, 2, disorder=1.0, rescale=8.7, seed=3).build_ham_csr()
+    bes = bessel_series(math.pi)
+    _, per = f2py.tbpm_dos_segmented(bes, h.indptr, h.indices, h.data, [0, h.shape[0]], ns, 11,
+                                     50000, 128, 1e-9, per_state=True)
+    for b in range(ns):
+        ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 50000, seed=11 * (b + 1),
+                              n_samples=1)
+        assert rel_err(per[0, b], ref) < 1e-10

@@ -799,10 +799,12 @@ void launch_persist(tbpm_ctx* c, const PersistShape& s, const PersistArgs<R, V>&
 #ifndef TBPM_CLUSTER_ITEMS
 #define TBPM_CLUSTER_ITEMS kClusterItems  // (0: off)
 #endif
-// The moments' terms 1..K of a tiny problem by cheb_cluster_kernel: block partials
-// to c->partials, the number of blocks returned (0: it does not apply).
+// The moments' terms k0..k1 of a tiny problem by cheb_cluster_kernel: block partials
+// to c->partials, the number of blocks returned (0: it does not apply).  The even
+// vectors are in A, the odd ones in X; both are written back when `keep`.
 template <typename R, int V>
-int launch_cluster(tbpm_ctx* c, double alpha, int K, int ld, const Pack<R, V>* p0) {
+int launch_cluster(tbpm_ctx* c, double alpha, int k0, int k1, bool keep, int ld, Pack<R, V>* A,
+                   Pack<R, V>* X) {
   const tbpm_options& o = c->opts;
   if (o.term_kernel != 0 || o.threads_per_block > 0 || o.rows_per_tile > 0) return 0;
   const Ham& h = c->ham;
@@ -838,7 +840,7 @@ int launch_cluster(tbpm_ctx* c, double alpha, int K, int ld, const Pack<R, V>* p
     (void)cudaGetLastError();
     return 0;
   }
-  ensure_partials(c, (size_t)K * ld * 2 * kClusterBlocks);
+  ensure_partials(c, (size_t)(k1 - k0 + 1) * ld * 2 * kClusterBlocks);
   ClusterArgs<R, V> a;
   a.indptr = h.indptr.as<int32_t>();
   a.indices = h.indices.as<int32_t>();
@@ -846,9 +848,12 @@ int launch_cluster(tbpm_ctx* c, double alpha, int K, int ld, const Pack<R, V>* p
   a.diag = h.has_diag ? h.diag.as<typename Cx<R>::t>() : nullptr;
   a.n_rows = (int)h.n;
   a.tpr = tpr;
-  a.p0 = p0;
+  a.even = A;
+  a.odd = X;
   a.alpha = alpha;
-  a.n_terms = K;
+  a.k0 = k0;
+  a.k1 = k1;
+  a.keep = keep ? 1 : 0;
   a.rows = rows;
   a.magic = (unsigned)(((1ull << 32) + rows - 1) / rows);
   a.partials = c->partials.as<double>();
@@ -1548,58 +1553,61 @@ TermArgs<R, V> poly_term2(const tbpm_ctx* c, const PolyPlan& pp, int k, int tpr,
   return poly_term<R, V>(c, pp, k, tpr, (k & 1) ? A : X, dst, dst);
 }
 
+// Terms whose block partials are reduced together: as many as fit 64 MB.
+int moment_chunk(int terms, int64_t doubles_per_term) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(terms, (64ll << 20) / (doubles_per_term * 8)));
+}
+
 // Terms 1..K with the products of every term: sums[((k-1)*ld + col)*2 + q],
 // q = 0: <p_k|p_k>, 1: Re <p_k|p_{k-1}>.  p_0 is in A, X is scratch.
 template <typename R, int V>
 void enqueue_moment_terms(tbpm_ctx* c, const PolyPlan& pp, int K, int ld, Pack<R, V>* A,
                           Pack<R, V>* X, double* sums) {
-  const PersistShape ps = persist_shape<R, V>(c, ld, kPersistMoments);
-  const int64_t n_vals = (int64_t)K * ld * 2;
-  const double all_bytes =
-      K * (matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R));
-  if (const int blocks = launch_cluster<R, V>(c, pp.alpha, K, ld, A)) {
+  const double bytes = matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R);
+  int k0 = 1;
+  // every route leaves p_k in A (k even) or X (k odd), where the next chunk takes it
+  auto reduce = [&](int terms, int blocks) {
+    const int64_t n_vals = (int64_t)terms * ld * 2;
     reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), blocks, n_vals, sums);
+        c->partials.as<double>(), blocks, n_vals, sums + (int64_t)(k0 - 1) * ld * 2);
     TBPM_CK(cudaGetLastError());
     c->launches++;
-    c->model_bytes += all_bytes;
-    return;
+    c->model_bytes += terms * bytes;
+    k0 += terms;
+  };
+  while (k0 <= K) {
+    const int m = moment_chunk(K - k0 + 1, (int64_t)ld * 2 * kClusterBlocks);
+    const int blocks = launch_cluster<R, V>(c, pp.alpha, k0, k0 + m - 1, k0 + m <= K, ld, A, X);
+    if (blocks == 0) break;
+    reduce(m, blocks);
   }
-  if (ps.grid > 0) {
-    ensure_partials(c, (size_t)n_vals * ps.grid);
+  if (k0 > K) return;
+  const PersistShape ps = persist_shape<R, V>(c, ld, kPersistMoments);
+  while (ps.grid > 0 && k0 <= K) {
+    const int m = moment_chunk(K - k0 + 1, (int64_t)ld * 2 * ps.grid);
+    ensure_partials(c, (size_t)m * ld * 2 * ps.grid);
     Pack<R, V>* ring[2] = {A, X};
-    PersistArgs<R, V> a = persist_args<R, V>(c, pp.alpha, 1, K, ld, A, ring, 2, false);
+    PersistArgs<R, V> a =
+        persist_args<R, V>(c, pp.alpha, k0, k0 + m - 1, ld, A, ring, 2, false);
     a.k_dots = K;
     a.partials = c->partials.as<double>();
     launch_persist<false>(c, ps, a);
-    c->model_bytes += all_bytes;
-    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), ps.grid, n_vals, sums);
-    TBPM_CK(cudaGetLastError());
-    c->launches++;
-    return;
+    reduce(m, ps.grid);
   }
+  if (k0 > K) return;
   const int tpr = ld / V;
   const TermTiles tt = term_tiles<R, V>(c, c->ham.n, tpr);
   const int grid = tt.t[3].grid;
   const int64_t per_term = (int64_t)ld * 2 * grid;
-  // block partials of as many terms as fit 64 MB, then one reduction of them all
-  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(K, (64ll << 20) / (per_term * 8)));
-  ensure_partials(c, (size_t)chunk * per_term);
-  const double bytes = matrix_bytes(c->ham) + 3.0 * (double)c->ham.n * ld * 2 * sizeof(R);
-  for (int k0 = 1; k0 <= K; k0 += chunk) {
-    const int m = std::min(chunk, K - k0 + 1);
+  ensure_partials(c, (size_t)moment_chunk(K, per_term) * per_term);
+  while (k0 <= K) {
+    const int m = moment_chunk(K - k0 + 1, per_term);
     for (int i = 0; i < m; ++i) {
       TermArgs<R, V> a = poly_term2<R, V>(c, pp, k0 + i, tpr, A, X);
       a.partials = c->partials.as<double>() + (int64_t)i * per_term;
       launch_term<R, V>(c, tt, a);
-      c->model_bytes += bytes;
     }
-    const int64_t n_vals = (int64_t)m * ld * 2;
-    reduce_rows_kernel<<<(int)std::min<int64_t>(n_vals, 65535), 256, 0, c->stream>>>(
-        c->partials.as<double>(), grid, n_vals, sums + (int64_t)(k0 - 1) * ld * 2);
-    TBPM_CK(cudaGetLastError());
-    c->launches++;
+    reduce(m, grid);
   }
 }
 
@@ -2451,7 +2459,7 @@ void dc_filter(tbpm_ctx* c, const PolyPlan& pp, int nb, const Pack<R, V>* W, int
   const TermTiles tt = term_tiles<R, V>(c, n, tpr);
   const int grid3 = tt.t[3].grid;
   const int64_t per_term = (int64_t)nb * 2 * grid3;
-  const int chunk = (int)std::max<int64_t>(1, std::min<int64_t>(K, (64ll << 20) / (per_term * 8)));
+  const int chunk = moment_chunk(K, per_term);
   ensure_partials(c, (size_t)chunk * per_term);
   auto vec = [&](int k) -> Pack<R, V>* {
     return k == 0 ? const_cast<Pack<R, V>*>(W)

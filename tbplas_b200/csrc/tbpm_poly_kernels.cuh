@@ -520,12 +520,14 @@ struct ClusterArgs {
   const typename Cx<R>::t* diag;
   int n_rows;
   int tpr;
-  const Pack<R, V>* p0;
+  Pack<R, V>* even;    // p_{k0-1} and p_{k0-2} (absent at k0 = 1) by their parity;
+  Pack<R, V>* odd;     // with `keep`, p_{k1} and p_{k1-1} on return
   double alpha;        // 2 / a
-  int n_terms;
+  int k0, k1;          // terms k0 <= k <= k1 of this launch
+  int keep;
   int rows;            // rows per block: block q owns rows [q*rows, (q+1)*rows)
   unsigned int magic;  // ceil(2^32 / rows): c / rows = umulhi(c, magic) for c*rows < 2^32
-  double* partials;    // [((k-1)*ld*2 + col*2 + q) * gridDim.x + block]
+  double* partials;    // [((k-k0)*ld*2 + col*2 + q) * gridDim.x + block]
 };
 
 constexpr int kClusterBlocks = 16;
@@ -592,8 +594,11 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
   const uint32_t odd = (uint32_t)(vec * sizeof(Pack<R, V>));
   const int width = tpr * V * 2;
   const bool any = slot < rpp && slot < n_own;
-  for (int q = threadIdx.x; q < n_own * tpr; q += blockDim.x)
-    buf[q] = a.p0[(int64_t)r_base * tpr + q];
+  for (int q = threadIdx.x; q < n_own * tpr; q += blockDim.x) {
+    const int64_t e = (int64_t)r_base * tpr + q;
+    buf[q] = a.even[e];
+    if (a.k0 > 1) buf[vec + q] = a.odd[e];
+  }
   // matrix entries of the thread's items; ca: address of a neighbour in p_even
   constexpr int NI = kClusterItems;
   int j0[NI], j1[NI];
@@ -624,7 +629,7 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
   }
   cluster_sync();
   const R alpha2 = (R)a.alpha, alpha1 = (R)(0.5 * a.alpha);
-  for (int k = 1; k <= a.n_terms; ++k) {
+  for (int k = a.k0; k <= a.k1; ++k) {
     const uint32_t so = (k & 1) ? 0u : odd;  // p_{k-1}
     const Pack<R, V>* src = buf + ((k & 1) ? 0 : vec);
     Pack<R, V>* dst = buf + ((k & 1) ? vec : 0);
@@ -686,7 +691,7 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
       }
     }
     // products per thread, reduced in batches as in cheb_persist_kernel
-    const int bs = (k - 1) % kPersistBatch;
+    const int bs = (k - a.k0) % kPersistBatch;
     if (slot < rpp) {
 #pragma unroll
       for (int v = 0; v < V; ++v) {
@@ -695,10 +700,10 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
       }
     }
     cluster_sync();
-    if (bs == kPersistBatch - 1 || k == a.n_terms) {
+    if (bs == kPersistBatch - 1 || k == a.k1) {
       const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31;
       const int full = blockDim.x >> 5;  // a partial last warp takes no part
-      const int64_t k_first = k - 1 - bs;
+      const int64_t k_first = k - a.k0 - bs;
       for (int q = warp < full ? warp : (bs + 1) * width; q < (bs + 1) * width; q += full) {
         double t = 0.0;
         for (int i = wl; i < rpp; i += 32) t += psm[q * rpp + i];
@@ -708,6 +713,12 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
       __syncthreads();  // the batch's slots are free again
     }
   }
+  if (a.keep)
+    for (int q = threadIdx.x; q < n_own * tpr; q += blockDim.x) {
+      const int64_t e = (int64_t)r_base * tpr + q;
+      a.even[e] = buf[q];
+      a.odd[e] = buf[vec + q];
+    }
 }
 
 // ---- packed realisations ------------------------------------------------------

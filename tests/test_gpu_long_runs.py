@@ -90,3 +90,30 @@ def test_packed_run_of_more_terms_than_a_grid_axis(ns):
         ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 50000, seed=11 * (b + 1),
                               n_samples=1)
         assert rel_err(per[0, b], ref) < 1e-10
+
+
+@pytest.mark.parametrize("nx,ns,n_t", [(40, 16, 8192), (16, 64, 16384)])
+def test_memory_of_long_runs_is_bounded(nx, ns, n_t):
+    """The one-launch and the cluster route in several launches (block partials of 450
+    and 400 MB all together): the context grows by 64 MB of them, and the curve is the
+    ring route's."""
+    import torch
+    h = tb.make_graphene_sample(nx, nx, disorder=1.0, rescale=9.0, seed=3).build_ham_csr()
+    bes = bessel_series(math.pi)
+    f2py.set_backend(batch=64)
+    kept, nat._contexts = nat._contexts, {0: nat.Context(0)}
+    try:
+        def run(steps, states):
+            return f2py.tbpm_dos(bes, h.indptr, h.indices, h.data, 7, steps, states, "", 0, 128,
+                                 1e-9)
+        run(2, 1)
+        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info(0)
+        got = run(n_t, ns)
+        used = free - torch.cuda.mem_get_info(0)[0]
+        f2py.set_backend(term_kernel=2)
+        assert rel_err(got, run(n_t, ns)) < 1e-10
+        assert used < 200e6
+    finally:
+        nat._contexts[0].close()
+        nat._contexts = kept

@@ -2209,27 +2209,36 @@ struct StepsShape {
   int window = 0;
 };
 
-// The largest shape whose states and ring, beside `other` bytes, fit the memory
-// that is free or held by the buffers they go into.  Model of a step of phase
-// pi/2 in passes over the block (time stepping: 57): 18 at (16, 32), 20 at (16, 16),
-// 24 at (8, 16), 27 at (8, 8), 36 at (4, 8).  Windows of 32 instead of 16 vectors: AC
-// 561 -> 541 ms (256,000 cells x 8 states), FP32 DC 201 -> 183 ms.  FP32 states take 8
-// steps at most: the 16 outputs' FP64 products cost more than the terms they save
-// (DC 183 ms at 8, 212 ms at 16).
-StepsShape steps_that_fit(size_t vb, size_t other, size_t held, int m_max,
-                          size_t cap = SIZE_MAX) {
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return StepsShape{};
-  }
+// Reserves `mem` for the states and the window of the largest shape that fits, with
+// `extra` further blocks: m + window + extra blocks of vb bytes, beside `other` bytes of
+// buffers to come, in the memory that is free or held by `mem` itself.  (What another
+// buffer holds from an earlier, larger call is not free.)  Someone else may take memory
+// after the query; a shape whose allocation fails is passed over for the next one.
+// Model of a step of phase pi/2 in passes over the block (time stepping: 57): 18 at
+// (16, 32), 20 at (16, 16), 24 at (8, 16), 27 at (8, 8), 36 at (4, 8).  Windows of 32
+// instead of 16 vectors: AC 561 -> 541 ms (256,000 cells x 8 states), FP32 DC 201 -> 183
+// ms.  FP32 states take 8 steps at most: the 16 outputs' FP64 products cost more than the
+// terms they save (DC 183 ms at 8, 212 ms at 16).
+StepsShape reserve_steps(DevMem& mem, size_t vb, int extra, size_t other, int m_max,
+                         size_t cap = SIZE_MAX) {
   const size_t reserve = (size_t)2 << 30;
   for (const StepsShape s : {StepsShape{16, kCombineWindow}, StepsShape{16, 16},
                              StepsShape{8, kCombineWindow}, StepsShape{8, 16}, StepsShape{8, 8},
-                             StepsShape{4, 8}})
-    if (const size_t need = vb * (size_t)(s.m + s.window + 2) + other;
-        s.m <= m_max && need <= cap && need + reserve <= free_b + held)
+                             StepsShape{4, 8}}) {
+    const size_t need = vb * (size_t)(s.m + s.window + extra);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return StepsShape{};
+    }
+    if (s.m > m_max || need > cap || need + other + reserve > free_b + mem.bytes) continue;
+    try {
+      mem.ensure(need);
       return s;
+    } catch (const Error& e) {
+      if (e.code != TBPM_ERR_OOM) throw;
+    }
+  }
   return StepsShape{};
 }
 
@@ -2244,14 +2253,16 @@ void trim(DevMem& m) {
 // and Y serve as two blocks of the ring), reserved before c->A is filled.
 template <typename R>
 StepsShape steps_room(tbpm_ctx* c, const PolyPlan* pp, int ld, int ref_ld) {
-  if (!pp) return StepsShape{};
-  const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
-  // the reference block, and the staging of states that come from the host
-  const size_t ref = (size_t)c->ham.n * ref_ld * (2 * sizeof(R) + 16);
-  const StepsShape s =
-      steps_that_fit(vb, vb + ref, c->A.bytes + c->X.bytes + c->Y.bytes + c->wf0.bytes,
-                     most_steps<R>);
-  if (s.m > 0) c->A.ensure(vb * (size_t)(1 + s.window + s.m));
+  StepsShape s;
+  if (pp) {
+    const size_t vb = (size_t)c->ham.n * ld * 2 * sizeof(R);
+    c->X.ensure(vb);
+    c->Y.ensure(vb);
+    c->wf0.ensure((size_t)c->ham.n * ref_ld * 2 * sizeof(R));
+    // still to come: the staging of states that come from the host
+    s = reserve_steps(c->A, vb, 1, (size_t)c->ham.n * ref_ld * 16, most_steps<R>);
+  }
+  ensure_vectors(c, ld, ref_ld);
   return s;
 }
 
@@ -2297,7 +2308,6 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
   const int ld = 3 * nb;
   c->graph.reset();
   const StepsShape shape = steps_room<R>(c, pp, ld, nb);
-  ensure_vectors(c, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * nb * 9 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
   auto* X = c->X.as<Pack<R, V>>();
@@ -2756,11 +2766,8 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
       const size_t budget = (size_t)(c->opts.dc_budget_gb * 1073741824.0);
       cap = budget > qe_bytes ? budget - qe_bytes : 0;
     }
-    shape = steps_that_fit(vb, vb * T2, c->A.bytes + c->X.bytes + c->Y.bytes, most_steps<R>,
-                           cap);
-    if (shape.m > 0) {
-      c->A.ensure(vb * (size_t)(shape.m + shape.window + 2 + T2));
-    } else {
+    shape = reserve_steps(c->A, vb, 2 + T2, 0, most_steps<R>, cap);
+    if (shape.m == 0) {
       c->X.ensure(vb);
       c->Y.ensure(vb);
       c->A.ensure(vb * (size_t)(T2 + 1));
@@ -2847,7 +2854,6 @@ void dynpol_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fer
   const int tpr = nq * nb;
   c->graph.reset();
   const StepsShape shape = steps_room<R>(c, pp, ld, nb);
-  ensure_vectors(c, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * tpr * 3 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
   auto* X = c->X.as<Pack<R, V>>();

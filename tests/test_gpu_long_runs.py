@@ -117,3 +117,31 @@ def test_memory_of_long_runs_is_bounded(nx, ns, n_t):
     finally:
         nat._contexts[0].close()
         nat._contexts = kept
+
+
+def test_buffers_of_an_earlier_call_are_not_free_memory():
+    """Vectors of 1.07 GB held from a larger call and 0.13 GB free: several steps per
+    expansion (1.4 GB) do not fit, although 3.3 GB are free or held together."""
+    import torch
+    s = tb.make_graphene_sample(192, 192, disorder=1.0, rescale=9.0, seed=2)
+    ip, ix, hv, dx, dy = s.build_ham_dxy()
+    bes = bessel_series(math.pi / 2)
+    args = (bes, 40.0, 0.0, ip, ix, hv, s.rescale, dx, dy, 3, 64, 8, 2 ** 12, 1e-12, "", 0, 128,
+            1e-9)
+    want = f2py.tbpm_accond(*args)
+    big = tb.make_graphene_device_sample(1024, 512, rescale=9.0, seed=2).build_ham_csr()
+    kept, nat._contexts = nat._contexts, {0: nat.Context(0)}
+    hold = None
+    try:
+        f2py.set_backend(batch=64)
+        f2py.tbpm_dos(bes, big.indptr, big.indices, big.data, 7, 2, 64, "", 0, 128, 1e-9)
+        f2py.set_backend(batch=16)
+        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info(0)
+        hold = torch.empty(free - (128 << 20), dtype=torch.uint8, device="cuda")
+        assert rel_err(f2py.tbpm_accond(*args), want) < 1e-12
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+        nat._contexts[0].close()
+        nat._contexts = kept

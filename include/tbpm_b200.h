@@ -415,6 +415,13 @@ int tbpm_cheb_timestep_noalloc(tbpm_ctx* ctx, const double* bes, int n_bes,
  * propagation whose wait ran out would, and the context stays usable. */
 int tbpm_selftest_wait_timeout(tbpm_ctx* ctx);
 
+/* The same for the kernels with a grid barrier (kernel 0: all terms of a small
+ * problem in one launch, 1: the Haydock recursion): two blocks wait for an arrival
+ * that never comes, give up after 10 ms and record it.  report != 0: the call returns
+ * TBPM_ERR_TIMEOUT; 0: the record is left for the next driver call on the context,
+ * which has to report it as if one of its own waits had run out. */
+int tbpm_selftest_grid_wait(tbpm_ctx* ctx, int kernel, int report);
+
 /* ---- Analyzer transforms on the device ---------------------------------- */
 
 /* Window-weighted trigonometric sums of correlation functions, the

@@ -45,6 +45,7 @@ void drv_dos_segmented(tbpm_ctx* c, const double* bes, int n_bes, const int64_t*
 void drv_session_advance(tbpm_ctx* c, int n_steps);
 void drv_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done);
 void drv_selftest_wait_timeout(tbpm_ctx* c);
+void drv_selftest_grid_wait(tbpm_ctx* c, int kernel, int report);
 void drv_session_dos_resume(tbpm_ctx* c, const double* bes, int n_bes, int n_states,
                             const double* wf0, const double* psi, const double* corr,
                             const double* norms, int n_done, int n_timestep);
@@ -549,6 +550,10 @@ int tbpm_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done) {
 
 int tbpm_selftest_wait_timeout(tbpm_ctx* c) {
   return guarded(c, [&] { tbpm::drv_selftest_wait_timeout(c); });
+}
+
+int tbpm_selftest_grid_wait(tbpm_ctx* c, int kernel, int report) {
+  return guarded(c, [&] { tbpm::drv_selftest_grid_wait(c, kernel, report); });
 }
 
 int tbpm_session_export(tbpm_ctx* c, double* wf0, double* psi) {

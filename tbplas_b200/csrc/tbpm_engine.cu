@@ -702,6 +702,9 @@ void qe_smem_attr(K kernel, size_t bytes) {
   TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
+// Longest wait on a grid barrier.
+constexpr unsigned long long kGridWaitNs = 2000000000ull;
+
 // Launch of a kernel with a grid barrier: every block is resident at once, so the
 // barrier cannot wait on a block that has not started.
 template <class K, class Args>
@@ -782,6 +785,8 @@ PersistArgs<R, V> persist_args(const tbpm_ctx* c, double alpha, int k0, int k1, 
   a.k1 = k1;
   a.bar = c->ctr.as<unsigned int>() + 12;
   a.status = c->status.as<unsigned int>();
+  a.absent = 0;
+  a.wait_ns = kGridWaitNs;
   return a;
 }
 
@@ -1301,8 +1306,8 @@ void check_status(tbpm_ctx* c) {
   if (st) {
     TBPM_CK(cudaMemset(c->status.p, 0, sizeof st));
     throw Error{TBPM_ERR_TIMEOUT,
-                "a bounded device-side wait of a Chebyshev-term kernel ran out; the results "
-                "of this call are invalid"};
+                "a bounded device-side wait of a kernel ran out; the results of this call are "
+                "invalid"};
   }
 }
 
@@ -3096,6 +3101,8 @@ void haydock_state(tbpm_ctx* c, int n_depth, double h_rescale, double* sc) {
   a.cap = (int)std::min<int64_t>(items, (int64_t)(kHaydockSmem / item_bytes));
   a.bar = c->ctr.as<unsigned int>() + 12;
   a.status = c->status.as<unsigned int>();
+  a.absent = 0;
+  a.wait_ns = kGridWaitNs;
   TBPM_CK(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), c->stream));
   qe_smem_attr(kernel, a.cap * item_bytes);
   launch_cooperative(c, kernel, grid, threads, a.cap * item_bytes, a);
@@ -4184,6 +4191,64 @@ void drv_selftest_wait_timeout(tbpm_ctx* c) {
   TBPM_CK(cudaGetLastError());
   TBPM_CK(cudaStreamSynchronize(c->stream));
   check_status(c);  // throws TBPM_ERR_TIMEOUT when the wait ran out
+}
+
+// A tiny launch of a kernel with a grid barrier (0: cheb_persist_kernel, 1:
+// haydock_kernel) on two blocks and an empty matrix, whose first barrier expects one
+// arrival more than there are blocks: every block gives up after 10 ms.
+void drv_selftest_grid_wait(tbpm_ctx* c, int kernel, int report) {
+  if (kernel < 0 || kernel > 1) throw Error{TBPM_ERR_ARG, "kernel must be 0 or 1"};
+  constexpr int n = 64, threads = 128, grid = 2;
+  constexpr unsigned long long wait_ns = 10000000ull;
+  c->ctr.ensure(16 * sizeof(int));
+  unsigned int* bar = c->ctr.as<unsigned int>() + 12;
+  unsigned int* status = c->status.as<unsigned int>();
+  ScratchScope scope(c->scratch);
+  TempMem mem(c->scratch);
+  const size_t vec = n * sizeof(double2), bytes = 3 * vec + 64 * sizeof(double) + (n + 1) * 4;
+  mem.ensure(bytes);
+  TBPM_CK(cudaMemsetAsync(mem.p, 0, bytes, c->stream));
+  TBPM_CK(cudaMemsetAsync(bar, 0, sizeof(unsigned int), c->stream));
+  auto* v = mem.as<double2>();
+  double* sums = reinterpret_cast<double*>(v + 3 * n);
+  const int32_t* indptr = reinterpret_cast<const int32_t*>(sums + 64);  // rows without entries
+  if (kernel == 0) {
+    PersistArgs<double, 1> a{};
+    a.indptr = indptr;
+    a.n_rows = n;
+    a.tpr = 1;
+    a.p0 = reinterpret_cast<Pack<double, 1>*>(v);
+    a.ring[0] = reinterpret_cast<Pack<double, 1>*>(v + n);
+    a.ring[1] = reinterpret_cast<Pack<double, 1>*>(v + 2 * n);
+    a.slots = 2;
+    a.alpha = 1.0;
+    a.k0 = 1;
+    a.k1 = 2;
+    a.bar = bar;
+    a.status = status;
+    a.absent = 1;
+    a.wait_ns = wait_ns;
+    launch_cooperative(c, cheb_persist_kernel<double, 1, false>, grid, threads, 0, a);
+  } else {
+    HaydockArgs<double> a{};
+    a.indptr = indptr;
+    a.n_rows = n;
+    a.rescale = 1.0;
+    a.w0 = v;
+    a.w1 = v + n;
+    a.y = v + 2 * n;
+    a.n_depth = 1;
+    a.a = sums;
+    a.b = sums + 2;
+    a.partials = sums + 8;
+    a.bar = bar;
+    a.status = status;
+    a.absent = 1;
+    a.wait_ns = wait_ns;
+    launch_cooperative(c, haydock_kernel<double, 768>, grid, threads, 0, a);
+  }
+  TBPM_CK(cudaStreamSynchronize(c->stream));
+  if (report) check_status(c);
 }
 
 void drv_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done) {

@@ -145,3 +145,20 @@ def test_buffers_of_an_earlier_call_are_not_free_memory():
         torch.cuda.empty_cache()
         nat._contexts[0].close()
         nat._contexts = kept
+
+
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_grid_barrier_gives_up_and_the_context_stays_usable(kernel):
+    """A grid barrier that one arrival never reaches: a time-out error, and the next
+    run on the context is right."""
+    ctx = f2py._ctx()
+    with pytest.raises(nat.DeviceTimeoutError):
+        ctx.call("tbpm_selftest_grid_wait", kernel, 1)
+    h = tb.make_graphene_sample(8, 9, disorder=1.0, rescale=9.0, seed=4).build_ham_csr()
+    wf0 = unit_states(2, h.shape[0], seed=9)
+    bes = bessel_series(math.pi)
+    got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf0, 70, 64, 1e-9)
+    ref = oracle.tbpm_dos(bes, h.indptr, h.indices, h.data, 70, wf0=wf0)
+    assert rel_err(got, ref) < 1e-10
+    with pytest.raises(ValueError):
+        ctx.call("tbpm_selftest_grid_wait", 2, 1)

@@ -2714,6 +2714,7 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
     c->launches += 3;
     c->model_bytes += 2.0 * (double)n * n_ib * 2 * sizeof(R) + 2.0 * total * 8;
     TBPM_CK(cudaStreamSynchronize(c->stream));
+    check_status(c);
     return;
   }
   if (!pp) read_out(c, host, (size_t)n_timestep * ld * 3);
@@ -2824,9 +2825,12 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
     const int64_t n_vals = (int64_t)2 * len * 2 * n_ib;
     c->model_bytes += (double)n * n_ib * 2 * sizeof(R) + (double)len * n * ld * 2 * sizeof(R);
     vals.resize(n_vals);
+    unsigned int st = 0;
     TBPM_CK(cudaMemcpyAsync(vals.data(), c->small.p, n_vals * sizeof(double),
                             cudaMemcpyDeviceToHost, c->stream));
+    TBPM_CK(cudaMemcpyAsync(&st, c->status.p, sizeof st, cudaMemcpyDeviceToHost, c->stream));
     TBPM_CK(cudaStreamSynchronize(c->stream));
+    if (st) check_status(c);  // before these values are added to the caller's arrays
     for (int tau = 0; tau < len; ++tau)
       for (int k = 0; k < 2; ++k)
         for (int i = 0; i < n_en; ++i)

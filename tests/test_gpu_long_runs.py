@@ -162,3 +162,20 @@ def test_grid_barrier_gives_up_and_the_context_stays_usable(kernel):
     assert rel_err(got, ref) < 1e-10
     with pytest.raises(ValueError):
         ctx.call("tbpm_selftest_grid_wait", 2, 1)
+
+
+@pytest.mark.parametrize("n_t", [20, 70])
+def test_eigenstates_without_a_norm_check_report_a_wait_that_ran_out(n_t):
+    """Time-stepped and filtered quasi-eigenstates whose check step lies past the run."""
+    s = tb.make_graphene_sample(8, 9, disorder=1.0, rescale=9.0, seed=4)
+    h = s.build_ham_csr()
+    wf0 = unit_states(2, h.shape[0], seed=9)
+    t_step = 2 * math.pi / s.energy_range
+    args = (bessel_series(math.pi), h.indptr, h.indices, h.data)
+    energies = np.array([-0.4, 0.1, 0.3])
+    f2py._ctx().call("tbpm_selftest_grid_wait", 0, 0)
+    with pytest.raises(nat.DeviceTimeoutError):
+        f2py.tbpm_eigenstates_states(*args, wf0, n_t, t_step, energies, 128, 1e-9)
+    got = f2py.tbpm_eigenstates_states(*args, wf0, n_t, t_step, energies, 128, 1e-9)
+    ref = oracle.tbpm_eigenstates(*args, n_t, t_step, energies, wf0=wf0)
+    assert rel_err(got, ref) < 1e-10

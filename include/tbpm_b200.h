@@ -422,6 +422,14 @@ int tbpm_selftest_wait_timeout(tbpm_ctx* ctx);
  * which has to report it as if one of its own waits had run out. */
 int tbpm_selftest_grid_wait(tbpm_ctx* ctx, int kernel, int report);
 
+/* Self-test of the last stage of long DOS runs: the correlation function (complex128
+ * [n_timestep+1]) of one state of norm 1 from sums[n_terms][2] = <p_k|p_k> and
+ * Re <p_k|p_{k-1}>, k = 1..n_terms, of its Chebyshev vectors p_k = T_k(H) psi, with
+ * the norm check at the last step (threshold 1e-9): sums that no state can have, e.g.
+ * of a recurrence that left its bounds, return TBPM_ERR_NORM or TBPM_ERR_NAN. */
+int tbpm_selftest_moments(tbpm_ctx* ctx, const double* bes, int n_bes, const double* sums,
+                          int n_terms, int n_timestep, double* corr);
+
 /* ---- Analyzer transforms on the device ---------------------------------- */
 
 /* Window-weighted trigonometric sums of correlation functions, the

@@ -48,7 +48,7 @@ EXPORTED_SYMBOLS = (
     "tbpm_cond_from_trace", "tbpm_session_export", "tbpm_session_dos_resume",
     "tbpm_nn_gemm_tn_mma", "tbpm_nn_tc_status", "tbpm_trig_sums", "tbpm_trig_cumtrapz",
     "tbpm_selftest_wait_timeout", "tbpm_dccond_accumulate", "tbpm_haydock_green",
-    "tbpm_selftest_grid_wait",
+    "tbpm_selftest_grid_wait", "tbpm_selftest_moments",
 )
 
 
@@ -211,6 +211,7 @@ _SIGNATURES = {
                                     ctypes.POINTER(_c_dbl), _vp, _vp, _vp, _vp, _vp]),
     "tbpm_selftest_wait_timeout": (_c_int, [_vp]),
     "tbpm_selftest_grid_wait": (_c_int, [_vp, _c_int, _c_int]),
+    "tbpm_selftest_moments": (_c_int, [_vp, _vp, _c_int, _vp, _c_int, _c_int, _vp]),
     "tbpm_dccond_accumulate": (_c_int, [_vp, _vp, _c_int, _vp, _c_int, _c_int, _c_int, _c_int,
                                         _c_int, _c_int, _c_dbl, _vp, _c_int, _vp, _c_int,
                                         _c_int, _c_dbl, _vp, _vp]),

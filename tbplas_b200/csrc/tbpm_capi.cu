@@ -46,6 +46,8 @@ void drv_session_advance(tbpm_ctx* c, int n_steps);
 void drv_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done);
 void drv_selftest_wait_timeout(tbpm_ctx* c);
 void drv_selftest_grid_wait(tbpm_ctx* c, int kernel, int report);
+void drv_selftest_moments(tbpm_ctx* c, const double* bes, int n_bes, const double* sums,
+                          int n_terms, int T, double* corr);
 void drv_session_dos_resume(tbpm_ctx* c, const double* bes, int n_bes, int n_states,
                             const double* wf0, const double* psi, const double* corr,
                             const double* norms, int n_done, int n_timestep);
@@ -550,6 +552,13 @@ int tbpm_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done) {
 
 int tbpm_selftest_wait_timeout(tbpm_ctx* c) {
   return guarded(c, [&] { tbpm::drv_selftest_wait_timeout(c); });
+}
+
+int tbpm_selftest_moments(tbpm_ctx* c, const double* bes, int n_bes, const double* sums,
+                          int n_terms, int n_timestep, double* corr) {
+  return guarded(c, [&] {
+    tbpm::drv_selftest_moments(c, bes, n_bes, sums, n_terms, n_timestep, corr);
+  });
 }
 
 int tbpm_selftest_grid_wait(tbpm_ctx* c, int kernel, int report) {

@@ -1634,9 +1634,26 @@ void enqueue_moment_curves(tbpm_ctx* c, const PolyPlan& pp, int M, int T, int n_
                             c->stream));
   }
   moment_curve_kernel<<<dim3((unsigned)(T + 3), cg), 128, 0, c->stream>>>(
-      nodes, rho, n_cols, M, T, t_ref, std::max(chk_step - 1, 1), c->out.as<double>());
+      nodes, mu, rho, n_cols, M, T, t_ref, std::max(chk_step - 1, 1), c->out.as<double>());
   TBPM_CK(cudaGetLastError());
   c->launches += 3;
+}
+
+// check_norm on the curves of enqueue_moment_curves (host: c->out): the norms after t_chk
+// and t_ref steps, and no moment above mu_0.  A recurrence of M/2 terms whose rounding
+// errors grow by at most 7 each leaves a moment within 7 M rounding errors of mu_0.
+void check_moments(const tbpm_ctx* c, const std::vector<double>& host, int T, int M, int n_cols,
+                   int chk_step, double chk_thr, const char* who) {
+  if (chk_step < 2 || chk_step > T) return;
+  const double thr = effective_thr(c, chk_thr);
+  const double eps = c->ham.prec == TBPM_PREC_FP64 ? 1.1e-16 : 6e-8;
+  for (int v = 0; v < n_cols; ++v) {
+    const double* ref = &host[((size_t)(T + 1) * n_cols + v) * 2];
+    const double* chk = &host[((size_t)(T + 2) * n_cols + v) * 2];
+    if (const int bad = norm_broken(chk[0], ref[0], thr)) raise_norm(who, chk_step, bad);
+    if (!(chk[1] <= ref[0] * (1 + 1e-12 + 64.0 * M * eps)))
+      raise_norm(who, chk_step, TBPM_ERR_NORM);
+  }
 }
 
 // dos_batch by moments of the whole run: C(t) = <wf0|P(H)^t|wf0>.
@@ -1674,14 +1691,8 @@ void dos_moments(tbpm_ctx* c, const PolyPlan& pp, int ns, const StateKeys* keys,
                         rho, nodes, chk_step);
   std::vector<double> host;
   read_out(c, host, (size_t)(T + 3) * ns * 2);
-  // check_norm as in dos_batch: after chk_step - 1 steps against after the first
-  if (chk_step >= 2 && chk_step <= T) {
-    const double thr = effective_thr(c, chk_thr);
-    for (int b = 0; b < ns; ++b)
-      if (const int bad = norm_broken(host[((size_t)(T + 2) * ns + b) * 2],
-                                      host[((size_t)(T + 1) * ns + b) * 2], thr))
-        raise_norm("tbpm_dos", chk_step, bad);
-  }
+  // as in dos_batch: after chk_step - 1 steps against after the first
+  check_moments(c, host, T, M, ns, chk_step, chk_thr, "tbpm_dos");
   for (int b = 0; b < ns; ++b)
     for (int t = 0; t <= T; ++t) {
       const double* v = &host[((size_t)t * ns + b) * 2];
@@ -2093,13 +2104,7 @@ bool dos_segmented_moments(tbpm_ctx* c, const PolyPlan& pp, const std::vector<in
                         sums, 2, mu, rho, nodes, chk_step);
   std::vector<double> host;
   read_out(c, host, (size_t)(T + 3) * n_cols * 2);
-  if (chk_step >= 2 && chk_step <= T) {
-    const double thr = effective_thr(c, chk_thr);
-    for (int v = 0; v < n_cols; ++v)
-      if (const int bad = norm_broken(host[((size_t)(T + 2) * n_cols + v) * 2],
-                                      host[((size_t)(T + 1) * n_cols + v) * 2], thr))
-        raise_norm("tbpm_dos_segmented", chk_step, bad);
-  }
+  check_moments(c, host, T, M, n_cols, chk_step, chk_thr, "tbpm_dos_segmented");
   for (int k = 0; k < n_seg; ++k)
     for (int t = 0; t <= T; ++t) {
       double re = 0, im = 0;
@@ -2541,15 +2546,9 @@ void dc_filter(tbpm_ctx* c, const PolyPlan& pp, int nb, const Pack<R, V>* W, int
                         rho, nodes, chk_step, 0, true);
   std::vector<double> host;
   read_out(c, host, (size_t)(T + 3) * nb * 2);
-  if (check) {
-    // tbpm.f90:611-614: after chk_step - 1 steps against <wf0|wf0>; P and its
-    // conjugate have the same norms
-    const double thr = effective_thr(c, chk_thr);
-    for (int b = 0; b < nb; ++b)
-      if (const int bad = norm_broken(host[((size_t)(T + 2) * nb + b) * 2],
-                                      host[((size_t)(T + 1) * nb + b) * 2], thr))
-        raise_norm(who, chk_step, bad);
-  }
+  // tbpm.f90:611-614: after chk_step - 1 steps against <wf0|wf0>; P and its
+  // conjugate have the same norms
+  check_moments(c, host, T, M, nb, chk_step, chk_thr, who);
   if (dos) dos->assign(host.begin() + (size_t)nb * 2, host.begin() + (size_t)(T + 1) * nb * 2);
 }
 
@@ -4253,6 +4252,35 @@ void drv_selftest_grid_wait(tbpm_ctx* c, int kernel, int report) {
   }
   TBPM_CK(cudaStreamSynchronize(c->stream));
   if (report) check_status(c);
+}
+
+// Curves and norm check of a run of T steps, checked at its end, from given sums of its
+// terms (one column, <p_0|p_0> = 1, y = H): what dos_moments does with its own.
+void drv_selftest_moments(tbpm_ctx* c, const double* bes, int n_bes, const double* sums,
+                          int n_terms, int T, double* corr) {
+  if (!bes || n_bes < 3 || !sums || n_terms < 2 || T < 2 || !corr)
+    throw Error{TBPM_ERR_ARG, "series, sums and an output required"};
+  PolyPlan pp;
+  pp.alpha = 2.0f;
+  pp.a = 1.0L;
+  pp.bes = bes;
+  pp.n_bes = n_bes;
+  const int M = 2 * n_terms;
+  c->out.ensure((size_t)(T + 3) * 2 * sizeof(double));
+  const size_t n_sums = 2 * (size_t)n_terms;
+  c->poly.ensure((n_sums + 1 + 2 * (size_t)M) * sizeof(double) + sizeof(PolyNode) * M);
+  double* d = c->poly.as<double>();
+  std::vector<double> in(sums, sums + n_sums);
+  in.push_back(1.0);
+  TBPM_CK(cudaMemcpyAsync(d, in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice,
+                          c->stream));
+  double* mu = d + in.size();
+  enqueue_moment_curves(c, pp, M, T, 1, d, 2, d + n_sums, 1, mu, mu + M,
+                        reinterpret_cast<PolyNode*>(mu + 2 * M), T);
+  std::vector<double> host;
+  read_out(c, host, (size_t)(T + 3) * 2);
+  check_moments(c, host, T, M, 1, T, 1e-9, "tbpm_selftest_moments");
+  std::copy(host.begin(), host.begin() + 2 * (T + 1), corr);
 }
 
 void drv_session_read(tbpm_ctx* c, double* corr, double* norms, int* n_done) {

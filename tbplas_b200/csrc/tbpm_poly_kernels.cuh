@@ -195,8 +195,11 @@ static __global__ void __launch_bounds__(128) moment_density_kernel(const double
 
 // Block (row, column chunk).  Rows 0..T: out = sum_j P(x_j)^t rho_j (re, im);
 // rows T+1, T+2: the norm sum_j |P(x_j)|^(2t) rho_j after t = t_ref, t_chk
-// steps.  out[(row*n_cols + col)*2 + {re, im}].
+// steps, and the largest |mu_m|: for unitary P the norms are mu_0 whatever the terms
+// computed, but no moment of a state with spectrum in [-1, 1] exceeds mu_0.
+// out[(row*n_cols + col)*2 + {re, im}].
 static __global__ void __launch_bounds__(128) moment_curve_kernel(const PolyNode* nodes,
+                                                                  const double* mu,
                                                                   const double* rho, int n_cols,
                                                                   int M, int T, int t_ref,
                                                                   int t_chk, double* out) {
@@ -214,6 +217,9 @@ static __global__ void __launch_bounds__(128) moment_curve_kernel(const PolyNode
     double re, im;
     if (norm) {
       re = exp(2.0 * t * p.lnabs);
+#pragma unroll
+      for (int c = 0; c < kMomentCols; ++c)
+        if (c < nc) ai[c] = fmax(ai[c], fabs(mu[(int64_t)(c0 + c) * M + j]));
       im = 0.0;
     } else {
       node_power(p, t, &re, &im);
@@ -233,7 +239,8 @@ static __global__ void __launch_bounds__(128) moment_curve_kernel(const PolyNode
   for (int c = 0; c < kMomentCols; ++c) {
     for (int s = 16; s > 0; s >>= 1) {
       ar[c] += __shfl_xor_sync(0xffffffffu, ar[c], s);
-      ai[c] += __shfl_xor_sync(0xffffffffu, ai[c], s);
+      const double o = __shfl_xor_sync(0xffffffffu, ai[c], s);
+      ai[c] = norm ? fmax(ai[c], o) : ai[c] + o;
     }
     if ((threadIdx.x & 31) == 0) {
       red[threadIdx.x >> 5][2 * c] = ar[c];
@@ -241,9 +248,12 @@ static __global__ void __launch_bounds__(128) moment_curve_kernel(const PolyNode
     }
   }
   __syncthreads();
-  if (threadIdx.x < 2 * nc)
+  if (threadIdx.x < 2 * nc) {
+    const double a = red[0][threadIdx.x], b = red[1][threadIdx.x], c = red[2][threadIdx.x],
+                 d = red[3][threadIdx.x];
     out[((int64_t)row * n_cols + c0) * 2 + threadIdx.x] =
-        (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
+        norm && (threadIdx.x & 1) ? fmax(fmax(a, b), fmax(c, d)) : (a + b) + (c + d);
+  }
 }
 
 // ---- all terms of a small problem in one launch -----------------------------

@@ -179,3 +179,30 @@ def test_eigenstates_without_a_norm_check_report_a_wait_that_ran_out(n_t):
     got = f2py.tbpm_eigenstates_states(*args, wf0, n_t, t_step, energies, 128, 1e-9)
     ref = oracle.tbpm_eigenstates(*args, n_t, t_step, energies, wf0=wf0)
     assert rel_err(got, ref) < 1e-10
+
+
+def test_norm_check_refuses_moments_that_no_state_has():
+    """The sums of a state with three levels give its curve; with one of them beyond the
+    state's norm, or not a number, the norm check refuses the run."""
+    x, w, n_t = np.array([-0.9, 0.2, 0.7]), np.array([0.5, 0.2, 0.3]), 80
+    bes = np.array(bessel_series(math.pi))
+    k = np.arange(200)
+    t = np.cos(k[:, None] * np.arccos(x))
+    sums = np.stack([(w * t[1:] ** 2).sum(1), (w * t[1:] * t[:-1]).sum(1)], 1)
+    corr = np.zeros(n_t + 1, dtype=complex)
+    f2py.set_backend(precision="fp64")
+    f2py.tbpm_dos([1.0, 0.1, 0.01], [0, 0], [], [], 1, 1, 1, "", 0, 128, 1e-9)  # FP64 resident
+
+    def run(s):
+        f2py._ctx().call("tbpm_selftest_moments", nat.ptr(bes), bes.size, nat.ptr(s), len(s), n_t,
+                         nat.ptr(corr))
+    run(sums)
+    ref = (w * np.exp(-1j * math.pi * x * np.arange(n_t + 1)[:, None])).sum(1)
+    assert rel_err(corr, ref) < 1e-12
+    for row, col, value, err in ((120, 0, 1.0 + 1e-6, nat.NormError),
+                                 (33, 1, -1.1, nat.NormError), (150, 0, 1e30, nat.NormError),
+                                 (7, 1, np.nan, nat.NanError)):
+        bad = sums.copy()
+        bad[row, col] = value
+        with pytest.raises(err):
+            run(bad)

@@ -13,9 +13,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <optional>
 #include <type_traits>
 
@@ -124,7 +126,7 @@ void dispatch(int prec, int V, F&& f) {
 inline size_t real_size(int prec) { return prec == TBPM_PREC_FP64 ? 8 : 4; }
 
 int num_sms(int device) {
-  static int cached[64] = {0};
+  static std::atomic<int> cached[64];
   if (device < 0 || device >= 64) return kSMs;
   if (!cached[device]) {
     int v = 0;
@@ -138,10 +140,13 @@ int num_sms(int device) {
   return cached[device];
 }
 
-// Resident blocks per SM of `kernel` at the given block shape (cached).
+// Resident blocks per SM of `kernel` at the given block shape (cached for all contexts
+// of the process, which may be driven from several threads).
 template <class K>
 int resident_per_sm(K kernel, int threads, size_t smem) {
+  static std::mutex mutex;
   static std::vector<std::pair<std::pair<const void*, long long>, int>> cache;
+  std::lock_guard<std::mutex> lock(mutex);
   const void* key = reinterpret_cast<const void*>(kernel);
   const long long shape = (long long)threads * (1ll << 32) + (long long)smem;
   for (const auto& e : cache)
@@ -347,7 +352,7 @@ RingShape ring_shape(const tbpm_ctx* c, int tpr, int mode, int ref_tpr, bool win
 
 template <typename R, int V, int MODE, bool WIN>
 int ring_blocks_per_sm(const tbpm_ctx* c, const RingShape& rs) {
-  static bool attr_set[64] = {false};
+  static std::atomic<bool> attr_set[64];
   const int dev = c->device;
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     TBPM_CK(cudaFuncSetAttribute(cheb_ring_kernel<R, V, MODE, WIN>,
@@ -554,7 +559,7 @@ void launch_seg_term(tbpm_ctx* c, const SegTiles& t, const int2* tiles,
 
 template <typename R, int V>
 int pair_blocks_per_sm(const tbpm_ctx* c, size_t smem) {
-  static bool attr_set[64] = {false};
+  static std::atomic<bool> attr_set[64];
   const int dev = c->device;
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     TBPM_CK(cudaFuncSetAttribute(cheb_pair_kernel<R, V>,
@@ -695,11 +700,17 @@ double matrix_bytes(const Ham& h) {
   return (double)(h.n + 1) * 4 + (double)h.nnz * (4 + s) + (h.has_diag ? (double)h.n * s : 0.0);
 }
 
+// Allows `kernel` the shared memory of its next launch.  The limit belongs to the
+// function, not to the launch, and other threads launch it for other contexts: it is
+// always set to the most the kernel can have, never down to what one launch needs.
 template <class K>
 void qe_smem_attr(K kernel, size_t bytes) {
   // (a kernel's static shared memory counts towards the default 48 KB too)
   if (bytes <= 40 * 1024) return;
-  TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  cudaFuncAttributes fa;
+  TBPM_CK(cudaFuncGetAttributes(&fa, kernel));
+  TBPM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               227 * 1024 - (int)fa.sharedSizeBytes));
 }
 
 // Longest wait on a grid barrier.
@@ -3970,9 +3981,7 @@ void drv_cond_from_trace(tbpm_ctx* c, const double* mu_mn, int nk, const double*
   TBPM_CK(cudaMemcpyAsync(dmu.p, mu_mn, sizeof(double2) * (size_t)nk * nk,
                           cudaMemcpyHostToDevice, c->stream));
   const size_t smem = (size_t)nk * 2 * sizeof(double);
-  if (smem > 48 * 1024)
-    TBPM_CK(cudaFuncSetAttribute(gamma_trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  qe_smem_attr(gamma_trace_kernel, smem);
   gamma_trace_kernel<<<ne, 256, smem, c->stream>>>(dmu.as<double2>(), nk, ne_integral,
                                                    dsum.as<double>());
   TBPM_CK(cudaGetLastError());

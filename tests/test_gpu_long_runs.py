@@ -5,6 +5,7 @@ The oracle and dense diagonalisation are the reference, FP64 to a relative 1e-10
 """
 
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -206,3 +207,37 @@ def test_norm_check_refuses_moments_that_no_state_has():
         bad[row, col] = value
         with pytest.raises(err):
             run(bad)
+
+
+def test_contexts_in_several_threads():
+    """Twelve threads, each with its own context and a block shape of its own (launches
+    of one kernel with different shared memory): every call returns the thread's first
+    result bit for bit."""
+    bes = nat.as_c(bessel_series(math.pi), np.float64)
+    failed = []
+
+    def work(nx):
+        h = tb.make_graphene_sample(nx, 100, disorder=1.0, rescale=9.0, seed=2).build_ham_csr()
+        ip, ix = nat.as_c(h.indptr, np.int32), nat.as_c(h.indices, np.int32)
+        hv = nat.as_c(h.data, np.complex128)
+        ctx = nat.Context(0)
+        first = None
+        try:
+            for _ in range(500):
+                corr = np.zeros(65, dtype=np.complex128)
+                ctx.call("tbpm_dos", nat.ptr(bes), bes.size, nat.ptr(ip), nat.ptr(ix), nat.ptr(hv),
+                         ip.size - 1, hv.size, 7, 64, 1, 0, 128, 1e-9, nat.ptr(corr))
+                first = corr if first is None else first
+                if not np.array_equal(first, corr):
+                    failed.append((nx, rel_err(corr, first)))
+        except nat.TbpmError as e:
+            failed.append((nx, str(e)))
+        finally:
+            ctx.close()
+
+    threads = [threading.Thread(target=work, args=(40 + 2 * i,)) for i in range(12)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed

@@ -241,3 +241,107 @@ def test_contexts_in_several_threads():
     for t in threads:
         t.join()
     assert not failed
+
+
+@pytest.fixture(scope="module")
+def sample():
+    s = tb.make_graphene_sample(9, 11, disorder=1.0, rescale=9.0, seed=21)
+    s.set_magnetic_field(30.0)
+    return s
+
+
+KERNELS = pytest.mark.parametrize("kernel", [1, 2])  # grid-stride, ring: a launch per term
+PRECS = pytest.mark.parametrize("prec", ["fp64", "fp32"])
+
+
+@KERNELS
+@PRECS
+def test_eigenstates_by_launched_terms(sample, kernel, prec):
+    h = sample.build_ham_csr()
+    wf = unit_states(3, h.shape[0], seed=6)
+    t_step = 2 * math.pi / sample.energy_range
+    energies = np.linspace(-2.0, 2.0, 9) + 0.01
+    args = (bessel_series(math.pi), h.indptr, h.indices, h.data)
+    f2py.set_backend(precision=prec, term_kernel=kernel)
+    got = f2py.tbpm_eigenstates_states(*args, wf, 97, t_step, energies, 64, 1e-9)
+    ref = oracle.tbpm_eigenstates(*args, 97, t_step, energies, wf0=wf)
+    assert rel_err(got, ref) < {"fp64": 1e-10, "fp32": 5e-5}[prec]
+
+
+@KERNELS
+@PRECS
+def test_ac_and_polarisation_by_launched_terms(sample, kernel, prec):
+    """Expansions of 57 (FP32: 36) vectors in windows of 32: several window borders."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    h = sample.build_ham_csr()
+    wf = unit_states(3, h.shape[0], seed=21)
+    bes = bessel_series(math.pi / 2)
+    beta = sample.rescale / (tb.KB * 3000.0)
+    f2py.set_backend(precision=prec, term_kernel=kernel)
+    tol = {"fp64": 1e-10, "fp32": 2e-5}[prec]
+    args = (bes, beta, 0.05, ip, ix, hv, sample.rescale, dx, dy)
+    got = f2py.tbpm_accond_states(*args, wf, 90, 2 ** 15, 1e-12, 64, 1e-9)
+    assert rel_err(got, oracle.tbpm_accond(*args, 90, wf0=wf)) < tol
+    q = [[1.3, 0.2, 0.0], [0.0, 2.0, 0.0]]
+    args = (bes, beta, 0.0, h.indptr, h.indices, h.data, *sample.orb_pos.T.copy(), q)
+    got = f2py.tbpm_dyn_pol_states(*args, wf, 90, 2 ** 15, 1e-12, 64, 1e-9)
+    assert rel_err(got, oracle.tbpm_dyn_pol(*args, 90, wf0=wf)) < tol
+
+
+@pytest.mark.parametrize("kernel", [0, 1, 2])
+@PRECS
+def test_dc_by_launched_terms(sample, kernel, prec):
+    """Energies inside the populated spectrum.  FP32: a recurrence of M = 280 terms loses
+    at most 7 M rounding errors of 6e-8, 1.2e-4, and a value divides by |<wf0|QE>|, which
+    is above a quarter of |QE| there."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf0 = unit_states(3, ip.size - 1, seed=31)
+    n_t = 89
+    e = np.array([0.5 * i * sample.energy_range / n_t - sample.energy_range / 2.
+                  for i in range(2 * n_t)])
+    sel = np.where((e >= 1.0) & (e <= 3.0))[0]
+    t_step = 2 * math.pi / sample.energy_range
+    args = (bessel_series(math.pi), ip, ix, hv, sample.rescale, dx, dy)
+    f2py.set_backend(precision=prec, term_kernel=kernel)
+    got = f2py.tbpm_dccond_states(*args, wf0, n_t, t_step, e, sel, 60, 1e-9)
+    ref = oracle.tbpm_dccond(*args, n_t, t_step, e, sel, wf0=wf0)
+    assert rel_err(got[0], ref[0]) < {"fp64": 1e-10, "fp32": 3e-5}[prec]
+    assert rel_err(got[1], ref[1]) < {"fp64": 1e-10, "fp32": 5e-4}[prec]
+
+
+@KERNELS
+def test_dc_block_partials_in_several_reductions(kernel):
+    """32 states of 5000 orbitals: the launched terms' block partials are reduced in
+    several chunks of 64 MB, those of the one-launch route window by window."""
+    s = tb.make_graphene_sample(50, 50, disorder=1.0, rescale=9.0, seed=3)
+    ip, ix, hv, dx, dy = s.build_ham_dxy()
+    bes = bessel_series(math.pi)
+    energies, sel = np.array([1.5, 2.0]), np.arange(2)
+    out = []
+    for k in (0, kernel):
+        f2py.set_backend(batch=32, term_kernel=k)
+        out.append(f2py.tbpm_dccond(bes, 40.0, 0.0, ip, ix, hv, s.rescale, dx, dy, 5, 300, 32,
+                                    math.pi / s.rescale, energies, sel, "", "", 0, 128, 1e-9))
+    assert rel_err(out[1][0], out[0][0]) < 1e-12
+    assert rel_err(out[1][1], out[0][1]) < 1e-10
+
+
+@pytest.mark.parametrize("n", [150, 221])
+def test_dc_of_general_matrices_inside_the_spectrum(n):
+    """Rows of no entry up to twelve, unsorted columns, energies where the levels lie."""
+    rng = np.random.default_rng(n)
+    m = sp.random(n, n, density=3.0 / n, random_state=rng, format="csr")
+    m = m + 1j * sp.random(n, n, density=3.0 / n, random_state=rng, format="csr")
+    m = sp.csr_matrix(m + m.conj().T)
+    m = sp.csr_matrix(m * (0.9 / abs(m).sum(1).max()))
+    pos = rng.standard_normal((2, n))
+    rows = np.repeat(np.arange(n), np.diff(m.indptr))
+    dx, dy = pos[:, m.indices] - pos[:, rows]
+    wf0 = unit_states(3, n, seed=21)
+    levels = np.linalg.eigvalsh(m.toarray())
+    energies, sel = np.quantile(levels, [0.2, 0.4, 0.6, 0.8]), np.arange(4)
+    args = (bessel_series(math.pi), m.indptr, m.indices, m.data, 1.0, dx, dy)
+    got = f2py.tbpm_dccond_states(*args, wf0, 70, math.pi, energies, sel, 64, 1e-9)
+    ref = oracle.tbpm_dccond(*args, 70, math.pi, energies, sel, wf0=wf0)
+    assert rel_err(got[0], ref[0]) < 1e-10
+    assert rel_err(got[1], ref[1]) < 1e-10

@@ -507,7 +507,8 @@ int tbpm_nn_cast_bf16(const float* in, int64_t n, void* out, void* stream);
  * tbpm_random_states with first_sample = 1) on the uploaded Hamiltonian, with
  * room for n_timestep steps.  Records corr(0).  With CUDA graphs enabled the
  * graph of opts.steps_per_graph steps is captured and uploaded here, so that
- * tbpm_session_advance only replays it. */
+ * tbpm_session_advance only replays it.  The session lives in the context's vectors:
+ * a driver call on the context ends it (TBPM_ERR_STATE from the session calls). */
 int tbpm_session_dos_begin(tbpm_ctx* ctx, const double* bes, int n_bes, int n_states,
                            int seed, int rank, int n_ran_samples, int n_timestep);
 /* Enqueue n_steps time steps on the context stream; returns without waiting. */

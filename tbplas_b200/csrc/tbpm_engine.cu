@@ -2328,6 +2328,7 @@ void ac_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fermi, 
               double chk_thr, int n_avg, double* corr, const PolyPlan* pp) {
   const int ld = 3 * nb;
   c->graph.reset();
+  c->sess.active = false;
   const StepsShape shape = steps_room<R>(c, pp, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * nb * 9 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
@@ -2579,6 +2580,7 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   const int T2 = std::min(8, std::max(n_timestep, 1));           // phase-2 window
   const size_t vb = (size_t)n * ld * 2 * sizeof(R);
   c->graph.reset();
+  c->sess.active = false;
   if (!pp) {
     c->X.ensure(vb);
     c->Y.ensure(vb);
@@ -2872,6 +2874,7 @@ void dynpol_batch(tbpm_ctx* c, const Expansion& ex_time, const Expansion& ex_fer
   const int ld = (nq + 1) * nb;
   const int tpr = nq * nb;
   c->graph.reset();
+  c->sess.active = false;
   const StepsShape shape = steps_room<R>(c, pp, ld, nb);
   c->out.ensure((size_t)std::max(n_timestep, 1) * tpr * 3 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
@@ -3177,6 +3180,7 @@ void psi_t_run(tbpm_ctx* c, const Expansion& ex, const double* bes, int n_bes,
                int chk_step, double chk_thr, double* psi_t) {
   constexpr int V = 1;
   c->graph.reset();
+  c->sess.active = false;
   ensure_vectors(c, 1, 1);
   c->out.ensure((size_t)(n_timestep + 1) * 3 * sizeof(double));
   auto* A = c->A.as<Pack<R, V>>();
@@ -4111,6 +4115,7 @@ void drv_expansion_apply(tbpm_ctx* c, const Expansion& ex, double* wf, int n_sta
   require_ham(c, false);
   if (n_states < 1 || n_states > kMaxCols) throw Error{TBPM_ERR_ARG, "1..64 states"};
   c->graph.reset();
+  c->sess.active = false;
   const int ld = n_states;
   ensure_vectors(c, ld, 1);
   dispatch(c->ham.prec, pick_V(c->ham.prec, ld, ld, c->opts.vector_width), [&](auto tag) {
@@ -4269,6 +4274,7 @@ void drv_selftest_moments(tbpm_ctx* c, const double* bes, int n_bes, const doubl
                           int n_terms, int T, double* corr) {
   if (!bes || n_bes < 3 || !sums || n_terms < 2 || T < 2 || !corr)
     throw Error{TBPM_ERR_ARG, "series, sums and an output required"};
+  c->sess.active = false;
   PolyPlan pp;
   pp.alpha = 2.0f;
   pp.a = 1.0L;

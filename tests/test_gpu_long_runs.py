@@ -345,3 +345,34 @@ def test_dc_of_general_matrices_inside_the_spectrum(n):
     ref = oracle.tbpm_dccond(*args, 70, math.pi, energies, sel, wf0=wf0)
     assert rel_err(got[0], ref[0]) < 1e-10
     assert rel_err(got[1], ref[1]) < 1e-10
+
+
+@pytest.mark.parametrize("driver", ["ac", "dc", "psi_t"])
+def test_driver_calls_end_a_session(sample, driver):
+    """A driver's call takes the vectors over (and may give them back to the device): the
+    session is over, not continued on what is left."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    bes = nat.as_c(bessel_series(math.pi), np.float64)
+    wf = unit_states(2, ip.size - 1, seed=1)
+    ctx = f2py._ctx()
+    arrays = [nat.as_c(a, t) for a, t in ((ip, np.int32), (ix, np.int32), (hv, np.complex128),
+                                          (dx, np.float64), (dy, np.float64))]
+    ctx.call("tbpm_ham_upload", *map(nat.ptr, arrays[:3]), ip.size - 1, ix.size,
+             *map(nat.ptr, arrays[3:]), sample.rescale)
+    ctx.call("tbpm_session_dos_begin", nat.ptr(bes), bes.size, 4, 7, 0, 4, 40)
+    ctx.call("tbpm_session_advance", 4)
+
+    class Uploaded:  # calls with this in the place of indptr run on the uploaded Hamiltonian
+        @staticmethod
+        def make_resident(_):
+            return ip.size - 1, ix.size
+    args = (bes, Uploaded, None, None)
+    if driver == "ac":
+        f2py.tbpm_accond_states(bes, 8.0, 0.0, *args[1:], sample.rescale, None, None, wf, 64,
+                                2 ** 12, 1e-12, 128, 1e-9)
+    elif driver == "dc":
+        f2py.tbpm_eigenstates_states(*args, wf, 64, 0.3, [0.1], 128, 1e-9)
+    else:
+        f2py.tbpm_psi_t(*args, wf[0], np.array([0, 64]), 64, 128, 1e-9)
+    with pytest.raises(nat.TbpmError):
+        ctx.call("tbpm_session_advance", 4)

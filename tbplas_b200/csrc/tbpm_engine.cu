@@ -820,9 +820,6 @@ void launch_persist(tbpm_ctx* c, const PersistShape& s, const PersistArgs<R, V>&
   c->launches++;
 }
 
-#ifndef TBPM_CLUSTER_ITEMS
-#define TBPM_CLUSTER_ITEMS kClusterItems  // (0: off)
-#endif
 // The moments' terms k0..k1 of a tiny problem by cheb_cluster_kernel: block partials
 // to c->partials, the number of blocks returned (0: it does not apply).  The even
 // vectors are in A, the odd ones in X; both are written back when `keep`.
@@ -839,7 +836,7 @@ int launch_cluster(tbpm_ctx* c, double alpha, int k0, int k1, bool keep, int ld,
   const int rows = std::max(2, (int)((h.n + kClusterBlocks - 1) / kClusterBlocks));
   const int rpp = std::max(std::min(rows, TMAX / tpr), (128 + tpr - 1) / tpr);
   const int threads = rpp * tpr;
-  if (rows > TBPM_CLUSTER_ITEMS * rpp) return 0;
+  if (rows > kClusterItems * rpp) return 0;
   const size_t smem = 2 * (size_t)rows * tpr * sizeof(Pack<R, V>) +
                       (size_t)kPersistBatch * threads * V * 2 * sizeof(double);
   // (the products' slots start at a multiple of 8 bytes: packs are that or more)

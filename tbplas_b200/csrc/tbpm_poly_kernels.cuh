@@ -288,13 +288,10 @@ struct PersistArgs {
   unsigned long long wait_ns;  // longest wait
 };
 
-// most threads of a block: 128 registers a thread for 32-byte packs, 102 for
+// most threads of a block: 128 registers a thread for 32-byte packs, 85 for
 // 16-byte ones, 64 for 8-byte ones
-#ifndef TBPM_PERSIST_T16
-#define TBPM_PERSIST_T16 768
-#endif
 template <typename R, int V>
-constexpr int kPersistThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? TBPM_PERSIST_T16 : 1024);
+constexpr int kPersistThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? 768 : 1024);
 // the same of the cluster kernel, whose items take more registers
 template <typename R, int V>
 constexpr int kClusterThreads = sizeof(R) * V == 16 ? 512 : (sizeof(R) * V == 8 ? 640 : 768);

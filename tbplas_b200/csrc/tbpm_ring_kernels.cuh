@@ -52,12 +52,6 @@ namespace tbpm {
 #ifndef TBPM_RING_WARPS
 #define TBPM_RING_WARPS 15  // consumer warps per block
 #endif
-#ifndef TBPM_RING_WARPS_SMALL
-#define TBPM_RING_WARPS_SMALL 22  // the same for packs of 16 or 8 bytes
-#endif
-#ifndef TBPM_RING_WARPS_PLAIN
-#define TBPM_RING_WARPS_PLAIN 19  // the same for mode 0 (recurrence only)
-#endif
 #ifndef TBPM_RING_MINB
 #define TBPM_RING_MINB 1  // resident blocks per SM the stages are sized for
 #endif
@@ -88,8 +82,7 @@ constexpr unsigned long long kRingWaitNs = 2000000000ull;  // 2 s per wait
 // FP64 100 ms with 15 and 107 with 16, FP32 42.7 with 15 and 44.4 with 19.
 template <typename R, int V, int MODE, bool WIN>
 constexpr int kRingWarps =
-    sizeof(R) * V == 16 ? (MODE == 0 && !WIN ? TBPM_RING_WARPS_PLAIN : kRingConsumerWarps)
-                        : TBPM_RING_WARPS_SMALL;
+    sizeof(R) * V == 16 ? (MODE == 0 && !WIN ? 19 : kRingConsumerWarps) : 22;
 template <typename R, int V, int MODE, bool WIN>
 constexpr int kRingItems = kRingWarps<R, V, MODE, WIN> * 32;
 

@@ -351,7 +351,7 @@ __device__ __forceinline__ float2 ld_c(const float2* p) {
 // before the barrier), its gathers are issued together, and a thread's own rows of
 // w, w_prev and y (as many as fit the shared memory: `cap` per thread) never leave
 // the SM: the second half of a depth then reads nothing from L2.  524,288
-// orbitals, per depth: 12.5 us, 16.5 us with the entries in the loop and all
+// orbitals, per depth: 12.6 us, 16.5 us with the entries in the loop and all
 // vectors in L2, 35 us as five launches.
 template <typename R, int T_MAX>
 __global__ void __launch_bounds__(T_MAX, 1)

@@ -10,9 +10,9 @@
 // tau*a*T products, not (n_Bes - 1)*T: for the DOS 3.0 per step instead of 19,
 // and half of that again because <p_k|p_k> and <p_k|p_{k-1}> give the moments
 // mu_2k and mu_2k-1.  Measured on B200, whole calls, before -> after: DOS of
-// 1600 x 1500 graphene, 16 FP64 states, 64 steps: 1017 -> 103 ms; 1024 x 1000, 16
-// FP32 states, 128 steps: 482 -> 45 ms; 100 x 100, one state, 256 steps: 14.3 ->
-// 1.8 ms; 20 packed samples, 4 states, 128 steps: 178 -> 40 ms.  The error against
+// 1600 x 1500 graphene, 16 FP64 states, 64 steps: 1061 -> 99 ms; 1024 x 1000, 16
+// FP32 states, 128 steps: 494 -> 43 ms; 100 x 100, one state, 256 steps: 14.2 ->
+// 1.04 ms; 20 packed samples, 4 states, 128 steps: 178 -> 27 ms.  The error against
 // exact propagation stays where it was (1e-15 to 1e-14).
 //
 //  ham_spectrum_kernel    Gershgorin bounds of H and of its anti-Hermitian part.
@@ -299,7 +299,8 @@ constexpr int kPersistDeg = 3;  // row entries whose gathers are issued together
 constexpr int kPersistBatch = 4;  // terms whose products are reduced together
 
 // The terms p_k = (2/a) H p_{k-1} - p_{k-2}, k0 <= k <= k1, of a problem whose
-// vectors stay in L2, under one cooperative launch: a grid barrier per
+// vectors stay in L2 for the most part (persist_shape: up to 160 MB of matrix and
+// vectors, where L2 has 126), under one cooperative launch: a grid barrier per
 // term instead of a launch per term.  What bounds it is latency, not bytes: a
 // barrier round trip and a gather per item of a thread (a row's pack of V columns).
 // So nothing else waits: an item's columns (up to kPersistDeg) are in registers when
@@ -731,7 +732,8 @@ __global__ void __launch_bounds__((kClusterThreads<R, V>), 1)
 
 // ---- packed realisations ------------------------------------------------------
 
-// *coupled becomes nonzero when an entry leads from one realisation to another.
+// *coupled becomes nonzero when an entry leads from one realisation to another
+// (1.4M rows: 14 us beside 16 ms of terms).
 // Block (row chunk, realisation), threads over rows.
 static __global__ void __launch_bounds__(256) seg_closed_kernel(const int64_t* seg_off,
                                                                 const int32_t* indptr,

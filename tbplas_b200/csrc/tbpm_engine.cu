@@ -1385,9 +1385,11 @@ const Spectrum& ham_spectrum(tbpm_ctx* c) {
     using C = typename Cx<R>::t;
     // values that are conjugates in FP64 stay so when rounded to FP32
     const double tol = sizeof(R) == 8 ? 1e-14 : 1.2e-7;
+    const double rounding = sizeof(R) == 8 ? 4.5e-16 : 1.2e-7;  // two ulps, one
     ham_spectrum_kernel<R><<<grid, 256, 0, c->stream>>>(
         h.indptr.as<int32_t>(), h.indices.as<int32_t>(), h.hop.as<C>(),
-        h.has_diag ? h.diag.as<C>() : nullptr, h.n, tol, c->poly.as<unsigned long long>());
+        h.has_diag ? h.diag.as<C>() : nullptr, h.n, tol, rounding,
+        c->poly.as<unsigned long long>());
   };
   if (h.prec == TBPM_PREC_FP64)
     launch(double{});

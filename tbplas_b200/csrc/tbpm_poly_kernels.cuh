@@ -41,8 +41,10 @@ namespace tbpm {
 constexpr int kSpectrumMaxRow = 64;
 
 // info[0]: largest row sum |D_r| + sum_j |O_rj| (the bits of a non-negative
-// double, ordered like it), info[1]: the same of the anti-Hermitian part
-// (H - H^+)/2, info[2]: nonzero when an entry is not the conjugate of its transpose
+// double, ordered like it), info[1]: the same of the anti-Hermitian part (H - H^+)/2,
+// off-diagonal deviations of up to `rounding` (relative) left out: those have no
+// common sign and average out, info[2]: nonzero when an entry is not the conjugate of
+// its transpose
 // to `tol` (relative) or a row is longer than kSpectrumMaxRow.  One thread per row; a
 // row's transposed entries lie in its neighbours' rows, which are near in
 // memory.  Runs once per Hamiltonian.
@@ -52,6 +54,7 @@ __global__ void __launch_bounds__(256) ham_spectrum_kernel(const int32_t* indptr
                                                            const typename Cx<R>::t* hop,
                                                            const typename Cx<R>::t* diag,
                                                            int64_t n, double tol,
+                                                           double rounding,
                                                            unsigned long long* info) {
   double bound = 0.0, skew = 0.0;
   bool bad = false;
@@ -92,7 +95,8 @@ __global__ void __launch_bounds__(256) ham_spectrum_kernel(const int32_t* indptr
         }
       const double lim = tol * (fabs(fr) + fabs(fi));
       if (!(fabs(fr - br) <= lim && fabs(fi + bi) <= lim)) bad = true;
-      sk += 0.5 * hypot(fr - br, fi + bi);
+      const double dev = hypot(fr - br, fi + bi);
+      if (dev > rounding * (fabs(fr) + fabs(fi))) sk += 0.5 * dev;
     }
     if (!(s <= 1e300)) bad = true;
     bound = fmax(bound, s);

@@ -79,6 +79,29 @@ def test_loss_below_the_hermiticity_tolerance_over_long_runs(n_t):
     assert rel_err(got, ref) < 1e-10
 
 
+@pytest.mark.parametrize("prec,size,nx,n_t,tol", [("fp64", 2e-16, 3, 60000, 1e-9),
+                                                  ("fp32", 3e-8, 20, 600, 3e-5)])
+def test_conjugates_to_rounding_stay_on_the_short_route(prec, size, nx, n_t, tol):
+    """Off-diagonal entries whose transposes differ by a rounding: a launch or less per
+    step, not the 19 of time stepping; against the levels of the matrix without them
+    (FP64: their own error, 4e-16 pi 60000 = 8e-11)."""
+    s = tb.make_graphene_sample(nx, nx, disorder=1.0, rescale=9.0, seed=5)
+    s.set_magnetic_field(60.0)
+    h = s.build_ham_csr()
+    rng = np.random.default_rng(2)
+    off = h.indices != np.repeat(np.arange(h.shape[0]), np.diff(h.indptr))
+    data = h.data * (1 + off * size * rng.choice([-1, 0, 1], h.data.size))
+    wf0 = unit_states(1, h.shape[0], seed=1)
+    f2py.set_backend(precision=prec)
+    got = f2py.tbpm_dos_states(bessel_series(math.pi), h.indptr, h.indices, data, wf0, n_t, 128,
+                               1e-9)
+    assert f2py._ctx().last_stats()[0] < n_t
+    e, v = np.linalg.eigh(h.toarray())
+    w = abs(v.conj().T @ wf0[0]) ** 2
+    ref = np.exp(-1j * math.pi * np.outer(np.arange(n_t + 1), e)) @ w
+    assert rel_err(got, ref) < tol
+
+
 @pytest.mark.parametrize("ns", [1, 2])
 def test_packed_run_of_more_terms_than_a_grid_axis(ns):
     """50,000 steps of one tiny realisation: 75,000 terms whose sums are reduced

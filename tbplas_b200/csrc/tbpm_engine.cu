@@ -1345,8 +1345,7 @@ void read_out(tbpm_ctx* c, std::vector<double>& host, size_t n_doubles) {
 // state, 20 steps 2.2 / 0.34, 63 steps 4.7 / 0.47; 2M x 16, 20 steps 131 / 17, 63 steps
 // 411 / 41).
 constexpr int kPolyMinSteps = 64;
-// The transforms between moments and curves grow with the square of the run, the
-// terms only linearly; beyond this length they would be the longer part.
+// Longest run (moments_pay and filters_pay judge the runs below it).
 constexpr int kPolyMaxSteps = 65536;
 // Largest deviation |P(x) - exp(-i tau x)| over the spectrum for which powers
 // of P count as unitary (the default Bessel precision leaves 1e-14).
@@ -1460,6 +1459,25 @@ bool poly_route(tbpm_ctx* c, const double* bes, int n_bes, int n_timestep, int c
       return false;
   }
   return true;
+}
+
+// Seconds of one term on a block of ld columns: a launch and the bytes (measured on
+// B200, about 6 TB/s; small problems 2.2 us in a CUDA graph or the one-launch kernel,
+// 4.5 us as single launches, 8 us a time-stepped term of packed samples with its sums).
+double term_seconds(const tbpm_ctx* c, int ld, double launch) {
+  const double vec = (double)c->ham.n * ld * 2 * real_size(c->ham.prec);
+  return launch + (matrix_bytes(c->ham) + 3.0 * vec) / 6e12;
+}
+
+// Whether moments are the faster side.  The terms grow with the run, the transforms
+// from moments to curves with its square: M (M + T) cosines and powers per 8 columns
+// take 7.5 ps each (measured: 2.2e6 nodes x 60,000 steps 38 s, where 200 orbitals are
+// time-stepped in 9.7 s; 1.5e5 x 4096 0.26 s against 0.67 s).
+bool moments_pay(const tbpm_ctx* c, const PolyPlan& pp, int T, int ld, int n_cols,
+                 double step_launch) {
+  const double M = std::fabs(pp.tau) * (double)pp.a * T;
+  return 7.5e-12 * M * (M + T) * ((n_cols + 7) / 8) + 0.5 * M * term_seconds(c, ld, 2.2e-6) <
+         (double)T * (pp.n_bes - 1) * term_seconds(c, ld, step_launch);
 }
 
 // Number of Chebyshev coefficients of exp(-i z y) on [-1, 1] above 1e-17, i.e.
@@ -2437,11 +2455,18 @@ void qe_accum_attr(size_t bytes) {
   qe_smem_attr(qe_accum_kernel<R>, bytes);
 }
 
-// The tables of n_en energies' filters for T steps (values on the nodes,
-// coefficients, window factors) have to stay small beside QE.
-bool filters_fit(const PolyPlan& pp, int T, int n_en) {
-  const double M = bessel_degree(pp.tau * (double)pp.a * T);
-  return 16.0 * n_en * (M + T) < 1e9;
+// Whether nb states' quasi-eigenstates at n_en energies come from filters.  Their
+// tables (values on the nodes, coefficients, window factors) have to stay small beside
+// QE, and the transforms of the filters, M^2 n_en products of 1.9 ps, are to cost less
+// than the steps they save: 8192 steps, 911 energies, 200 orbitals 1017 ms with filters,
+// 739 ms time-stepped; 183 energies 263 and 709 ms; 4096 steps, 455 energies 162 and 354.
+bool filters_pay(const tbpm_ctx* c, const PolyPlan& pp, int T, int nb, int n_en) {
+  const double M = std::fabs(pp.tau) * (double)pp.a * T;
+  const double transform =
+      1.9e-12 * M * M * n_en + 7.5e-12 * M * (M + T) * ((nb + 7) / 8);
+  return 16.0 * n_en * (M + T) < 1e9 &&
+         transform + M * term_seconds(c, nb, 2.2e-6) <
+             (double)T * (pp.n_bes - 1) * term_seconds(c, 2 * nb, 4.5e-6);
 }
 
 // Phase 1 on the polynomial route: QE_i = f_i(H) wf0 by the energies' filters
@@ -2582,6 +2607,7 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
               int n_energies, double* dos_corr, double* dc_corr, double* qe_acc = nullptr,
               const char* who = "tbpm_dccond", int en_out0 = 0, bool add_dos = true,
               const PolyPlan* pp = nullptr) {
+  const bool filters = pp && filters_pay(c, *pp, n_timestep, nb, (int)en_sel.size());
   using C = typename Cx<R>::t;
   const Ham& h = c->ham;
   const int64_t n = h.n;
@@ -2592,7 +2618,7 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   const size_t vb = (size_t)n * ld * 2 * sizeof(R);
   c->graph.reset();
   c->sess.active = false;
-  if (!pp) {
+  if (!filters) {
     c->X.ensure(vb);
     c->Y.ensure(vb);
     c->A.ensure(vb * (size_t)(std::max(T1, T2) + 1));
@@ -2615,7 +2641,7 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
   std::optional<Phase> phase;
   phase.emplace("tbpm_dccond: quasi-eigenstates");
   int t = 1;
-  if (pp) {
+  if (filters) {
     std::vector<double> dos;
     dc_filter<R, V>(c, *pp, nb, W, n_timestep, t_step, en_sel, chk_step, chk_thr, who,
                     dos_corr && add_dos ? &dos : nullptr);
@@ -2740,8 +2766,8 @@ void dc_batch(tbpm_ctx* c, const Expansion& ex_pm, const Expansion& ex_fwd, int 
     check_status(c);
     return;
   }
-  if (!pp) read_out(c, host, (size_t)n_timestep * ld * 3);
-  if (!pp && add_dos)
+  if (!filters) read_out(c, host, (size_t)n_timestep * ld * 3);
+  if (!filters && add_dos)
     for (int b = 0; b < nb; ++b)
       for (int tt = 1; tt <= n_timestep; ++tt) {
         dos_corr[2 * (tt - 1)] += host[((size_t)(tt - 1) * ld + b) * 3 + 0] / n_avg;
@@ -3553,7 +3579,7 @@ void drv_dos(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, int n
     const double* hw = wf0 ? wf0 + 2 * (size_t)s0 * c->ham.n : nullptr;
     dispatch(c->ham.prec, pick_V(c->ham.prec, ns, ns, c->opts.vector_width), [&](auto tag) {
       using P = decltype(tag);
-      if (poly)
+      if (poly && moments_pay(c, pp, n_timestep, ns, ns, 2.2e-6))
         dos_moments<typename P::Real, P::V>(c, pp, ns, kp, hw, n_timestep, chk_step, chk_thr,
                                             n_states, corr, corr_per_state, s0);
       else
@@ -3673,8 +3699,7 @@ void drv_dc_part(tbpm_ctx* c, const double* bes, int n_bes, const double* wf0, i
     (void)cudaGetLastError();
   }
   PolyPlan pp;
-  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
-                    filters_fit(pp, n_timestep, en_chunk);
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;
@@ -3811,8 +3836,7 @@ void drv_eigenstates(tbpm_ctx* c, const double* bes, int n_bes, const double* wf
     (void)cudaGetLastError();
   }
   PolyPlan pp;
-  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
-                    filters_fit(pp, n_timestep, n_energies);
+  const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp);
   for (int s0 = 0; s0 < n_states; s0 += B) {
     const int nb = std::min(B, n_states - s0);
     Expansion ex_pm = ex_fwd;
@@ -4047,6 +4071,7 @@ void drv_dos_segmented(tbpm_ctx* c, const double* bes, int n_bes, const int64_t*
   const Expansion ex = time_step_expansion(bes, n_bes);
   PolyPlan pp;
   const bool poly = poly_route(c, bes, n_bes, n_timestep, chk_step, chk_thr, &pp) &&
+                    moments_pay(c, pp, n_timestep, n_states, n_seg * n_states, 8e-6) &&
                     segments_closed(c, off);
   dispatch(c->ham.prec, pick_V(c->ham.prec, n_states, n_states, c->opts.vector_width),
            [&](auto tag) {

@@ -399,3 +399,58 @@ def test_driver_calls_end_a_session(sample, driver):
         f2py.tbpm_psi_t(*args, wf[0], np.array([0, 64]), 64, 128, 1e-9)
     with pytest.raises(nat.TbpmError):
         ctx.call("tbpm_session_advance", 4)
+
+
+def _launches():
+    return f2py._ctx().last_stats()[0]
+
+
+@pytest.mark.parametrize("n_en,filtered", [(4, True), (1000, False)])
+def test_long_runs_whose_filters_cost_more_than_the_steps(sample, n_en, filtered):
+    """8192 steps: a few energies by filters (a vector per 0.33 steps), 1000 of them time-stepped
+    as a transform of 25,000 x 25,000 x 1000 products would take longer; both routes' densities
+    at the energies they share agree."""
+    h = sample.build_ham_csr()
+    wf = unit_states(1, h.shape[0], seed=6)
+    energies = np.linspace(-2.0, 2.0, n_en) + 0.003
+    t_step = 2 * math.pi / sample.energy_range
+    args = (bessel_series(math.pi), h.indptr, h.indices, h.data, wf, 8192, t_step)
+    got = f2py.tbpm_eigenstates_states(*args, energies, 128, 1e-9)
+    assert (_launches() < 8192) == filtered
+    if not filtered:
+        pick = [0, 333, 999]
+        few = f2py.tbpm_eigenstates_states(*args, energies[pick], 128, 1e-9)
+        assert _launches() < 8192
+        assert rel_err(got[pick], few) < 1e-8
+
+
+def test_dc_with_stepped_quasi_eigenstates_and_expanded_currents(sample):
+    """The same choice in tbpm_dccond: phase 1 time-stepped (its filters would cost more),
+    phase 2 by several steps per expansion, against both phases of the short route."""
+    ip, ix, hv, dx, dy = sample.build_ham_dxy()
+    wf = unit_states(2, ip.size - 1, seed=6)
+    energies = np.linspace(1.0, 3.0, 1000)
+    t_step = 2 * math.pi / sample.energy_range
+    args = (bessel_series(math.pi), ip, ix, hv, sample.rescale, dx, dy, wf, 6000, t_step, energies)
+    dos, dc = f2py.tbpm_dccond_states(*args, np.arange(1000), 128, 1e-9)
+    stepped = _launches()
+    pick = np.array([0, 500, 999])
+    dos3, dc3 = f2py.tbpm_dccond_states(*args, pick, 128, 1e-9)
+    assert _launches() < 6000 * 4 < 6000 * 19 < stepped < 6000 * 26
+    assert rel_err(dos, dos3) < 1e-10
+    assert rel_err(dc[:, pick], dc3[:, :3]) < 1e-8
+
+
+def test_dos_of_a_large_time_step_over_a_long_run(sample):
+    """Twelve times the usual time step, 60,000 steps: two million moments would cost more than
+    the products they save; 2000 steps take the moments."""
+    h = sample.build_ham_csr()
+    wf = unit_states(1, h.shape[0], seed=6)
+    bes = bessel_series(12 * math.pi)
+    e, v = np.linalg.eigh(h.toarray())
+    w = abs(v.conj().T @ wf[0]) ** 2
+    for n_t, moments in ((2000, True), (60000, False)):
+        got = f2py.tbpm_dos_states(bes, h.indptr, h.indices, h.data, wf, n_t, 128, 1e-9)
+        assert (_launches() < n_t) == moments
+        ref = np.exp(-12j * math.pi * np.outer(np.arange(n_t + 1), e)) @ w
+        assert rel_err(got, ref) < 1e-8

@@ -348,8 +348,9 @@ int tbpm_cond_from_trace(tbpm_ctx* ctx, const double* mu_mn, int n_kernel, const
  * [seg_offsets[k], seg_offsets[k+1]) (seg_offsets[0] = 0,
  * seg_offsets[n_seg] = n_rows) and n_states random states drawn over its own
  * rows with iseed = seed*(k*n_states + s + 1) and normalised there.  All
- * realisations share the Bessel series (one rescale factor).  The whole
- * propagation is captured as one CUDA graph and launched once.
+ * realisations share the Bessel series (one rescale factor).  Runs of 64 steps or
+ * more are evaluated from Chebyshev moments; shorter ones, and matrices with entries
+ * between the realisations' rows, are time-stepped as one CUDA graph.
  * corr: complex128 [n_seg][n_timestep+1] (state average per realisation);
  * corr_per_state (optional): complex128 [n_seg][n_states][n_timestep+1]. */
 int tbpm_dos_segmented(tbpm_ctx* ctx, const double* bes, int n_bes, const int32_t* indptr,
